@@ -27,6 +27,7 @@
 #include "pmf_bulk.cuh"
 #include "pmf_dense.cuh"
 #include "pmf_kernels.h"
+#include "pmf_rr.cuh"
 #include "tune.h"
 
 namespace pmf {
@@ -585,12 +586,8 @@ struct PhaseClock {
   }
 };
 
-// sc: scratch of the tridiagonal eigensolver (>= 2 400 doubles); null: mt.stile and the tiles after it.  The
-// phase-batched Rayleigh-Ritz passes mt.GM: GM, GA and U are dead by then, so its shared memory ends at stile.
 __device__ int cta_rayleigh_ritz(LbSmall& sm, LbMats& mt, int nS, int m, double drop, double jtol,
-                                 PhaseClock* pc = nullptr, double* sc = nullptr);
-__device__ int cta_rayleigh_ritz(LbSmall& sm, LbMats& mt, int nS, int m, double drop, double jtol, PhaseClock* pc,
-                                 double* sc) {
+                                 PhaseClock* pc = nullptr) {
   for (int e = threadIdx.x; e < nS * nS; e += blockDim.x) {
     const int a = e / nS, b = e % nS;
     if (a < b) {
@@ -693,7 +690,7 @@ __device__ int cta_rayleigh_ritz(LbSmall& sm, LbMats& mt, int nS, int m, double 
   __syncthreads();
   if (pc) pc->lap(11);
   // only the lowest min(m, q) eigenpairs of H are needed
-  cta_sym_lowest(mt.H, mt.V, sm.th, q, min(m, q), LB_LD, sc ? sc : mt.stile);
+  cta_sym_lowest(mt.H, mt.V, sm.th, q, min(m, q), LB_LD, mt.stile);
   (void)jtol;
   if (pc) pc->lap(12);
   const int mm = min(m, q);
@@ -1654,43 +1651,46 @@ __global__ void __launch_bounds__(256, 2) k_eb_gram(EbArgs a) {
     cta_gram2_mma<T, double, 4>(sS, sA, sl.Md + c0, cn, G, G + LB_LD * LB_LD, red);
 }
 
-// Rayleigh-Ritz on the chunk-summed Grams (k_lobpcg's cta_rayleigh_ritz).
-__global__ void __launch_bounds__(256) k_eb_rr(EbArgs a, double drop) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  LbSmall& sm = *reinterpret_cast<LbSmall*>(smraw);
-  LbMats& mt = *reinterpret_cast<LbMats*>(smraw + sizeof(LbSmall));
+// Rayleigh-Ritz on the chunk-summed Grams, one warp per subdomain (pmf_rr.cuh).
+// NX: the basis size rounded up (3m), MX: the block size rounded up.
+template <int NX, int MX>
+__global__ void __launch_bounds__(32) k_eb_rr(EbArgs a, double drop) {
+  __shared__ WarpRR<NX, MX> sm;
   const int s = eb_sub(a, blockIdx.x);
   EbState& es = a.state[s];
   if (es.done) return;
   const SubInfo S = a.subs[s];
   const int nc = S.nx * S.ny * S.nz;
   const int nch = (nc + EB_CHUNK - 1) / EB_CHUNK;
-  const int nS = es.nS, m = a.m;
-  for (int e = threadIdx.x; e < nS * nS; e += blockDim.x) {
-    const int r = e / nS, c = e % nS;
-    double gm = 0.0, ga = 0.0;
-    for (int q = 0; q < nch; ++q) {
-      const double* G = a.gpart + ((size_t)s * a.nchunk + q) * 2 * LB_LD * LB_LD;
-      gm += G[r * LB_LD + c];
-      ga += G[LB_LD * LB_LD + r * LB_LD + c];
+  const int nS = es.nS, m = a.m, lane = threadIdx.x;
+  const double* G0 = a.gpart + (size_t)s * a.nchunk * 2 * LB_LD * LB_LD;
+  auto load = [&](int which, double (&g)[NX]) {
+#pragma unroll
+    for (int j = 0; j < NX; ++j) g[j] = 0.0;
+    for (int c = 0; c < nch; ++c) {
+      const double* G = G0 + ((size_t)c * 2 + which) * LB_LD * LB_LD + lane;
+#pragma unroll
+      for (int j = 0; j < NX; ++j)
+        if (j < nS && lane < nS) g[j] += G[j * LB_LD];
     }
-    mt.GM[r * LB_LD + c] = gm;
-    mt.GA[r * LB_LD + c] = ga;
-  }
-  if (threadIdx.x < LB_MM) sm.lam[threadIdx.x] = threadIdx.x < m ? es.lam[threadIdx.x] : 0.0;
-  if (threadIdx.x == 0) sm.scal[0] = es.lscale;
-  __syncthreads();
-  const int q = cta_rayleigh_ritz(sm, mt, nS, m, drop, 1e-11, nullptr, mt.GM);
-  double* Y = a.Ybuf + (size_t)s * LB_LD * LB_LD;
-  for (int e = threadIdx.x; e < nS * m; e += blockDim.x) {
-    const int r = e / m, c = e % m;
-    Y[r * LB_LD + c] = mt.Y[r * LB_LD + c];
-  }
-  if (threadIdx.x < m) es.lam[threadIdx.x] = sm.lam[threadIdx.x];
-  if (threadIdx.x == 0) {
+  };
+  const int q = warp_rayleigh_ritz<NX, MX>(sm, nS, m, drop, load, a.Ybuf + (size_t)s * LB_LD * LB_LD, LB_LD);
+  if (lane < min(m, q)) es.lam[lane] = sm.lam[lane];
+  if (lane == 0) {
     es.restart = q < m ? 1 : 0;  // basis collapsed: no update, next iteration without P
     es.hasP = q < m ? 0 : 1;
   }
+}
+static void launch_eb_rr(const EbArgs& e, int nact, double drop, cudaStream_t st) {
+  note_launch();
+  if (e.m <= 5)
+    k_eb_rr<16, 8><<<nact, 32, 0, st>>>(e, drop);
+  else if (e.m == 6)
+    k_eb_rr<20, 8><<<nact, 32, 0, st>>>(e, drop);
+  else if (e.m <= 8)
+    k_eb_rr<24, 8><<<nact, 32, 0, st>>>(e, drop);
+  else
+    k_eb_rr<32, 10><<<nact, 32, 0, st>>>(e, drop);
 }
 
 // X <- S Y, P <- [W P] Y_WP (and the FP64 A-images in FP64 storage), per chunk.
@@ -2199,7 +2199,6 @@ int launch_lobpcg_batched(const LobpcgArgs& a_in, const EbBuffers& b, const int*
   size_t pre_smem_max = 0;
   for (int q = 0; q < nmb; ++q) pre_smem_max = std::max(pre_smem_max, coef + (size_t)4 * e.ldc * mb_c[q]);
   const size_t gram_smem = (size_t)8 * 32 * 32 * sizeof(double);
-  const size_t rr_smem = sizeof(LbSmall) + offsetof(LbMats, stile);  // k_eb_rr stops at the tiles: 3 CTAs / SM
   cudaFuncSetAttribute(k_eb_precond<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pre_smem_max);
   // basis update tiles: <6,1> (3 CTAs per SM) is the built-in for m <= 8, <8,2> the alternative;
   // candidates 2 / 3 are the same tiles with two groups of cells loading ahead per warp
@@ -2223,7 +2222,6 @@ int launch_lobpcg_batched(const LobpcgArgs& a_in, const EbBuffers& b, const int*
     prev_pc = -1;
   };
   cudaFuncSetAttribute(k_eb_gram<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gram_smem);
-  cudaFuncSetAttribute(k_eb_rr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rr_smem);
   const double drop = sizeof(T) == 4 ? 1e-9 : 1e-13;
   // optional phase timing (b.phase_ms, or PMF_PROFILE_EIGEN): device time per phase
   const bool prof = b.phase_ms != nullptr || getenv("PMF_PROFILE_EIGEN") != nullptr;
@@ -2268,7 +2266,7 @@ int launch_lobpcg_batched(const LobpcgArgs& a_in, const EbBuffers& b, const int*
     mark(3);
     { note_launch(); k_eb_gram<T><<<gchunk, 256, gram_smem, st>>>(e); }
     mark(4);
-    { note_launch(); k_eb_rr<<<nact, 256, rr_smem, st>>>(e, drop); }
+    launch_eb_rr(e, nact, drop, st);
     mark(5);
     note_launch();
     cudaEventRecord(tev[2], st);
