@@ -1,14 +1,12 @@
 // Coarse-space kernels (FP64): level-2 Galerkin assembly, batched dense SPD
 // inverses, the level-3 eigenproblem and the small coarse products used by the
 // cycle executor.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <cstdio>
 
 #include "pmf_dense.cuh"
 #include "pmf_kernels.h"
-#include "tune.h"
+#include "pmf_rr.cuh"
 
 namespace pmf {
 
@@ -479,513 +477,344 @@ __global__ void k_spd_inverse(int n, double* a_all, double tol, int* nnull) {
   }
   if (threadIdx.x == 0 && nnull) atomicAdd(nnull, nul);
 }
-// The same Gauss-Jordan inverse by a cluster of kSpdCl CTAs per matrix, for
-// n <= 32 * NM.  CTA c of the cluster owns rows [c R, c R + R), R = ceil(n /
-// kSpdCl); warp w holds rows c R + w + 16 s (s < RW) in registers, lane l the
-// columns l + 32 m.  Per pivot the owning warp publishes the scaled pivot row
-// in its CTA's shared memory, one cluster barrier makes it visible, and every
-// CTA copies it through distributed shared memory and updates its rows.  The
-// arithmetic per element is that of k_spd_inverse, so the results agree bit
-// for bit.
-constexpr int kSpdCl = 8;
-constexpr int kSpdWarps = 16;
-
-template <int NM, int RW>
-__global__ void __launch_bounds__(kSpdWarps * 32, 1)
-    k_spd_inverse_cl(int n, double* a_all, double tol, int* nnull) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  const int crank = (int)cluster.block_rank();
-  const int mat = blockIdx.x / kSpdCl;
-  double* a = a_all + (long long)mat * n * n;
-  const int R = (n + kSpdCl - 1) / kSpdCl;
-  const int r0 = crank * R;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  __shared__ double pub[2][NM * 32];  // published pivot rows (read by the whole cluster)
-  __shared__ double prow[NM * 32];    // local copy of the current pivot row
-  __shared__ int pnull[2];
-  __shared__ double cmax[kSpdWarps];
-  __shared__ double smax;
-  double v[RW][NM];
-  int rows[RW];
-#pragma unroll
-  for (int s = 0; s < RW; ++s) {
-    const int i = r0 + w + kSpdWarps * s;
-    rows[s] = (w + kSpdWarps * s < R && i < n) ? i : -1;
-#pragma unroll
-    for (int m = 0; m < NM; ++m) {
-      const int j = lane + 32 * m;
-      v[s][m] = (rows[s] >= 0 && j < n) ? a[(long long)i * n + j] : 0.0;
-    }
-  }
-  // scale = max |a_ii| over the whole matrix
-  double mx = 0.0;
-#pragma unroll
-  for (int s = 0; s < RW; ++s)
-#pragma unroll
-    for (int m = 0; m < NM; ++m)
-      if (rows[s] >= 0 && lane + 32 * m == rows[s]) mx = fmax(mx, fabs(v[s][m]));
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if (lane == 0) cmax[w] = mx;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double m2 = 0.0;
-    for (int q = 0; q < kSpdWarps; ++q) m2 = fmax(m2, cmax[q]);
-    smax = m2;
-  }
-  cluster.sync();
-  if (threadIdx.x == 0) {
-    double m2 = 0.0;
-    for (int c = 0; c < kSpdCl; ++c) m2 = fmax(m2, *cluster.map_shared_rank(&smax, c));
-    cmax[0] = m2 > 0 ? m2 : 1.0;
-  }
-  cluster.sync();  // every CTA has read the others' maxima before smax is reused
-  const double scale = cmax[0];
-  int nul = 0;
-  for (int k = 0; k < n; ++k) {
-    const int o = k / R, ok = k - o * R;
-    const int ow = ok % kSpdWarps, os = ok / kSpdWarps;
-    const int km = k >> 5, kl = k & 31;
-    if (crank == o && w == ow) {  // owner warp: publish row k scaled by its pivot
-#pragma unroll
-      for (int s = 0; s < RW; ++s)
-        if (s == os) {
-          double pv = 0.0;
-#pragma unroll
-          for (int m = 0; m < NM; ++m)
-            if (m == km) pv = v[s][m];
-          const double piv = __shfl_sync(0xffffffffu, pv, kl);
-          const bool isnull = !(piv > tol * scale);
-#pragma unroll
-          for (int m = 0; m < NM; ++m) {
-            const int j = lane + 32 * m;
-            pub[k & 1][j] = isnull ? 0.0 : (j == k ? 1.0 : v[s][m]) / piv;
-          }
-          if (lane == 0) pnull[k & 1] = isnull ? 1 : 0;
-        }
-    }
-    cluster.sync();
-    {
-      const double* src = cluster.map_shared_rank(&pub[k & 1][0], o);
-      for (int j = threadIdx.x; j < NM * 32; j += blockDim.x) prow[j] = src[j];
-    }
-    const bool isnull = *cluster.map_shared_rank(&pnull[k & 1], o) != 0;
-    __syncthreads();
-    if (isnull) {
-      if (crank == o && threadIdx.x == 0) ++nul;
-#pragma unroll
-      for (int s = 0; s < RW; ++s) {
-        if (rows[s] < 0) continue;
-#pragma unroll
-        for (int m = 0; m < NM; ++m)
-          if (rows[s] == k || (m == km && lane == kl)) v[s][m] = 0.0;
-      }
-    } else {
-#pragma unroll
-      for (int s = 0; s < RW; ++s) {
-        if (rows[s] < 0) continue;
-        if (rows[s] == k) {
-#pragma unroll
-          for (int m = 0; m < NM; ++m) v[s][m] = prow[lane + 32 * m];
-        } else {
-          double cv = 0.0;
-#pragma unroll
-          for (int m = 0; m < NM; ++m)
-            if (m == km) cv = v[s][m];
-          const double ci = __shfl_sync(0xffffffffu, cv, kl);
-#pragma unroll
-          for (int m = 0; m < NM; ++m) {
-            const int j = lane + 32 * m;
-            v[s][m] = (j == k ? 0.0 : v[s][m]) - ci * prow[j];
-          }
-        }
-      }
-    }
-  }
-  // rows back to global memory, then the symmetrisation of k_spd_inverse by the
-  // owner of the lower row index of each pair
-#pragma unroll
-  for (int s = 0; s < RW; ++s)
-    if (rows[s] >= 0)
-#pragma unroll
-      for (int m = 0; m < NM; ++m) {
-        const int j = lane + 32 * m;
-        if (j < n) a[(long long)rows[s] * n + j] = v[s][m];
-      }
-  cluster.sync();
-#pragma unroll
-  for (int s = 0; s < RW; ++s) {
-    const int i = rows[s];
-    if (i < 0) continue;
-#pragma unroll
-    for (int m = 0; m < NM; ++m) {
-      const int j = lane + 32 * m;
-      if (j > i && j < n) {
-        const double sv = 0.5 * (v[s][m] + a[(long long)j * n + i]);
-        a[(long long)i * n + j] = sv;
-        a[(long long)j * n + i] = sv;
-      }
-    }
-  }
-  if (threadIdx.x == 0 && nnull && nul) atomicAdd(nnull, nul);
+// D += A B for one 8 x 8 tile, k = 4, on the FP64 tensor cores.
+__device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
 }
 
-template <int NM, int RW>
-static bool spd_inverse_cl(int nb, int n, double* a, double tol, int* nnull, cudaStream_t st) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nb * kSpdCl);
-  cfg.blockDim = dim3(kSpdWarps * 32);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kSpdCl;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, k_spd_inverse_cl<NM, RW>, n, a, tol, nnull) != cudaSuccess) {
-    (void)cudaGetLastError();  // cluster launch refused: the caller falls back to one CTA per matrix
-    return false;
-  }
-  note_launch();
-  return true;
-}
-
-// The same Gauss-Jordan inverse spread over the whole GPU, for matrices too
-// large for one cluster, in panels of kGjPB pivots.  Eliminating the pivots P
-// of a panel turns [A_PP A_PR; A_RP A_RR] into
+// The same Gauss-Jordan inverse spread over the whole GPU, in panels of kGjPB
+// pivots.  Eliminating the pivots P of a panel turns [A_PP A_PR; A_RP A_RR] into
 //   A_PP <- Z = A_PP^-1,  A_PR <- Z A_PR,  A_RP <- -A_RP Z,  A_RR <- A_RR - A_RP Z A_PR,
 // which is what the pivots one at a time give in exact arithmetic; Z comes
-// from the pivot-by-pivot Gauss-Jordan of the diagonal block with
-// k_spd_inverse's arithmetic and null-pivot rule (a pivot at or below
-// tol x max|diag| drops its row and column), so a null pivot zeroes its row
-// and column of the result as before.  Per panel: k_gjb_diag (one CTA per
-// matrix), k_gjb_rows (R = Z A_PR), k_gjb_update (the rank-kGjPB update of
-// every element outside the panel: 64 x 64 tiles, 2 n^2 kGjPB flops per
-// panel), k_gjb_cols (A_RP) and k_gjb_prow (A_PR, A_PP).  Matrix b has order
-// nv[b] (or n) and starts at off[b] (or b n^2); panels past a matrix's order
-// leave it alone.
+// from the pivot-by-pivot Gauss-Jordan of the diagonal block with the
+// null-pivot rule above (a pivot at or below tol x max|diag| drops its row and
+// column), so a null pivot zeroes its row and column of the result as before.
+//
+// The matrix stays symmetric up to sign: with s_i = -1 for the pivots already
+// eliminated and +1 for the others, A_ij = s_i s_j A_ji.  So A_RP is s A_PR^T,
+// its new value -s (Z A_PR)^T, and only the tiles on and below the diagonal
+// are updated, each writing its mirror image as well: half the operations of
+// the full update, and one kernel (k_gj_rows: R = Z A_PR) before it instead of
+// three around it.  The products run on the FP64 tensor cores (m8n8k4) from
+// shared memory whose pitch keeps fragment loads at their two wavefronts.  The
+// CTA that updates the next panel's diagonal block also inverts it, so a panel
+// costs two launches; the inversion, the longest chain, runs next to the other
+// tiles' updates.  Matrix b has order ord(b) and starts at at(b); panels past a
+// matrix's order leave it alone.
+//
+// Bound by FP64 arithmetic for many or large matrices and by the chain of
+// panels for few small ones.  The two inverses of a set-up with four matrices of
+// 2 244: 10.7 ms instead of 36.5 by the full update on the CUDA cores in five
+// launches a panel; one of 256: 0.18 ms instead of 0.58 by a cluster of 8 CTAs
+// with the rows in registers.
 struct GjShape {
-  const int* nv;         // per matrix order, or null (all n)
-  const long long* off;  // per matrix offset, or null (b n^2)
-  int n;
-  __device__ int ord(int b) const { return nv ? nv[b] : n; }
+  const int* first;      // per-matrix orders (first[b+1] - first[b]) kmax, or null (all n)
+  const long long* off;  // per-matrix offsets, or null (b n^2)
+  int n, kmax;
+  __device__ int ord(int b) const { return first ? (first[b + 1] - first[b]) * kmax : n; }
   __device__ long long at(int b) const { return off ? off[b] : (long long)b * n * n; }
 };
-constexpr int kGjPB = 64;  // pivots per panel
-constexpr int kGjT = 64;   // tile edge of the update
-constexpr int kGjLd = kGjPB + 1;
+constexpr int kGjPB = 64;   // pivots per panel and tile edge
+constexpr int kGjLd = 72;   // pitch of operands stored [k][row or column]: 8 mod 16 doubles
+constexpr int kGjLdZ = 68;  // pitch of an operand stored [row][k]: 4 mod 16 doubles
+constexpr int kGjLdT = 65;  // pitch of a tile read by rows and by columns
 
-__global__ void k_gj_scale(GjShape sh, const double* a_all, double* scale) {
-  const int nb = sh.ord(blockIdx.x);
-  const double* a = a_all + sh.at(blockIdx.x);
-  __shared__ double red[32];
-  double mx = 0.0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) mx = fmax(mx, fabs(a[(long long)i * nb + i]));
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if (lane == 0) red[wid] = mx;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double m = 0.0;
-    for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) m = fmax(m, red[w]);
-    scale[blockIdx.x] = m > 0 ? m : 1.0;
+// Inverse of the pb x pb matrix t (pitch kGjLdT) in place, pivot by pivot, by 256 threads holding 4 x 4
+// entries each (rows ty + 16 a, columns tx + 16 b); a pivot at or below thr drops its row and column.
+// buf: 4 x kGjPB doubles.  Returns the number of dropped pivots.
+__device__ __forceinline__ int gj_invert_tile(double* t, int pb, double thr, double* buf) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  double v[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int i = ty + 16 * a, j = tx + 16 * b;
+      v[a][b] = (i < pb && j < pb) ? t[i * kGjLdT + j] : 0.0;
+    }
+  int nul = 0;
+#pragma unroll
+  for (int ka = 0; ka < 4; ++ka) {
+#pragma unroll 1
+    for (int kl = 0; kl < 16; ++kl) {
+      const int kk = 16 * ka + kl;
+      if (kk >= pb) break;
+      double* row = buf + (kk & 1) * 2 * kGjPB;
+      double* col = row + kGjPB;
+      if (ty == kl) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) row[tx + 16 * b] = v[ka][b];
+      }
+      if (tx == kl) {
+#pragma unroll
+        for (int a = 0; a < 4; ++a) col[ty + 16 * a] = v[a][ka];
+      }
+      __syncthreads();
+      const double piv = row[kk];
+      const bool isnull = !(piv > thr);
+      const double rp = isnull ? 0.0 : 1.0 / piv;
+      nul += isnull ? 1 : 0;
+      double rk[4], ck[4];
+#pragma unroll
+      for (int b = 0; b < 4; ++b) rk[b] = (tx + 16 * b == kk ? 1.0 : row[tx + 16 * b]) * rp;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) ck[a] = isnull ? 0.0 : col[ty + 16 * a];
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const bool pr = a == ka && ty == kl, pc = b == ka && tx == kl;
+          v[a][b] = pr ? rk[b] : (pc ? 0.0 : v[a][b]) - ck[a] * rk[b];
+        }
+    }
   }
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int i = ty + 16 * a, j = tx + 16 * b;
+      if (i < pb && j < pb) t[i * kGjLdT + j] = v[a][b];
+    }
+  __syncthreads();
+  return nul;
 }
 
-// Z = inverse of the panel's diagonal block, pivot by pivot in shared memory.
-__global__ void __launch_bounds__(256) k_gjb_diag(GjShape sh, const double* a_all, int k0, double tol,
-                                                  const double* scale, double* zbuf, int* nnull) {
+// scale = max |a_ii| and Z of the first panel
+__global__ void __launch_bounds__(256) k_gj_first(GjShape sh, const double* a_all, double tol, double* scale,
+                                                  double* zbuf, int* nnull) {
   const int b = blockIdx.x;
   const int n = sh.ord(b);
-  if (k0 >= n) return;
-  const int pb = min(kGjPB, n - k0);
   const double* a = a_all + sh.at(b);
-  __shared__ double z[kGjPB][kGjLd];
-  __shared__ double colk[kGjPB], rowk[kGjPB];
-  const int tid = threadIdx.x, bd = blockDim.x;
-  for (int e = tid; e < pb * pb; e += bd) {
-    const int i = e / pb, j = e % pb;
-    z[i][j] = a[(long long)(k0 + i) * n + k0 + j];
+  __shared__ double t[kGjPB * kGjLdT], buf[4 * kGjPB], red[8];
+  const int tid = threadIdx.x, pb = min(kGjPB, n);
+  double mx = 0.0;
+  for (int i = tid; i < n; i += 256) mx = fmax(mx, fabs(a[(long long)i * n + i]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((tid & 31) == 0) red[tid >> 5] = mx;
+  for (int e = tid; e < pb * kGjPB; e += 256) {
+    const int i = e / kGjPB, j = e % kGjPB;
+    if (j < pb) t[i * kGjLdT + j] = a[(long long)i * n + j];
   }
   __syncthreads();
-  const double thr = tol * scale[b];
-  int nul = 0;
-  for (int kk = 0; kk < pb; ++kk) {
-    const double piv = z[kk][kk];
-    const bool isnull = !(piv > thr);
-    for (int i = tid; i < pb; i += bd) {
-      colk[i] = z[i][kk];
-      rowk[i] = isnull ? 0.0 : (i == kk ? 1.0 : z[kk][i]) / piv;
-    }
-    __syncthreads();
-    for (int e = tid; e < pb * pb; e += bd) {
-      const int i = e / pb, j = e % pb;
-      if (isnull) {
-        if (i == kk || j == kk) z[i][j] = 0.0;
-      } else if (i == kk) {
-        z[i][j] = rowk[j];
-      } else {
-        z[i][j] = (j == kk ? 0.0 : z[i][j]) - colk[i] * rowk[j];
-      }
-    }
-    __syncthreads();
-    nul += isnull ? 1 : 0;
-  }
+  double m = 0.0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) m = fmax(m, red[w]);
+  m = m > 0 ? m : 1.0;
+  if (tid == 0) scale[b] = m;
+  const int nul = gj_invert_tile(t, pb, tol * m, buf);
   double* zb = zbuf + (long long)b * kGjPB * kGjPB;
-  for (int e = tid; e < pb * pb; e += bd) zb[(e / pb) * kGjPB + e % pb] = z[e / pb][e % pb];
+  for (int e = tid; e < kGjPB * kGjPB; e += 256) {
+    const int i = e / kGjPB, j = e % kGjPB;
+    zb[e] = (i < pb && j < pb) ? t[i * kGjLdT + j] : 0.0;
+  }
   if (tid == 0 && nnull && nul) atomicAdd(nnull, nul);
 }
 
-// R[c][j] = sum_c' Z[c][c'] A[k0 + c'][j] for the columns j outside the panel; 64 columns per CTA.
-__global__ void __launch_bounds__(256) k_gjb_rows(GjShape sh, const double* a_all, int k0, const double* zbuf,
-                                                  double* rbuf) {
+// acc += X^T Y over kGjPB k-values, X and Y stored [k][.] at pitch kGjLd: the warp's 16 x 32 part at
+// (wi, wj) of a 64 x 64 tile.
+template <bool XZ>
+__device__ __forceinline__ void gj_mma_tile(const double* X, const double* Y, int wi, int wj, double (&acc)[2][4][2]) {
+  const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+#pragma unroll 4
+  for (int k = 0; k < kGjPB; k += 4) {
+    double x[2], y[4];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+      x[a] = XZ ? X[(wi + 8 * a + r) * kGjLdZ + k + q] : X[(k + q) * kGjLd + wi + 8 * a + r];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) y[b] = Y[(k + q) * kGjLd + wj + 8 * b + r];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) dmma_8x8x4(acc[a][b][0], acc[a][b][1], x[a], y[b]);
+  }
+}
+
+// R = Z A_PR and a copy of A_PR, 64 columns per CTA (none for the panel's own columns)
+__global__ void __launch_bounds__(256) k_gj_rows(GjShape sh, const double* a_all, int k0, const double* zbuf,
+                                                 double* rbuf, double* lbuf) {
   const int b = blockIdx.y;
   const int n = sh.ord(b);
-  const int j0 = blockIdx.x * kGjT;
-  if (k0 >= n || j0 >= n) return;
+  const int j0 = blockIdx.x * kGjPB;
+  if (k0 >= n || j0 >= n || j0 == k0) return;
   const int pb = min(kGjPB, n - k0);
   const double* a = a_all + sh.at(b);
-  extern __shared__ double gj_sm[];
-  double* zs = gj_sm;                 // [kGjPB][kGjLd]
-  double* as = gj_sm + kGjPB * kGjLd;  // [kGjPB][kGjT + 1]
+  extern __shared__ __align__(16) double gj_sm[];
+  double* zs = gj_sm;                   // [c][c'] at kGjLdZ
+  double* as = gj_sm + kGjPB * kGjLdZ;  // [c'][j] at kGjLd
   const double* zb = zbuf + (long long)b * kGjPB * kGjPB;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < pb * pb; e += blockDim.x) zs[(e / pb) * kGjLd + e % pb] = zb[(e / pb) * kGjPB + e % pb];
-  for (int e = tid; e < pb * kGjT; e += blockDim.x) {
-    const int c = e / kGjT, jj = e % kGjT, j = j0 + jj;
-    as[c * (kGjT + 1) + jj] = j < n ? a[(long long)(k0 + c) * n + j] : 0.0;
-  }
-  __syncthreads();
   double* rb = rbuf + (long long)b * kGjPB * sh.n;
-  const int tx = tid & 15, ty = tid >> 4;
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int c = ty + 16 * r;
-    if (c >= pb) continue;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int q = 0; q < pb; ++q) {
-      const double zv = zs[c * kGjLd + q];
-#pragma unroll
-      for (int s2 = 0; s2 < 4; ++s2) acc[s2] += zv * as[q * (kGjT + 1) + tx + 16 * s2];
-    }
-#pragma unroll
-    for (int s2 = 0; s2 < 4; ++s2) {
-      const int j = j0 + tx + 16 * s2;
-      if (j < n && (j < k0 || j >= k0 + pb)) rb[(long long)c * sh.n + j] = acc[s2];
-    }
-  }
-}
-
-// A[i][j] -= sum_c A[i][k0 + c] R[c][j] for i, j outside the panel; one 64 x 64 tile per CTA.
-__global__ void __launch_bounds__(256) k_gjb_update(GjShape sh, double* a_all, int k0, const double* rbuf,
-                                                    int ntile) {
-  const int b = blockIdx.y;
-  const int n = sh.ord(b);
-  const int i0 = (blockIdx.x / ntile) * kGjT, j0 = (blockIdx.x % ntile) * kGjT;
-  if (k0 >= n || i0 >= n || j0 >= n) return;
-  const int pb = min(kGjPB, n - k0);
-  double* a = a_all + sh.at(b);
-  extern __shared__ double gj_sm[];
-  double* ls = gj_sm;                 // [kGjT][kGjLd]: A[i0 + ii][k0 + c]
-  double* rs = gj_sm + kGjT * kGjLd;  // [kGjPB][kGjT + 1]: R[c][j0 + jj]
-  const double* rb = rbuf + (long long)b * kGjPB * sh.n;
+  double* lb = lbuf + (long long)b * kGjPB * sh.n;
   const int tid = threadIdx.x;
-  for (int e = tid; e < kGjT * pb; e += blockDim.x) {
-    const int ii = e / pb, c = e % pb, i = i0 + ii;
-    ls[ii * kGjLd + c] = i < n ? a[(long long)i * n + k0 + c] : 0.0;
-  }
-  for (int e = tid; e < pb * kGjT; e += blockDim.x) {
-    const int c = e / kGjT, jj = e % kGjT, j = j0 + jj;
-    rs[c * (kGjT + 1) + jj] = (j < n && (j < k0 || j >= k0 + pb)) ? rb[(long long)c * sh.n + j] : 0.0;
+  for (int e = tid; e < kGjPB * kGjPB; e += 256) {
+    const int c = e / kGjPB, j = e % kGjPB;
+    zs[c * kGjLdZ + j] = zb[e];
+    const double v = (c < pb && j0 + j < n) ? a[(long long)(k0 + c) * n + j0 + j] : 0.0;
+    as[c * kGjLd + j] = v;
+    if (j0 + j < n) lb[(long long)c * sh.n + j0 + j] = v;
   }
   __syncthreads();
-  const int tx = tid & 15, ty = tid >> 4;
-  double acc[4][4];
+  const int w = tid >> 5, wi = (w >> 1) * 16, wj = (w & 1) * 32, r = (tid & 31) >> 2, q = tid & 3;
+  double acc[2][4][2] = {};
+  gj_mma_tile<true>(zs, as, wi, wj, acc);
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (int x = 0; x < 2; ++x)
 #pragma unroll
-    for (int s2 = 0; s2 < 4; ++s2) acc[r][s2] = 0.0;
-  for (int c = 0; c < pb; ++c) {
-    double lv[4], rv[4];
+    for (int y = 0; y < 4; ++y)
 #pragma unroll
-    for (int r = 0; r < 4; ++r) lv[r] = ls[(ty + 16 * r) * kGjLd + c];
-#pragma unroll
-    for (int s2 = 0; s2 < 4; ++s2) rv[s2] = rs[c * (kGjT + 1) + tx + 16 * s2];
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int s2 = 0; s2 < 4; ++s2) acc[r][s2] += lv[r] * rv[s2];
-  }
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = i0 + ty + 16 * r;
-    if (i >= n || (i >= k0 && i < k0 + pb)) continue;
-#pragma unroll
-    for (int s2 = 0; s2 < 4; ++s2) {
-      const int j = j0 + tx + 16 * s2;
-      if (j < n && (j < k0 || j >= k0 + pb)) a[(long long)i * n + j] -= acc[r][s2];
-    }
-  }
+      for (int h = 0; h < 2; ++h) {
+        const int c = wi + 8 * x + r, j = j0 + wj + 8 * y + 2 * q + h;
+        if (j < n) rb[(long long)c * sh.n + j] = acc[x][y][h];
+      }
 }
 
-// A[i][k0 + c] = -sum_c' A[i][k0 + c'] Z[c'][c] for the rows i outside the panel; 64 rows per CTA.
-__global__ void __launch_bounds__(256) k_gjb_cols(GjShape sh, double* a_all, int k0, const double* zbuf) {
-  const int b = blockIdx.y;
-  const int n = sh.ord(b);
-  const int i0 = blockIdx.x * kGjT;
-  if (k0 >= n || i0 >= n) return;
-  const int pb = min(kGjPB, n - k0);
-  double* a = a_all + sh.at(b);
-  extern __shared__ double gj_sm[];
-  double* zs = gj_sm;                 // [kGjPB][kGjLd]
-  double* ls = gj_sm + kGjPB * kGjLd;  // [kGjT][kGjLd]
-  const double* zb = zbuf + (long long)b * kGjPB * kGjPB;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < pb * pb; e += blockDim.x) zs[(e / pb) * kGjLd + e % pb] = zb[(e / pb) * kGjPB + e % pb];
-  for (int e = tid; e < kGjT * pb; e += blockDim.x) {
-    const int ii = e / pb, c = e % pb, i = i0 + ii;
-    ls[ii * kGjLd + c] = i < n ? a[(long long)i * n + k0 + c] : 0.0;
-  }
-  __syncthreads();
-  const int tx = tid & 15, ty = tid >> 4;
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = i0 + ty + 16 * r;
-    if (i >= n || (i >= k0 && i < k0 + pb)) continue;
-#pragma unroll
-    for (int s2 = 0; s2 < 4; ++s2) {
-      const int c = tx + 16 * s2;
-      if (c >= pb) continue;
-      double acc = 0.0;
-      for (int q = 0; q < pb; ++q) acc += ls[(ty + 16 * r) * kGjLd + q] * zs[q * kGjLd + c];
-      a[(long long)i * n + k0 + c] = -acc;
-    }
-  }
-}
-
-// the panel's rows: A[k0 + c][j] = R[c][j] outside the panel, Z[c][j - k0] inside
-__global__ void k_gjb_prow(GjShape sh, double* a_all, int k0, const double* zbuf, const double* rbuf) {
+// One tile (ti >= tj) of the panel's update and its mirror image: the rank-64
+// update outside the panel, R and -s R^T in its row and column, Z on its
+// diagonal.  CTA 0 takes the next panel's diagonal tile and inverts it.
+__global__ void __launch_bounds__(256) k_gj_update(GjShape sh, double* a_all, int k0, const double* zbuf, double* znext,
+                                                   const double* rbuf, const double* lbuf, int ntile, double tol,
+                                                   const double* scale, int* nnull) {
   const int b = blockIdx.y;
   const int n = sh.ord(b);
   if (k0 >= n) return;
-  const int pb = min(kGjPB, n - k0);
+  const int tp = k0 / kGjPB, tn = min(tp + 1, ntile - 1);
+  // tile list in row order, with the next panel's diagonal tile first
+  int id = blockIdx.x;
+  const int dn = tn * (tn + 1) / 2 + tn;
+  id = id == 0 ? dn : (id <= dn ? id - 1 : id);
+  int ti = (int)((sqrtf(8.0f * (float)id + 1.0f) - 1.0f) * 0.5f);
+  while ((ti + 1) * (ti + 2) / 2 <= id) ++ti;
+  while (ti * (ti + 1) / 2 > id) --ti;
+  const int tj = id - ti * (ti + 1) / 2;
+  const int i0 = ti * kGjPB, j0 = tj * kGjPB;
+  if (i0 >= n) return;
   double* a = a_all + sh.at(b);
-  const double* zb = zbuf + (long long)b * kGjPB * kGjPB;
   const double* rb = rbuf + (long long)b * kGjPB * sh.n;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)pb * n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(e / n), j = (int)(e % n);
-    a[(long long)(k0 + c) * n + j] =
-        (j >= k0 && j < k0 + pb) ? zb[c * kGjPB + (j - k0)] : rb[(long long)c * sh.n + j];
+  const double* lb = lbuf + (long long)b * kGjPB * sh.n;
+  extern __shared__ __align__(16) double gj_sm[];
+  double* xs = gj_sm;                   // [c][i], old A_PR at the rows' columns; then the new tile
+  double* ys = gj_sm + kGjPB * kGjLd;   // [c][j], R
+  const int tid = threadIdx.x, c64 = tid & 63, r64 = tid >> 6;
+  if (ti == tp && tj == tp) {
+    const double* zb = zbuf + (long long)b * kGjPB * kGjPB;
+    for (int c = r64; c < kGjPB; c += 4)
+      if (k0 + c < n && k0 + c64 < n) a[(long long)(k0 + c) * n + k0 + c64] = zb[c * kGjPB + c64];
+    return;
+  }
+  if (ti == tp || tj == tp) {
+    const int o0 = ti == tp ? j0 : i0;  // the tile's rows and columns outside the panel
+    const double s = o0 < k0 ? 1.0 : -1.0;
+    for (int c = r64; c < kGjPB; c += 4) {
+      const double v = o0 + c64 < n ? rb[(long long)c * sh.n + o0 + c64] : 0.0;
+      if (k0 + c < n && o0 + c64 < n) a[(long long)(k0 + c) * n + o0 + c64] = v;
+      xs[c * kGjLdT + c64] = v;
+    }
+    __syncthreads();
+    for (int i = r64; i < kGjPB; i += 4)
+      if (o0 + i < n && k0 + c64 < n) a[(long long)(o0 + i) * n + k0 + c64] = s * xs[c64 * kGjLdT + i];
+    return;
+  }
+  double old[16];
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {
+    const int i = i0 + r64 + 4 * u, j = j0 + c64;
+    old[u] = (i < n && j < n) ? a[(long long)i * n + j] : 0.0;
+  }
+  for (int c = r64; c < kGjPB; c += 4) {
+    xs[c * kGjLd + c64] = i0 + c64 < n ? lb[(long long)c * sh.n + i0 + c64] : 0.0;
+    ys[c * kGjLd + c64] = j0 + c64 < n ? rb[(long long)c * sh.n + j0 + c64] : 0.0;
+  }
+  __syncthreads();
+  const int w = tid >> 5, wi = (w >> 1) * 16, wj = (w & 1) * 32, r = (tid & 31) >> 2, q = tid & 3;
+  double acc[2][4][2] = {};
+  gj_mma_tile<false>(xs, ys, wi, wj, acc);
+  __syncthreads();
+  double* t = xs;
+#pragma unroll
+  for (int x = 0; x < 2; ++x)
+#pragma unroll
+    for (int y = 0; y < 4; ++y)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) t[(wi + 8 * x + r) * kGjLdT + wj + 8 * y + 2 * q + h] = acc[x][y][h];
+  __syncthreads();
+  const double si = i0 < k0 ? -1.0 : 1.0, sj = j0 < k0 ? -1.0 : 1.0;
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {
+    const int il = r64 + 4 * u, i = i0 + il, j = j0 + c64;
+    const double v = old[u] - si * t[il * kGjLdT + c64];
+    t[il * kGjLdT + c64] = v;
+    if (i < n && j < n) a[(long long)i * n + j] = v;
+  }
+  __syncthreads();
+  if (ti != tj) {
+    const double sg = si * sj;
+    for (int jl = r64; jl < kGjPB; jl += 4)
+      if (j0 + jl < n && i0 + c64 < n) a[(long long)(j0 + jl) * n + i0 + c64] = sg * t[c64 * kGjLdT + jl];
+  } else if (ti == tp + 1) {
+    const int pb = min(kGjPB, n - i0);
+    const int nul = gj_invert_tile(t, pb, tol * scale[b], ys);
+    double* zb = znext + (long long)b * kGjPB * kGjPB;
+    for (int i = r64; i < kGjPB; i += 4)
+      zb[i * kGjPB + c64] = (i < pb && c64 < pb) ? t[i * kGjLdT + c64] : 0.0;
+    if (tid == 0 && nnull && nul) atomicAdd(nnull, nul);
   }
 }
 
-__global__ void k_gj_sym(GjShape sh, double* a_all) {
+// the diagonal tiles, the only ones whose two halves are computed separately
+__global__ void __launch_bounds__(256) k_gj_sym(GjShape sh, double* a_all) {
   const int b = blockIdx.y;
-  const int n = sh.ord(b);
+  const int n = sh.ord(b), i0 = blockIdx.x * kGjPB;
   double* a = a_all + sh.at(b);
-  const long long nn = (long long)n * n;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nn; e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e / n), j = (int)(e % n);
-    if (j > i) {
-      const double v = 0.5 * (a[e] + a[(long long)j * n + i]);
-      a[e] = v;
+  for (int e = threadIdx.x; e < kGjPB * kGjPB; e += 256) {
+    const int i = i0 + e / kGjPB, j = i0 + e % kGjPB;
+    if (i < n && j < n && j > i) {
+      const double v = 0.5 * (a[(long long)i * n + j] + a[(long long)j * n + i]);
+      a[(long long)i * n + j] = v;
       a[(long long)j * n + i] = v;
     }
   }
 }
-// nb matrices of orders <= n; returns false when the scratch could not be allocated
+// nb matrices of orders <= sh.n; returns false when the scratch could not be allocated
 static bool gj_inverse(int nb, GjShape sh, double* a, double tol, int* nnull, cudaStream_t st) {
   const int n = sh.n;
   double* scr = nullptr;
-  const size_t bytes = sizeof(double) * (size_t)nb * (1 + (size_t)kGjPB * kGjPB + (size_t)kGjPB * n);
-  if (cudaMallocAsync((void**)&scr, bytes, st) != cudaSuccess) {
+  const size_t zsz = (size_t)nb * kGjPB * kGjPB, psz = (size_t)nb * kGjPB * n;
+  if (cudaMallocAsync((void**)&scr, sizeof(double) * (nb + 2 * zsz + 2 * psz), st) != cudaSuccess) {
     (void)cudaGetLastError();
     return false;
   }
-  double* scale = scr;
-  double* zbuf = scr + nb;
-  double* rbuf = zbuf + (size_t)nb * kGjPB * kGjPB;
-  const int sm_rows = (int)(sizeof(double) * (kGjPB * kGjLd + kGjPB * (kGjT + 1)));
-  const int sm_upd = (int)(sizeof(double) * (kGjT * kGjLd + kGjPB * (kGjT + 1)));
-  const int sm_cols = (int)(sizeof(double) * (kGjPB * kGjLd + kGjT * kGjLd));
-  cudaFuncSetAttribute(k_gjb_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_rows);
-  cudaFuncSetAttribute(k_gjb_update, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_upd);
-  cudaFuncSetAttribute(k_gjb_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_cols);
-  { note_launch(); k_gj_scale<<<nb, 256, 0, st>>>(sh, a, scale); }
-  const int nt = (n + kGjT - 1) / kGjT;
-  const int gp = (int)std::max<long long>(1, std::min<long long>(((long long)kGjPB * n + 255) / 256, 64));
-  for (int k0 = 0; k0 < n; k0 += kGjPB) {
-    { note_launch(); k_gjb_diag<<<nb, 256, 0, st>>>(sh, a, k0, tol, scale, zbuf, nnull); }
-    { note_launch(); k_gjb_rows<<<dim3(nt, nb), 256, sm_rows, st>>>(sh, a, k0, zbuf, rbuf); }
-    { note_launch(); k_gjb_update<<<dim3(nt * nt, nb), 256, sm_upd, st>>>(sh, a, k0, rbuf, nt); }
-    { note_launch(); k_gjb_cols<<<dim3(nt, nb), 256, sm_cols, st>>>(sh, a, k0, zbuf); }
-    { note_launch(); k_gjb_prow<<<dim3(gp, nb), 256, 0, st>>>(sh, a, k0, zbuf, rbuf); }
+  double* zbuf = scr;
+  double* rbuf = scr + 2 * zsz;
+  double* lbuf = rbuf + psz;
+  double* scale = lbuf + psz;
+  const int sm_rows = (int)(sizeof(double) * kGjPB * (kGjLdZ + kGjLd));
+  const int sm_upd = (int)(sizeof(double) * kGjPB * 2 * kGjLd);
+  cudaFuncSetAttribute(k_gj_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_rows);
+  cudaFuncSetAttribute(k_gj_update, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_upd);
+  { note_launch(); k_gj_first<<<nb, 256, 0, st>>>(sh, a, tol, scale, zbuf, nnull); }
+  const int nt = (n + kGjPB - 1) / kGjPB;
+  for (int k0 = 0, p = 0; k0 < n; k0 += kGjPB, p ^= 1) {
+    double *z = zbuf + p * zsz, *zn = zbuf + (p ^ 1) * zsz;
+    if (nt > 1) { note_launch(); k_gj_rows<<<dim3(nt, nb), 256, sm_rows, st>>>(sh, a, k0, z, rbuf, lbuf); }
+    { note_launch(); k_gj_update<<<dim3(nt * (nt + 1) / 2, nb), 256, sm_upd, st>>>(sh, a, k0, z, zn, rbuf, lbuf, nt, tol, scale, nnull); }
   }
-  const long long nn = (long long)n * n;
-  const int gx = (int)std::max<long long>(1, std::min<long long>((nn + 255) / 256, (148 * 8 + nb - 1) / nb));
-  { note_launch(); k_gj_sym<<<dim3(gx, nb), 256, 0, st>>>(sh, a); }
+  { note_launch(); k_gj_sym<<<dim3(nt, nb), 256, 0, st>>>(sh, a); }
   cudaFreeAsync(scr, st);
   return true;
 }
 
 void launch_spd_inverse_r(const RankLayout& L, int nrank, int nr_max, double* dense, double tol, int* nnull,
                           cudaStream_t st) {
-  // the per-rank orders as an int array next to the layout: nr_r = (first[r+1] - first[r]) x kmax
-  int* nv = nullptr;
-  if (cudaMallocAsync((void**)&nv, sizeof(int) * nrank, st) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return;
-  }
-  std::vector<int> h_first(nrank + 1), h_nv(nrank);
-  cudaMemcpyAsync(h_first.data(), L.first, sizeof(int) * (nrank + 1), cudaMemcpyDeviceToHost, st);
-  cudaStreamSynchronize(st);
-  for (int r = 0; r < nrank; ++r) h_nv[r] = (h_first[r + 1] - h_first[r]) * L.kmax;
-  cudaMemcpyAsync(nv, h_nv.data(), sizeof(int) * nrank, cudaMemcpyHostToDevice, st);
-  GjShape sh{nv, L.off2, nr_max};
-  gj_inverse(nrank, sh, dense, tol, nnull, st);
-  cudaFreeAsync(nv, st);
-  cudaStreamSynchronize(st);  // the host vector must outlive the copy
-}
-
-// The cluster inverse for one of its three widths (false: the shape does not fit it, or the launch was refused).
-static bool spd_inverse_cluster(int nb, int n, double* a, double tol, int* nnull, cudaStream_t st) {
-  const int R = (n + kSpdCl - 1) / kSpdCl;
-  if (n <= 128 && R <= kSpdWarps) return spd_inverse_cl<4, 1>(nb, n, a, tol, nnull, st);
-  if (n > 128 && n <= 256 && R <= 2 * kSpdWarps) return spd_inverse_cl<8, 2>(nb, n, a, tol, nnull, st);
-  if (n > 256 && n <= 384 && R <= 3 * kSpdWarps) return spd_inverse_cl<12, 3>(nb, n, a, tol, nnull, st);
-  return false;
+  gj_inverse(nrank, GjShape{L.first, L.off2, nr_max, L.kmax}, dense, tol, nnull, st);
 }
 
 void launch_spd_inverse(int nb, int n, double* a, double tol, int* nnull, cudaStream_t st) {
-  if (n <= 384) {
-    // up to 384 unknowns both the cluster inverse and the panel Gauss-Jordan apply: the tuner times
-    // them on a scratch copy of the matrices (the inverse works in place; no null counts while tuning)
-    int choice = 0;
-    if (n > 64 && tune_enabled()) {
-      double* scr = nullptr;  // allocated only when the key is tuned (the candidates run on it)
-      const size_t bytes = sizeof(double) * (size_t)nb * n * n;
-      char key[64];
-      snprintf(key, sizeof(key), "spd_inverse|n%d|b%d", n, nb);
-      choice = tune_choose(key, 2, [&](int c) {
-        if (!scr && cudaMallocAsync((void**)&scr, bytes, st) != cudaSuccess) {
-          (void)cudaGetLastError();
-          scr = nullptr;
-          return false;
-        }
-        cudaMemcpyAsync(scr, a, bytes, cudaMemcpyDeviceToDevice, st);
-        return c == 0 ? spd_inverse_cluster(nb, n, scr, tol, nullptr, st)
-                      : gj_inverse(nb, GjShape{nullptr, nullptr, n}, scr, tol, nullptr, st);
-      }, st);
-      if (scr) cudaFreeAsync(scr, st);
-    }
-    if (choice == 1 && gj_inverse(nb, GjShape{nullptr, nullptr, n}, a, tol, nnull, st)) return;
-    if (spd_inverse_cluster(nb, n, a, tol, nnull, st)) return;
-  }
-  if (n > 384 && gj_inverse(nb, GjShape{nullptr, nullptr, n}, a, tol, nnull, st)) return;
-  const int smem = 2 * n * sizeof(double);
+  if (gj_inverse(nb, GjShape{nullptr, nullptr, n, 0}, a, tol, nnull, st)) return;
+  const int smem = 2 * n * sizeof(double);  // no room for the scratch: one CTA per matrix, in place
   if (smem > 48 * 1024) cudaFuncSetAttribute(k_spd_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   { note_launch(); k_spd_inverse<<<nb, 1024, smem, st>>>(n, a, tol, nnull); }
 }
@@ -1203,22 +1032,32 @@ __global__ void __launch_bounds__(512) k_dense_smallest_eig(RankLayout L, int en
   if (tid == 0) iters[r] = it + 1;
 }
 
-// The same iteration for ranks whose block does not fit in shared memory, in
-// phases over all ranks: the two dense products of an iteration (Y = inv X
-// and AY = A X) spread over CTAs of 32 rows each, the projected problems
-// (SVQB of Y, Rayleigh-Ritz on A) one CTA per rank.  The Ritz vectors' images
-// are rotated with the vectors (A (X U) = (A X) U) instead of recomputed, so an
-// iteration streams each rank's two matrices once.  A converged rank's
-// kernels return at once; the host checks every 8 iterations whether all
-// ranks have converged.
+// The same iteration in three launches over all ranks for p <= kL3Cols columns:
+// Y = inv X and A Y on the FP64 tensor cores, then one CTA per rank for the
+// projected problem.  Y is not orthonormalised first: the Rayleigh-Ritz step
+// takes the pencil (Y^T A Y, Y^T Y) on one warp (pmf_rr.cuh), whose Cholesky
+// drops dependent columns; in exact arithmetic the Ritz pairs are the same, and
+// from the second iteration on Y's columns are nearly orthogonal.  The Ritz
+// vectors' images are A Y C, so an iteration streams each rank's two matrices
+// once.  Dropped columns restart from random directions orthogonal to the kept
+// ones: without that the shift-inverse would turn them back into copies of the
+// lowest vector and they would be dropped again.  A converged rank's kernels
+// return at once; the host checks every 4 iterations whether all have converged.
+//
+// Bound by latency for few small ranks (one rank of 256 unknowns: 1.4 ms a
+// set-up, 4.6 ms with one CTA per rank for the whole iteration and CTA-wide
+// Jacobi for the projected problems) and by streaming the matrices for large
+// ones (four ranks of 2 244: 3.0 ms instead of 23).
 struct L3Rank {
   double anorm;
   double w[PMF_L3_MAXP];
   int q, conv, it;
 };
-constexpr int kL3Rows = 32;    // rows per CTA of the products
-constexpr int kL3Tile = 256;   // l-values per shared-memory tile of the block
-constexpr int kL3Cols = 16;    // columns the product kernel holds in registers
+constexpr int kL3Cols = 16;    // most columns of the block
+constexpr int kL3Rows = 32;    // rows per CTA of the products: 4 warps of 8
+constexpr int kL3Tile = 128;   // rows of the block staged in shared memory at a time
+constexpr int kL3Ld = 18;      // its pitch: 4 kL3Ld is 8 mod 16 doubles, so fragment loads take two wavefronts
+constexpr int kL3Thr = 512;    // threads of the projected problem
 
 __global__ void k_l3_init(RankLayout L, int p, const double* A_all, double* work_all, L3Rank* st) {
   const int r = blockIdx.x;
@@ -1245,186 +1084,219 @@ __global__ void k_l3_init(RankLayout L, int p, const double* A_all, double* work
     X[e] = hash_uniform(((unsigned long long)r << 40) ^ (unsigned long long)e);
 }
 
-// Out = M In for the rank's first `cols` columns (cols = p, or the kept count q): block src/dst of the
-// rank's workspace (0 X, 1 Y, 2 AY), 32 rows per CTA, 8 warps x 4 rows, lanes along the row.
-__global__ void __launch_bounds__(256) k_l3_mm(RankLayout L, int p, const double* M_all, double* work_all, int src,
-                                               int dst, int use_q, const L3Rank* st) {
-  const int r = blockIdx.y;
-  if (st[r].conv) return;
-  const int nr = rank_nr(L, r);
+// Out = M In, blocks src / dst of the rank's workspace (0 X, 1 Y, 2 A Y).  Lane (r, q) of a warp holds of
+// row r the entries k0 + 4 q + t, t < 4, of each 16: whole 128-byte row segments per load, used as the A
+// fragments of four k-steps (the order of k within a dot product is free as long as B follows it).
+__global__ void __launch_bounds__(128) k_l3_mm(RankLayout L, int p, const double* M_all, double* work_all, int src,
+                                               int dst, const L3Rank* st) {
+  const int rk = blockIdx.y;
+  if (st[rk].conv) return;
+  const int nr = rank_nr(L, rk);
+  const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
   const int i0 = blockIdx.x * kL3Rows;
   if (i0 >= nr) return;
-  const int cols = use_q ? st[r].q : p;
-  const double* M = M_all + L.off2[r];
-  const double* In = work_all + L.offw[r] + (long long)src * nr * p;
-  double* Out = work_all + L.offw[r] + (long long)dst * nr * p;
-  __shared__ double xs[kL3Tile][kL3Cols + 1];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  double acc[4][kL3Cols];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int c = 0; c < kL3Cols; ++c) acc[a][c] = 0.0;
+  const int i = i0 + (threadIdx.x >> 5) * 8 + r;
+  const double* M = M_all + L.off2[rk];
+  const double* In = work_all + L.offw[rk] + (long long)src * nr * p;
+  double* Out = work_all + L.offw[rk] + (long long)dst * nr * p;
+  __shared__ double xs[kL3Tile * kL3Ld];
+  const bool vec = (nr & 1) == 0 && (reinterpret_cast<unsigned long long>(M) & 15) == 0;  // 16-byte aligned rows
+  const double* row = M + (long long)min(i, nr - 1) * nr;
+  double acc[2][2][2] = {};  // two independent chains per 8-column tile
   for (int l0 = 0; l0 < nr; l0 += kL3Tile) {
+    const int lend = min(kL3Tile, nr - l0);
     for (int e = threadIdx.x; e < kL3Tile * kL3Cols; e += blockDim.x) {
       const int l = e / kL3Cols, c = e % kL3Cols;
-      xs[l][c] = (l0 + l < nr && c < cols) ? In[(long long)(l0 + l) * p + c] : 0.0;
+      xs[l * kL3Ld + c] = (l < lend && c < p) ? In[(long long)(l0 + l) * p + c] : 0.0;
     }
     __syncthreads();
-    const int lend = min(kL3Tile, nr - l0);
+    for (int k0 = 0; k0 < lend; k0 += 32) {
+      double m[2][4];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int i = i0 + wid * 4 + a;
-      if (i >= nr) continue;
-      const double* row = M + (long long)i * nr + l0;
-      for (int l = lane; l < lend; l += 32) {
-        const double mv = row[l];
+      for (int u = 0; u < 2; ++u) {
+        const int k = k0 + 16 * u + 4 * q;
+        if (vec && k + 3 < lend) {
+          const double2 lo = *reinterpret_cast<const double2*>(row + l0 + k);
+          const double2 hi = *reinterpret_cast<const double2*>(row + l0 + k + 2);
+          m[u][0] = lo.x;
+          m[u][1] = lo.y;
+          m[u][2] = hi.x;
+          m[u][3] = hi.y;
+        } else {
 #pragma unroll
-        for (int c = 0; c < kL3Cols; ++c) acc[a][c] += mv * xs[l][c];
+          for (int t = 0; t < 4; ++t) m[u][t] = k + t < lend ? row[l0 + k + t] : 0.0;
+        }
       }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const double* xk = xs + (k0 + 16 * u + 4 * q + t) * kL3Ld + r;
+          dmma_8x8x4(acc[u][0][0], acc[u][0][1], m[u][t], xk[0]);
+          dmma_8x8x4(acc[u][1][0], acc[u][1][1], m[u][t], xk[8]);
+        }
     }
     __syncthreads();
   }
+  if (i < nr) {
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int i = i0 + wid * 4 + a;
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
-    for (int c = 0; c < kL3Cols; ++c) {
-      const double v = warp_sum(acc[a][c]);
-      if (lane == 0 && i < nr && c < cols) Out[(long long)i * p + c] = v;
-    }
+      for (int h = 0; h < 2; ++h) {
+        const int c = 8 * n + 2 * q + h;
+        if (c < p) Out[(long long)i * p + c] = acc[0][n][h] + acc[1][n][h];
+      }
   }
 }
 
-// SVQB of Y: G = Y^T Y, D^-1/2 G D^-1/2 = U w U^T, X = Y D^-1/2 U w^-1/2 on the kept columns (q).
-__global__ void __launch_bounds__(512) k_l3_svqb(RankLayout L, int p, double* work_all, L3Rank* st) {
-  const int r = blockIdx.x;
-  if (st[r].conv) return;
-  const int nr = rank_nr(L, r);
-  double* X = work_all + L.offw[r];
+struct L3Smem {
+  WarpRR<kL3Cols, kL3Cols> rr;
+  double C[kL3Cols * kL3Cols];
+  double G[2 * kL3Cols * kL3Cols];
+  double part[kL3Thr / 32][kL3Cols * kL3Cols];  // per-warp partial Grams, then the pads' coefficients
+  double red[32];
+};
+
+// Rayleigh-Ritz on (Y^T A Y, Y^T Y), X <- Y C, residuals of the wanted pairs from A Y C - X w, and fresh
+// directions in place of dropped columns.
+__global__ void __launch_bounds__(kL3Thr) k_l3_rr(RankLayout L, int en2, int p, double* work_all, L3Rank* st,
+                                                  double tol, int it) {
+  const int rk = blockIdx.x;
+  if (st[rk].conv) return;
+  extern __shared__ __align__(16) unsigned char l3_raw[];
+  L3Smem& sm = *reinterpret_cast<L3Smem*>(l3_raw);
+  const int nr = rank_nr(L, rk);
+  double* X = work_all + L.offw[rk];
   const double* Y = X + (long long)nr * p;
-  __shared__ double G[PMF_L3_MAXP * PMF_L3_MAXP], U[PMF_L3_MAXP * PMF_L3_MAXP], w[PMF_L3_MAXP],
-      C[PMF_L3_MAXP * PMF_L3_MAXP], dsc[PMF_L3_MAXP], jac[64];
-  __shared__ int ijac[32];
-  __shared__ int keep;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int e = tid; e < p * p; e += nt) {
-    const int a = e / p, b = e % p;
-    double acc = 0.0;
-    for (int l = 0; l < nr; ++l) acc += Y[(long long)l * p + a] * Y[(long long)l * p + b];
-    G[a * PMF_L3_MAXP + b] = acc;
-  }
-  __syncthreads();
-  if (tid < p) dsc[tid] = 1.0 / sqrt(fmax(G[tid * PMF_L3_MAXP + tid], 1e-300));
-  __syncthreads();
-  for (int e = tid; e < p * p; e += nt) {
-    const int a = e / p, b = e % p;
-    G[a * PMF_L3_MAXP + b] *= dsc[a] * dsc[b];
-  }
-  __syncthreads();
-  cta_jacobi_eigh(G, U, w, p, PMF_L3_MAXP, ijac, jac);
-  if (tid == 0) {
-    int kk = 0;
-    const double wmax = w[p - 1];
-    for (int c = p - 1; c >= 0; --c)
-      if (w[c] > 1e-12 * wmax) ++kk;
-    keep = kk;
-    st[r].q = kk;
-  }
-  __syncthreads();
-  const int q = keep;  // kept columns are the last q (largest w)
-  for (int e = tid; e < p * q; e += nt) {
-    const int a = e / q, c = e % q;
-    const int cc = p - q + c;
-    C[a * PMF_L3_MAXP + c] = dsc[a] * U[a * PMF_L3_MAXP + cc] / sqrt(w[cc]);
-  }
-  __syncthreads();
-  for (long long e = tid; e < (long long)nr * q; e += nt) {
-    const int i = (int)(e / q), c = (int)(e % q);
-    double acc = 0.0;
-    for (int a = 0; a < p; ++a) acc += Y[(long long)i * p + a] * C[a * PMF_L3_MAXP + c];
-    X[(long long)i * p + c] = acc;
-  }
-}
-
-// Rayleigh-Ritz on A: H = X^T AY, H = U w U^T, X <- X U, AY <- AY U, residual test of the wanted pairs;
-// columns dropped by the SVQB get fresh random directions for the next iteration.
-__global__ void __launch_bounds__(512) k_l3_rr(RankLayout L, int en2, int p, double* work_all, L3Rank* st,
-                                               double tol, int it) {
-  const int r = blockIdx.x;
-  if (st[r].conv) return;
-  const int nr = rank_nr(L, r);
-  double* X = work_all + L.offw[r];
-  double* Y = X + (long long)nr * p;
-  double* AY = Y + (long long)nr * p;
-  __shared__ double G[PMF_L3_MAXP * PMF_L3_MAXP], U[PMF_L3_MAXP * PMF_L3_MAXP], w[PMF_L3_MAXP], jac[64];
-  __shared__ int ijac[32];
-  __shared__ int conv;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int q = st[r].q;
-  for (int e = tid; e < q * q; e += nt) {
-    const int a = e / q, b = e % q;
-    double acc = 0.0;
-    for (int l = 0; l < nr; ++l) acc += X[(long long)l * p + a] * AY[(long long)l * p + b];
-    G[a * PMF_L3_MAXP + b] = acc;
-  }
-  __syncthreads();
-  for (int e = tid; e < q * q; e += nt) {  // symmetrise
-    const int a = e / q, b = e % q;
-    if (a < b) {
-      const double v = 0.5 * (G[a * PMF_L3_MAXP + b] + G[b * PMF_L3_MAXP + a]);
-      G[a * PMF_L3_MAXP + b] = v;
-      G[b * PMF_L3_MAXP + a] = v;
+  const double* AY = Y + (long long)nr * p;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = kL3Thr / 32;
+  {
+    // Grams: rows l of four per step, tiles (0,0), (0,1), (1,1) of the 16 x 16 result
+    const int r = lane >> 2, q = lane & 3;
+    double g[2][3][2] = {};
+    const bool c0 = r < p, c1 = r + 8 < p;
+#pragma unroll 4
+    for (int l0 = 4 * wid; l0 < nr; l0 += 4 * nw) {
+      const int l = l0 + q;
+      const double* y = Y + (long long)l * p + r;
+      const double* ay = AY + (long long)l * p + r;
+      const bool in = l < nr;
+      const double y0 = in && c0 ? y[0] : 0.0, y1 = in && c1 ? y[8] : 0.0;
+      const double a0 = in && c0 ? ay[0] : 0.0, a1 = in && c1 ? ay[8] : 0.0;
+      dmma_8x8x4(g[0][0][0], g[0][0][1], y0, y0);
+      dmma_8x8x4(g[0][1][0], g[0][1][1], y0, y1);
+      dmma_8x8x4(g[0][2][0], g[0][2][1], y1, y1);
+      dmma_8x8x4(g[1][0][0], g[1][0][1], y0, a0);
+      dmma_8x8x4(g[1][1][0], g[1][1][1], y0, a1);
+      dmma_8x8x4(g[1][2][0], g[1][2][1], y1, a1);
+    }
+#pragma unroll
+    for (int which = 0; which < 2; ++which) {
+      double* o = sm.part[wid];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = 2 * q + h;
+        o[r * 16 + c] = g[which][0][h];
+        o[r * 16 + 8 + c] = g[which][1][h];
+        o[(8 + r) * 16 + 8 + c] = g[which][2][h];
+      }
+      __syncthreads();
+      if (tid < 256) {
+        int a = tid >> 4, b = tid & 15;
+        if (a >= 8 && b < 8) {  // the block below the diagonal is the mirror
+          const int x = a;
+          a = b;
+          b = x;
+        }
+        double v = 0.0;
+        for (int w = 0; w < nw; ++w) v += sm.part[w][a * 16 + b];
+        sm.G[which * 256 + tid] = v;
+      }
+      __syncthreads();
     }
   }
-  __syncthreads();
-  cta_jacobi_eigh(G, U, w, q, PMF_L3_MAXP, ijac, jac);
-  // X <- X U and AY <- AY U, through Y
-  for (long long e = tid; e < (long long)nr * q; e += nt) {
-    const int i = (int)(e / q), c = (int)(e % q);
-    double ax = 0.0;
-    for (int a = 0; a < q; ++a) ax += X[(long long)i * p + a] * U[a * PMF_L3_MAXP + c];
-    Y[(long long)i * p + c] = ax;
+  if (wid == 0) {
+    auto load = [&](int which, double(&g)[kL3Cols]) {
+#pragma unroll
+      for (int j = 0; j < kL3Cols; ++j) g[j] = (j < p && lane < p) ? sm.G[which * 256 + j * 16 + lane] : 0.0;
+    };
+    const int q = warp_rayleigh_ritz<kL3Cols, kL3Cols>(sm.rr, p, p, 1e-12, load, sm.C, kL3Cols);
+    if (lane == 0) st[rk].q = q;
+    if (lane < min(p, q)) st[rk].w[lane] = sm.rr.lam[lane];
+    sm.red[0] = q;
   }
   __syncthreads();
-  for (long long e = tid; e < (long long)nr * q; e += nt) {
-    const int i = (int)(e / q), c = (int)(e % q);
-    X[(long long)i * p + c] = Y[(long long)i * p + c];
-  }
+  const int q = (int)sm.red[0];
   __syncthreads();
-  for (long long e = tid; e < (long long)nr * q; e += nt) {
-    const int i = (int)(e / q), c = (int)(e % q);
-    double ay = 0.0;
-    for (int a = 0; a < q; ++a) ay += AY[(long long)i * p + a] * U[a * PMF_L3_MAXP + c];
-    Y[(long long)i * p + c] = ay;
-  }
-  __syncthreads();
-  for (long long e = tid; e < (long long)nr * q; e += nt) {
-    const int i = (int)(e / q), c = (int)(e % q);
-    AY[(long long)i * p + c] = Y[(long long)i * p + c];
-  }
-  if (tid == 0) conv = q >= en2 ? 1 : 0;
-  __syncthreads();
-  const double thr = tol * st[r].anorm;
-  for (int c = tid; c < min(en2, q); c += nt) {
-    double rr = 0.0;
-    for (int l = 0; l < nr; ++l) {
-      const double v = AY[(long long)l * p + c] - w[c] * X[(long long)l * p + c];
-      rr += v * v;
+  const int nw2 = min(en2, q);
+  double res[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) res[c] = 0.0;
+  for (int l = tid; l < nr; l += kL3Thr) {
+    double y[kL3Cols], ay[kL3Cols];
+#pragma unroll
+    for (int a = 0; a < kL3Cols; ++a) {
+      y[a] = a < p ? Y[(long long)l * p + a] : 0.0;
+      ay[a] = a < p ? AY[(long long)l * p + a] : 0.0;
     }
-    if (sqrt(rr) > thr) conv = 0;
+#pragma unroll
+    for (int c = 0; c < kL3Cols; ++c)
+      if (c < q) {
+        double x = 0.0;
+#pragma unroll
+        for (int a = 0; a < kL3Cols; ++a)
+          if (a < p) x += y[a] * sm.C[a * kL3Cols + c];
+        X[(long long)l * p + c] = x;
+        if (c < 8 && c < nw2) {
+          double ax = 0.0;
+#pragma unroll
+          for (int a = 0; a < kL3Cols; ++a)
+            if (a < p) ax += ay[a] * sm.C[a * kL3Cols + c];
+          const double d = ax - sm.rr.lam[c] * x;
+          res[c] += d * d;
+        }
+      }
+  }
+  bool conv = q >= en2;
+  const double thr = tol * st[rk].anorm;
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    if (c < nw2) {
+      const double rr = block_sum(res[c], sm.red);
+      __syncthreads();
+      if (tid == 0) sm.G[c] = rr;
+    }
+  __syncthreads();
+  for (int c = 0; c < nw2; ++c) conv = conv && sqrt(sm.G[c]) <= thr;
+  if (tid == 0) {
+    st[rk].it = it + 1;
+    st[rk].conv = conv ? 1 : 0;
+  }
+  if (conv || q == p) return;
+  // fresh directions for the dropped columns, orthogonal to the kept ones (X, complete after the barriers above)
+  auto rnd = [&](int l, int c) {
+    return hash_uniform(((unsigned long long)(rk + 7) << 44) ^ ((unsigned long long)it << 32) ^
+                        ((unsigned long long)l * (p - q) + (c - q)));
+  };
+  double* d = &sm.part[0][0];  // d[c * 16 + k] = <random column c, kept column k>
+  for (int e = wid; e < (p - q) * q; e += nw) {
+    const int c = q + e / q, k = e % q;
+    double v = 0.0, xx = 0.0;
+    for (int l = lane; l < nr; l += 32) {
+      const double x = X[(long long)l * p + k];
+      v += rnd(l, c) * x;
+      xx += x * x;
+    }
+    v = warp_sum(v);
+    xx = warp_sum(xx);
+    if (lane == 0) d[c * 16 + k] = xx > 0.0 ? v / xx : 0.0;
   }
   __syncthreads();
-  if (tid < q) st[r].w[tid] = w[tid];
-  if (tid == 0) {
-    st[r].it = it + 1;
-    st[r].conv = conv;
-  }
-  if (!conv)
-    for (long long e = tid; e < (long long)nr * (p - q); e += nt) {
-      const int i = (int)(e / (p - q)), c = q + (int)(e % (p - q));
-      X[(long long)i * p + c] = hash_uniform(((unsigned long long)(r + 7) << 44) ^ ((unsigned long long)it << 32) ^
-                                             (unsigned long long)e);
+  for (int l = tid; l < nr; l += kL3Thr)
+    for (int c = q; c < p; ++c) {
+      double v = rnd(l, c);
+      for (int k = 0; k < q; ++k) v -= d[c * 16 + k] * X[(long long)l * p + k];
+      X[(long long)l * p + c] = v;
     }
 }
 
@@ -1455,21 +1327,18 @@ __global__ void k_l3_out(RankLayout L, int en2, int p, const double* work_all, c
 void launch_dense_smallest_eig(const RankLayout& L, int nrank, int nr, int en2, int p, const double* A,
                                const double* inv, double* V, double* evals, int* iters, double tol, int max_it,
                                double* work, cudaStream_t st) {
-  // stage the iteration block in shared memory (odd leading dimension: no bank conflicts) when it fits
-  const int ldx = p | 1;
-  const size_t smem = (size_t)nr * ldx * sizeof(double);
   L3Rank* rs = nullptr;
   int* left = nullptr;
-  if (smem > 160 * 1024 && p <= kL3Cols && cudaMallocAsync((void**)&rs, sizeof(L3Rank) * nrank + 16, st) == cudaSuccess) {
+  if (p <= kL3Cols && en2 <= 8 && cudaMallocAsync((void**)&rs, sizeof(L3Rank) * nrank + 16, st) == cudaSuccess) {
     left = reinterpret_cast<int*>(rs + nrank);
     const int gx = (nr + kL3Rows - 1) / kL3Rows;
+    cudaFuncSetAttribute(k_l3_rr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(L3Smem));
     { note_launch(); k_l3_init<<<nrank, 256, 0, st>>>(L, p, A, work, rs); }
     for (int it = 0; it < max_it; ++it) {
-      { note_launch(); k_l3_mm<<<dim3(gx, nrank), 256, 0, st>>>(L, p, inv, work, 0, 1, 0, rs); }
-      { note_launch(); k_l3_svqb<<<nrank, 512, 0, st>>>(L, p, work, rs); }
-      { note_launch(); k_l3_mm<<<dim3(gx, nrank), 256, 0, st>>>(L, p, A, work, 0, 2, 1, rs); }
-      { note_launch(); k_l3_rr<<<nrank, 512, 0, st>>>(L, en2, p, work, rs, tol, it); }
-      if ((it + 1) % 8 == 0 || it + 1 == max_it) {
+      { note_launch(); k_l3_mm<<<dim3(gx, nrank), 128, 0, st>>>(L, p, inv, work, 0, 1, rs); }
+      { note_launch(); k_l3_mm<<<dim3(gx, nrank), 128, 0, st>>>(L, p, A, work, 1, 2, rs); }
+      { note_launch(); k_l3_rr<<<nrank, kL3Thr, sizeof(L3Smem), st>>>(L, en2, p, work, rs, tol, it); }
+      if ((it + 1) % 4 == 0 || it + 1 == max_it) {
         int h = 1;
         { note_launch(); k_l3_count<<<1, 256, 0, st>>>(rs, nrank, left); }
         if (cudaMemcpyAsync(&h, left, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -1483,8 +1352,10 @@ void launch_dense_smallest_eig(const RankLayout& L, int nrank, int nr, int en2, 
     return;
   }
   (void)cudaGetLastError();
-  int ld = ldx;
-  size_t sm = smem;
+  // wider blocks: one CTA per rank, the iteration block staged in shared memory (odd leading dimension: no
+  // bank conflicts) when it fits
+  int ld = p | 1;
+  size_t sm = (size_t)nr * ld * sizeof(double);
   if (sm > 160 * 1024) {
     ld = 0;
     sm = 0;

@@ -125,7 +125,7 @@ class Solver {
   long long band_len = 0;
   void* phi = nullptr;
   double *blk = nullptr, *gface = nullptr, *A2inv = nullptr, *AN = nullptr, *ANinv = nullptr, *V3 = nullptr,
-         *A3inv = nullptr, *d_eig1 = nullptr, *d_eig3 = nullptr;
+         *A3inv = nullptr, *a3part = nullptr, *d_eig1 = nullptr, *d_eig3 = nullptr;
   int *d_ks = nullptr, *d_iters = nullptr, *d_status = nullptr, *d_l3it = nullptr, *d_flag = nullptr;
   int* d_rank_nb = nullptr;
   bool coarse_ok = false;  // the level-2/3 arrays above are allocated
