@@ -98,6 +98,9 @@ class Net {
   int cap_ = 0;  // batch capacity of the workspace
   __nv_bfloat16* act_[NET_ACTS] = {};
   float* dact_[NET_ACTS] = {};
+  double* bpart_ = nullptr;  // partial bias gradients
+  float* dyal_ = nullptr;    // 16-byte aligned copy of a misaligned dL/dy
+  int dyal_cap_ = 0;
   const __nv_bfloat16* x_ = nullptr;
   int ensure(int B);
   void refresh(int layer, cudaStream_t st);
