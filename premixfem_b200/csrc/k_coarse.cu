@@ -10,95 +10,7 @@
 
 namespace pmf {
 
-// ---------------------------------------------------------------------------
-// out = base - A2 v with A2 = Phi^T A Phi stored as 7 kmax x kmax blocks per
-// subdomain row (diagonal + six face neighbours).
-__global__ void k_a2_mult(const SubInfo* subs, int nsub, int kmax, const double* blk, const double* v,
-                          const double* base, double* out, const int* done) {
-  if (done && *done) return;
-  const long long row = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (row >= (long long)nsub * kmax) return;
-  const int s = (int)(row / kmax), i = (int)(row % kmax);
-  const SubInfo& S = subs[s];
-  double acc = 0.0;
-  for (int b = 0; b < 7; ++b) {
-    const int nb = b == 0 ? s : S.nb[b - 1];
-    if (nb < 0) continue;
-    const double* B = blk + (((long long)s * 7 + b) * kmax + i) * kmax;
-    const double* vv = v + (long long)nb * kmax;
-    for (int j = 0; j < kmax; ++j) acc += B[j] * vv[j];
-  }
-  out[row] = (base ? base[row] : 0.0) - acc;
-}
-void launch_a2_mult(const SubInfo* subs, int nsub, int kmax, const double* blk, const double* v, const double* base,
-                    double* out, const int* done, cudaStream_t st) {
-  long long n = (long long)nsub * kmax;
-  { note_launch(); k_a2_mult<<<(int)((n + 255) / 256), 256, 0, st>>>(subs, nsub, kmax, blk, v, base, out, done); }
-}
-
-// Batched dense GEMV, one warp per row.
-__global__ void k_block_gemv(int nrank, int nr, const double* inv, const double* in, double* out, int accumulate,
-                             const int* done) {
-  if (done && *done) return;
-  const long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (row >= (long long)nrank * nr) return;
-  const long long r = row / nr;
-  const double* A = inv + row * nr;
-  const double* x = in + r * nr;
-  double acc = 0.0;
-  for (int j = lane; j < nr; j += 32) acc += A[j] * x[j];
-  acc = warp_sum(acc);
-  if (lane == 0) out[row] = accumulate ? out[row] + acc : acc;
-}
-void launch_block_gemv(int nrank, int nr, const double* inv, const double* in, double* out, int accumulate,
-                       const int* done, cudaStream_t st) {
-  long long threads = (long long)nrank * nr * 32;
-  { note_launch(); k_block_gemv<<<(int)((threads + 255) / 256), 256, 0, st>>>(nrank, nr, inv, in, out, accumulate, done); }
-}
-
-// d[r][j] = sum_i V[r][i][j] c[r][i]  (Psi^T r = V^T Phi^T r, per rank)
-__global__ void k_lv3_restrict(int nrank, int nr, int en2, const double* V, const double* c, double* d,
-                               const int* done) {
-  if (done && *done) return;
-  const long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (row >= (long long)nrank * en2) return;
-  const long long r = row / en2;
-  const int j = (int)(row % en2);
-  const double* Vr = V + r * nr * en2;
-  const double* cr = c + r * nr;
-  double acc = 0.0;
-  for (int i = lane; i < nr; i += 32) acc += Vr[(long long)i * en2 + j] * cr[i];
-  acc = warp_sum(acc);
-  if (lane == 0) d[row] = acc;
-}
-void launch_lv3_restrict(int nrank, int nr, int en2, const double* V, const double* c, double* d, const int* done,
-                         cudaStream_t st) {
-  long long threads = (long long)nrank * en2 * 32;
-  { note_launch(); k_lv3_restrict<<<(int)((threads + 255) / 256), 256, 0, st>>>(nrank, nr, en2, V, c, d, done); }
-}
-
-// dz[r][i] = sum_j V[r][i][j] w[r][j]
-__global__ void k_lv3_prolong(int nrank, int nr, int en2, const double* V, const double* w, double* dz,
-                              const int* done) {
-  if (done && *done) return;
-  const long long row = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (row >= (long long)nrank * nr) return;
-  const long long r = row / nr;
-  const double* Vi = V + row * en2;
-  const double* wr = w + r * en2;
-  double acc = 0.0;
-  for (int j = 0; j < en2; ++j) acc += Vi[j] * wr[j];
-  dz[row] = acc;
-}
-void launch_lv3_prolong(int nrank, int nr, int en2, const double* V, const double* w, double* dz, const int* done,
-                        cudaStream_t st) {
-  long long n = (long long)nrank * nr;
-  { note_launch(); k_lv3_prolong<<<(int)((n + 255) / 256), 256, 0, st>>>(nrank, nr, en2, V, w, dz, done); }
-}
-
-// ---- the same products over ranks of different sizes (RankLayout) ----------
+// ---- coarse products over ranks of different sizes (RankLayout) -------------
 __device__ __forceinline__ int rank_nr(const RankLayout& L, int r) { return (L.first[r + 1] - L.first[r]) * L.kmax; }
 __device__ __forceinline__ long long rank_dof0(const RankLayout& L, int r) { return (long long)L.first[r] * L.kmax; }
 // the rank whose range [off[r], off[r+1]) holds e (binary search)
@@ -114,63 +26,148 @@ __device__ __forceinline__ int rank_of(const long long* off, int nrank, long lon
   return lo;
 }
 
-// out[g] = sum_j inv_r[i][j] in[dof0_r + j] for coarse dof g = dof0_r + i, one warp per dof
-__global__ void k_block_gemv_r(RankLayout L, long long ncoarse, const double* inv, const double* in, double* out,
-                               const int* done) {
+// The cycle's coarse visits are short and follow one another, so they are bound
+// by launches and the latency of a few dependent loads: one launch for the
+// level-2 product with its accumulation into Z, one for the coarse residual's
+// update with the level-3 restriction, and one for the level-3 solve with its
+// prolongation and accumulation; five launches a V-cycle instead of ten.
+// Coarse part of an iteration: 33 us instead of 53 (one rank of 256 unknowns),
+// 40 instead of 72 (eight of 384), 100 instead of 153 (four of 2 244, whose two
+// products with the inverses stream 161 MB each).
+
+// Rows go in chunks of kCoarseRows within one rank, one CTA each; a chunk's table entry holds all a CTA
+// needs to start loading, so that no chain of index loads precedes the data.
+
+// out[g] = sum_j inv_r[i][j] in[dof0_r + j] for coarse dof g = dof0_r + i, four rows per warp at a time;
+// Z = out (first) or Z += out
+__global__ void __launch_bounds__(256) k_block_gemv_r(const CoarseChunk* chunks, const double* inv, const double* in,
+                                                      double* out, double* Z, int first, const int* done) {
   if (done && *done) return;
-  const long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (g >= ncoarse) return;
-  const int r = L.dof_rank[g];
-  const int nr = rank_nr(L, r);
-  const long long d0 = rank_dof0(L, r);
-  const double* A = inv + L.off2[r] + (g - d0) * nr;
-  const double* x = in + d0;
-  double acc = 0.0;
-  for (int j = lane; j < nr; j += 32) acc += A[j] * x[j];
-  acc = warp_sum(acc);
-  if (lane == 0) out[g] = acc;
+  const CoarseChunk ch = chunks[blockIdx.x];
+  const int lane = threadIdx.x & 31, i0 = (threadIdx.x >> 5) * 4;
+  if (i0 >= ch.rows) return;
+  const double* x = in + ch.dof0;
+  const double* A = inv + ch.a_off + (long long)i0 * ch.nr;
+  const int n1 = min(1, ch.rows - 1 - i0), n2 = min(2, ch.rows - 1 - i0), n3 = min(3, ch.rows - 1 - i0);
+  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;  // rows past the chunk repeat its last one
+#pragma unroll 4
+  for (int j = lane; j < ch.nr; j += 32) {
+    const double v = x[j];
+    a0 += A[j] * v;
+    a1 += A[(long long)n1 * ch.nr + j] * v;
+    a2 += A[(long long)n2 * ch.nr + j] * v;
+    a3 += A[(long long)n3 * ch.nr + j] * v;
+  }
+  a0 = warp_sum(a0);
+  a1 = warp_sum(a1);
+  a2 = warp_sum(a2);
+  a3 = warp_sum(a3);
+  if (lane < 4 && i0 + lane < ch.rows) {
+    const double v = lane == 0 ? a0 : lane == 1 ? a1 : lane == 2 ? a2 : a3;
+    const long long g = ch.g0 + i0 + lane;
+    out[g] = v;
+    Z[g] = first ? v : Z[g] + v;
+  }
 }
-void launch_block_gemv_r(const RankLayout& L, long long ncoarse, const double* inv, const double* in, double* out,
+void launch_block_gemv_r(const RankLayout& L, const double* inv, const double* in, double* out, double* Z, int first,
                          const int* done, cudaStream_t st) {
-  const long long threads = ncoarse * 32;
-  { note_launch(); k_block_gemv_r<<<(int)((threads + 255) / 256), 256, 0, st>>>(L, ncoarse, inv, in, out, done); }
+  { note_launch(); k_block_gemv_r<<<L.nchunk, 256, 0, st>>>(L.chunks, inv, in, out, Z, first, done); }
 }
-__global__ void k_lv3_restrict_r(RankLayout L, int nrank, int en2, const double* V, const double* c, double* d,
-                                 const int* done) {
+
+// c -= A2 dz (when dz is given) with A2 = Phi^T A Phi stored as 7 kmax x kmax
+// blocks per subdomain row (diagonal + six face neighbours), then, when V is
+// given, this chunk of rows' part of the level-3 restriction
+// part[chunk][j] = sum_i V[i][j] c[i].  Eight lanes per row, a block each.
+__global__ void __launch_bounds__(256) k_coarse_resid(const CoarseChunk* chunks, const SubInfo* subs, int kmax,
+                                                      const double* blk, const double* dz, double* c, int en2,
+                                                      const double* V, double* part, const int* done) {
   if (done && *done) return;
-  const long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  __shared__ double cs[kCoarseRows];
+  const CoarseChunk ch = chunks[blockIdx.x];
+  const int b = threadIdx.x & 7, q = threadIdx.x >> 3;
+  const long long g = ch.g0 + q;
+  double acc = 0.0;
+  if (q < ch.rows && dz) {
+    const int s = (int)(g / kmax), i = (int)(g - (long long)s * kmax);
+    const int nb = b == 0 ? s : (b < 7 ? subs[s].nb[b - 1] : -1);
+    if (nb >= 0) {
+      const double* B = blk + (((long long)s * 7 + b) * kmax + i) * kmax;
+      const double* v = dz + (long long)nb * kmax;
+#pragma unroll 8
+      for (int j = 0; j < kmax; ++j) acc += B[j] * v[j];
+    }
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (b == 0 && q < ch.rows) {
+    const double v = c[g] - acc;
+    if (dz) c[g] = v;
+    cs[q] = v;
+  }
+  if (!V) return;
+  __syncthreads();
   const int lane = threadIdx.x & 31;
-  if (row >= (long long)nrank * en2) return;
-  const int r = (int)(row / en2), j = (int)(row % en2);
-  const int nr = rank_nr(L, r);
-  const double* Vr = V + L.offv[r];
-  const double* cr = c + rank_dof0(L, r);
-  double acc = 0.0;
-  for (int i = lane; i < nr; i += 32) acc += Vr[(long long)i * en2 + j] * cr[i];
-  acc = warp_sum(acc);
-  if (lane == 0) d[row] = acc;
+  static_assert(kCoarseRows == 32, "a lane per row");
+  for (int j = threadIdx.x >> 5; j < en2; j += 8) {
+    const double v = warp_sum(lane < ch.rows ? V[ch.v_off + (long long)lane * en2 + j] * cs[lane] : 0.0);
+    if (lane == 0) part[(long long)blockIdx.x * en2 + j] = v;
+  }
 }
-void launch_lv3_restrict_r(const RankLayout& L, int nrank, int en2, const double* V, const double* c, double* d,
-                           const int* done, cudaStream_t st) {
-  const long long threads = (long long)nrank * en2 * 32;
-  { note_launch(); k_lv3_restrict_r<<<(int)((threads + 255) / 256), 256, 0, st>>>(L, nrank, en2, V, c, d, done); }
+void launch_coarse_resid(const RankLayout& L, const SubInfo* subs, const double* blk, const double* dz, double* c,
+                         int en2, const double* V, double* part, const int* done, cudaStream_t st) {
+  { note_launch(); k_coarse_resid<<<L.nchunk, 256, 0, st>>>(L.chunks, subs, L.kmax, blk, dz, c, en2, V, part, done); }
 }
-__global__ void k_lv3_prolong_r(RankLayout L, long long ncoarse, int en2, const double* V, const double* w, double* dz,
-                                const int* done) {
+
+// Level-3 solve and prolongation for this chunk of rows: d = the ranks' sums of
+// part, w = the rank's rows of A3^-1 d, dz = V w, Z = dz (first) or Z += dz.
+// Every CTA adds up d (gs lanes per entry) and forms its rank's en2 entries of w itself.
+__global__ void __launch_bounds__(256) k_lv3_solve(const CoarseChunk* chunks, const int* chunk_first, int n3, int en2,
+                                                   int gs, const double* part, const double* A3inv, const double* V,
+                                                   double* dz, double* Z, int first, const int* done) {
   if (done && *done) return;
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (g >= ncoarse) return;
-  const int r = L.dof_rank[g];
-  const double* Vi = V + L.offv[r] + (g - rank_dof0(L, r)) * en2;
-  const double* wr = w + (long long)r * en2;
-  double acc = 0.0;
-  for (int j = 0; j < en2; ++j) acc += Vi[j] * wr[j];
-  dz[g] = acc;
+  extern __shared__ double l3s[];
+  double* d = l3s;       // n3
+  double* w = l3s + n3;  // en2
+  const CoarseChunk ch = chunks[blockIdx.x];
+  const int lane = threadIdx.x & 31, gl = threadIdx.x % gs;
+  for (int e0 = 0; e0 < n3; e0 += 256 / gs) {
+    const int e = e0 + threadIdx.x / gs;
+    double v = 0.0;
+    if (e < n3) {
+      const int rr = e / en2, j = e - rr * en2, c1 = chunk_first[rr + 1];
+#pragma unroll 4
+      for (int k = chunk_first[rr] + gl; k < c1; k += gs) v += part[(long long)k * en2 + j];
+    }
+    for (int o = gs >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (e < n3 && gl == 0) d[e] = v;
+  }
+  __syncthreads();
+  for (int j = threadIdx.x >> 5; j < en2; j += 8) {
+    const double* row = A3inv + (long long)(ch.rank * en2 + j) * n3;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int e = lane; e < n3; e += 32) acc += row[e] * d[e];
+    acc = warp_sum(acc);
+    if (lane == 0) w[j] = acc;
+  }
+  __syncthreads();
+  const int q = threadIdx.x;
+  if (q < ch.rows) {
+    const double* Vi = V + ch.v_off + (long long)q * en2;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int j = 0; j < en2; ++j) acc += Vi[j] * w[j];
+    dz[ch.g0 + q] = acc;
+    Z[ch.g0 + q] = first ? acc : Z[ch.g0 + q] + acc;
+  }
 }
-void launch_lv3_prolong_r(const RankLayout& L, long long ncoarse, int en2, const double* V, const double* w,
-                          double* dz, const int* done, cudaStream_t st) {
-  { note_launch(); k_lv3_prolong_r<<<(int)((ncoarse + 255) / 256), 256, 0, st>>>(L, ncoarse, en2, V, w, dz, done); }
+void launch_lv3_solve(const RankLayout& L, int n3, int en2, const double* part, const double* A3inv, const double* V,
+                      double* dz, double* Z, int first, const int* done, cudaStream_t st) {
+  const int smem = (n3 + en2) * (int)sizeof(double);
+  int gs = 1;  // lanes per entry of d: as many as leave no second pass
+  while (gs < 32 && n3 * gs * 2 <= 256) gs *= 2;
+  if (smem > 48 * 1024) cudaFuncSetAttribute(k_lv3_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  { note_launch(); k_lv3_solve<<<L.nchunk, 256, smem, st>>>(L.chunks, L.chunk_first, n3, en2, gs, part, A3inv, V, dz, Z, first, done); }
 }
 
 __global__ void k_axpy(long long n, double a, const double* x, double* y, const int* done) {
@@ -325,33 +322,6 @@ template void launch_galerkin<double>(const Grid&, const SubInfo*, int, int, con
 // Phi^T A Phi (level-2 matrix of _PC_setup_lv2_J); mode 1: the rank-Neumann
 // matrix of _PC_setup_lv3_eigen (:938-1076), i.e. without the boundary-face
 // terms of faces that leave the rank.  Padded dofs (j >= k_s) are identity.
-__global__ void k_assemble_dense(const SubInfo* subs, int nrank, int spr, int kmax, const double* blk,
-                                 const double* gface, int mode, double* dense) {
-  const long long nr = (long long)spr * kmax;
-  const long long total = (long long)nrank * nr * nr;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(e / (nr * nr));
-    const long long rem = e % (nr * nr);
-    const int row = (int)(rem / nr), col = (int)(rem % nr);
-    const int a = row / kmax, i = row % kmax, b = col / kmax, j = col % kmax;
-    const int s = r * spr + a, s2 = r * spr + b;
-    const SubInfo& S = subs[s];
-    double v = 0.0;
-    if (i >= S.k || j >= subs[s2].k) {
-      v = (row == col) ? 1.0 : 0.0;
-    } else if (a == b) {
-      v = blk[(((long long)s * 7) * kmax + i) * kmax + j];
-      if (mode == 1)
-        for (int f = 0; f < 6; ++f)
-          if (S.nb[f] >= 0 && subs[S.nb[f]].rank != r) v -= gface[(((long long)s * 6 + f) * kmax + i) * kmax + j];
-    } else {
-      for (int f = 0; f < 6; ++f)
-        if (S.nb[f] == s2) v = blk[(((long long)s * 7 + 1 + f) * kmax + i) * kmax + j];
-    }
-    dense[e] = v;
-  }
-}
 __global__ void k_assemble_dense_r(const SubInfo* subs, int nrank, RankLayout L, long long total, const double* blk,
                                    const double* gface, int mode, double* dense) {
   const int kmax = L.kmax;
@@ -399,14 +369,6 @@ __global__ void k_add_diag_r(RankLayout L, double* dense, double mu, int relativ
 }
 void launch_add_diag_r(const RankLayout& L, int nrank, double* dense, double mu, int relative, cudaStream_t st) {
   { note_launch(); k_add_diag_r<<<nrank, 256, 0, st>>>(L, dense, mu, relative); }
-}
-
-void launch_assemble_dense(const SubInfo* subs, int nsub, int nrank, int spr, int kmax, const double* blk,
-                           const double* gface, int mode, double* dense, cudaStream_t st) {
-  (void)nsub;
-  long long total = (long long)nrank * spr * kmax * spr * kmax;
-  int nb = (int)std::min<long long>((total + 255) / 256, 148 * 32);
-  { note_launch(); k_assemble_dense<<<nb, 256, 0, st>>>(subs, nrank, spr, kmax, blk, gface, mode, dense); }
 }
 
 // In-place Gauss-Jordan inverse of SPD matrices (one CTA per matrix).

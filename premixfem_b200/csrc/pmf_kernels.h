@@ -156,6 +156,13 @@ void launch_prolong(const Grid& g, const SubInfo* subs, int nsub, int kmax, cons
 // first[r] = r spr, off2[r] = r nr^2 ...; a batch of problems has one rank per
 // problem and ragged sizes.  All arrays are device arrays of nrank + 1 entries;
 // dof_rank (nsub x kmax) maps a coarse dof to its rank.
+// kCoarseRows rows of one rank's coarse dofs: a CTA of the level-2 / level-3 products
+struct CoarseChunk {
+  int rank, rows, nr, pad;
+  long long g0, dof0;     // first dof of the chunk and of its rank
+  long long a_off, v_off;  // the chunk's first row in the dense blocks (off2) and in V (offv)
+};
+constexpr int kCoarseRows = 32;
 struct RankLayout {
   const int* first = nullptr;
   const long long* off2 = nullptr;
@@ -163,13 +170,21 @@ struct RankLayout {
   const long long* offw = nullptr;
   const int* dof_rank = nullptr;
   int kmax = 0;
+  // chunks of rank r: chunk_first[r] .. chunk_first[r+1]-1
+  int nchunk = 0;
+  const CoarseChunk* chunks = nullptr;
+  const int* chunk_first = nullptr;
 };
-void launch_block_gemv_r(const RankLayout& L, long long ncoarse, const double* inv, const double* in, double* out,
+// out = inv_r in per rank; Z = out (first) or Z += out
+void launch_block_gemv_r(const RankLayout& L, const double* inv, const double* in, double* out, double* Z, int first,
                          const int* done, cudaStream_t st);
-void launch_lv3_restrict_r(const RankLayout& L, int nrank, int en2, const double* V, const double* c, double* d,
-                           const int* done, cudaStream_t st);
-void launch_lv3_prolong_r(const RankLayout& L, long long ncoarse, int en2, const double* V, const double* w,
-                          double* dz, const int* done, cudaStream_t st);
+// c -= A2 dz (dz not null; A2 block sparse: blk[s][b][kmax][kmax], b = 0 diagonal, 1..6 couplings to nb[b-1]),
+// then part[chunk][j] = the chunk's rows of V^T c (V not null)
+void launch_coarse_resid(const RankLayout& L, const SubInfo* subs, const double* blk, const double* dz, double* c,
+                         int en2, const double* V, double* part, const int* done, cudaStream_t st);
+// dz = V A3^-1 (sum of part), Z = dz (first) or Z += dz
+void launch_lv3_solve(const RankLayout& L, int n3, int en2, const double* part, const double* A3inv, const double* V,
+                      double* dz, double* Z, int first, const int* done, cudaStream_t st);
 void launch_assemble_dense_r(const SubInfo* subs, int nrank, const RankLayout& L, long long total, const double* blk,
                              const double* gface, int mode, double* dense, cudaStream_t st);
 // dense[r] += mu (relative != 0: mu x max |diag| of the block) on the diagonal, one CTA per rank
@@ -177,18 +192,6 @@ void launch_add_diag_r(const RankLayout& L, int nrank, double* dense, double mu,
 // Gauss-Jordan inverses of the ragged blocks (the multi-CTA form of launch_spd_inverse)
 void launch_spd_inverse_r(const RankLayout& L, int nrank, int nr_max, double* dense, double tol, int* nnull,
                           cudaStream_t st);
-// out = alpha*v_in_out_base - A2 * v   where A2 is block sparse: blk[s][b][kmax][kmax],
-// b = 0 diagonal, 1..6 couplings to nb[b-1].  If base is null the base term is 0.
-void launch_a2_mult(const SubInfo* subs, int nsub, int kmax, const double* blk, const double* v, const double* base,
-                    double* out, const int* done, cudaStream_t st);
-// out[r][i] = sum_j inv[r][i][j] * in[r][j] for nrank dense blocks of size nr (batched GEMV).
-void launch_block_gemv(int nrank, int nr, const double* inv, const double* in, double* out, int accumulate,
-                       const int* done, cudaStream_t st);
-// Level-3 restriction / prolongation with the per-rank eigenvector blocks V[r][nr][en2].
-void launch_lv3_restrict(int nrank, int nr, int en2, const double* V, const double* c, double* d, const int* done,
-                         cudaStream_t st);
-void launch_lv3_prolong(int nrank, int nr, int en2, const double* V, const double* w, double* dz, const int* done,
-                        cudaStream_t st);
 void launch_axpy(long long n, double a, const double* x, double* y, const int* done, cudaStream_t st);
 void launch_copy(long long n, const double* x, double* y, const int* done, cudaStream_t st);
 
@@ -199,8 +202,6 @@ void launch_galerkin(const Grid& g, const SubInfo* subs, int nsub, int kmax, con
                      cudaStream_t st);
 // dense per-rank matrices from the block-sparse coarse operator.
 // mode 0: principal block of Phi^T A Phi (level 2); mode 1: rank-Neumann (level 3 eigen)
-void launch_assemble_dense(const SubInfo* subs, int nsub, int nrank, int spr, int kmax, const double* blk,
-                           const double* gface, int mode, double* dense, cudaStream_t st);
 // In-place batched SPD inverse by Gauss-Jordan; pivots <= tol*max|diag| are null directions.
 void launch_spd_inverse(int nb, int n, double* a, double tol, int* nnull, cudaStream_t st);
 

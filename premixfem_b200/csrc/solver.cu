@@ -423,7 +423,7 @@ Solver::~Solver() {
   void* ptrs[] = {d_subs, kx,    ky,    kz,    tx,     ty,    tz,     diag,     db,       bval,    tx32,  ty32,
                   tz32,   diag32, inv32, inv64, phi,    blk,   gface,  A2inv,    AN,       ANinv,   V3,    A3inv, a3part,
                   d_eig1, d_eig3, d_ks,  d_iters, d_status, d_l3it, d_flag, d_rank_nb, eig_work, c,     dz,    Zacc,
-                  d3,     w3,     y0,    y1,    vb,     vx,    r,      z,        p0,       p1,      w,     part,
+                  l3part, y0,    y1,    vb,     vx,    r,      z,        p0,       p1,      w,     part,
                   state};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -450,7 +450,7 @@ Solver::~Solver() {
   for (auto& e : prof_ev)
     if (e) cudaEventDestroy(e);
   for (void* q : {(void*)d_coff, ic_coef, (void*)d_kerr, (void*)phi64, (void*)d_rl_first, (void*)d_rl_off,
-                  (void*)d_rl_dof_rank, (void*)d_probs, (void*)d_layer_prob})
+                  (void*)d_rl_dof_rank, (void*)d_rl_chunk, (void*)d_rl_chunks, (void*)d_probs, (void*)d_layer_prob})
     if (q) cudaFree(q);
   if (st) cudaStreamDestroy(st);
 }
@@ -667,16 +667,35 @@ int Solver::rank_layout() {
     off[(nrank + 1) + r + 1] = off[(nrank + 1) + r] + n * en2;
     off[2 * (nrank + 1) + r + 1] = off[2 * (nrank + 1) + r] + 3 * n * l3p;
   }
-  std::vector<int> dof_rank((size_t)nsub * kmax);
+  std::vector<int> dof_rank((size_t)nsub * kmax), chunk(nrank + 1, 0);
+  for (int r = 0; r < nrank; ++r)
+    chunk[r + 1] = chunk[r] + ((rank_first[r + 1] - rank_first[r]) * kmax + kCoarseRows - 1) / kCoarseRows;
+  const int nchunk = chunk[nrank];
+  std::vector<CoarseChunk> chunks(nchunk);
+  for (int r = 0; r < nrank; ++r) {
+    const int n = (rank_first[r + 1] - rank_first[r]) * kmax;
+    for (int q = chunk[r], i = 0; q < chunk[r + 1]; ++q, i += kCoarseRows) {
+      const long long d0 = (long long)rank_first[r] * kmax;
+      chunks[q] = CoarseChunk{r, std::min(kCoarseRows, n - i), n, 0, d0 + i, d0, off[r] + (long long)i * n,
+                              off[(nrank + 1) + r] + (long long)i * en2};
+    }
+  }
   for (int r = 0; r < nrank; ++r)
     for (long long g = (long long)rank_first[r] * kmax; g < (long long)rank_first[r + 1] * kmax; ++g) dof_rank[g] = r;
   int e = dalloc((void**)&d_rl_first, sizeof(int) * (nrank + 1), "rank layout");
   if (!e) e = dalloc((void**)&d_rl_off, sizeof(long long) * off.size(), "rank layout");
   if (!e) e = dalloc((void**)&d_rl_dof_rank, sizeof(int) * dof_rank.size(), "rank layout");
+  if (!e) e = dalloc((void**)&d_rl_chunk, sizeof(int) * chunk.size(), "rank layout");
+  if (!e) e = dalloc((void**)&d_rl_chunks, sizeof(CoarseChunk) * chunks.size(), "rank layout");
   if (e) return e;
   cudaMemcpyAsync(d_rl_first, rank_first.data(), sizeof(int) * (nrank + 1), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(d_rl_off, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(d_rl_dof_rank, dof_rank.data(), sizeof(int) * dof_rank.size(), cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(d_rl_chunk, chunk.data(), sizeof(int) * chunk.size(), cudaMemcpyHostToDevice, st);
+  rl.chunk_first = d_rl_chunk;
+  cudaMemcpyAsync(d_rl_chunks, chunks.data(), sizeof(CoarseChunk) * chunks.size(), cudaMemcpyHostToDevice, st);
+  rl.chunks = d_rl_chunks;
+  rl.nchunk = nchunk;
   rl.first = d_rl_first;
   rl.off2 = d_rl_off;
   rl.offv = d_rl_off + (nrank + 1);
@@ -1226,8 +1245,7 @@ int Solver::setup() {
                       {(void**)&c, sizeof(double) * nsub * kmax, "coarse residual"},
                       {(void**)&dz, sizeof(double) * nsub * kmax, "coarse correction"},
                       {(void**)&Zacc, sizeof(double) * nsub * kmax, "coarse accumulator"},
-                      {(void**)&d3, sizeof(double) * n3, "level-3 right-hand side"},
-                      {(void**)&w3, sizeof(double) * n3, "level-3 solution"},
+                      {(void**)&l3part, sizeof(double) * rl.nchunk * en2, "level-3 right-hand side"},
                       {(void**)&d_rank_nb, sizeof(int) * nrank * 6, "rank neighbours"}};
     const int nl = (int)(sizeof(list) / sizeof(list[0]));
     for (int i = 0; i < nl; ++i) {
@@ -1628,7 +1646,7 @@ void Solver::apply_impl(const double* x, double* out, double* partial, const int
   T* yb[2] = {(T*)y0, (T*)y1};
   const std::vector<int> sch = schedule();
   int cur = 0;
-  bool y_zero = true, z_pend = false, c_valid = false;
+  bool y_zero = true, z_pend = false, c_valid = false, dz_pend = false;
   const long long ncoarse = (long long)nsub * kmax;
   for (size_t idx = 0; idx < sch.size(); ++idx) {
     const int v = sch[idx];
@@ -1672,25 +1690,25 @@ void Solver::apply_impl(const double* x, double* out, double* partial, const int
         prof_mark(PROF_RESTRICT);
         c_valid = true;
       }
-      if (v == 2) {
-        launch_block_gemv_r(rl, ncoarse, A2inv, c, dz, done, st);
-      } else if (v == 4) {  // _PC_apply_vec_lv2_2level (:1481-1537)
-        launch_cband_solve(cb_perm, cband, cb_T, cb_X, c, dz, cb_v, cb_y, cb_t, cb_part, done, st);
+      if (v == 3) {
+        launch_coarse_resid(rl, d_subs, blk, dz_pend ? dz : nullptr, c, en2, V3, l3part, done, st);
+        launch_lv3_solve(rl, n3, en2, l3part, A3inv, V3, dz, Zacc, z_pend ? 0 : 1, done, st);
       } else {
-        launch_lv3_restrict_r(rl, nrank, en2, V3, c, d3, done, st);
-        launch_block_gemv(1, n3, A3inv, d3, w3, 0, done, st);
-        launch_lv3_prolong_r(rl, ncoarse, en2, V3, w3, dz, done, st);
+        if (dz_pend) launch_coarse_resid(rl, d_subs, blk, dz, c, en2, nullptr, nullptr, done, st);
+        if (v == 2) {
+          launch_block_gemv_r(rl, A2inv, c, dz, Zacc, z_pend ? 0 : 1, done, st);
+        } else {  // _PC_apply_vec_lv2_2level (:1481-1537)
+          launch_cband_solve(cb_perm, cband, cb_T, cb_X, c, dz, cb_v, cb_y, cb_t, cb_part, done, st);
+          if (z_pend)
+            launch_axpy(ncoarse, 1.0, dz, Zacc, done, st);
+          else
+            launch_copy(ncoarse, dz, Zacc, done, st);
+        }
       }
-      if (z_pend)
-        launch_axpy(ncoarse, 1.0, dz, Zacc, done, st);
-      else
-        launch_copy(ncoarse, dz, Zacc, done, st);
       z_pend = true;
-      const bool next_coarse = !last && sch[idx + 1] != 1;
-      if (next_coarse)
-        launch_a2_mult(d_subs, nsub, kmax, blk, dz, c, c, done, st);
-      else
-        c_valid = false;
+      // the next coarse visit starts from c - A2 dz
+      dz_pend = !last && sch[idx + 1] != 1;
+      c_valid = dz_pend;
       prof_mark(PROF_COARSE);
     }
   }

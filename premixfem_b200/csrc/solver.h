@@ -139,6 +139,8 @@ class Solver {
   int* d_rl_first = nullptr;
   long long* d_rl_off = nullptr;  // off2, offv, offw: 3 x (nrank + 1)
   int* d_rl_dof_rank = nullptr;
+  int* d_rl_chunk = nullptr;
+  CoarseChunk* d_rl_chunks = nullptr;
   void rank_sizes();   // host: nr, nr_min, en2, n3, l3p, tot2, totv, totw from rank_first
   int rank_layout();   // device copies of the layout
   // a batch of problems (0: one problem)
@@ -163,7 +165,7 @@ class Solver {
   int bpcg_blocks() const { return 32; }
   void* eig_work = nullptr;
   size_t eig_work_bytes = 0;
-  double *c = nullptr, *dz = nullptr, *Zacc = nullptr, *d3 = nullptr, *w3 = nullptr;
+  double *c = nullptr, *dz = nullptr, *Zacc = nullptr, *l3part = nullptr;
   void *y0 = nullptr, *y1 = nullptr;
   double *vb = nullptr, *vx = nullptr, *r = nullptr, *z = nullptr, *p0 = nullptr, *p1 = nullptr, *w = nullptr,
          *part = nullptr;
