@@ -601,7 +601,8 @@ def _lv1_kernel(tune, prec, kind):
     """Name of the level-1 kernel the tuner chose for a visit kind (0: first
     visit, 1: with the iterate, timed in its final-visit form).  Candidates:
     the natural-order kernel at each thread count, then (b2 / b3 in the key)
-    the blocked kernel at 512 and 256 threads and its staged form."""
+    the blocked kernel at 512 and 256 threads and its staged form, then (w1 in
+    the key) the kernel with one warp per subdomain."""
     ty = "float" if prec == "f32" else "double"
     args = f"<{ty},1,1>" if kind else f"<{ty},0,0>"
     for key, (choice, us) in tune.items():
@@ -609,7 +610,10 @@ def _lv1_kernel(tune, prec, kind):
         if parts[0] != "ic_apply" or parts[1] != prec or f"y{kind}" not in parts:
             continue
         nblk = int(next((q[1:] for q in parts if q.startswith("b") and q[1:].isdigit()), "0"))
-        nnat = len(us) - nblk
+        nwarp = 1 if "w1" in parts else 0
+        if choice >= len(us) - nwarp:
+            return "k_ic_warp" + args
+        nnat = len(us) - nblk - nwarp
         if choice < nnat:
             return "k_ic_apply" + args
         return ("k_ic_apply_blk" if choice - nnat < 2 else "k_ic_apply_stg") + args

@@ -6,7 +6,10 @@
 // in between is the shared three-level cycle of the whole batch (its
 // operators are block diagonal over the problems); it runs while any problem
 // is still iterating, and the CG kernels of a finished problem do nothing.
+#include <algorithm>
+
 #include "pmf_kernels.h"
+#include "pmf_stencil.cuh"
 
 namespace pmf {
 
@@ -28,7 +31,8 @@ __device__ __forceinline__ double bfixed_sum(const double* part, int n, double* 
 }  // namespace
 
 // r = b, x = 0, partial r.r per (problem, block)
-__global__ void k_bpcg_start(const ProbInfo* probs, const double* b, double* x, double* r, double* part, int nblk) {
+__global__ void k_bpcg_start(const ProbInfo* probs, const double* b, double* x, double* r, float* r32, double* part,
+                             int nblk) {
   __shared__ double red[32];
   const int q = blockIdx.y;
   const ProbCells pc = prob_cells(probs[q], nblk);
@@ -37,6 +41,7 @@ __global__ void k_bpcg_start(const ProbInfo* probs, const double* b, double* x, 
     const double bc = b[c];
     x[c] = 0.0;
     r[c] = bc;
+    if (r32) r32[c] = (float)bc;
     v += bc * bc;
   }
   v = block_sum(v, red);
@@ -76,102 +81,41 @@ __global__ void k_bpcg_beta_fin(const ProbInfo* probs, const double* part, PcgSt
   }
 }
 
-// p <- z (first) or z + (beta/betaold) p; w <- A p; partial p.w (the single-problem kernel per problem)
-__global__ void k_bpcg_iter_a(Grid g, const ProbInfo* probs, const double* tx, const double* ty, const double* tz,
-                              const double* diag, const double* z, const double* pin, double* pout, double* w,
-                              double* part, const PcgState* st, int nblk) {
-  __shared__ double red[32];
-  const int q = blockIdx.y;
-  const PcgState& s = st[q];
-  if (s.done) return;
-  const bool first = s.first != 0;
-  const double b = first ? 0.0 : s.beta / s.betaold;
-  const ProbCells pc = prob_cells(probs[q], nblk);
-  double v = 0.0;
-  for (long long c = pc.c0; c < pc.c1; c += pc.stride) {
-    const int ex = (int)(c % g.M);
-    const long long t = c / g.M;
-    const int ey = (int)(t % g.N), ez = (int)(t / g.N);
-#define PNEW(i) (first ? z[i] : z[i] + b * pin[i])
-    const double pcv = PNEW(c);
-    double a = diag[c] * pcv;
-    if (ex > 0) a -= tx[c] * PNEW(c - 1);
-    if (ex < g.M - 1) a -= tx[c + 1] * PNEW(c + 1);
-    if (ey > 0) a -= ty[c] * PNEW(c - g.M);
-    if (ey < g.N - 1) a -= ty[c + g.M] * PNEW(c + g.M);
-    if (ez > 0) a -= tz[c] * PNEW(c - g.MN);
-    if (ez < g.P - 1) a -= tz[c + g.MN] * PNEW(c + g.MN);
-#undef PNEW
-    pout[c] = pcv;
-    w[c] = a;
-    v += pcv * a;
-  }
-  v = block_sum(v, red);
-  if (threadIdx.x == 0) part[(long long)q * nblk + blockIdx.x] = v;
-}
-__global__ void k_bpcg_iter_a_fin(const double* part, int nblk, PcgState* st) {
-  __shared__ double red[32];
-  const int q = blockIdx.x;
-  PcgState& s = st[q];
-  if (s.done) return;
-  const double dpi = bfixed_sum(part + (long long)q * nblk, nblk, red);
-  if (threadIdx.x == 0) {
-    s.dpiold = s.dpi;
-    s.dpi = dpi;
-    s.betaold = s.beta;
-    const bool flip = !s.first && ((dpi > 0) != (s.dpiold > 0));
-    s.first = 0;
-    if (dpi == 0.0 || flip) {
-      s.its += 1;
-      s.done = 3;  // KSP_DIVERGED_INDEFINITE_MAT
-    } else {
-      s.alpha = s.beta / dpi;
-    }
-  }
-}
-
-// The same step one cell per thread: a (32 x 4)-thread CTA covers 32 x 4 cells of
+// p <- z (first) or z + (beta/betaold) p; w <- A p: a CTA covers a 32 x 8 tile of
 // one layer of the shared mesh, whose problem is layer_prob[z] (separator
-// layers: none); partial (z gy + y) gx + x, so problem q's partials are the
-// contiguous range of its layers.
-__global__ void __launch_bounds__(128) k_bpcg_iter_a1(Grid g, const int* layer_prob, const double* __restrict__ tx,
-                                                     const double* __restrict__ ty, const double* __restrict__ tz,
-                                                     const double* __restrict__ diag, const double* __restrict__ z,
-                                                     const double* __restrict__ pin, double* pout, double* w,
-                                                     double* part, const PcgState* st) {
-  __shared__ double red[4];
-  const int ez = blockIdx.z;
-  const int q = layer_prob[ez];
-  if (q < 0) return;
-  const PcgState& s = st[q];
-  if (s.done) return;
-  const bool first = s.first != 0;
-  const double b = first ? 0.0 : s.beta / s.betaold;
-  const int ex = blockIdx.x * 32 + threadIdx.x, ey = blockIdx.y * 4 + threadIdx.y;
-  double v = 0.0;
-  if (ex < g.M && ey < g.N) {
-    const long long c = ((long long)ez * g.N + ey) * g.M + ex;
-#define PNEW(i) (first ? z[i] : z[i] + b * pin[i])
-    const double pcv = PNEW(c);
-    double a = diag[c] * pcv;
-    if (ex > 0) a -= tx[c] * PNEW(c - 1);
-    if (ex < g.M - 1) a -= tx[c + 1] * PNEW(c + 1);
-    if (ey > 0) a -= ty[c] * PNEW(c - g.M);
-    if (ey < g.N - 1) a -= ty[c + g.M] * PNEW(c + g.M);
-    if (ez > 0) a -= tz[c] * PNEW(c - g.MN);
-    if (ez < g.P - 1) a -= tz[c + g.MN] * PNEW(c + g.MN);
-#undef PNEW
-    pout[c] = pcv;
-    w[c] = a;
-    v = pcv * a;
+// layers: none); layers past the grid's y limit are taken in turn.  Tiles past
+// the problem's own extent (the shared mesh is the largest of all problems in x
+// and y) only report a zero partial; everything there is zero and stays so.
+// Partial z tiles + tile of p.w, so problem q's partials are the contiguous range
+// of its layers.  (A solve of 16 problems of 24..80 cells per axis takes 18.4 ms;
+// with this step and the next over the whole shared mesh 25.)
+__global__ void __launch_bounds__(kStX * kStY) k_bpcg_iter_a(Grid g, const ProbInfo* probs, const int* layer_prob,
+                                                             const double* tx, const double* ty, const double* tz,
+                                                             const double* diag, const double* __restrict__ z,
+                                                             const double* __restrict__ pin,
+                                                             double* __restrict__ pout, double* __restrict__ w,
+                                                             double* __restrict__ part, const PcgState* st) {
+  const int2 xy = stencil_xy(g);
+  for (int ez = blockIdx.y; ez < g.P; ez += gridDim.y) {
+    const int q = layer_prob[ez];
+    if (q < 0) continue;
+    const PcgState& s = st[q];
+    if (s.done) continue;
+    const double b = s.first ? 0.0 : s.beta / s.betaold;  // the first step: pin is zero
+    double v = 0.0;
+    if (xy.x < probs[q].M && xy.y < probs[q].N)
+      stencil_march(g, tx, ty, tz, diag, ez, ez + 1, [&](long long c) { return z[c] + b * pin[c]; },
+                    [&](long long c, double pc, double a) {
+                      pout[c] = pc;
+                      w[c] = a;
+                      v = pc * a;
+                    });
+    v = stencil_sum(v);
+    if (threadIdx.x == 0 && threadIdx.y == 0) part[(long long)ez * gridDim.x + blockIdx.x] = v;
+    __syncthreads();  // the sum's scratch is reused
   }
-  v = warp_sum(v);
-  if (threadIdx.x == 0) red[threadIdx.y] = v;
-  __syncthreads();
-  if (threadIdx.x == 0 && threadIdx.y == 0)
-    part[((long long)ez * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = ((red[0] + red[1]) + red[2]) + red[3];
 }
-__global__ void __launch_bounds__(1024) k_bpcg_iter_a1_fin(const ProbInfo* probs, const double* part, int per_layer,
+__global__ void __launch_bounds__(1024) k_bpcg_iter_a_fin(const ProbInfo* probs, const double* part, int per_layer,
                                                            PcgState* st) {
   __shared__ double red[32];
   const int q = blockIdx.x;
@@ -206,45 +150,70 @@ __global__ void __launch_bounds__(1024) k_bpcg_iter_a1_fin(const ProbInfo* probs
   }
 }
 
-// x += alpha p, r -= alpha w, partial r.r
-__global__ void k_bpcg_iter_b(const ProbInfo* probs, double* x, double* r, const double* p, const double* w,
-                              double* part, const PcgState* st, int nblk) {
+// x += alpha p, r -= alpha w, partial r.r over the problem's own cells: gridDim.x CTAs per layer
+__global__ void __launch_bounds__(kBT) k_bpcg_iter_b(Grid g, const ProbInfo* probs, const int* layer_prob, double* x,
+                                                     double* r, float* r32, const double* p, const double* w,
+                                                     double* part, const PcgState* st) {
   __shared__ double red[32];
-  const int q = blockIdx.y;
-  const PcgState& s = st[q];
-  if (s.done) return;
-  const double a = s.alpha;
-  const ProbCells pc = prob_cells(probs[q], nblk);
-  double v = 0.0;
-  for (long long c = pc.c0; c < pc.c1; c += pc.stride) {
-    x[c] += a * p[c];
-    const double rc = r[c] - a * w[c];
-    r[c] = rc;
-    v += rc * rc;
-  }
-  v = block_sum(v, red);
-  if (threadIdx.x == 0) part[(long long)q * nblk + blockIdx.x] = v;
-}
-__global__ void k_bpcg_iter_b_fin(const double* part, int nblk, PcgState* st) {
-  __shared__ double red[32];
-  const int q = blockIdx.x;
-  PcgState& s = st[q];
-  if (s.done) return;
-  const double v = bfixed_sum(part + (long long)q * nblk, nblk, red);
-  if (threadIdx.x == 0) {
-    const double dp = sqrt(v);
-    s.dp = dp;
-    s.its += 1;
-    if (!(dp == dp) || isinf(dp))
-      s.done = 4;
-    else if (dp <= s.ttol)
-      s.done = 1;
-    else if (s.its >= s.max_it)
-      s.done = 2;
+  for (int ez = blockIdx.y; ez < g.P; ez += gridDim.y) {
+    const int q = layer_prob[ez];
+    if (q < 0) continue;
+    const PcgState& s = st[q];
+    if (s.done) continue;
+    const double a = s.alpha;
+    const int M = probs[q].M, n = M * probs[q].N;
+    const long long c0 = (long long)ez * g.MN;
+    double v = 0.0;
+#pragma unroll 4
+    for (int i = blockIdx.x * kBT + threadIdx.x; i < n; i += gridDim.x * kBT) {
+      const int ey = i / M;
+      const long long c = c0 + (long long)ey * g.M + (i - ey * M);
+      x[c] += a * p[c];
+      const double rc = r[c] - a * w[c];
+      r[c] = rc;
+      if (r32) r32[c] = (float)rc;
+      v += rc * rc;
+    }
+    v = block_sum(v, red);
+    if (threadIdx.x == 0) part[(long long)ez * gridDim.x + blockIdx.x] = v;
   }
 }
-
+// the residual norms, iteration counts and stop codes (a warp per problem, its partials in order), then
 // all_done = 1 when every problem has stopped (the shared preconditioner kernels test it)
+__global__ void __launch_bounds__(1024) k_bpcg_iter_b_fin(const ProbInfo* probs, int nprob, const double* part,
+                                                          int per_layer, PcgState* st, int* all_done) {
+  __shared__ int any;
+  if (threadIdx.x == 0) any = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int q = threadIdx.x >> 5; q < nprob; q += 32) {
+    PcgState& s = st[q];
+    int d = s.done;
+    if (!d) {
+      const double* pp = part + (long long)probs[q].z0 * per_layer;
+      const int n = probs[q].P * per_layer;
+      double v = 0.0;
+#pragma unroll 4
+      for (int i = lane; i < n; i += 32) v += pp[i];
+      v = warp_sum(v);
+      if (lane == 0) {
+        const double dp = sqrt(v);
+        s.dp = dp;
+        s.its += 1;
+        if (!(dp == dp) || isinf(dp))
+          d = 4;
+        else if (dp <= s.ttol)
+          d = 1;
+        else if (s.its >= s.max_it)
+          d = 2;
+        s.done = d;
+      }
+    }
+    if (lane == 0 && !d) any = 1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *all_done = any ? 0 : 1;
+}
 __global__ void k_bpcg_all_done(const PcgState* st, int nprob, int* all_done) {
   __shared__ int any;
   if (threadIdx.x == 0) any = 0;
@@ -255,9 +224,9 @@ __global__ void k_bpcg_all_done(const PcgState* st, int nprob, int* all_done) {
   if (threadIdx.x == 0) *all_done = any ? 0 : 1;
 }
 
-void launch_bpcg_start(const ProbInfo* probs, int nprob, const double* b, double* x, double* r, double* part,
-                       PcgState* st, double rtol, double atol, int max_it, int* all_done, int nblk, cudaStream_t s) {
-  { note_launch(); k_bpcg_start<<<dim3(nblk, nprob), kBT, 0, s>>>(probs, b, x, r, part, nblk); }
+void launch_bpcg_start(const ProbInfo* probs, int nprob, const double* b, double* x, double* r, float* r32,
+                       double* part, PcgState* st, double rtol, double atol, int max_it, int* all_done, int nblk, cudaStream_t s) {
+  { note_launch(); k_bpcg_start<<<dim3(nblk, nprob), kBT, 0, s>>>(probs, b, x, r, r32, part, nblk); }
   { note_launch(); k_bpcg_start_fin<<<nprob, 256, 0, s>>>(part, nblk, st, rtol, atol, max_it); }
   { note_launch(); k_bpcg_all_done<<<1, 256, 0, s>>>(st, nprob, all_done); }
 }
@@ -266,22 +235,18 @@ void launch_bpcg_beta(const ProbInfo* probs, int nprob, const double* part, PcgS
 }
 void launch_bpcg_iter_a(const Grid& g, const ProbInfo* probs, const int* layer_prob, int nprob, const double* tx,
                         const double* ty, const double* tz, const double* diag, const double* z, const double* pin,
-                        double* pout, double* w, double* part, PcgState* st, int nblk, cudaStream_t s) {
-  // one cell per thread (pcg_part_capacity(g) partials) where the grid fits, else the grid-stride form
-  const dim3 grid((g.M + 31) / 32, (g.N + 3) / 4, g.P);
-  if (layer_prob && grid.y <= 65535 && grid.z <= 65535) {
-    { note_launch(); k_bpcg_iter_a1<<<grid, dim3(32, 4), 0, s>>>(g, layer_prob, tx, ty, tz, diag, z, pin, pout, w, part, st); }
-    { note_launch(); k_bpcg_iter_a1_fin<<<nprob, 1024, 0, s>>>(probs, part, (int)(grid.x * grid.y), st); }
-    return;
-  }
-  { note_launch(); k_bpcg_iter_a<<<dim3(nblk, nprob), kBT, 0, s>>>(g, probs, tx, ty, tz, diag, z, pin, pout, w, part, st, nblk); }
-  { note_launch(); k_bpcg_iter_a_fin<<<nprob, 256, 0, s>>>(part, nblk, st); }
+                        double* pout, double* w, double* part, PcgState* st, cudaStream_t s) {
+  // a partial per tile and layer: pcg_part_capacity(g) of them at most
+  const dim3 grid((g.M + kStX - 1) / kStX * ((g.N + kStY - 1) / kStY), std::min(g.P, 65535));
+  { note_launch(); k_bpcg_iter_a<<<grid, dim3(kStX, kStY), 0, s>>>(g, probs, layer_prob, tx, ty, tz, diag, z, pin, pout, w, part, st); }
+  { note_launch(); k_bpcg_iter_a_fin<<<nprob, 1024, 0, s>>>(probs, part, (int)grid.x, st); }
 }
-void launch_bpcg_iter_b(const ProbInfo* probs, int nprob, double* x, double* r, const double* p, const double* w,
-                        double* part, PcgState* st, int* all_done, int nblk, cudaStream_t s) {
-  { note_launch(); k_bpcg_iter_b<<<dim3(nblk, nprob), kBT, 0, s>>>(probs, x, r, p, w, part, st, nblk); }
-  { note_launch(); k_bpcg_iter_b_fin<<<nprob, 256, 0, s>>>(part, nblk, st); }
-  { note_launch(); k_bpcg_all_done<<<1, 256, 0, s>>>(st, nprob, all_done); }
+void launch_bpcg_iter_b(const Grid& g, const ProbInfo* probs, const int* layer_prob, int nprob, double* x, double* r,
+                        float* r32, const double* p, const double* w, double* part, PcgState* st, int* all_done,
+                        cudaStream_t s) {
+  const int sub = std::max(1, std::min(32, (int)(g.MN / 2048)));  // CTAs per layer, fewer than its tiles
+  { note_launch(); k_bpcg_iter_b<<<dim3(sub, std::min(g.P, 65535)), kBT, 0, s>>>(g, probs, layer_prob, x, r, r32, p, w, part, st); }
+  { note_launch(); k_bpcg_iter_b_fin<<<1, 1024, 0, s>>>(probs, nprob, part, sub, st, all_done); }
 }
 
 }  // namespace pmf

@@ -1,8 +1,10 @@
 // Fine-grid kernels: operator assembly, stencil products, CG vector updates,
 // level-1 IC(0) block solves and the level-2 restriction / prolongation.
 #include <algorithm>
+#include <type_traits>
 
 #include "pmf_kernels.h"
+#include "pmf_stencil.cuh"
 
 namespace pmf {
 
@@ -146,19 +148,19 @@ __device__ __forceinline__ T apply_A(const Grid& g, long long c, int ex, int ey,
   return v;
 }
 
-__global__ void k_spmv(Grid g, const double* tx, const double* ty, const double* tz, const double* diag,
-                       const double* x, double* y) {
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.ncell;
-       c += (long long)gridDim.x * blockDim.x) {
-    int ex, ey, ez;
-    decode(c, g, ex, ey, ez);
-    y[c] = apply_A(g, c, ex, ey, ez, tx, ty, tz, diag, x);
-  }
+// 135 us at 256^3 (5.96 TB/s of its 48 B per cell); one cell per thread with a decoded index took 185.
+__global__ void __launch_bounds__(kStX * kStY) k_spmv(Grid g, const double* tx, const double* ty, const double* tz,
+                                                      const double* diag, const double* __restrict__ x,
+                                                      double* __restrict__ y, int zc) {
+  const int z0 = blockIdx.y * zc;
+  stencil_march(g, tx, ty, tz, diag, z0, min(g.P, z0 + zc), [&](long long c) { return x[c]; },
+                [&](long long c, double, double a) { y[c] = a; });
 }
 
 void launch_spmv(const Grid& g, const double* tx, const double* ty, const double* tz, const double* diag,
                  const double* x, double* y, cudaStream_t st) {
-  { note_launch(); k_spmv<<<cell_blocks(g.ncell), kCellThreads, 0, st>>>(g, tx, ty, tz, diag, x, y); }
+  const StencilShape s = stencil_shape(g);
+  { note_launch(); k_spmv<<<s.grid, dim3(kStX, kStY), 0, st>>>(g, tx, ty, tz, diag, x, y, s.zc); }
 }
 
 // ---------------------------------------------------------------------------
@@ -207,7 +209,7 @@ void launch_dot(const double* a, const double* b, long long n, double* part, dou
 }
 
 // --- KSPSolve_CG (PETSc src/ksp/ksp/impls/cg/cg.c) with the unpreconditioned norm ---
-__global__ void k_pcg_start(long long n, const double* b, double* x, double* r, double* part) {
+__global__ void k_pcg_start(long long n, const double* b, double* x, double* r, float* r32, double* part) {
   __shared__ double red[32];
   double v = 0.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -215,6 +217,7 @@ __global__ void k_pcg_start(long long n, const double* b, double* x, double* r, 
     const double bi = b[i];
     x[i] = 0.0;
     r[i] = bi;
+    if (r32) r32[i] = (float)bi;
     v += bi * bi;
   }
   v = block_sum(v, red);
@@ -236,10 +239,10 @@ __global__ void k_pcg_start_fin(const double* part, int nb, PcgState* s, double 
     s->done = (!(dp == dp) || isinf(dp)) ? 4 : (dp <= s->ttol) ? 1 : 0;
   }
 }
-void launch_pcg_start(const Grid& g, const double* b, double* x, double* r, double* part, PcgState* s, double rtol,
-                      double atol, int max_it, cudaStream_t st) {
+void launch_pcg_start(const Grid& g, const double* b, double* x, double* r, float* r32, double* part, PcgState* s,
+                      double rtol, double atol, int max_it, cudaStream_t st) {
   int nb = cell_blocks(g.ncell);
-  { note_launch(); k_pcg_start<<<nb, kCellThreads, 0, st>>>(g.ncell, b, x, r, part); }
+  { note_launch(); k_pcg_start<<<nb, kCellThreads, 0, st>>>(g.ncell, b, x, r, r32, part); }
   { note_launch(); k_pcg_start_fin<<<1, 256, 0, st>>>(part, nb, s, rtol, atol, max_it); }
 }
 
@@ -306,37 +309,30 @@ void launch_pcg_null_beta(double* z, const double* r, long long n, double* part,
   { note_launch(); k_pcg_beta_fin<<<1, 256, 0, st>>>(part, nb, s); }
 }
 
-// p <- z (first) or z + (beta/betaold) p; w <- A p; partial p.w.
+// p <- z (first) or z + (beta/betaold) p; w <- A p; one partial of p.w per CTA.
 // In-place on p: the stencil reads p at neighbours, so p_new is formed from z
-// and the old p of each neighbour on the fly, and written to pout != pin.
-__global__ void k_pcg_iter_a(Grid g, const double* tx, const double* ty, const double* tz, const double* diag,
-                             const double* z, const double* pin, double* pout, double* w, double* part,
-                             const PcgState* s) {
-  __shared__ double red[32];
+// and the old p of each neighbour on the fly, and written to pout != pin.  The
+// first step takes beta = 0 with pin zero.  The outputs alias nothing, which
+// lets the next plane's loads pass this plane's stores: 186 us at 256^3 (5.8
+// TB/s of its 64 B per cell) instead of 275; one cell per thread took 290.
+__global__ void __launch_bounds__(kStX * kStY) k_pcg_iter_a(Grid g, const double* tx, const double* ty,
+                                                            const double* tz, const double* diag,
+                                                            const double* __restrict__ z,
+                                                            const double* __restrict__ pin, double* __restrict__ pout,
+                                                            double* __restrict__ w, double* __restrict__ part,
+                                                            const PcgState* __restrict__ s, int zc) {
+  const double b = s->first ? 0.0 : s->beta / s->betaold;
   if (s->done) return;
-  const bool first = s->first != 0;
-  const double b = first ? 0.0 : s->beta / s->betaold;
+  const int z0 = blockIdx.y * zc;
   double v = 0.0;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.ncell;
-       c += (long long)gridDim.x * blockDim.x) {
-    int ex, ey, ez;
-    decode(c, g, ex, ey, ez);
-#define PNEW(i) (first ? z[i] : z[i] + b * pin[i])
-    const double pc = PNEW(c);
-    double a = diag[c] * pc;
-    if (ex > 0) a -= tx[c] * PNEW(c - 1);
-    if (ex < g.M - 1) a -= tx[c + 1] * PNEW(c + 1);
-    if (ey > 0) a -= ty[c] * PNEW(c - g.M);
-    if (ey < g.N - 1) a -= ty[c + g.M] * PNEW(c + g.M);
-    if (ez > 0) a -= tz[c] * PNEW(c - g.MN);
-    if (ez < g.P - 1) a -= tz[c + g.MN] * PNEW(c + g.MN);
-#undef PNEW
-    pout[c] = pc;
-    w[c] = a;
-    v += pc * a;
-  }
-  v = block_sum(v, red);
-  if (threadIdx.x == 0) part[blockIdx.x] = v;
+  stencil_march(g, tx, ty, tz, diag, z0, min(g.P, z0 + zc), [&](long long c) { return z[c] + b * pin[c]; },
+                [&](long long c, double pc, double a) {
+                  pout[c] = pc;
+                  w[c] = a;
+                  v += pc * a;
+                });
+  v = stencil_sum(v);
+  if (threadIdx.x == 0 && threadIdx.y == 0) part[(long long)blockIdx.y * gridDim.x + blockIdx.x] = v;
 }
 __global__ void __launch_bounds__(1024) k_pcg_iter_a_fin(const double* part, int nb, PcgState* s) {
   __shared__ double red[32];
@@ -356,161 +352,53 @@ __global__ void __launch_bounds__(1024) k_pcg_iter_a_fin(const double* part, int
     }
   }
 }
-// The same step as a 2.5-D march: a CTA owns a 32 x 16 tile of x-lines and a
-// stretch of z-planes; the new p of the current plane sits in shared memory
-// with a one-cell halo, the planes below and above in registers, so z and p
-// are read once per cell (plus the tile halo) instead of at all seven stencil
-// points.  The operator is evaluated in apply_A's order (same w bit for bit).
-// One cell per thread: a (32 x 4)-thread CTA covers 32 x 4 cells of one z-plane,
-// the grid covers the mesh, so no thread decodes a linear index and every load
-// has the whole GPU's parallelism behind it; the seven-point stencil reads its
-// neighbours through L1/L2.  Same arithmetic as k_pcg_iter_a, in the same
-// order.  One partial of p.w per CTA.
-constexpr int kP1X = 32, kP1Y = 4;
-__global__ void __launch_bounds__(kP1X * kP1Y) k_pcg_iter_a1(Grid g, const double* __restrict__ tx,
-                                                            const double* __restrict__ ty,
-                                                            const double* __restrict__ tz,
-                                                            const double* __restrict__ diag,
-                                                            const double* __restrict__ z,
-                                                            const double* __restrict__ pin, double* pout, double* w,
-                                                            double* part, const PcgState* s) {
-  __shared__ double red[kP1Y];
-  if (s->done) return;
-  const bool first = s->first != 0;
-  const double b = first ? 0.0 : s->beta / s->betaold;
-  const int ex = blockIdx.x * kP1X + threadIdx.x, ey = blockIdx.y * kP1Y + threadIdx.y, ez = blockIdx.z;
-  double v = 0.0;
-  if (ex < g.M && ey < g.N) {
-    const long long c = ((long long)ez * g.N + ey) * g.M + ex;
-#define PNEW(i) (first ? z[i] : z[i] + b * pin[i])
-    const double pc = PNEW(c);
-    double a = diag[c] * pc;
-    if (ex > 0) a -= tx[c] * PNEW(c - 1);
-    if (ex < g.M - 1) a -= tx[c + 1] * PNEW(c + 1);
-    if (ey > 0) a -= ty[c] * PNEW(c - g.M);
-    if (ey < g.N - 1) a -= ty[c + g.M] * PNEW(c + g.M);
-    if (ez > 0) a -= tz[c] * PNEW(c - g.MN);
-    if (ez < g.P - 1) a -= tz[c + g.MN] * PNEW(c + g.MN);
-#undef PNEW
-    pout[c] = pc;
-    w[c] = a;
-    v = pc * a;
-  }
-  v = warp_sum(v);
-  if (threadIdx.x == 0) red[threadIdx.y] = v;
-  __syncthreads();
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    double t = 0.0;
-    for (int i = 0; i < kP1Y; ++i) t += red[i];
-    part[((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = t;
-  }
-}
-
+// one partial per x-y tile and plane: the batch's CG step, the largest user
 int pcg_part_capacity(const Grid& g) {
-  const long long n1 = (long long)((g.M + kP1X - 1) / kP1X) * ((g.N + kP1Y - 1) / kP1Y) * g.P;
-  return (int)std::max<long long>(cell_blocks(g.ncell), n1);
-}
-
-constexpr int kPaX = 32, kPaY = 16;
-__global__ void __launch_bounds__(kPaX * kPaY) k_pcg_iter_a25(Grid g, const double* __restrict__ tx,
-                                                             const double* __restrict__ ty,
-                                                             const double* __restrict__ tz,
-                                                             const double* __restrict__ diag,
-                                                             const double* __restrict__ z,
-                                                             const double* __restrict__ pin, double* pout,
-                                                             double* w, double* part, const PcgState* s, int zc) {
-  __shared__ double sp[kPaY + 2][kPaX + 2];
-  __shared__ double red[32];
-  if (s->done) return;
-  const bool first = s->first != 0;
-  const double b = first ? 0.0 : s->beta / s->betaold;
-  const int lx = threadIdx.x % kPaX, ly = threadIdx.x / kPaX;
-  const int ex = blockIdx.x * kPaX + lx, ey = blockIdx.y * kPaY + ly;
-  const int zb = blockIdx.z * zc, ze = min(g.P, zb + zc);
-  const bool in = ex < g.M && ey < g.N;
-  auto pn = [&](long long c) { return first ? z[c] : z[c] + b * pin[c]; };
-  const long long row = (long long)ey * g.M + ex;
-  double pprev = 0.0, pcur = 0.0;
-  if (in) {
-    pcur = pn((long long)zb * g.MN + row);
-    if (zb > 0) pprev = pn((long long)(zb - 1) * g.MN + row);
-  }
-  double v = 0.0;
-  for (int ez = zb; ez < ze; ++ez) {
-    const long long c = (long long)ez * g.MN + row;
-    const double pnext = (in && ez + 1 < g.P) ? pn(c + g.MN) : 0.0;
-    sp[ly + 1][lx + 1] = pcur;
-    if (lx == 0) sp[ly + 1][0] = (in && ex > 0) ? pn(c - 1) : 0.0;
-    if (lx == kPaX - 1) sp[ly + 1][kPaX + 1] = (in && ex + 1 < g.M) ? pn(c + 1) : 0.0;
-    if (ly == 0) sp[0][lx + 1] = (in && ey > 0) ? pn(c - g.M) : 0.0;
-    if (ly == kPaY - 1) sp[kPaY + 1][lx + 1] = (in && ey + 1 < g.N) ? pn(c + g.M) : 0.0;
-    __syncthreads();
-    if (in) {
-      double a = diag[c] * pcur;
-      if (ex > 0) a -= tx[c] * sp[ly + 1][lx];
-      if (ex < g.M - 1) a -= tx[c + 1] * sp[ly + 1][lx + 2];
-      if (ey > 0) a -= ty[c] * sp[ly][lx + 1];
-      if (ey < g.N - 1) a -= ty[c + g.M] * sp[ly + 2][lx + 1];
-      if (ez > 0) a -= tz[c] * pprev;
-      if (ez < g.P - 1) a -= tz[c + g.MN] * pnext;
-      pout[c] = pcur;
-      w[c] = a;
-      v += pcur * a;
-    }
-    __syncthreads();  // the next plane overwrites sp
-    pprev = pcur;
-    pcur = pnext;
-  }
-  v = block_sum(v, red);
-  if (threadIdx.x == 0) part[((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = v;
-}
-
-int launch_pcg_iter_a_main(const Grid& g, const double* tx, const double* ty, const double* tz, const double* diag,
-                           const double* z, const double* pin, double* pout, double* w, double* part,
-                           const PcgState* s, cudaStream_t st, int variant) {
-  // variant 0: one cell per thread (pcg_part_capacity(g) partials, the size the caller's buffer holds);
-  // 1: the 2.5-D march; 2: grid-stride.  Variants 1 and 2 use at most cell_blocks(ncell) partials.
-  if (variant == 0) {
-    const dim3 grid((g.M + kP1X - 1) / kP1X, (g.N + kP1Y - 1) / kP1Y, g.P);
-    if (grid.y <= 65535 && grid.z <= 65535) {
-      { note_launch(); k_pcg_iter_a1<<<grid, dim3(kP1X, kP1Y), 0, st>>>(g, tx, ty, tz, diag, z, pin, pout, w, part, s); }
-      return (int)(grid.x * grid.y * grid.z);
-    }
-    variant = 1;
-  }
-  const int cap = cell_blocks(g.ncell);
-  const int bx = (g.M + kPaX - 1) / kPaX, by = (g.N + kPaY - 1) / kPaY;
-  const int per_z = std::max(1, cap / std::max(1, bx * by));
-  const int zc = std::max(16, (g.P + per_z - 1) / per_z);
-  const int bz = (g.P + zc - 1) / zc;
-  const long long nb25 = (long long)bx * by * bz;
-  if (variant == 1 && nb25 <= cap && by <= 65535 && bz <= 65535) {
-    { note_launch(); k_pcg_iter_a25<<<dim3(bx, by, bz), kPaX * kPaY, 0, st>>>(g, tx, ty, tz, diag, z, pin, pout, w, part, s, zc); }
-    return (int)nb25;
-  }
-  { note_launch(); k_pcg_iter_a<<<cap, kCellThreads, 0, st>>>(g, tx, ty, tz, diag, z, pin, pout, w, part, s); }
-  return cap;
+  const long long n = (long long)((g.M + kStX - 1) / kStX) * ((g.N + kStY - 1) / kStY) * g.P;
+  return (int)std::max<long long>(cell_blocks(g.ncell), n);
 }
 
 void launch_pcg_iter_a(const Grid& g, const double* tx, const double* ty, const double* tz, const double* diag,
                        const double* z, const double* pin, double* pout, double* w, double* part, PcgState* s,
-                       cudaStream_t st, int variant) {
-  const int nb = launch_pcg_iter_a_main(g, tx, ty, tz, diag, z, pin, pout, w, part, s, st, variant);
-  { note_launch(); k_pcg_iter_a_fin<<<1, 1024, 0, st>>>(part, nb, s); }
+                       cudaStream_t st) {
+  const StencilShape sh = stencil_shape(g);
+  { note_launch(); k_pcg_iter_a<<<sh.grid, dim3(kStX, kStY), 0, st>>>(g, tx, ty, tz, diag, z, pin, pout, w, part, s, sh.zc); }
+  { note_launch(); k_pcg_iter_a_fin<<<1, 1024, 0, st>>>(part, sh.blocks(), s); }
 }
 
 // x += alpha p; r -= alpha w; partial r.r; then dp, its and the convergence test.
-__global__ void k_pcg_iter_b(long long n, double* x, double* r, const double* p, const double* w, double* part,
-                             const PcgState* s) {
+// Two cells per load where x is 16-byte aligned (a caller's pointer may not be; the solver's own arrays are).
+__global__ void __launch_bounds__(kCellThreads) k_pcg_iter_b(long long n, double* x, double* r, float* r32,
+                                                             const double* p, const double* w, double* part,
+                                                             const PcgState* s) {
   __shared__ double red[32];
   if (s->done) return;
   const double a = s->alpha;
   double v = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
+  const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, str = (long long)gridDim.x * blockDim.x;
+  long long n2 = 0;  // cells done in pairs
+  if ((reinterpret_cast<unsigned long long>(x) & 15) == 0) {
+    n2 = n & ~1LL;
+#pragma unroll 2
+    for (long long i = t0; i < n2 / 2; i += str) {
+      double2 xv = reinterpret_cast<double2*>(x)[i], rv = reinterpret_cast<double2*>(r)[i];
+      const double2 pv = reinterpret_cast<const double2*>(p)[i], wv = reinterpret_cast<const double2*>(w)[i];
+      xv.x += a * pv.x;
+      xv.y += a * pv.y;
+      rv.x -= a * wv.x;
+      rv.y -= a * wv.y;
+      reinterpret_cast<double2*>(x)[i] = xv;
+      reinterpret_cast<double2*>(r)[i] = rv;
+      if (r32) reinterpret_cast<float2*>(r32)[i] = make_float2((float)rv.x, (float)rv.y);
+      v += rv.x * rv.x;
+      v += rv.y * rv.y;
+    }
+  }
+  for (long long i = n2 + t0; i < n; i += str) {
     x[i] += a * p[i];
     const double ri = r[i] - a * w[i];
     r[i] = ri;
+    if (r32) r32[i] = (float)ri;
     v += ri * ri;
   }
   v = block_sum(v, red);
@@ -532,10 +420,10 @@ __global__ void k_pcg_iter_b_fin(const double* part, int nb, PcgState* s) {
       s->done = 2;
   }
 }
-void launch_pcg_iter_b(long long n, double* x, double* r, const double* p, const double* w, double* part,
+void launch_pcg_iter_b(long long n, double* x, double* r, float* r32, const double* p, const double* w, double* part,
                        PcgState* s, cudaStream_t st) {
   int nb = cell_blocks(n);
-  { note_launch(); k_pcg_iter_b<<<nb, kCellThreads, 0, st>>>(n, x, r, p, w, part, s); }
+  { note_launch(); k_pcg_iter_b<<<nb, kCellThreads, 0, st>>>(n, x, r, r32, p, w, part, s); }
   { note_launch(); k_pcg_iter_b_fin<<<1, 256, 0, st>>>(part, nb, s); }
 }
 
@@ -733,26 +621,63 @@ void launch_ic_apply(const Grid& g, const SubInfo* subs, int nsub, int max_lines
 // Level-2 restriction c_s = Phi_s^T (x - A y)|_s  (VecMDot in
 // _PC_apply_vec_lv2, src/PreMixFEM_3D.c:1564) fused with the residual update
 // r = x - A y of PC_apply_vec (:1859-1926): the residual is never stored.
+// KM is the number of basis vectors exactly, and a cell's row of Phi is read by
+// the widest loads that every row's alignment allows: one load per vector under a
+// run-time bound cost the prolongation 94 us at 256^3 with six FP32 vectors, this
+// 90 (its 1.2 GB of traffic need 82); the restriction stays at 185 to 190 either way.
+template <typename T, int KM>
+__device__ __forceinline__ void load_phi(const T* __restrict__ p, T (&v)[KM]) {
+  constexpr int B = KM * sizeof(T) % 16 == 0 ? 16 : KM * sizeof(T) % 8 == 0 ? 8 : 4;  // row alignment in bytes
+  if constexpr (B == 16 && sizeof(T) == 4) {
+#pragma unroll
+    for (int j = 0; j < KM; j += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(p + j);
+      v[j] = f.x;
+      v[j + 1] = f.y;
+      v[j + 2] = f.z;
+      v[j + 3] = f.w;
+    }
+  } else if constexpr (B == 16) {
+#pragma unroll
+    for (int j = 0; j < KM; j += 2) {
+      const double2 f = *reinterpret_cast<const double2*>(p + j);
+      v[j] = f.x;
+      v[j + 1] = f.y;
+    }
+  } else if constexpr (B == 8 && sizeof(T) == 4) {
+#pragma unroll
+    for (int j = 0; j < KM; j += 2) {
+      const float2 f = *reinterpret_cast<const float2*>(p + j);
+      v[j] = f.x;
+      v[j + 1] = f.y;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < KM; ++j) v[j] = p[j];
+  }
+}
+
 template <typename T, int KM, bool HAS_Y>
-__global__ void k_resid_restrict(Grid g, const SubInfo* subs, int kmax, const T* tx, const T* ty, const T* tz,
-                                 const T* diag, const T* phi, const double* x, const T* y, double* c,
-                                 const int* done) {
+__global__ void k_resid_restrict(Grid g, const SubInfo* subs, const T* __restrict__ tx, const T* __restrict__ ty,
+                                 const T* __restrict__ tz, const T* __restrict__ diag, const T* __restrict__ phi,
+                                 const T* __restrict__ x, const T* __restrict__ y, double* c, const int* done) {
   if (done && *done) return;
   __shared__ double red[KM][33];
   const SubGeom q = sub_geom(subs[blockIdx.x]);
   double acc[KM];
 #pragma unroll
   for (int j = 0; j < KM; ++j) acc[j] = 0.0;
+#pragma unroll 1
   for (int cl = threadIdx.x; cl < q.ncells; cl += blockDim.x) {
     const int i = cl % q.nx, tt = cl / q.nx, jj = tt % q.ny, k = tt / q.ny;
     const int ex = q.x0 + i, ey = q.y0 + jj, ez = q.z0 + k;
     const long long cg = ((long long)ez * g.N + ey) * g.M + ex;
-    T r = (T)x[cg];
+    T ph[KM];
+    load_phi<T, KM>(phi + cg * KM, ph);
+    T r = x[cg];
     if (HAS_Y) r -= apply_A(g, cg, ex, ey, ez, tx, ty, tz, diag, y);
-    const T* ph = phi + cg * kmax;
 #pragma unroll
-    for (int j = 0; j < KM; ++j)
-      if (j < kmax) acc[j] += (double)(ph[j] * r);
+    for (int j = 0; j < KM; ++j) acc[j] += (double)(ph[j] * r);
   }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
@@ -761,53 +686,61 @@ __global__ void k_resid_restrict(Grid g, const SubInfo* subs, int kmax, const T*
     if (lane == 0) red[j][wid] = v;
   }
   __syncthreads();
-  if (threadIdx.x < kmax) {
+  if (threadIdx.x < KM) {
     double v = 0.0;
     for (int w = 0; w < nw; ++w) v += red[threadIdx.x][w];
-    c[(long long)blockIdx.x * kmax + threadIdx.x] = v;
+    c[(long long)blockIdx.x * KM + threadIdx.x] = v;
   }
 }
 
-template <typename T, int KM>
-static void rr_dispatch(const Grid& g, const SubInfo* subs, int nsub, int kmax, const T* tx, const T* ty,
-                        const T* tz, const T* diag, const T* phi, const double* x, const T* y, double* c,
-                        const int* done, cudaStream_t st, int threads) {
-  if (y)
-    { note_launch(); k_resid_restrict<T, KM, true><<<nsub, threads, 0, st>>>(g, subs, kmax, tx, ty, tz, diag, phi, x, y, c, done); }
-  else
-    { note_launch(); k_resid_restrict<T, KM, false><<<nsub, threads, 0, st>>>(g, subs, kmax, tx, ty, tz, diag, phi, x, y, c, done); }
+// f(std::integral_constant<int, kmax>) for 1 <= kmax <= 8 (the partition's limit)
+template <class F>
+static void with_km(int kmax, F f) {
+  switch (kmax) {
+    case 1: return f(std::integral_constant<int, 1>());
+    case 2: return f(std::integral_constant<int, 2>());
+    case 3: return f(std::integral_constant<int, 3>());
+    case 4: return f(std::integral_constant<int, 4>());
+    case 5: return f(std::integral_constant<int, 5>());
+    case 6: return f(std::integral_constant<int, 6>());
+    case 7: return f(std::integral_constant<int, 7>());
+    default: return f(std::integral_constant<int, 8>());
+  }
 }
 
 template <typename T>
 void launch_resid_restrict(const Grid& g, const SubInfo* subs, int nsub, int kmax, const T* tx, const T* ty,
-                           const T* tz, const T* diag, const T* phi, const double* x, const T* y, double* c,
+                           const T* tz, const T* diag, const T* phi, const T* x, const T* y, double* c,
                            const int* done, cudaStream_t st, int threads) {
   threads = (threads >= 32 && threads <= 1024 && threads % 32 == 0) ? threads : 256;
-  if (kmax <= 4)
-    rr_dispatch<T, 4>(g, subs, nsub, kmax, tx, ty, tz, diag, phi, x, y, c, done, st, threads);
-  else if (kmax <= 8)
-    rr_dispatch<T, 8>(g, subs, nsub, kmax, tx, ty, tz, diag, phi, x, y, c, done, st, threads);
-  else
-    rr_dispatch<T, 16>(g, subs, nsub, kmax, tx, ty, tz, diag, phi, x, y, c, done, st, threads);
+  note_launch();
+  with_km(kmax, [&](auto km) {
+    constexpr int KM = decltype(km)::value;
+    if (y)
+      k_resid_restrict<T, KM, true><<<nsub, threads, 0, st>>>(g, subs, tx, ty, tz, diag, phi, x, y, c, done);
+    else
+      k_resid_restrict<T, KM, false><<<nsub, threads, 0, st>>>(g, subs, tx, ty, tz, diag, phi, x, y, c, done);
+  });
 }
 
 // Prolongation y += Phi_s Z_s (VecMAXPY in _PC_apply_vec_lv2, :1578).
 template <typename T, int KM>
-__global__ void k_prolong(Grid g, const SubInfo* subs, int kmax, const T* phi, const double* Z, T* y,
-                          const int* done) {
+__global__ void k_prolong(Grid g, const SubInfo* subs, const T* __restrict__ phi, const double* __restrict__ Z,
+                          T* __restrict__ y, const int* done) {
   if (done && *done) return;
   const SubGeom q = sub_geom(subs[blockIdx.x]);
   T z[KM];
 #pragma unroll
-  for (int j = 0; j < KM; ++j) z[j] = j < kmax ? (T)Z[(long long)blockIdx.x * kmax + j] : (T)0;
+  for (int j = 0; j < KM; ++j) z[j] = (T)Z[(long long)blockIdx.x * KM + j];
+#pragma unroll 2
   for (int cl = threadIdx.x; cl < q.ncells; cl += blockDim.x) {
     const int i = cl % q.nx, tt = cl / q.nx, jj = tt % q.ny, k = tt / q.ny;
     const long long cg = ((long long)(q.z0 + k) * g.N + (q.y0 + jj)) * g.M + (q.x0 + i);
-    const T* ph = phi + cg * kmax;
+    T ph[KM];
+    load_phi<T, KM>(phi + cg * KM, ph);
     T v = y[cg];
 #pragma unroll
-    for (int j = 0; j < KM; ++j)
-      if (j < kmax) v += ph[j] * z[j];
+    for (int j = 0; j < KM; ++j) v += ph[j] * z[j];
     y[cg] = v;
   }
 }
@@ -816,12 +749,11 @@ template <typename T>
 void launch_prolong(const Grid& g, const SubInfo* subs, int nsub, int kmax, const T* phi, const double* Z, T* y,
                     const int* done, cudaStream_t st, int threads) {
   threads = (threads >= 32 && threads <= 1024 && threads % 32 == 0) ? threads : 256;
-  if (kmax <= 4)
-    { note_launch(); k_prolong<T, 4><<<nsub, threads, 0, st>>>(g, subs, kmax, phi, Z, y, done); }
-  else if (kmax <= 8)
-    { note_launch(); k_prolong<T, 8><<<nsub, threads, 0, st>>>(g, subs, kmax, phi, Z, y, done); }
-  else
-    { note_launch(); k_prolong<T, 16><<<nsub, threads, 0, st>>>(g, subs, kmax, phi, Z, y, done); }
+  note_launch();
+  with_km(kmax, [&](auto km) {
+    constexpr int KM = decltype(km)::value;
+    k_prolong<T, KM><<<nsub, threads, 0, st>>>(g, subs, phi, Z, y, done);
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -1023,7 +955,7 @@ void launch_band_chol_apply(const Grid& g, const SubInfo* subs, int nsub, int ma
                                    const T*, const T*, const double*, const T*, T*, double*, double*, const int*, \
                                    cudaStream_t, int);                                                           \
   template void launch_resid_restrict<T>(const Grid&, const SubInfo*, int, int, const T*, const T*, const T*,     \
-                                         const T*, const T*, const double*, const T*, double*, const int*,        \
+                                         const T*, const T*, const T*, const T*, double*, const int*,             \
                                          cudaStream_t, int);                                                      \
   template void launch_prolong<T>(const Grid&, const SubInfo*, int, int, const T*, const double*, T*, const int*, \
                                   cudaStream_t, int);                                                           \

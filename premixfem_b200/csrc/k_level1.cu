@@ -39,6 +39,7 @@
 
 #include "pmf_bulk.cuh"
 #include "pmf_kernels.h"
+#include "pmf_stencil.cuh"
 
 namespace pmf {
 
@@ -436,6 +437,364 @@ __global__ void __launch_bounds__(BD, sizeof(T) == 4 ? 2 : 1)
   }
 }
 
+// One warp per subdomain.
+//
+// The sweeps are a chain of nx + ny + nz - 2 dependent steps each way, and a
+// CTA that runs them with a barrier per step (the kernels above) is bound by
+// that latency: 14 000 to 20 000 cycles a sweep for 16^3 cells, two CTAs per SM.
+// Here a warp owns a subdomain.  Lane (j, kl), j < ny, kl < KL = min(32 / ny,
+// nx - 3, nz), walks the x-lines (., j, kl), (., j, kl + KL), (., j, kl + 2 KL), ... one
+// after another, lane (j, kl) running j + kl steps behind lane (0, 0):
+// at step t it handles position t - j - kl of its chain of lines.  The j - 1 and
+// k - 1 neighbours were handled one step before by lanes of the same warp
+// (shuffles), except below kl = 0, where the value comes from shared memory,
+// written nx - KL + 1 >= 4 steps before.  A sweep is one stream of
+// nx nz / KL + ny + KL - 2 steps with no CTA barrier and no drained pipeline
+// between groups of lines, and about ten warps per SM hide each other's
+// latency.
+//
+// The factor {tx, ty, tz, 1/D}, masked at the subdomain's faces so that the
+// sweeps have no branches, is stored in step order (entry step * 32 + lane):
+// a warp copies 512 contiguous FP32 bytes per step, asynchronously, into a ring
+// of four groups of four steps, after one bulk prefetch of the whole block into
+// L2 at the kernel's start; the backward sweep reads it again, from L2 for the
+// subdomains in flight.  (Loads ahead into registers stall on the scoreboard:
+// 245 cycles a step against 130 with the ring.)  Beside the ring shared memory
+// holds only the vector, at pitch 34 per position: consecutive positions of a
+// line and consecutive lines at one step then both fall on different banks.
+//
+// The backward sweep passes the products t_ij z_j down instead of z_j, because
+// the coupling belongs to the upper cell: its sums round the products where the
+// other kernels contract them into multiply-adds (1e-12 in FP64, 1e-5 in mixed
+// precision per application, the bar between those kernels).
+//
+// Measured against the better of the other kernels: 256^3 cells in 4 096 mixed-
+// precision subdomains, 165 us the first visit (270) and 303 with the iterate,
+// its residual kernel included (411; the bytes of one pass need 72 and 113);
+// 192^3 FP64, 140 and 230 (219 and 320); 128^3 mixed, 512 subdomains, 30 and 56
+// (37 and 58).
+namespace {
+constexpr int kWarpPitch = 34;
+constexpr int kWarpBatch = 4;  // steps between warp synchronisations
+constexpr int kWarpRing = 4;   // batches of the factor in shared memory: one in use, three on their way
+}  // namespace
+
+struct IcWarpGeom {
+  int kl, nslab, npos, nstep;  // planes per group, groups, positions per lane, steps
+};
+__host__ __device__ inline IcWarpGeom ic_warp_geom(int nx, int ny, int nz) {
+  IcWarpGeom w;
+  w.kl = 32 / ny;
+  if (w.kl > nx + 1 - kWarpBatch) w.kl = nx + 1 - kWarpBatch;
+  if (w.kl > nz) w.kl = nz;
+  w.nslab = (nz + w.kl - 1) / w.kl;
+  w.npos = nx * w.nslab;
+  w.nstep = w.npos + ny + w.kl - 2;
+  return w;
+}
+
+// n / d for n, d < 2^13 by one multiplication: ceil(2^32 / d) is exact there (d = 1 apart)
+struct SmallDiv {
+  unsigned d, m;
+  __device__ explicit SmallDiv(int v) : d((unsigned)v), m((unsigned)(0xffffffffu / (unsigned)v) + 1u) {}
+  __device__ __forceinline__ int quot(int n) const { return d == 1u ? n : (int)__umulhi((unsigned)n, m); }
+};
+
+// asynchronous 16-byte copies, global to shared
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+template <int B>
+__device__ __forceinline__ void cp_async_elem(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(B) : "memory");
+}
+
+// r: the right-hand side of the sweeps, the first visit's x in precision T or the residual x - A y that
+// k_lv1_resid wrote; x: for the z.r partials of the final visit.
+template <typename T, bool HAS_Y, bool FINAL>
+__global__ void __launch_bounds__(32, 8) k_ic_warp(Grid g, const SubInfo* subs, const long long* woff,
+                                                const typename Coef4<T>::type* coef, const T* __restrict__ r,
+                                                const double* __restrict__ x, const T* __restrict__ yin,
+                                                T* __restrict__ out_t, double* __restrict__ out_d, double* part,
+                                                const int* done, int ldu) {
+  typedef typename Coef4<T>::type V4;
+  constexpr int P = kWarpPitch, BS = kWarpBatch, NB = kWarpRing;
+  if (done && *done) return;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  V4* ring = reinterpret_cast<V4*>(smem_raw);  // ring[(batch % NB) * BS * 32 + step * 32 + lane]
+  T* us = reinterpret_cast<T*>(ring + NB * BS * 32);  // us[position * P + lane]
+  T* pzs = us + ldu;                                  // products to the group below, [i * ny + j]
+  const unsigned full = 0xffffffffu;
+  const SubInfo S = subs[blockIdx.x];
+  const int nx = S.nx, ny = S.ny, nz = S.nz, nc = nx * ny * nz;
+  const IcWarpGeom w = ic_warp_geom(nx, ny, nz);
+  const int KL = w.kl, lane = threadIdx.x;
+  const V4* cw = coef + woff[blockIdx.x];
+  if (lane == 0)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(cw), "r"((uint32_t)(w.nstep * 32 * sizeof(V4)))
+                 : "memory");
+  const int MN = g.M * g.N;  // offsets within a subdomain's reach stay below the mesh size, which fits an int
+  const long long c00 = ((long long)S.z0 * g.N + S.y0) * g.M + S.x0;
+  const SmallDiv dnx(nx), dny(ny), dkl(KL);
+  struct Cell {
+    int loc, slot;  // offset from the subdomain's first cell, slot in us
+  };
+  auto place = [&](int cl) {
+    const int line = dnx.quot(cl), i = cl - line * nx, k = dny.quot(line), j = line - k * ny, grp = dkl.quot(k);
+    Cell q;
+    q.loc = k * MN + j * g.M + i;
+    q.slot = (grp * nx + i) * P + j + (k - grp * KL) * ny;
+    return q;
+  };
+  // right-hand side, cells in natural order straight into their slots, all copies in flight together
+  {
+    const T* rs = r + c00;
+#pragma unroll 4
+    for (int cl = lane; cl < nc; cl += 32) {
+      const Cell q = place(cl);
+      cp_async_elem<sizeof(T)>(us + q.slot, rs + q.loc);
+    }
+    cp_async_commit();
+    for (int e = lane; e < nx * ny; e += 32) pzs[e] = (T)0;
+  }
+  const int kl = dny.quot(lane), j = lane - kl * ny, off = j + kl;
+  // positions of this lane: whole lines with k = group * KL + kl < nz
+  const int np = kl < KL ? nx * ((nz - kl + KL - 1) / KL) : 0;
+  const bool below = kl == 0, above = kl == KL - 1;
+  T* const u0 = us + (lane - off * P);  // u0[t * P]: this lane's slot at step t
+  const int nbatch = (w.nstep + BS - 1) / BS;
+  // batch b of the factor into its ring slot (nothing past the ends; a group is committed either way)
+  auto stage = [&](int b) {
+    if (b >= 0 && b < nbatch) {
+      V4* dst = ring + (b % NB) * BS * 32 + lane;
+#pragma unroll
+      for (int q = 0; q < BS; ++q) {
+        const int t = b * BS + q;
+        if ((unsigned)(t - off) < (unsigned)np) {
+          const V4* src = cw + t * 32 + lane;
+          cp_async16(dst + q * 32, src);
+          if (sizeof(V4) == 32) cp_async16(reinterpret_cast<char*>(dst + q * 32) + 16, reinterpret_cast<const char*>(src) + 16);
+        }
+      }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int b = 0; b < NB - 1; ++b) stage(b);
+  cp_async_wait<NB - 1>();  // the right-hand side
+  __syncwarp();
+  // Forward: (D + L) u = r  ->  u_i = (r_i + sum_{lower} t_ij u_j) / D_i.  What a batch of BS steps reads from
+  // shared memory (its own slots and, for kl = 0, the group below, written nx - KL + 1 >= BS steps before) is
+  // read at its start, so a step's chain is a shuffle and four operations.
+  {
+    T up = (T)0;
+    const int dk = (KL - 1) * ny - nx * P;
+    for (int b = 0; b < nbatch; ++b) {
+      cp_async_wait<NB - 2>();  // a lane reads only what it copied itself
+      const V4* cb = ring + (b % NB) * BS * 32 + lane;
+      V4 cc[BS];
+      T rr[BS], d[BS], o[BS];
+      bool act[BS];
+#pragma unroll
+      for (int q = 0; q < BS; ++q) {
+        const int pos = b * BS + q - off;
+        act[q] = (unsigned)pos < (unsigned)np;
+        rr[q] = d[q] = (T)0;
+        cc[q] = cb[q * 32];
+        const T* s0 = u0 + (b * BS + q) * P;
+        if (act[q]) rr[q] = *s0;
+        if (below && act[q] && pos >= nx) d[q] = s0[dk];
+      }
+      stage(b + NB - 1);
+#pragma unroll
+      for (int q = 0; q < BS; ++q) {
+        const T um = __shfl_up_sync(full, up, 1);
+        T uk = __shfl_sync(full, up, (lane - ny) & 31);
+        uk = below ? d[q] : uk;
+        T s = rr[q];
+        s += cc[q].z * uk;
+        s += cc[q].y * um;
+        s += cc[q].x * up;
+        o[q] = s * cc[q].w;
+        up = act[q] ? o[q] : up;
+      }
+#pragma unroll
+      for (int q = 0; q < BS; ++q)
+        if (act[q]) u0[(b * BS + q) * P] = o[q];
+      __syncwarp();
+    }
+  }
+  cp_async_wait<0>();
+  // backward: (D + L^T) z = D u  ->  z_i = u_i + (sum_{upper} t_ij z_j) / D_i, in batches as well
+  {
+    T px = (T)0, py = (T)0, pz = (T)0;
+    const bool top = lane == 31;  // no lane above
+#pragma unroll
+    for (int b = 0; b < NB - 1; ++b) stage(nbatch - 1 - b);
+    for (int b = nbatch - 1; b >= 0; --b) {
+      cp_async_wait<NB - 2>();
+      const V4* cb = ring + (b % NB) * BS * 32 + lane;
+      V4 cc[BS];
+      T un[BS], gn[BS], o[BS], oz[BS];
+      bool act[BS];
+      T* pp[BS];
+      const int p0 = b * BS + BS - 1 - off;  // position of the batch's first step
+      int i = p0 - dnx.quot(max(p0, 0)) * nx;
+#pragma unroll
+      for (int q = 0; q < BS; ++q) {
+        act[q] = (unsigned)(p0 - q) < (unsigned)np;
+        cc[q] = cb[(BS - 1 - q) * 32];
+        un[q] = gn[q] = (T)0;
+        pp[q] = pzs + i * ny + j;
+        if (act[q]) un[q] = u0[(b * BS + BS - 1 - q) * P];
+        if (act[q] && above) gn[q] = *pp[q];
+        i = i == 0 ? nx - 1 : i - 1;
+      }
+      stage(b - (NB - 1));
+#pragma unroll
+      for (int q = 0; q < BS; ++q) {
+        T qy = __shfl_down_sync(full, py, 1);
+        T qz = __shfl_sync(full, pz, (lane + ny) & 31);
+        qy = top ? (T)0 : qy;
+        qz = above ? gn[q] : qz;
+        T s = px;
+        s += qy;
+        s += qz;
+        o[q] = un[q] + s * cc[q].w;
+        px = act[q] ? cc[q].x * o[q] : px;
+        py = act[q] ? cc[q].y * o[q] : py;
+        pz = act[q] ? cc[q].z * o[q] : pz;
+        oz[q] = pz;
+      }
+#pragma unroll
+      for (int q = 0; q < BS; ++q) {
+        if (act[q]) u0[(b * BS + BS - 1 - q) * P] = o[q];
+        if (act[q] && below) *pp[q] = oz[q];
+      }
+      __syncwarp();
+    }
+  }
+  cp_async_wait<0>();
+  // out = y + z, the loads of 16 cells in flight together
+  double dot = 0.0;
+  {
+    constexpr int UO = 16;
+    const double* xs = x + c00;
+    const T* ys = yin + c00;
+    for (int b0 = lane; b0 < nc; b0 += 32 * UO) {
+      T o[UO];
+      double xv[UO];
+      int loc[UO];
+#pragma unroll
+      for (int u = 0; u < UO; ++u) {
+        const Cell q = place(min(b0 + 32 * u, nc - 1));
+        loc[u] = q.loc;
+        o[u] = us[q.slot];
+        if (FINAL) xv[u] = xs[q.loc];
+        if (HAS_Y) o[u] += ys[q.loc];
+      }
+#pragma unroll
+      for (int u = 0; u < UO; ++u)
+        if (b0 + 32 * u < nc) {
+          if (FINAL) {
+            const double od = (double)o[u];
+            out_d[c00 + loc[u]] = od;
+            dot += xv[u] * od;
+          } else {
+            out_t[c00 + loc[u]] = o[u];
+          }
+        }
+    }
+  }
+  if (FINAL) {
+    dot = warp_sum(dot);
+    if (lane == 0) part[blockIdx.x] = dot;
+  }
+}
+
+template <typename T>
+__global__ void k_pack_ic_warp(Grid g, const SubInfo* subs, const long long* woff, const T* tx, const T* ty,
+                               const T* tz, const T* inv, typename Coef4<T>::type* coef) {
+  typedef typename Coef4<T>::type V4;
+  const SubInfo S = subs[blockIdx.x];
+  const int nx = S.nx, ny = S.ny, nc = nx * ny * S.nz;
+  const int KL = ic_warp_geom(nx, ny, S.nz).kl;
+  V4* out = coef + woff[blockIdx.x];
+  for (int cl = threadIdx.x; cl < nc; cl += blockDim.x) {
+    const int i = cl % nx, tt = cl / nx, j = tt % ny, k = tt / ny;
+    const long long cg = ((long long)(S.z0 + k) * g.N + (S.y0 + j)) * g.M + (S.x0 + i);
+    const int kl = k % KL, pos = (k / KL) * nx + i;
+    V4 c;
+    c.x = i > 0 ? tx[cg] : (T)0;
+    c.y = j > 0 ? ty[cg] : (T)0;
+    c.z = k > 0 ? tz[cg] : (T)0;
+    c.w = inv[cg];
+    out[(long long)(pos + j + kl) * 32 + j + kl * ny] = c;
+  }
+}
+
+// entries of the step-ordered factor of an nx x ny x nz subdomain, and elements of its vector in shared memory
+long long ic_warp_coef_len(int nx, int ny, int nz) { return (long long)ic_warp_geom(nx, ny, nz).nstep * 32; }
+size_t ic_warp_smem_bytes(int smem_len, int max_face, int prec_bytes) {
+  return ((size_t)kWarpRing * kWarpBatch * 32 * 4 + smem_len + max_face) * prec_bytes;
+}
+int ic_warp_smem_len(int nx, int ny, int nz) { return (ic_warp_geom(nx, ny, nz).npos * kWarpPitch + 3) & ~3; }
+
+template <typename T>
+void launch_pack_ic_warp(const Grid& g, const SubInfo* subs, int nsub, const long long* woff, const T* tx, const T* ty,
+                         const T* tz, const T* inv, void* coef, cudaStream_t st) {
+  note_launch();
+  k_pack_ic_warp<T><<<nsub, 256, 0, st>>>(g, subs, woff, tx, ty, tz, inv,
+                                          reinterpret_cast<typename Coef4<T>::type*>(coef));
+}
+
+// r = x - A y in precision T
+template <typename T>
+__global__ void __launch_bounds__(kStX * kStY) k_lv1_resid(Grid g, const T* tx, const T* ty, const T* tz, const T* diag,
+                                                           const T* __restrict__ x, const T* __restrict__ y,
+                                                           T* __restrict__ r,
+                                                           const int* done, int zc) {
+  if (done && *done) return;
+  const int z0 = blockIdx.y * zc;
+  stencil_march(g, tx, ty, tz, diag, z0, min(g.P, z0 + zc), [&](long long c) { return y[c]; },
+                [&](long long c, T, T a) { r[c] = x[c] - a; });
+}
+
+template <typename T>
+void launch_ic_warp(const Grid& g, const SubInfo* subs, int nsub, int smem_len, int max_face, const long long* woff,
+                    const void* coef, const T* tx, const T* ty, const T* tz, const T* diag, const double* x,
+                    const T* xt, const T* yin, T* rbuf, T* out_t, double* out_d, double* part, const int* done,
+                    cudaStream_t st) {
+  typedef typename Coef4<T>::type V4;
+  const int smem = (int)ic_warp_smem_bytes(smem_len, max_face, sizeof(T));
+  const V4* c4 = reinterpret_cast<const V4*>(coef);
+  const T* r = xt;
+  if (yin) {
+    const StencilShape sh = stencil_shape(g);
+    { note_launch(); k_lv1_resid<T><<<sh.grid, dim3(kStX, kStY), 0, st>>>(g, tx, ty, tz, diag, xt, yin, rbuf, done, sh.zc); }
+    r = rbuf;
+  }
+#define PMF_WRP(HY, FN)                                                                                           \
+  {                                                                                                               \
+    cudaFuncSetAttribute(k_ic_warp<T, HY, FN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);                \
+    note_launch();                                                                                                \
+    k_ic_warp<T, HY, FN><<<nsub, 32, smem, st>>>(g, subs, woff, c4, r, x, yin, out_t, out_d, part, done,          \
+                                                 smem_len);                                                       \
+  }
+  if (yin) {
+    if (out_d) PMF_WRP(true, true) else PMF_WRP(true, false)
+  } else {
+    if (out_d) PMF_WRP(false, true) else PMF_WRP(false, false)
+  }
+#undef PMF_WRP
+}
+
 template <typename T>
 __global__ void k_pack_ic_coef(Grid g, const SubInfo* subs, const long long* coff, const T* tx, const T* ty,
                                const T* tz, const T* inv, typename Coef4<T>::type* coef) {
@@ -533,6 +892,11 @@ void launch_ic_apply_stg(const Grid& g, const SubInfo* subs, int nsub, int max_c
   template void launch_ic_apply_blk<T>(const Grid&, const SubInfo*, int, int, const long long*, const void*,     \
                                        const T*, const T*, const T*, const T*, const double*, const T*, T*,      \
                                        double*, double*, const int*, int*, cudaStream_t, int);                   \
+  template void launch_pack_ic_warp<T>(const Grid&, const SubInfo*, int, const long long*, const T*, const T*,   \
+                                       const T*, const T*, void*, cudaStream_t);                                 \
+  template void launch_ic_warp<T>(const Grid&, const SubInfo*, int, int, int, const long long*, const void*,     \
+                                  const T*, const T*, const T*, const T*, const double*, const T*, const T*, T*, \
+                                  T*, double*, double*, const int*, cudaStream_t);                                            \
   template size_t ic_stg_smem_bytes<T>(int);                                                                     \
   template void launch_ic_apply_stg<T>(const Grid&, const SubInfo*, int, int, const long long*, const void*,     \
                                        const T*, const T*, const T*, const T*, const double*, const T*, T*,      \

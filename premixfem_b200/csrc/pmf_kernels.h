@@ -50,8 +50,9 @@ void launch_spmv(const Grid& g, const double* tx, const double* ty, const double
                  const double* x, double* y, cudaStream_t st);
 
 // ---- PCG -----------------------------------------------------------------------
-void launch_pcg_start(const Grid& g, const double* b, double* x, double* r, double* part, PcgState* s, double rtol,
-                      double atol, int max_it, cudaStream_t st);
+// r32: FP32 copy of the residual for the mixed form's preconditioner, or null
+void launch_pcg_start(const Grid& g, const double* b, double* x, double* r, float* r32, double* part, PcgState* s,
+                      double rtol, double atol, int max_it, cudaStream_t st);
 // beta = z.r from nparts per-block partials (written by the preconditioner's last kernel).
 void launch_pcg_beta_fin(const double* part, int nparts, PcgState* s, cudaStream_t st);
 // same, computing the partials itself
@@ -61,27 +62,23 @@ void launch_pcg_null_beta(double* z, const double* r, long long n, double* part,
                           cudaStream_t st);
 void launch_pcg_iter_a(const Grid& g, const double* tx, const double* ty, const double* tz, const double* diag,
                        const double* z, const double* pin, double* pout, double* w, double* part, PcgState* s,
-                       cudaStream_t st, int variant = 0);
-// The main kernel of launch_pcg_iter_a alone (no state update): variant 0 the
-// 2.5-D march where the mesh allows it, 1 the grid-stride kernel.  Returns the
-// number of partial sums written.
-int launch_pcg_iter_a_main(const Grid& g, const double* tx, const double* ty, const double* tz, const double* diag,
-                           const double* z, const double* pin, double* pout, double* w, double* part,
-                           const PcgState* s, cudaStream_t st, int variant);
-void launch_pcg_iter_b(long long n, double* x, double* r, const double* p, const double* w, double* part,
+                       cudaStream_t st);
+void launch_pcg_iter_b(long long n, double* x, double* r, float* r32, const double* p, const double* w, double* part,
                        PcgState* s, cudaStream_t st);
 void launch_dot(const double* a, const double* b, long long n, double* part, double* out, cudaStream_t st);
 
 // ---- CG over a batch of problems (k_batch.cu): per-problem scalars, 2-D grids
 // (blocks x problems); all_done is set when every problem has stopped
-void launch_bpcg_start(const ProbInfo* probs, int nprob, const double* b, double* x, double* r, double* part,
-                       PcgState* st, double rtol, double atol, int max_it, int* all_done, int nblk, cudaStream_t s);
+void launch_bpcg_start(const ProbInfo* probs, int nprob, const double* b, double* x, double* r, float* r32,
+                       double* part, PcgState* st, double rtol, double atol, int max_it, int* all_done, int nblk,
+                       cudaStream_t s);
 void launch_bpcg_beta(const ProbInfo* probs, int nprob, const double* part, PcgState* st, cudaStream_t s);
 void launch_bpcg_iter_a(const Grid& g, const ProbInfo* probs, const int* layer_prob, int nprob, const double* tx,
                         const double* ty, const double* tz, const double* diag, const double* z, const double* pin,
-                        double* pout, double* w, double* part, PcgState* st, int nblk, cudaStream_t s);
-void launch_bpcg_iter_b(const ProbInfo* probs, int nprob, double* x, double* r, const double* p, const double* w,
-                        double* part, PcgState* st, int* all_done, int nblk, cudaStream_t s);
+                        double* pout, double* w, double* part, PcgState* st, cudaStream_t s);
+void launch_bpcg_iter_b(const Grid& g, const ProbInfo* probs, const int* layer_prob, int nprob, double* x, double* r,
+                        float* r32, const double* p, const double* w, double* part, PcgState* st, int* all_done,
+                        cudaStream_t s);
 
 // ---- level 1 (IC(0) block solves) -------------------------------------------
 void launch_ic_factor(const Grid& g, const SubInfo* subs, int nsub, int max_lines, const double* tx, const double* ty,
@@ -123,6 +120,22 @@ void launch_ic_apply_stg(const Grid& g, const SubInfo* subs, int nsub, int max_c
                          const T* yin, T* out_t, double* out_d, double* part, const int* done, int* err,
                          cudaStream_t st);
 
+// The same solve by one warp per subdomain with the factor in step order (k_level1.cu): the entries of
+// subdomain s start at coef[woff[s]], ic_warp_coef_len of them.  Needs ny <= 32 and nx >= 4; smem_len and max_face are
+// the largest ic_warp_smem_len and nx*ny of the subdomains.
+long long ic_warp_coef_len(int nx, int ny, int nz);
+int ic_warp_smem_len(int nx, int ny, int nz);
+size_t ic_warp_smem_bytes(int smem_len, int max_face, int prec_bytes);
+template <typename T>
+void launch_pack_ic_warp(const Grid& g, const SubInfo* subs, int nsub, const long long* woff, const T* tx, const T* ty,
+                         const T* tz, const T* inv, void* coef, cudaStream_t st);
+// xt: x in precision T; rbuf: ncell values for the residual of visits with an iterate
+template <typename T>
+void launch_ic_warp(const Grid& g, const SubInfo* subs, int nsub, int smem_len, int max_face, const long long* woff,
+                    const void* coef, const T* tx, const T* ty, const T* tz, const T* diag, const double* x,
+                    const T* xt, const T* yin, T* rbuf, T* out_t, double* out_d, double* part, const int* done,
+                    cudaStream_t st);
+
 // Exact level-1 solves (-use_full_Cholesky_lv1): banded Cholesky of every
 // subdomain block in natural order, column j of L at band[boff[s] + j*band_ld(b)],
 // b = nx*ny; bad counts non-positive pivots.
@@ -139,8 +152,8 @@ void launch_band_chol_apply(const Grid& g, const SubInfo* subs, int nsub, int ma
 // c[s*kmax + j] = sum_{cells of s} phi[c*kmax + j] * (x - A y)[c]   (y may be null)
 template <typename T>
 void launch_resid_restrict(const Grid& g, const SubInfo* subs, int nsub, int kmax, const T* tx, const T* ty,
-                           const T* tz, const T* diag, const T* phi, const double* x, const T* y, double* c,
-                           const int* done, cudaStream_t st, int threads = 256);
+                           const T* tz, const T* diag, const T* phi, const T* x, const T* y, double* c, const int* done,
+                           cudaStream_t st, int threads = 256);
 
 // y[c] += sum_j phi[c*kmax + j] * Z[s*kmax + j]
 template <typename T>

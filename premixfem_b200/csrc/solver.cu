@@ -449,8 +449,9 @@ Solver::~Solver() {
   if (ev1) cudaEventDestroy(ev1);
   for (auto& e : prof_ev)
     if (e) cudaEventDestroy(e);
-  for (void* q : {(void*)d_coff, ic_coef, (void*)d_kerr, (void*)phi64, (void*)d_rl_first, (void*)d_rl_off,
-                  (void*)d_rl_dof_rank, (void*)d_rl_chunk, (void*)d_rl_chunks, (void*)d_probs, (void*)d_layer_prob})
+  for (void* q : {(void*)d_coff, ic_coef, (void*)d_woff, ic_wcoef, rt, (void*)r32, (void*)d_kerr, (void*)phi64,
+                  (void*)d_rl_first, (void*)d_rl_off, (void*)d_rl_dof_rank, (void*)d_rl_chunk, (void*)d_rl_chunks,
+                  (void*)d_probs, (void*)d_layer_prob})
     if (q) cudaFree(q);
   if (st) cudaStreamDestroy(st);
 }
@@ -725,7 +726,7 @@ int Solver::dalloc(void** p, size_t bytes, const char* what) {
 int Solver::alloc_fine() {
   const size_t n = (size_t)g.ncell;
   const size_t pb = opt.precision == 1 ? 4 : 8;
-  const int nparts = std::max(pcg_part_capacity(g), nsub) + 64;  // partial slots of the CG and level-1 kernels
+  const int nparts = std::max({pcg_part_capacity(g), nsub, nprob * bpcg_blocks()}) + 64;  // partial slots of the CG and level-1 kernels
   struct A {
     void** p;
     size_t bytes;
@@ -739,6 +740,7 @@ int Solver::alloc_fine() {
                          {(void**)&z, n * 8, "z"},        {(void**)&p0, n * 8, "p0"},
                          {(void**)&p1, n * 8, "p1"},      {(void**)&w, n * 8, "w"},
                          {(void**)&y0, n * pb, "y0"},     {(void**)&y1, n * pb, "y1"},
+                         {&rt, n * pb, "rt"},
                          {(void**)&phi, n * kmax * pb, "phi"},
                          {(void**)&part, (size_t)(nparts + cell_blocks(g.ncell)) * 8, "part"},
                          {(void**)&state, sizeof(PcgState), "state"}};
@@ -748,6 +750,7 @@ int Solver::alloc_fine() {
     list.push_back({(void**)&tz32, n * 4, "tz32"});
     list.push_back({(void**)&diag32, n * 4, "diag32"});
     list.push_back({(void**)&inv32, n * 4, "inv32"});
+    list.push_back({(void**)&r32, n * 4, "r32"});
   }
   for (size_t i = 0; i < list.size(); ++i) {
     if (int e = dalloc(list[i].p, list[i].bytes, list[i].what)) {
@@ -1066,6 +1069,7 @@ int Solver::setup() {
   }
   if (!opt.use_full_Cholesky_lv1) {
     if (int er = setup_ic_blocked(mixed)) return er;
+    if (int er = setup_ic_warp(mixed)) return er;
     if (opt.lv1_kernel == 2 && !ic_blk_ok) {
       err = "-pmf_lv1_kernel blocked needs every subdomain 16 cells wide in x with x0 % 4 == 0, M % 4 == 0 and "
             "ny*nz <= 256";
@@ -1496,6 +1500,44 @@ int Solver::setup_ic_blocked(bool mixed) {
   return 0;
 }
 
+// The step-ordered copy of the IC(0) factor for k_ic_warp, rebuilt by every
+// set-up, unless another kernel is forced by option.
+int Solver::setup_ic_warp(bool mixed) {
+  ic_wrp_ok = opt.lv1_kernel == 0;
+  ic_wrp_smem = ic_wrp_face = 0;
+  for (const SubInfo& S : subs) {
+    if (S.ny > 32 || S.nx < 4) ic_wrp_ok = false;
+    if (!ic_wrp_ok) return 0;
+    ic_wrp_smem = std::max(ic_wrp_smem, ic_warp_smem_len(S.nx, S.ny, S.nz));
+    ic_wrp_face = std::max(ic_wrp_face, S.nx * S.ny);
+  }
+  const size_t tb = mixed ? 4 : 8;
+  if (ic_warp_smem_bytes(ic_wrp_smem, ic_wrp_face, (int)tb) > 227 * 1024) ic_wrp_ok = false;
+  if (!ic_wrp_ok) return 0;
+  if (!d_woff) {
+    std::vector<long long> off(nsub);
+    long long acc = 0;
+    for (int s = 0; s < nsub; ++s) {
+      off[s] = acc;
+      acc += ic_warp_coef_len(subs[s].nx, subs[s].ny, subs[s].nz);
+    }
+    if (int e = dalloc((void**)&d_woff, sizeof(long long) * nsub, "step-ordered factor offsets")) return e;
+    if (int e = dalloc(&ic_wcoef, (size_t)acc * 4 * tb, "step-ordered IC(0) factor")) {
+      cudaFree(d_woff);
+      d_woff = nullptr;
+      return e;
+    }
+    cudaMemcpyAsync(d_woff, off.data(), sizeof(long long) * nsub, cudaMemcpyHostToDevice, st);
+    // the host vector must outlive the asynchronous copy
+    if (int e = check(cudaStreamSynchronize(st), "step-ordered factor offsets")) return e;
+  }
+  if (mixed)
+    launch_pack_ic_warp<float>(g, d_subs, nsub, d_woff, tx32, ty32, tz32, inv32, ic_wcoef, st);
+  else
+    launch_pack_ic_warp<double>(g, d_subs, nsub, d_woff, tx, ty, tz, inv64, ic_wcoef, st);
+  return 0;
+}
+
 // A bounded wait inside a kernel ran out (the kernel recorded it and returned
 // without computing): report it as a library failure.
 int Solver::check_kernel_flag(const char* what) {
@@ -1512,14 +1554,17 @@ int Solver::check_kernel_flag(const char* what) {
 
 // One level-1 visit: out = yin + IC^-1 (x - A yin) with the tuned kernel.
 template <typename T>
-void Solver::launch_lv1(const double* x, const T* yin, T* out_t, double* out_d, double* partial, const int* done) {
+void Solver::launch_lv1(const double* x, const T* xt, const T* yin, T* out_t, double* out_d, double* partial, const int* done) {
   const bool f32 = sizeof(T) == 4;
   const T* ttx = f32 ? (const T*)tx32 : (const T*)tx;
   const T* tty = f32 ? (const T*)ty32 : (const T*)ty;
   const T* ttz = f32 ? (const T*)tz32 : (const T*)tz;
   const T* tdg = f32 ? (const T*)diag32 : (const T*)diag;
   const int kind = yin ? 1 : 0;
-  if (ic_variant[kind] == 2 && ic_stg_ok) {
+  if (ic_variant[kind] == 3 && ic_wrp_ok) {
+    launch_ic_warp<T>(g, d_subs, nsub, ic_wrp_smem, ic_wrp_face, d_woff, ic_wcoef, ttx, tty, ttz, tdg, x, xt, yin,
+                      (T*)rt, out_t, out_d, partial, done, st);
+  } else if (ic_variant[kind] == 2 && ic_stg_ok) {
     launch_ic_apply_stg<T>(g, d_subs, nsub, max_cells, d_coff, ic_coef, ttx, tty, ttz, tdg, x, yin, out_t, out_d,
                            partial, done, d_kerr, st);
   } else if (ic_variant[kind] >= 1 && ic_blk_ok) {
@@ -1548,9 +1593,11 @@ void Solver::tune_pc() {
   T* yo = (T*)y1;
   cudaMemsetAsync(ya, 0, sizeof(T) * g.ncell, st);
   cudaMemsetAsync(z, 0, sizeof(double) * g.ncell, st);
+  const T* zt = f32 ? (const T*)r32 : (const T*)z;
+  if (f32) cudaMemsetAsync(r32, 0, sizeof(float) * g.ncell, st);
   cudaMemsetAsync(Zacc, 0, sizeof(double) * nsub * kmax, st);
-  const int old[8] = {ic_threads,    rr_threads,    pr_threads,        pcga_variant,
-                      ic_variant[0], ic_variant[1], ic_blk_threads[0], ic_blk_threads[1]};
+  const int old[7] = {ic_threads,    rr_threads,        pr_threads,       ic_variant[0],
+                      ic_variant[1], ic_blk_threads[0], ic_blk_threads[1]};
   char key[192];
   const char* prec = f32 ? "f32" : "f64";
   if (!opt.use_full_Cholesky_lv1) {
@@ -1561,46 +1608,54 @@ void Solver::tune_pc() {
     // candidates per visit kind (first visit: no iterate; later visits: with
     // one): the natural-order kernel with each thread count, then the blocked
     // kernel with 512 and 256 threads (when every subdomain fits it) and its
-    // staged form (when every subdomain also has ny, nz <= 16).  The natural
-    // kernel's thread count is tuned on the visits with an iterate.
+    // staged form (when every subdomain also has ny, nz <= 16), then one warp
+    // per subdomain (ny <= 32).  The natural kernel's thread count is tuned on
+    // the visits with an iterate.
     const int nnat = (int)cand.size();
     const int nblk = ic_blk_ok ? (ic_stg_ok ? 3 : 2) : 0;
+    const int nwrp = ic_wrp_ok ? 1 : 0;
     const int blk_threads[2] = {512, 256};
     // The visits with an iterate are timed in the form the V-cycle's last
     // visit takes (FP64 result and the z.r partials, into p0 and part, which
     // hold nothing yet); the first visit writes the preconditioner's iterate.
     for (int kind = 1; kind >= 0; --kind) {
-      snprintf(key, sizeof(key), "ic_apply|%s|n%d|c%d|l%d|b%d|y%d|f", prec, nsub, max_cells, max_lines, nblk, kind);
-      const int ncand = kind == 1 ? nnat + nblk : 1 + nblk;
+      snprintf(key, sizeof(key), "ic_apply|%s|n%d|c%d|l%d|b%d|w%d|y%d|f", prec, nsub, max_cells, max_lines, nblk, nwrp,
+               kind);
       T* o_t = kind ? nullptr : yo;
       double* o_d = kind ? p0 : nullptr;
       double* o_p = kind ? part : nullptr;
+      const int nn = kind == 1 ? nnat : 1;
+      // where only the natural and the warp kernel apply, the first visit takes the other visits' choice
+      const bool follow = kind == 0 && nblk == 0;
+      const int ncand = follow ? 1 : nn + nblk + nwrp;
+      auto variant = [&](int i) { return i < nn ? 0 : (i < nn + nblk ? (i - nn < 2 ? 1 : 2) : 3); };
       const int ci = tune_choose(key, ncand, [&](int i) {
-        const int nn = kind == 1 ? nnat : 1;
-        if (i < nn)
-          launch_ic_apply<T>(g, d_subs, nsub, max_lines, max_cells, ttx, tty, ttz, tdg, tinv, z, kind ? ya : nullptr,
-                             o_t, o_d, o_p, nullptr, st, kind ? cand[i] : ic_threads);
-        else if (i - nn < 2)
-          launch_ic_apply_blk<T>(g, d_subs, nsub, max_cells, d_coff, ic_coef, ttx, tty, ttz, tdg, z,
-                                 kind ? ya : nullptr, o_t, o_d, o_p, nullptr, d_kerr, st, blk_threads[i - nn]);
+        const T* yi = kind ? ya : nullptr;
+        const int v = variant(i);
+        if (v == 0)
+          launch_ic_apply<T>(g, d_subs, nsub, max_lines, max_cells, ttx, tty, ttz, tdg, tinv, z, yi, o_t, o_d, o_p,
+                             nullptr, st, kind ? cand[i] : ic_threads);
+        else if (v == 1)
+          launch_ic_apply_blk<T>(g, d_subs, nsub, max_cells, d_coff, ic_coef, ttx, tty, ttz, tdg, z, yi, o_t, o_d, o_p,
+                                 nullptr, d_kerr, st, blk_threads[i - nn]);
+        else if (v == 2)
+          launch_ic_apply_stg<T>(g, d_subs, nsub, max_cells, d_coff, ic_coef, ttx, tty, ttz, tdg, z, yi, o_t, o_d, o_p,
+                                 nullptr, d_kerr, st);
         else
-          launch_ic_apply_stg<T>(g, d_subs, nsub, max_cells, d_coff, ic_coef, ttx, tty, ttz, tdg, z,
-                                 kind ? ya : nullptr, o_t, o_d, o_p, nullptr, d_kerr, st);
+          launch_ic_warp<T>(g, d_subs, nsub, ic_wrp_smem, ic_wrp_face, d_woff, ic_wcoef, ttx, tty, ttz, tdg, z, zt, yi,
+                            (T*)rt, o_t, o_d, o_p, nullptr, st);
         return true;
       }, st);
-      const int nn = kind == 1 ? nnat : 1;
-      ic_variant[kind] = ci < nn ? 0 : (ci - nn < 2 ? 1 : 2);
-      if (ci >= nn && ci - nn < 2) ic_blk_threads[kind] = blk_threads[ci - nn];
+      ic_variant[kind] = follow ? ic_variant[1] : variant(ci);
+      if (ic_variant[kind] == 1) ic_blk_threads[kind] = blk_threads[ci - nn];
       if (kind == 1) ic_threads = cand[std::min(ci, nnat - 1)];
-      if (opt.lv1_kernel == 1) ic_variant[kind] = 0;
-      if (opt.lv1_kernel == 2) ic_variant[kind] = 1;  // eligibility checked by setup()
-      if (opt.lv1_kernel == 3) ic_variant[kind] = 2;
+      if (opt.lv1_kernel > 0) ic_variant[kind] = opt.lv1_kernel - 1;  // eligibility checked by setup()
     }
   }
   const int rcand[3] = {256, 128, 512};
   snprintf(key, sizeof(key), "resid_restrict|%s|n%d|c%d|k%d", prec, nsub, max_cells, kmax);
   rr_threads = rcand[tune_choose(key, 3, [&](int i) {
-    launch_resid_restrict<T>(g, d_subs, nsub, kmax, ttx, tty, ttz, tdg, tphi, z, ya, c, nullptr, st, rcand[i]);
+    launch_resid_restrict<T>(g, d_subs, nsub, kmax, ttx, tty, ttz, tdg, tphi, zt, ya, c, nullptr, st, rcand[i]);
     return true;
   }, st)];
   snprintf(key, sizeof(key), "prolong|%s|n%d|c%d|k%d", prec, nsub, max_cells, kmax);
@@ -1608,27 +1663,8 @@ void Solver::tune_pc() {
     launch_prolong<T>(g, d_subs, nsub, kmax, tphi, Zacc, yo, nullptr, st, rcand[i]);
     return true;
   }, st)];
-  // the CG step's fused p-update + operator kernel: 2.5-D march or grid-stride
-  // (the main kernel alone is timed, in the state of a later iteration, whose
-  // p = z + (beta/betaold) p reads the previous p; not done)
-  {
-    PcgState hs;
-    memset(&hs, 0, sizeof(hs));
-    hs.first = 0;
-    hs.beta = hs.betaold = 1.0;
-    hs.dpi = 1.0;
-    cudaMemsetAsync(p0, 0, sizeof(double) * g.ncell, st);
-    cudaMemcpyAsync(state, &hs, sizeof(hs), cudaMemcpyHostToDevice, st);
-    cudaStreamSynchronize(st);
-    snprintf(key, sizeof(key), "pcg_iter_a|M%d|N%d|P%d|p3", g.M, g.N, g.P);
-    pcga_variant = tune_choose(key, 3, [&](int i) {
-      launch_pcg_iter_a_main(g, tx, ty, tz, diag, z, p0, p1, w, part, state, st, i);
-      return true;
-    }, st);
-  }
-  if (pcg_exec && (old[0] != ic_threads || old[1] != rr_threads || old[2] != pr_threads || old[3] != pcga_variant ||
-                   old[4] != ic_variant[0] || old[5] != ic_variant[1] || old[6] != ic_blk_threads[0] ||
-                   old[7] != ic_blk_threads[1])) {
+  if (pcg_exec && (old[0] != ic_threads || old[1] != rr_threads || old[2] != pr_threads || old[3] != ic_variant[0] ||
+                   old[4] != ic_variant[1] || old[5] != ic_blk_threads[0] || old[6] != ic_blk_threads[1])) {
     cudaGraphExecDestroy(pcg_exec);  // captured with other launch shapes
     pcg_exec = nullptr;
     pcg_graph_x = nullptr;
@@ -1636,7 +1672,7 @@ void Solver::tune_pc() {
 }
 
 template <typename T>
-void Solver::apply_impl(const double* x, double* out, double* partial, const int* done) {
+void Solver::apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done) {
   const bool f32 = sizeof(T) == 4;
   const T* ttx = f32 ? (const T*)tx32 : (const T*)tx;
   const T* tty = f32 ? (const T*)ty32 : (const T*)ty;
@@ -1670,9 +1706,9 @@ void Solver::apply_impl(const double* x, double* out, double* partial, const int
           cur = 1 - cur;
         }
       } else if (last)
-        launch_lv1<T>(x, yin, nullptr, out, partial, done);
+        launch_lv1<T>(x, xt, yin, nullptr, out, partial, done);
       else {
-        launch_lv1<T>(x, yin, yb[1 - cur], nullptr, nullptr, done);
+        launch_lv1<T>(x, xt, yin, yb[1 - cur], nullptr, nullptr, done);
         cur = 1 - cur;
       }
       prof_mark(lv1_slot);
@@ -1685,7 +1721,7 @@ void Solver::apply_impl(const double* x, double* out, double* partial, const int
           prof_mark(PROF_PROLONG);
           z_pend = false;
         }
-        launch_resid_restrict<T>(g, d_subs, nsub, kmax, ttx, tty, ttz, tdg, tphi, x, y_zero ? nullptr : yb[cur], c,
+        launch_resid_restrict<T>(g, d_subs, nsub, kmax, ttx, tty, ttz, tdg, tphi, xt, y_zero ? nullptr : yb[cur], c,
                                  done, st, rr_threads);
         prof_mark(PROF_RESTRICT);
         c_valid = true;
@@ -1748,9 +1784,10 @@ int Solver::solve_batch(const double* b_in, double* x_out, bool on_device, int* 
   }
   // entries outside every problem stay zero in every CG vector
   for (double* v : {z, p0, p1, w, r, xs}) cudaMemsetAsync(v, 0, n * 8, st);
+  if (r32) cudaMemsetAsync(r32, 0, n * 4, st);
   const int nblk = bpcg_blocks();
   cudaEventRecord(ev0, st);
-  launch_bpcg_start(d_probs, nprob, bs, xs, r, part, bstate, opt.rtol, opt.atol, opt.max_it, d_all_done, nblk, st);
+  launch_bpcg_start(d_probs, nprob, bs, xs, r, r32, part, bstate, opt.rtol, opt.atol, opt.max_it, d_all_done, nblk, st);
   apply(r, z, part, d_all_done);
   launch_bpcg_beta(d_probs, nprob, part, bstate, st);
   double* pin = p0;
@@ -1758,8 +1795,8 @@ int Solver::solve_batch(const double* b_in, double* x_out, bool on_device, int* 
   const int chunk = std::max(2, opt.pcg_chunk & ~1);  // even: the p buffers return to their roles
   auto enqueue_chunk = [&]() {
     for (int c_ = 0; c_ < chunk; ++c_) {
-      launch_bpcg_iter_a(g, d_probs, d_layer_prob, nprob, tx, ty, tz, diag, z, pin, pout, w, part, bstate, nblk, st);
-      launch_bpcg_iter_b(d_probs, nprob, xs, r, pout, w, part, bstate, d_all_done, nblk, st);
+      launch_bpcg_iter_a(g, d_probs, d_layer_prob, nprob, tx, ty, tz, diag, z, pin, pout, w, part, bstate, st);
+      launch_bpcg_iter_b(g, d_probs, d_layer_prob, nprob, xs, r, r32, pout, w, part, bstate, d_all_done, st);
       apply(r, z, part, d_all_done);
       launch_bpcg_beta(d_probs, nprob, part, bstate, st);
       std::swap(pin, pout);
@@ -1852,9 +1889,9 @@ int Solver::profile_iteration(int reps, double ms[PROF_SLOTS], int launches[PROF
     prof_n = 0;
     prof_on = true;
     prof_mark(-1);
-    launch_pcg_iter_a(g, tx, ty, tz, diag, z, p0, p1, w, part, state, st, pcga_variant);
+    launch_pcg_iter_a(g, tx, ty, tz, diag, z, p0, p1, w, part, state, st);
     prof_mark(PROF_CG_A);
-    launch_pcg_iter_b(g.ncell, vx, vb, p1, w, part, state, st);
+    launch_pcg_iter_b(g.ncell, vx, vb, r32, p1, w, part, state, st);
     prof_mark(PROF_CG_B);
     apply(vb, z, part, nullptr);
     if (opt.null_space)
@@ -1879,11 +1916,12 @@ int Solver::profile_iteration(int reps, double ms[PROF_SLOTS], int launches[PROF
   return 0;
 }
 
+// In the mixed form r32 holds x in FP32 (written by the CG kernels with the residual).
 void Solver::apply(const double* x, double* out, double* partial, const int* done) {
   if (opt.precision == 1)
-    apply_impl<float>(x, out, partial, done);
+    apply_impl<float>(x, r32, out, partial, done);
   else
-    apply_impl<double>(x, out, partial, done);
+    apply_impl<double>(x, x, out, partial, done);
 }
 
 int Solver::rhs(const double* source, double* out, bool on_device) {
@@ -1930,6 +1968,7 @@ int Solver::pc_apply(const double* x_in, double* y_out, bool on_device) {
     ys = z;
   }
   cudaEventRecord(ev0, st);
+  if (opt.precision == 1) launch_to_f32(xs, r32, g.ncell, st);
   apply(xs, ys, part, nullptr);
   cudaEventRecord(ev1, st);
   if (!on_device) cudaMemcpyAsync(y_out, ys, n * 8, cudaMemcpyDeviceToHost, st);
@@ -1960,7 +1999,8 @@ int Solver::solve(const double* b_in, double* x_out, bool on_device, int* its, d
     xs = vx;
   }
   cudaEventRecord(ev0, st);
-  launch_pcg_start(g, bs, xs, r, part, state, opt.rtol, opt.atol, opt.max_it, st);
+  launch_pcg_start(g, bs, xs, r, r32, part, state, opt.rtol, opt.atol, opt.max_it, st);
+  cudaMemsetAsync(p0, 0, n * 8, st);  // the first step takes p = z + 0 p
   const int* done = &state->done;
   // beta = z.r from the preconditioner's partials, or of the projected z when
   // the operator carries the constant null space
@@ -1978,8 +2018,8 @@ int Solver::solve(const double* b_in, double* x_out, bool on_device, int* its, d
   const int chunk = std::max(1, opt.pcg_chunk);
   auto enqueue_chunk = [&]() {
     for (int c_ = 0; c_ < chunk; ++c_) {
-      launch_pcg_iter_a(g, tx, ty, tz, diag, z, pin, pout, w, part, state, st, pcga_variant);
-      launch_pcg_iter_b(g.ncell, xs, r, pout, w, part, state, st);
+      launch_pcg_iter_a(g, tx, ty, tz, diag, z, pin, pout, w, part, state, st);
+      launch_pcg_iter_b(g.ncell, xs, r, r32, pout, w, part, state, st);
       apply(r, z, part, done);
       beta();
       std::swap(pin, pout);

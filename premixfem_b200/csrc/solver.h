@@ -180,7 +180,7 @@ class Solver {
   int alloc_fine();
   void assemble_launch();
   template <typename T>
-  void apply_impl(const double* x, double* out, double* partial, const int* done);
+  void apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done);
   void apply(const double* x, double* out, double* partial, const int* done);
   std::vector<int> schedule() const;
   int dir_on_[6] = {0, 0, 0, 0, 0, 0};
@@ -203,21 +203,29 @@ class Solver {
   int setup_band_cholesky(bool mixed);
   template <typename T>
   void tune_pc();
-  int ic_threads = 0, rr_threads = 256, pr_threads = 256, pcga_variant = 0;  // tuned launch shapes
+  int ic_threads = 0, rr_threads = 256, pr_threads = 256;  // tuned launch shapes
   // level-1 solve with the subdomain-blocked IC(0) factor (k_ic_apply_blk)
   bool ic_blk_ok = false;  // every subdomain fits the blocked kernel
   bool ic_stg_ok = false;  // ... and its staged form (k_ic_apply_stg: ny, nz <= 16)
   // per visit kind (0: first visit, no iterate; 1: visits with an iterate):
-  // 0 natural-order kernel, 1 blocked kernel, 2 its staged form (tuner's
-  // choice), and the blocked kernel's threads
+  // 0 natural-order kernel, 1 blocked kernel, 2 its staged form, 3 one warp per
+  // subdomain (tuner's choice), and the blocked kernel's threads
   int ic_variant[2] = {0, 0}, ic_blk_threads[2] = {512, 512};
   long long* d_coff = nullptr;  // per subdomain: first cell in the blocked arrays
   void* ic_coef = nullptr;      // blocked {tx, ty, tz, 1/D} (precision of the preconditioner)
+  // level-1 solve by one warp per subdomain (k_ic_warp): the factor in step order
+  bool ic_wrp_ok = false;
+  int ic_wrp_smem = 0, ic_wrp_face = 0;
+  long long* d_woff = nullptr;
+  void* ic_wcoef = nullptr;
+  void* rt = nullptr;     // residual x - A y of the level-1 visits with an iterate (k_lv1_resid)
+  float* r32 = nullptr;   // mixed form: FP32 copy of the vector the preconditioner is applied to
+  int setup_ic_warp(bool mixed);
   int* d_kerr = nullptr;        // set by a kernel whose bounded wait ran out
   int check_kernel_flag(const char* what);
   int setup_ic_blocked(bool mixed);
   template <typename T>
-  void launch_lv1(const double* x, const T* yin, T* out_t, double* out_d, double* partial, const int* done);
+  void launch_lv1(const double* x, const T* xt, const T* yin, T* out_t, double* out_d, double* partial, const int* done);
   int run_eigen(LobpcgArgs& la, const int* list, int nlist, int eig_blocks, double eb1);
   // the local eigensolves run on FP32 vectors (the mixed form's default)
   bool eig32() const { return opt.precision == 1 && opt.eig_precision != 0; }

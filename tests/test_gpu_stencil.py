@@ -1,0 +1,53 @@
+"""The z-march of the 7-point operator (32 x 8 tiles, stretches of 1 to 16
+planes by the number of tiles) at its edges, the fused CG step built on it, and
+the restriction and prolongation for every basis size, against the sparse
+operator of the oracle.
+
+Bars: an operator product is a sum of at most seven products per cell, so 1e-13
+of its norm; a solve at rtol 1e-11 leaves a true residual within 1e-10."""
+import numpy as np
+import pytest
+
+from oracle import pmf_oracle as O
+from premixfem_b200 import fields
+from premixfem_b200.solver import DarcySolver
+
+pytestmark = pytest.mark.gpu
+
+MESHES = [(2, 2, 2), (31, 9, 17), (32, 8, 16), (33, 7, 5), (64, 16, 33), (65, 17, 31), (5, 3, 130), (130, 2, 3),
+          (3, 100, 4), (96, 96, 48)]
+
+
+@pytest.mark.parametrize("mesh", MESHES, ids=lambda m: "x".join(map(str, m)))
+def test_operator_and_cg_step(native, mesh):
+    prob = fields.random_box(mesh, seed=4, sigma=2.0, dirichlet={"x-": 1.0, "z+": 0.5})
+    op = O.Operator(prob)
+    sd = tuple(max(1, (n + 7) // 8) for n in mesh)
+    s = DarcySolver.from_problem(prob, f"-pmf_sd {sd[0]},{sd[1]},{sd[2]} -en_lv1 1 -en_lv2 1 -ksp_rtol 1e-11")
+    s.setup()
+    x = np.random.default_rng(1).standard_normal(op.n)
+    ref = op.A @ x
+    assert np.linalg.norm(s.apply_A(x) - ref) <= 1e-13 * np.linalg.norm(ref)
+    b = s.rhs(prob["source"].ravel())
+    u, _, _, reason = s.solve(b)
+    s.close()
+    assert reason == "converged"
+    assert np.linalg.norm(b - op.A @ u) <= 1e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("k", range(1, 9))
+def test_basis_sizes(native, k, precision):
+    """The W-cycle visits the restriction with an iterate, the V-cycle without; one basis vector more
+    never leaves the solve unconverged."""
+    prob = fields.random_box((17, 15, 19), seed=5, sigma=1.5)
+    op = O.Operator(prob)
+    for extra in ("", " -use_W_cycle"):
+        s = DarcySolver.from_problem(prob, f"-pmf_sd 2,2,3 -en_lv1 {k} -en_lv2 2 -pmf_precision {precision} "
+                                           f"-ksp_rtol 1e-11{extra}")
+        s.setup()
+        b = s.rhs(prob["source"].ravel())
+        u, _, _, reason = s.solve(b)
+        s.close()
+        assert reason == "converged"
+        assert np.linalg.norm(b - op.A @ u) <= 1e-10 * np.linalg.norm(b)
