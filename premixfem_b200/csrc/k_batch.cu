@@ -47,13 +47,15 @@ __global__ void k_bpcg_start(const ProbInfo* probs, const double* b, double* x, 
   v = block_sum(v, red);
   if (threadIdx.x == 0) part[(long long)q * nblk + blockIdx.x] = v;
 }
-__global__ void k_bpcg_start_fin(const double* part, int nblk, PcgState* st, double rtol, double atol, int max_it) {
+__global__ void k_bpcg_start_fin(const double* part, int nblk, PcgState* st, double* x, double rtol, double atol,
+                                 int max_it) {
   __shared__ double red[32];
   const int q = blockIdx.x;
   const double v = bfixed_sum(part + (long long)q * nblk, nblk, red);
   if (threadIdx.x == 0) {
     PcgState& s = st[q];
     const double dp = sqrt(v);
+    s.x = x;
     s.dp = dp;
     s.rnorm0 = dp;
     s.ttol = fmax(rtol * dp, atol);  // KSPConvergedDefault
@@ -151,8 +153,8 @@ __global__ void __launch_bounds__(1024) k_bpcg_iter_a_fin(const ProbInfo* probs,
 }
 
 // x += alpha p, r -= alpha w, partial r.r over the problem's own cells: gridDim.x CTAs per layer
-__global__ void __launch_bounds__(kBT) k_bpcg_iter_b(Grid g, const ProbInfo* probs, const int* layer_prob, double* x,
-                                                     double* r, float* r32, const double* p, const double* w,
+__global__ void __launch_bounds__(kBT) k_bpcg_iter_b(Grid g, const ProbInfo* probs, const int* layer_prob, double* r,
+                                                     float* r32, const double* p, const double* w,
                                                      double* part, const PcgState* st) {
   __shared__ double red[32];
   for (int ez = blockIdx.y; ez < g.P; ez += gridDim.y) {
@@ -161,6 +163,7 @@ __global__ void __launch_bounds__(kBT) k_bpcg_iter_b(Grid g, const ProbInfo* pro
     const PcgState& s = st[q];
     if (s.done) continue;
     const double a = s.alpha;
+    double* x = s.x;
     const int M = probs[q].M, n = M * probs[q].N;
     const long long c0 = (long long)ez * g.MN;
     double v = 0.0;
@@ -181,7 +184,7 @@ __global__ void __launch_bounds__(kBT) k_bpcg_iter_b(Grid g, const ProbInfo* pro
 // the residual norms, iteration counts and stop codes (a warp per problem, its partials in order), then
 // all_done = 1 when every problem has stopped (the shared preconditioner kernels test it)
 __global__ void __launch_bounds__(1024) k_bpcg_iter_b_fin(const ProbInfo* probs, int nprob, const double* part,
-                                                          int per_layer, PcgState* st, int* all_done) {
+                                                          int per_layer, PcgState* st, int* all_done, LoopCond loop) {
   __shared__ int any;
   if (threadIdx.x == 0) any = 0;
   __syncthreads();
@@ -212,7 +215,10 @@ __global__ void __launch_bounds__(1024) k_bpcg_iter_b_fin(const ProbInfo* probs,
     if (lane == 0 && !d) any = 1;
   }
   __syncthreads();
-  if (threadIdx.x == 0) *all_done = any ? 0 : 1;
+  if (threadIdx.x == 0) {
+    *all_done = any ? 0 : 1;
+    loop_while(loop, any);
+  }
 }
 __global__ void k_bpcg_all_done(const PcgState* st, int nprob, int* all_done) {
   __shared__ int any;
@@ -227,7 +233,7 @@ __global__ void k_bpcg_all_done(const PcgState* st, int nprob, int* all_done) {
 void launch_bpcg_start(const ProbInfo* probs, int nprob, const double* b, double* x, double* r, float* r32,
                        double* part, PcgState* st, double rtol, double atol, int max_it, int* all_done, int nblk, cudaStream_t s) {
   { note_launch(); k_bpcg_start<<<dim3(nblk, nprob), kBT, 0, s>>>(probs, b, x, r, r32, part, nblk); }
-  { note_launch(); k_bpcg_start_fin<<<nprob, 256, 0, s>>>(part, nblk, st, rtol, atol, max_it); }
+  { note_launch(); k_bpcg_start_fin<<<nprob, 256, 0, s>>>(part, nblk, st, x, rtol, atol, max_it); }
   { note_launch(); k_bpcg_all_done<<<1, 256, 0, s>>>(st, nprob, all_done); }
 }
 void launch_bpcg_beta(const ProbInfo* probs, int nprob, const double* part, PcgState* st, cudaStream_t s) {
@@ -241,12 +247,12 @@ void launch_bpcg_iter_a(const Grid& g, const ProbInfo* probs, const int* layer_p
   { note_launch(); k_bpcg_iter_a<<<grid, dim3(kStX, kStY), 0, s>>>(g, probs, layer_prob, tx, ty, tz, diag, z, pin, pout, w, part, st); }
   { note_launch(); k_bpcg_iter_a_fin<<<nprob, 1024, 0, s>>>(probs, part, (int)grid.x, st); }
 }
-void launch_bpcg_iter_b(const Grid& g, const ProbInfo* probs, const int* layer_prob, int nprob, double* x, double* r,
-                        float* r32, const double* p, const double* w, double* part, PcgState* st, int* all_done,
+void launch_bpcg_iter_b(const Grid& g, const ProbInfo* probs, const int* layer_prob, int nprob, double* r, float* r32,
+                        const double* p, const double* w, double* part, PcgState* st, int* all_done, LoopCond loop,
                         cudaStream_t s) {
   const int sub = std::max(1, std::min(32, (int)(g.MN / 2048)));  // CTAs per layer, fewer than its tiles
-  { note_launch(); k_bpcg_iter_b<<<dim3(sub, std::min(g.P, 65535)), kBT, 0, s>>>(g, probs, layer_prob, x, r, r32, p, w, part, st); }
-  { note_launch(); k_bpcg_iter_b_fin<<<1, 1024, 0, s>>>(probs, nprob, part, sub, st, all_done); }
+  { note_launch(); k_bpcg_iter_b<<<dim3(sub, std::min(g.P, 65535)), kBT, 0, s>>>(g, probs, layer_prob, r, r32, p, w, part, st); }
+  { note_launch(); k_bpcg_iter_b_fin<<<1, 1024, 0, s>>>(probs, nprob, part, sub, st, all_done, loop); }
 }
 
 }  // namespace pmf

@@ -223,11 +223,13 @@ __global__ void k_pcg_start(long long n, const double* b, double* x, double* r, 
   v = block_sum(v, red);
   if (threadIdx.x == 0) part[blockIdx.x] = v;
 }
-__global__ void k_pcg_start_fin(const double* part, int nb, PcgState* s, double rtol, double atol, int max_it) {
+__global__ void k_pcg_start_fin(const double* part, int nb, PcgState* s, double* x, double rtol, double atol,
+                                int max_it) {
   __shared__ double red[32];
   const double v = fixed_sum(part, nb, red);
   if (threadIdx.x == 0) {
     const double dp = sqrt(v);
+    s->x = x;
     s->dp = dp;
     s->rnorm0 = dp;
     s->ttol = fmax(rtol * dp, atol);  // KSPConvergedDefault: max(rtol*rnorm0, abstol)
@@ -243,15 +245,19 @@ void launch_pcg_start(const Grid& g, const double* b, double* x, double* r, floa
                       double rtol, double atol, int max_it, cudaStream_t st) {
   int nb = cell_blocks(g.ncell);
   { note_launch(); k_pcg_start<<<nb, kCellThreads, 0, st>>>(g.ncell, b, x, r, r32, part); }
-  { note_launch(); k_pcg_start_fin<<<1, 256, 0, st>>>(part, nb, s, rtol, atol, max_it); }
+  { note_launch(); k_pcg_start_fin<<<1, 256, 0, st>>>(part, nb, s, x, rtol, atol, max_it); }
 }
 
-// beta = z.r (the dot is written per block by the preconditioner's last kernel
-// or by k_dot); a zero beta ends the loop with done = 5 (KSP_CONVERGED_ATOL,
-// as KSPSolve_CG reports it).
-__global__ void k_pcg_beta_fin(const double* part, int nb, PcgState* s) {
+// beta = z.r (the dot is written per block by the preconditioner's last kernel);
+// a zero beta ends the loop with done = 5 (KSP_CONVERGED_ATOL, as KSPSolve_CG
+// reports it).  The last kernel of an iteration: it also tells the graph that
+// repeats the iterations whether to go on.
+__global__ void k_pcg_beta_fin(const double* part, int nb, PcgState* s, LoopCond loop) {
   __shared__ double red[32];
-  if (s->done) return;
+  if (s->done) {
+    if (threadIdx.x == 0) loop_while(loop, false);
+    return;
+  }
   const double v = fixed_sum(part, nb, red);
   if (threadIdx.x == 0) {
     s->beta = v;
@@ -259,15 +265,11 @@ __global__ void k_pcg_beta_fin(const double* part, int nb, PcgState* s) {
       s->its += 1;
       s->done = 5;
     }
+    loop_while(loop, v != 0.0);
   }
 }
-void launch_pcg_beta_fin(const double* part, int nparts, PcgState* s, cudaStream_t st) {
-  { note_launch(); k_pcg_beta_fin<<<1, 256, 0, st>>>(part, nparts, s); }
-}
-void launch_pcg_beta(const double* r, const double* z, long long n, double* part, PcgState* s, cudaStream_t st) {
-  int nb = cell_blocks(n);
-  { note_launch(); k_dot<<<nb, kCellThreads, 0, st>>>(r, z, n, part); }
-  { note_launch(); k_pcg_beta_fin<<<1, 256, 0, st>>>(part, nb, s); }
+void launch_pcg_beta_fin(const double* part, int nparts, PcgState* s, LoopCond loop, cudaStream_t st) {
+  { note_launch(); k_pcg_beta_fin<<<1, 256, 0, st>>>(part, nparts, s, loop); }
 }
 
 // Constant null space (-ksp_constant_null_space): PETSc's KSP_PCApply removes
@@ -302,11 +304,11 @@ __global__ void k_null_project(double* z, const double* r, long long n, const do
   if (threadIdx.x == 0) part[blockIdx.x] = v;
 }
 void launch_pcg_null_beta(double* z, const double* r, long long n, double* part, double* zpart, PcgState* s,
-                          cudaStream_t st) {
+                          LoopCond loop, cudaStream_t st) {
   const int nb = cell_blocks(n);
   { note_launch(); k_null_sum<<<nb, kCellThreads, 0, st>>>(z, n, zpart, &s->done); }
   { note_launch(); k_null_project<<<nb, kCellThreads, 0, st>>>(z, r, n, zpart, nb, part, &s->done); }
-  { note_launch(); k_pcg_beta_fin<<<1, 256, 0, st>>>(part, nb, s); }
+  { note_launch(); k_pcg_beta_fin<<<1, 256, 0, st>>>(part, nb, s, loop); }
 }
 
 // p <- z (first) or z + (beta/betaold) p; w <- A p; one partial of p.w per CTA.
@@ -368,12 +370,12 @@ void launch_pcg_iter_a(const Grid& g, const double* tx, const double* ty, const 
 
 // x += alpha p; r -= alpha w; partial r.r; then dp, its and the convergence test.
 // Two cells per load where x is 16-byte aligned (a caller's pointer may not be; the solver's own arrays are).
-__global__ void __launch_bounds__(kCellThreads) k_pcg_iter_b(long long n, double* x, double* r, float* r32,
-                                                             const double* p, const double* w, double* part,
-                                                             const PcgState* s) {
+__global__ void __launch_bounds__(kCellThreads) k_pcg_iter_b(long long n, double* r, float* r32, const double* p,
+                                                             const double* w, double* part, const PcgState* s) {
   __shared__ double red[32];
   if (s->done) return;
   const double a = s->alpha;
+  double* x = s->x;
   double v = 0.0;
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, str = (long long)gridDim.x * blockDim.x;
   long long n2 = 0;  // cells done in pairs
@@ -420,10 +422,10 @@ __global__ void k_pcg_iter_b_fin(const double* part, int nb, PcgState* s) {
       s->done = 2;
   }
 }
-void launch_pcg_iter_b(long long n, double* x, double* r, float* r32, const double* p, const double* w, double* part,
-                       PcgState* s, cudaStream_t st) {
+void launch_pcg_iter_b(long long n, double* r, float* r32, const double* p, const double* w, double* part, PcgState* s,
+                       cudaStream_t st) {
   int nb = cell_blocks(n);
-  { note_launch(); k_pcg_iter_b<<<nb, kCellThreads, 0, st>>>(n, x, r, r32, p, w, part, s); }
+  { note_launch(); k_pcg_iter_b<<<nb, kCellThreads, 0, st>>>(n, r, r32, p, w, part, s); }
   { note_launch(); k_pcg_iter_b_fin<<<1, 256, 0, st>>>(part, nb, s); }
 }
 

@@ -20,7 +20,20 @@ struct PcgState {
   // done: 0 running, 1 converged (residual test), 2 max_it, 3 indefinite, 4 nan/inf,
   // 5 converged because z.r = 0 (KSP_CONVERGED_ATOL)
   int its, max_it, first, done;
+  double* x;  // the solution: read from here so that a captured iteration serves every solution buffer
 };
+
+// The condition of the graph node that repeats a captured chunk of CG iterations
+// on the device (use = 0 outside such a graph).
+struct LoopCond {
+  unsigned long long handle = 0;
+  int use = 0;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void loop_while(const LoopCond& c, bool go) {
+  if (c.use) cudaGraphSetConditional(c.handle, go ? 1u : 0u);
+}
+#endif
 
 constexpr int kCellThreads = 256;
 int cell_blocks(long long n);  // grid size for grid-stride cell loops (fixed per n)
@@ -54,17 +67,15 @@ void launch_spmv(const Grid& g, const double* tx, const double* ty, const double
 void launch_pcg_start(const Grid& g, const double* b, double* x, double* r, float* r32, double* part, PcgState* s,
                       double rtol, double atol, int max_it, cudaStream_t st);
 // beta = z.r from nparts per-block partials (written by the preconditioner's last kernel).
-void launch_pcg_beta_fin(const double* part, int nparts, PcgState* s, cudaStream_t st);
-// same, computing the partials itself
-void launch_pcg_beta(const double* r, const double* z, long long n, double* part, PcgState* s, cudaStream_t st);
+void launch_pcg_beta_fin(const double* part, int nparts, PcgState* s, LoopCond loop, cudaStream_t st);
 // constant null space: z <- z - mean(z), then beta = z.r (zpart: cell_blocks(n) scratch partials)
 void launch_pcg_null_beta(double* z, const double* r, long long n, double* part, double* zpart, PcgState* s,
-                          cudaStream_t st);
+                          LoopCond loop, cudaStream_t st);
 void launch_pcg_iter_a(const Grid& g, const double* tx, const double* ty, const double* tz, const double* diag,
                        const double* z, const double* pin, double* pout, double* w, double* part, PcgState* s,
                        cudaStream_t st);
-void launch_pcg_iter_b(long long n, double* x, double* r, float* r32, const double* p, const double* w, double* part,
-                       PcgState* s, cudaStream_t st);
+void launch_pcg_iter_b(long long n, double* r, float* r32, const double* p, const double* w, double* part, PcgState* s,
+                       cudaStream_t st);
 void launch_dot(const double* a, const double* b, long long n, double* part, double* out, cudaStream_t st);
 
 // ---- CG over a batch of problems (k_batch.cu): per-problem scalars, 2-D grids
@@ -76,8 +87,8 @@ void launch_bpcg_beta(const ProbInfo* probs, int nprob, const double* part, PcgS
 void launch_bpcg_iter_a(const Grid& g, const ProbInfo* probs, const int* layer_prob, int nprob, const double* tx,
                         const double* ty, const double* tz, const double* diag, const double* z, const double* pin,
                         double* pout, double* w, double* part, PcgState* st, cudaStream_t s);
-void launch_bpcg_iter_b(const Grid& g, const ProbInfo* probs, const int* layer_prob, int nprob, double* x, double* r,
-                        float* r32, const double* p, const double* w, double* part, PcgState* st, int* all_done,
+void launch_bpcg_iter_b(const Grid& g, const ProbInfo* probs, const int* layer_prob, int nprob, double* r, float* r32,
+                        const double* p, const double* w, double* part, PcgState* st, int* all_done, LoopCond loop,
                         cudaStream_t s);
 
 // ---- level 1 (IC(0) block solves) -------------------------------------------

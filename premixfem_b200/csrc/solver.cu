@@ -427,8 +427,7 @@ Solver::~Solver() {
                   state};
   for (void* p : ptrs)
     if (p) cudaFree(p);
-  if (pcg_exec) cudaGraphExecDestroy(pcg_exec);
-  if (bpcg_exec) cudaGraphExecDestroy(bpcg_exec);
+  drop_graphs();
   for (void* p : {(void*)bstate, (void*)d_all_done})
     if (p) cudaFree(p);
   if (h_bstate) cudaFreeHost(h_bstate);
@@ -709,7 +708,15 @@ int Solver::rank_layout() {
 
 // cudaMalloc with its return code checked: on failure *p is null, err names
 // the array and the PETSc-style code 76 comes back.
+// The CG graphs hold addresses and launch shapes of what they were captured with.
+void Solver::drop_graphs() {
+  if (pcg_exec) cudaGraphExecDestroy(pcg_exec);
+  if (bpcg_exec) cudaGraphExecDestroy(bpcg_exec);
+  pcg_exec = bpcg_exec = nullptr;
+}
+
 int Solver::dalloc(void** p, size_t bytes, const char* what) {
+  drop_graphs();  // the new buffer may replace one that they hold
   *p = nullptr;
   const cudaError_t e = cudaMalloc(p, bytes);
   if (e == cudaSuccess) return 0;
@@ -866,7 +873,6 @@ int Solver::assemble() {
 int Solver::alloc_eb(int m, bool mixed) {
   const size_t stride = lobpcg_batched_slab_bytes(max_cells, m, mixed ? 4 : 8);
   if (eb.slab && eb.slab_stride == stride) return 0;
-  if (pcg_exec) cudaGraphExecDestroy(pcg_exec);
   for (void* p : {(void*)eb.slab, eb.state, (void*)eb.Ybuf, (void*)eb.gpart, (void*)eb.rpart})
     if (p) cudaFree(p);
   eb.slab_stride = stride;
@@ -1443,6 +1449,7 @@ int Solver::setup_band_cholesky(bool mixed) {
       err = "not enough device memory for the level-1 Cholesky factors";
       return 55;  // PETSC_ERR_MEM
     }
+    drop_graphs();
     if (int er = check(cudaMalloc(&band64, sizeof(double) * len), "cudaMalloc Cholesky factors")) return er;
     band_len = len;
   }
@@ -1663,12 +1670,9 @@ void Solver::tune_pc() {
     launch_prolong<T>(g, d_subs, nsub, kmax, tphi, Zacc, yo, nullptr, st, rcand[i]);
     return true;
   }, st)];
-  if (pcg_exec && (old[0] != ic_threads || old[1] != rr_threads || old[2] != pr_threads || old[3] != ic_variant[0] ||
-                   old[4] != ic_variant[1] || old[5] != ic_blk_threads[0] || old[6] != ic_blk_threads[1])) {
-    cudaGraphExecDestroy(pcg_exec);  // captured with other launch shapes
-    pcg_exec = nullptr;
-    pcg_graph_x = nullptr;
-  }
+  if (old[0] != ic_threads || old[1] != rr_threads || old[2] != pr_threads || old[3] != ic_variant[0] ||
+      old[4] != ic_variant[1] || old[5] != ic_blk_threads[0] || old[6] != ic_blk_threads[1])
+    drop_graphs();  // captured with other launch shapes
 }
 
 template <typename T>
@@ -1793,44 +1797,28 @@ int Solver::solve_batch(const double* b_in, double* x_out, bool on_device, int* 
   double* pin = p0;
   double* pout = p1;
   const int chunk = std::max(2, opt.pcg_chunk & ~1);  // even: the p buffers return to their roles
-  auto enqueue_chunk = [&]() {
+  auto enqueue_chunk = [&](LoopCond loop) {
     for (int c_ = 0; c_ < chunk; ++c_) {
       launch_bpcg_iter_a(g, d_probs, d_layer_prob, nprob, tx, ty, tz, diag, z, pin, pout, w, part, bstate, st);
-      launch_bpcg_iter_b(g, d_probs, d_layer_prob, nprob, xs, r, r32, pout, w, part, bstate, d_all_done, st);
+      launch_bpcg_iter_b(g, d_probs, d_layer_prob, nprob, r, r32, pout, w, part, bstate, d_all_done, loop, st);
       apply(r, z, part, d_all_done);
       launch_bpcg_beta(d_probs, nprob, part, bstate, st);
       std::swap(pin, pout);
     }
   };
-  const bool use_graph = opt.pcg_graph != 0;
-  if (use_graph && (!bpcg_exec || bpcg_graph_x != xs)) {
-    if (bpcg_exec) cudaGraphExecDestroy(bpcg_exec);
-    bpcg_exec = nullptr;
-    const unsigned long long l0 = __atomic_load_n(&g_launches, __ATOMIC_RELAXED);
-    cudaGraph_t graph = nullptr;
-    if (int e = check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "graph capture")) return e;
-    enqueue_chunk();
-    if (int e = check(cudaStreamEndCapture(st, &graph), "graph capture")) return e;
-    bpcg_graph_kernels = __atomic_load_n(&g_launches, __ATOMIC_RELAXED) - l0;
-    __atomic_fetch_sub(&g_launches, bpcg_graph_kernels, __ATOMIC_RELAXED);  // captured, not launched
-    const cudaError_t ie = cudaGraphInstantiate(&bpcg_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (int e = check(ie, "graph instantiate")) return e;
-    bpcg_graph_x = xs;
-  }
-  int guard = 0;
-  for (;;) {
-    if (use_graph) {
-      if (int e = check(cudaGraphLaunch(bpcg_exec, st), "graph launch")) return e;
-      __atomic_fetch_add(&g_launches, bpcg_graph_kernels, __ATOMIC_RELAXED);
-    } else {
-      enqueue_chunk();
+  if (opt.pcg_graph) {
+    if (!bpcg_exec)
+      if (int e = loop_graph(&bpcg_exec, &bpcg_graph_kernels, enqueue_chunk)) return e;
+    if (int e = check(cudaGraphLaunch(bpcg_exec, st), "graph launch")) return e;
+  } else {
+    for (int guard = 0;;) {
+      enqueue_chunk(LoopCond());
+      cudaMemcpyAsync(h_all_done, d_all_done, sizeof(int), cudaMemcpyDeviceToHost, st);
+      if (int e = check(cudaStreamSynchronize(st), "batch KSPSolve")) return e;
+      if (int e = check(cudaGetLastError(), "batch KSPSolve launch")) return e;
+      if (*h_all_done) break;
+      if (++guard * chunk > opt.max_it + 8) break;
     }
-    cudaMemcpyAsync(h_all_done, d_all_done, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (int e = check(cudaStreamSynchronize(st), "batch KSPSolve")) return e;
-    if (int e = check(cudaGetLastError(), "batch KSPSolve launch")) return e;
-    if (*h_all_done) break;
-    if (++guard * chunk > opt.max_it + 8) break;
   }
   cudaEventRecord(ev1, st);
   cudaMemcpyAsync(h_bstate, bstate, sizeof(PcgState) * nprob, cudaMemcpyDeviceToHost, st);
@@ -1848,7 +1836,54 @@ int Solver::solve_batch(const double* b_in, double* x_out, bool on_device, int* 
     if (reason) reason[q] = s.done ? s.done : 2;
     last_its = std::max(last_its, s.its);
   }
+  if (opt.pcg_graph) count_loop(bpcg_graph_kernels, last_its, chunk);
   return e;
+}
+
+// A CUDA graph that repeats `chunk` on the device while the condition its last
+// kernels set holds: the host is not asked between chunks, and because the
+// kernels read the solution's address from the CG state one graph serves every
+// solution buffer.  (45 x 37 x 29 cells, each solve into another buffer: 2.96 ms
+// instead of 3.57 with a capture per buffer and a synchronisation per chunk.)
+// The loop ends: the state's stop code is set at max_it at the latest, and a
+// stopped state ends it.
+int Solver::loop_graph(cudaGraphExec_t* exec, unsigned long long* kernels, const std::function<void(LoopCond)>& chunk) {
+  const unsigned long long l0 = __atomic_load_n(&g_launches, __ATOMIC_RELAXED);
+  cudaGraph_t graph = nullptr;
+  if (int e = check(cudaGraphCreate(&graph, 0), "graph")) return e;
+  cudaGraphConditionalHandle handle;
+  cudaError_t ce = cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault);
+  cudaGraph_t body = nullptr;
+  if (ce == cudaSuccess) {
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = handle;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    cudaGraphNode_t node;
+    ce = cudaGraphAddNode(&node, graph, nullptr, 0, &np);
+    if (ce == cudaSuccess) body = np.conditional.phGraph_out[0];
+  }
+  if (ce == cudaSuccess)
+    ce = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+  if (ce == cudaSuccess) {
+    LoopCond loop;
+    loop.handle = handle;
+    loop.use = 1;
+    chunk(loop);
+    ce = cudaStreamEndCapture(st, &body);
+  }
+  *kernels = __atomic_load_n(&g_launches, __ATOMIC_RELAXED) - l0;
+  __atomic_fetch_sub(&g_launches, *kernels, __ATOMIC_RELAXED);  // captured, not launched
+  if (ce == cudaSuccess) ce = cudaGraphInstantiate(exec, graph, 0);
+  cudaGraphDestroy(graph);
+  return check(ce, "CG graph");
+}
+
+// the kernels that a graph of loop_graph launched
+void Solver::count_loop(unsigned long long kernels, int its, int chunk) {
+  __atomic_fetch_add(&g_launches, kernels * (unsigned long long)std::max(1, (its + chunk - 1) / chunk),
+                     __ATOMIC_RELAXED);
 }
 
 void Solver::prof_mark(int slot) {
@@ -1880,6 +1915,7 @@ int Solver::profile_iteration(int reps, double ms[PROF_SLOTS], int launches[PROF
   hs.beta = hs.betaold = 1.0;
   hs.dpi = 1.0;  // a positive previous p.Ap: the indefinite test compares signs
   hs.max_it = 1 << 30;
+  hs.x = vx;
   cudaMemcpyAsync(vb, r, sizeof(double) * g.ncell, cudaMemcpyDeviceToDevice, st);
   cudaMemsetAsync(vx, 0, sizeof(double) * g.ncell, st);
   cudaMemsetAsync(p0, 0, sizeof(double) * g.ncell, st);
@@ -1891,13 +1927,13 @@ int Solver::profile_iteration(int reps, double ms[PROF_SLOTS], int launches[PROF
     prof_mark(-1);
     launch_pcg_iter_a(g, tx, ty, tz, diag, z, p0, p1, w, part, state, st);
     prof_mark(PROF_CG_A);
-    launch_pcg_iter_b(g.ncell, vx, vb, r32, p1, w, part, state, st);
+    launch_pcg_iter_b(g.ncell, vb, r32, p1, w, part, state, st);
     prof_mark(PROF_CG_B);
     apply(vb, z, part, nullptr);
     if (opt.null_space)
-      launch_pcg_null_beta(z, vb, g.ncell, part, zpart, state, st);
+      launch_pcg_null_beta(z, vb, g.ncell, part, zpart, state, LoopCond(), st);
     else
-      launch_pcg_beta_fin(part, nparts_apply(), state, st);
+      launch_pcg_beta_fin(part, nparts_apply(), state, LoopCond(), st);
     prof_mark(PROF_BETA);
     prof_on = false;
     if (int er = check(cudaStreamSynchronize(st), "profile iteration")) return er;
@@ -2004,66 +2040,56 @@ int Solver::solve(const double* b_in, double* x_out, bool on_device, int* its, d
   const int* done = &state->done;
   // beta = z.r from the preconditioner's partials, or of the projected z when
   // the operator carries the constant null space
-  auto beta = [&]() {
+  auto beta = [&](LoopCond loop) {
     if (opt.null_space)
-      launch_pcg_null_beta(z, r, g.ncell, part, zpart, state, st);
+      launch_pcg_null_beta(z, r, g.ncell, part, zpart, state, loop, st);
     else
-      launch_pcg_beta_fin(part, nparts_apply(), state, st);
+      launch_pcg_beta_fin(part, nparts_apply(), state, loop, st);
   };
   apply(r, z, part, done);
-  beta();
+  beta(LoopCond());
   double* pin = p0;
   double* pout = p1;
-  int guard = 0;
   const int chunk = std::max(1, opt.pcg_chunk);
-  auto enqueue_chunk = [&]() {
+  auto enqueue_chunk = [&](LoopCond loop) {
     for (int c_ = 0; c_ < chunk; ++c_) {
       launch_pcg_iter_a(g, tx, ty, tz, diag, z, pin, pout, w, part, state, st);
-      launch_pcg_iter_b(g.ncell, xs, r, r32, pout, w, part, state, st);
+      launch_pcg_iter_b(g.ncell, r, r32, pout, w, part, state, st);
       apply(r, z, part, done);
-      beta();
+      beta(loop);
       std::swap(pin, pout);
     }
   };
-  // A chunk of PCG iterations (each: p-update + A p, x/r update, the whole
-  // preconditioner application, beta) as one CUDA graph: captured once per
-  // solution buffer and replayed until the device-side `done` flag is set.
-  // An even chunk returns the p buffers to their roles, so replays chain.
+  // PCG iterations (each: p-update + A p, x/r update, the whole preconditioner
+  // application, beta) as one CUDA graph that repeats a chunk until the
+  // device-side `done` flag is set.  An even chunk returns the p buffers to
+  // their roles.
   const bool use_graph = opt.pcg_graph && chunk % 2 == 0;
-  if (use_graph && (!pcg_exec || pcg_graph_x != xs || pcg_graph_ns != opt.null_space)) {
-    if (pcg_exec) cudaGraphExecDestroy(pcg_exec);
-    pcg_exec = nullptr;
-    const unsigned long long l0 = __atomic_load_n(&g_launches, __ATOMIC_RELAXED);
-    cudaGraph_t graph = nullptr;
-    if (int e = check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "graph capture")) return e;
-    enqueue_chunk();
-    if (int e = check(cudaStreamEndCapture(st, &graph), "graph capture")) return e;
-    const unsigned long long l1 = __atomic_load_n(&g_launches, __ATOMIC_RELAXED);
-    pcg_graph_kernels = l1 - l0;
-    __atomic_fetch_sub(&g_launches, pcg_graph_kernels, __ATOMIC_RELAXED);  // captured, not launched
-    const cudaError_t ie = cudaGraphInstantiate(&pcg_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (int e = check(ie, "graph instantiate")) return e;
-    pcg_graph_x = xs;
-    pcg_graph_ns = opt.null_space;
-  }
-  for (;;) {
-    if (use_graph) {
-      if (int e = check(cudaGraphLaunch(pcg_exec, st), "graph launch")) return e;
-      __atomic_fetch_add(&g_launches, pcg_graph_kernels, __ATOMIC_RELAXED);
-    } else {
-      enqueue_chunk();
+  if (use_graph) {
+    if (!pcg_exec || pcg_graph_ns != opt.null_space) {
+      if (pcg_exec) cudaGraphExecDestroy(pcg_exec);
+      pcg_exec = nullptr;
+      if (int e = loop_graph(&pcg_exec, &pcg_graph_kernels, enqueue_chunk)) return e;
+      pcg_graph_ns = opt.null_space;
     }
+    if (int e = check(cudaGraphLaunch(pcg_exec, st), "graph launch")) return e;
     cudaMemcpyAsync(h_state, state, sizeof(PcgState), cudaMemcpyDeviceToHost, st);
-    if (int e = check(cudaStreamSynchronize(st), "KSPSolve")) return e;
-    if (int e = check(cudaGetLastError(), "KSPSolve launch")) return e;
-    if (h_state->done) break;
-    if (++guard > opt.max_it + 8) break;
+  } else {
+    for (int guard = 0;;) {
+      enqueue_chunk(LoopCond());
+      cudaMemcpyAsync(h_state, state, sizeof(PcgState), cudaMemcpyDeviceToHost, st);
+      if (int e = check(cudaStreamSynchronize(st), "KSPSolve")) return e;
+      if (int e = check(cudaGetLastError(), "KSPSolve launch")) return e;
+      if (h_state->done) break;
+      if (++guard > opt.max_it + 8) break;
+    }
   }
   cudaEventRecord(ev1, st);
   if (!on_device) cudaMemcpyAsync(x_out, xs, n * 8, cudaMemcpyDeviceToHost, st);
   int e = check(cudaStreamSynchronize(st), "KSPSolve");
+  if (!e) e = check(cudaGetLastError(), "KSPSolve launch");
   if (!e) e = check_kernel_flag("KSPSolve");
+  if (use_graph) count_loop(pcg_graph_kernels, h_state->its, chunk);
   float ms = 0;
   cudaEventElapsedTime(&ms, ev0, ev1);
   last_solve_ms = ms;

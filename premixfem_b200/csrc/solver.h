@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <map>
 #include <string>
 #include <vector>
@@ -160,7 +161,6 @@ class Solver {
   int* d_all_done = nullptr;
   int* h_all_done = nullptr;     // pinned
   cudaGraphExec_t bpcg_exec = nullptr;
-  const double* bpcg_graph_x = nullptr;
   unsigned long long bpcg_graph_kernels = 0;
   int bpcg_blocks() const { return 32; }
   void* eig_work = nullptr;
@@ -176,6 +176,9 @@ class Solver {
 
   int check(cudaError_t e, const char* what);
   int dalloc(void** p, size_t bytes, const char* what);
+  void drop_graphs();
+  int loop_graph(cudaGraphExec_t* exec, unsigned long long* kernels, const std::function<void(LoopCond)>& chunk);
+  static void count_loop(unsigned long long kernels, int its, int chunk);
   int build_partition();
   int alloc_fine();
   void assemble_launch();
@@ -194,8 +197,7 @@ class Solver {
   int* d_queue = nullptr;
   EbBuffers eb;  // phase-batched eigensolver storage
   double eig_phase_ms[8] = {0};
-  cudaGraphExec_t pcg_exec = nullptr;  // one chunk of PCG iterations
-  const double* pcg_graph_x = nullptr;
+  cudaGraphExec_t pcg_exec = nullptr;  // PCG iterations, repeated on the device
   bool pcg_graph_ns = false;  // the null-space setting the graph was captured with
   unsigned long long pcg_graph_kernels = 0;
   unsigned long long eig_colcells = 0;
