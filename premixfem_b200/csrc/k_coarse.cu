@@ -995,8 +995,11 @@ __global__ void __launch_bounds__(512) k_dense_smallest_eig(RankLayout L, int en
 }
 
 // The same iteration in three launches over all ranks for p <= kL3Cols columns:
-// Y = inv X and A Y on the FP64 tensor cores, then one CTA per rank for the
-// projected problem.  Y is not orthonormalised first: the Rayleigh-Ritz step
+// Y and A Y on the FP64 tensor cores, then one CTA per rank for the projected
+// problem.  Y = X - inv R with the residuals R = A X - X w is (A + mu I)^-1 X up to
+// a factor per column, formed so that the inverse's rounding errors are multiplied
+// by the residual: from Y = inv X a rank whose matrix is singular up to mu can stall
+// above the tolerance and run to the iteration limit.  Y is not orthonormalised first: the Rayleigh-Ritz step
 // takes the pencil (Y^T A Y, Y^T Y) on one warp (pmf_rr.cuh), whose Cholesky
 // drops dependent columns; in exact arithmetic the Ritz pairs are the same, and
 // from the second iteration on Y's columns are nearly orthogonal.  The Ritz
@@ -1042,13 +1045,17 @@ __global__ void k_l3_init(RankLayout L, int p, const double* A_all, double* work
     st[r].conv = 0;
     st[r].it = 0;
   }
-  for (long long e = threadIdx.x; e < (long long)nr * p; e += blockDim.x)
-    X[e] = hash_uniform(((unsigned long long)r << 40) ^ (unsigned long long)e);
+  double* R = X + 2 * (long long)nr * p;  // X = 0 and R = -(random columns): Y = inv (random columns)
+  for (long long e = threadIdx.x; e < (long long)nr * p; e += blockDim.x) {
+    X[e] = 0.0;
+    R[e] = -hash_uniform(((unsigned long long)r << 40) ^ (unsigned long long)e);
+  }
 }
 
-// Out = M In, blocks src / dst of the rank's workspace (0 X, 1 Y, 2 A Y).  Lane (r, q) of a warp holds of
+// Out = M In (REFINE: X - M In), blocks src / dst of the rank's workspace (0 X, 1 Y, 2 R or A Y).  Lane (r, q) of a warp holds of
 // row r the entries k0 + 4 q + t, t < 4, of each 16: whole 128-byte row segments per load, used as the A
 // fragments of four k-steps (the order of k within a dot product is free as long as B follows it).
+template <bool REFINE>
 __global__ void __launch_bounds__(128) k_l3_mm(RankLayout L, int p, const double* M_all, double* work_all, int src,
                                                int dst, const L3Rank* st) {
   const int rk = blockIdx.y;
@@ -1106,7 +1113,9 @@ __global__ void __launch_bounds__(128) k_l3_mm(RankLayout L, int p, const double
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int c = 8 * n + 2 * q + h;
-        if (c < p) Out[(long long)i * p + c] = acc[0][n][h] + acc[1][n][h];
+        const long long o = (long long)i * p + c;
+        const double v = acc[0][n][h] + acc[1][n][h];
+        if (c < p) Out[o] = REFINE ? work_all[L.offw[rk] + o] - v : v;
       }
   }
 }
@@ -1119,8 +1128,8 @@ struct L3Smem {
   double red[32];
 };
 
-// Rayleigh-Ritz on (Y^T A Y, Y^T Y), X <- Y C, residuals of the wanted pairs from A Y C - X w, and fresh
-// directions in place of dropped columns.
+// Rayleigh-Ritz on (Y^T A Y, Y^T Y), X <- Y C, R = A X - X w from A Y C in the place of A Y, the residual norms
+// of the wanted pairs, and fresh directions in place of dropped columns.
 __global__ void __launch_bounds__(kL3Thr) k_l3_rr(RankLayout L, int en2, int p, double* work_all, L3Rank* st,
                                                   double tol, int it) {
   const int rk = blockIdx.x;
@@ -1130,7 +1139,7 @@ __global__ void __launch_bounds__(kL3Thr) k_l3_rr(RankLayout L, int en2, int p, 
   const int nr = rank_nr(L, rk);
   double* X = work_all + L.offw[rk];
   const double* Y = X + (long long)nr * p;
-  const double* AY = Y + (long long)nr * p;
+  double* AY = X + 2 * (long long)nr * p;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = kL3Thr / 32;
   {
     // Grams: rows l of four per step, tiles (0,0), (0,1), (1,1) of the 16 x 16 result
@@ -1208,15 +1217,14 @@ __global__ void __launch_bounds__(kL3Thr) k_l3_rr(RankLayout L, int en2, int p, 
 #pragma unroll
         for (int a = 0; a < kL3Cols; ++a)
           if (a < p) x += y[a] * sm.C[a * kL3Cols + c];
-        X[(long long)l * p + c] = x;
-        if (c < 8 && c < nw2) {
-          double ax = 0.0;
+        double ax = 0.0;
 #pragma unroll
-          for (int a = 0; a < kL3Cols; ++a)
-            if (a < p) ax += ay[a] * sm.C[a * kL3Cols + c];
-          const double d = ax - sm.rr.lam[c] * x;
-          res[c] += d * d;
-        }
+        for (int a = 0; a < kL3Cols; ++a)
+          if (a < p) ax += ay[a] * sm.C[a * kL3Cols + c];
+        const double d = ax - sm.rr.lam[c] * x;
+        X[(long long)l * p + c] = x;
+        AY[(long long)l * p + c] = d;
+        if (c < 8 && c < nw2) res[c] += d * d;
       }
   }
   bool conv = q >= en2;
@@ -1258,7 +1266,8 @@ __global__ void __launch_bounds__(kL3Thr) k_l3_rr(RankLayout L, int en2, int p, 
     for (int c = q; c < p; ++c) {
       double v = rnd(l, c);
       for (int k = 0; k < q; ++k) v -= d[c * 16 + k] * X[(long long)l * p + k];
-      X[(long long)l * p + c] = v;
+      X[(long long)l * p + c] = 0.0;
+      AY[(long long)l * p + c] = -v;
     }
 }
 
@@ -1280,7 +1289,7 @@ __global__ void k_l3_out(RankLayout L, int en2, int p, const double* work_all, c
   double* V = V_all + L.offv[r];
   for (long long e = threadIdx.x; e < (long long)nr * en2; e += blockDim.x) {
     const int i = (int)(e / en2), j = (int)(e % en2);
-    V[e] = X[(long long)i * p + j];
+    V[e] = j < st[r].q ? X[(long long)i * p + j] : -X[((long long)2 * nr + i) * p + j];
   }
   if (threadIdx.x < en2) evals_all[(long long)r * en2 + threadIdx.x] = st[r].w[threadIdx.x];
   if (threadIdx.x == 0) iters[r] = st[r].it;
@@ -1297,8 +1306,8 @@ void launch_dense_smallest_eig(const RankLayout& L, int nrank, int nr, int en2, 
     cudaFuncSetAttribute(k_l3_rr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(L3Smem));
     { note_launch(); k_l3_init<<<nrank, 256, 0, st>>>(L, p, A, work, rs); }
     for (int it = 0; it < max_it; ++it) {
-      { note_launch(); k_l3_mm<<<dim3(gx, nrank), 128, 0, st>>>(L, p, inv, work, 0, 1, rs); }
-      { note_launch(); k_l3_mm<<<dim3(gx, nrank), 128, 0, st>>>(L, p, A, work, 1, 2, rs); }
+      { note_launch(); k_l3_mm<true><<<dim3(gx, nrank), 128, 0, st>>>(L, p, inv, work, 2, 1, rs); }
+      { note_launch(); k_l3_mm<false><<<dim3(gx, nrank), 128, 0, st>>>(L, p, A, work, 1, 2, rs); }
       { note_launch(); k_l3_rr<<<nrank, kL3Thr, sizeof(L3Smem), st>>>(L, en2, p, work, rs, tol, it); }
       if ((it + 1) % 4 == 0 || it + 1 == max_it) {
         int h = 1;

@@ -1,0 +1,57 @@
+"""The dense coarse problems at the edges of their tiles: inverses of order 1,
+63, 64, 65, 128, 130 and 192 (64-wide panels), the level-3 eigensolve with blocks
+of 6, 12 and 16 columns (tensor-core launches) and 18 and 20 (one CTA per rank),
+one rank and ragged ranks, a floating rank included.
+
+Level-3 eigenvalues and the preconditioner at 1e-6 against the oracle's level 2
+and 3 on the basis that the library computed, so that the local eigensolver's
+tolerance is not part of the difference; a block iteration of this kind
+needs some tens of steps, so 100 of the 500 allowed mean that it stalled."""
+import numpy as np
+import pytest
+
+from oracle import pmf_oracle as O
+from premixfem_b200 import fields
+from premixfem_b200.solver import DarcySolver, options_string
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "n1": ((6, 5, 4), (1, 1, 1), (2, 1, 1), 1, 1),
+    "n63": ((15, 15, 6), (3, 3, 1), (1, 1, 1), 7, 2),
+    "n64": ((16, 16, 16), (4, 4, 4), (1, 1, 1), 1, 4),
+    "n65": ((52, 4, 4), (13, 1, 1), (1, 1, 1), 5, 6),
+    "n66_wide": ((44, 4, 4), (11, 1, 1), (1, 1, 1), 6, 7),
+    "n128": ((16, 16, 8), (4, 4, 2), (1, 1, 1), 4, 4),
+    "n130": ((52, 8, 4), (13, 2, 1), (1, 1, 1), 5, 4),
+    "n192_wide": ((16, 16, 16), (4, 4, 4), (1, 1, 1), 3, 8),
+    "ragged": ((22, 18, 10), (2, 2, 2), (2, 2, 1), 5, 4),
+}
+
+
+@pytest.mark.parametrize("contrast", [1.0, 4.0])
+@pytest.mark.parametrize("name", list(CASES))
+def test_coarse_orders(native, monkeypatch, name, contrast):
+    mesh, sd, vr, k, en2 = CASES[name]
+    prob = fields.random_box(mesh, seed=3, sigma=contrast, dirichlet={"x-": 1.0})
+    op = O.Operator(prob)
+    s = DarcySolver.from_problem(prob, options_string({"pmf_sd": sd, "pmf_vranks": vr, "en_lv1": k, "en_lv2": en2}))
+    s.setup()
+    phi = s.phi()
+
+    def basis(op, box, o):
+        V = phi[O.box_cells(op.mesh, box)]
+        return np.zeros(k), V, k, 0.0
+
+    monkeypatch.setattr(O, "local_basis", basis)
+    pc = O.Preconditioner(op, O.Options(sd=sd, vranks=vr, en_lv1=k, en_lv2=en2))
+    ev, _, its = s.eigen_lv2()
+    assert np.max(its) <= 100
+    ref = np.stack(list(pc.eigvals_lv2))
+    # a rank of one unknown has the eigenvalue zero alone: its scale is the coarse matrix's
+    scale = np.maximum(np.abs(ref).max(axis=1, keepdims=True), 1e-3 * np.abs(pc.A2full).max())
+    assert (np.abs(ev - ref) / np.maximum(np.abs(ref), 1e-3 * scale)).max() <= 1e-6
+    x = np.random.default_rng(2).standard_normal(op.n)
+    y, yr = s.pc_apply(x), pc.apply(x)
+    s.close()
+    assert np.linalg.norm(y - yr) <= 1e-6 * np.linalg.norm(yr)
