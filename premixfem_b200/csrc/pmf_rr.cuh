@@ -8,10 +8,11 @@
 // warp-synchronous steps and lets a dozen problems share an SM.  Against one CTA
 // of 256 threads per problem: 64 problems of 18 unknowns 52 us a launch instead
 // of 95, the 38 iterations of 512 problems of 24 unknowns 3.5 ms instead of
-// 10.0, the 86 of 1 728 problems in FP64 storage 8.6 ms instead of 31.1.  Every loop over pivots is rolled: the
-// registers shift by one column per step (the shift is the destination of the
-// update's multiply-add), so all register indices are compile-time constants
-// and the code stays small enough for the instruction cache.
+// 10.0, the 86 of 1 728 problems in FP64 storage 8.6 ms instead of 31.1.  Every
+// loop over pivots is rolled: the registers shift by one column per step (the
+// shift is the destination of the update's multiply-add), so all register indices
+// are compile-time constants and the code stays small enough for the instruction
+// cache.
 #pragma once
 
 #include "pmf_dense.cuh"
@@ -326,8 +327,11 @@ __device__ __forceinline__ void warp_sym_lowest(WarpRR<NX, MX>& s, double (&a)[N
 // The basis is scaled to unit M-norm, D = diag(GM)^-1/2; Cholesky D GM D = L L^T
 // and H = L^-1 (D GA D) L^-T by two substitutions.  A vector whose pivot is at or
 // below `drop` depends on the ones before it and leaves the basis (its row of H is
-// decoupled above the spectrum), so a nearly dependent basis costs no more than
-// another one.
+// decoupled above the spectrum), so a nearly dependent basis costs little more than
+// another one.  A pivot d is known to eps / d, and one of that size enters the later
+// ones as eps / sqrt(d): below eps^(2/3) it can lift a dependent vector's pivot over
+// `drop`, and its Ritz value is noise.  So as soon as one vector is dropped the
+// factorisation is repeated with the pivots held above 1e-9.
 template <int NX, int MX, class F>
 __device__ __forceinline__ int warp_rayleigh_ritz(WarpRR<NX, MX>& s, int n, int m, double drop, F load, double* Y,
                                                   int ldy) {
@@ -346,23 +350,30 @@ __device__ __forceinline__ int warp_rayleigh_ritz(WarpRR<NX, MX>& s, int n, int 
   const double dsc = (lane < n && dl > 1e-28 * mx) ? 1.0 / sqrt(dl) : 0.0;
   if (lane < NX) s.dsc[lane] = dsc;
   __syncwarp();
-#pragma unroll
-  for (int j = 0; j < NX; ++j) a[j] *= dsc * s.dsc[j];
   // Cholesky, right-looking: at step c, a[j] = (trailing matrix)[lane][c + j]
   unsigned kept = 0;
-  for (int c = 0; c < n; ++c) {
-    const double d = __shfl_sync(full, a[0], c);
-    const bool keep = d > drop && s.dsc[c] != 0.0;
-    const double r = keep ? rsqrt(d) : 0.0;
-    const double lc = lane > c ? a[0] * r : (lane == c && keep ? d * r : 0.0);
-    const double lsh = __shfl_sync(full, lc, (c + lane) & 31);
-    if (lane < NX) s.Lc[c * NX + lane] = c + lane < n ? lsh : 0.0;
-    if (lane == 0) s.inv[c] = r;
-    kept |= (keep ? 1u : 0u) << c;
+#pragma unroll 1
+  for (double least = drop;; least = 1e-9) {
+    if (kept) load(0, a);
     __syncwarp();
 #pragma unroll
-    for (int j = 1; j < NX; ++j) a[j - 1] = a[j] - lc * s.Lc[c * NX + j];
-    a[NX - 1] = 0.0;
+    for (int j = 0; j < NX; ++j) a[j] *= dsc * s.dsc[j];
+    kept = 0;
+    for (int c = 0; c < n; ++c) {
+      const double d = __shfl_sync(full, a[0], c);
+      const bool keep = d > least && s.dsc[c] != 0.0;
+      const double r = keep ? rsqrt(d) : 0.0;
+      const double lc = lane > c ? a[0] * r : (lane == c && keep ? d * r : 0.0);
+      const double lsh = __shfl_sync(full, lc, (c + lane) & 31);
+      if (lane < NX) s.Lc[c * NX + lane] = c + lane < n ? lsh : 0.0;
+      if (lane == 0) s.inv[c] = r;
+      kept |= (keep ? 1u : 0u) << c;
+      __syncwarp();
+#pragma unroll
+      for (int j = 1; j < NX; ++j) a[j - 1] = a[j] - lc * s.Lc[c * NX + j];
+      a[NX - 1] = 0.0;
+    }
+    if (kept == 0 || __popc(kept) == n || least >= 1e-9) break;
   }
   const int q = __popc(kept);
   // B = D GA D, symmetrised

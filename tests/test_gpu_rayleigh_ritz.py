@@ -32,3 +32,24 @@ def test_local_eigenvalues_at_every_width(native, mesh, k):
     # error by its square over the gap; 1e-6 is the bar of the other eigenvalue tests
     assert (ks == k).all() and (status != 1).all()
     assert err.max() <= 1e-6, f"max rel eigen error {err.max():.2e}"
+
+
+@pytest.mark.parametrize("k", [4, 6, 8])
+@pytest.mark.parametrize("tile", [(2, 3, 4), (3, 3, 3), (4, 2, 2), (5, 3, 2), (4, 4, 4), (6, 5, 3)],
+                         ids=lambda t: "x".join(map(str, t)))
+def test_basis_wider_than_the_space(native, tile, k):
+    """Bases that fill or exceed the space of a small subdomain: dependent vectors have to be recognised as
+    such, else their Ritz values are noise and the lowest wanted ones are wrong.  27 subdomains of four
+    contrasts; the bars of the test above."""
+    for seed, sigma in enumerate([0.5, 1.5, 3.0, 4.0]):
+        prob = fields.random_box(tuple(3 * n for n in tile), seed=seed, sigma=sigma)
+        s = DarcySolver.from_problem(prob, options_string({"sd": 3, "en_lv1": k, "en_lv2": 2}))
+        s.setup()
+        ev, _, _, status = s.eigen_lv1()
+        boxes, _ = s.subdomains()
+        s.close()
+        ref = O.local_eigenvalues(prob, [tuple(b) for b in boxes], k, method="dense")
+        scale = np.abs(ref).max(axis=1, keepdims=True)
+        err = np.abs(ev - ref) / np.maximum(np.abs(ref), 1e-3 * scale)
+        assert (status != 1).all()
+        assert err.max() <= 1e-6, f"max rel eigen error {err.max():.2e}"
