@@ -12,7 +12,7 @@
 // is orthonormalised in the M inner product (Cholesky QR, SVQB of Stathopoulos
 // & Wu 2002 when it is nearly dependent) and the Rayleigh-Ritz projection is
 // formed and solved in FP64: the Grams and the basis update run on the FP64
-// tensor cores (mma.sync m8n8k4), the projected eigenproblem by Householder
+// tensor cores (mma.sync m16n8k4), the projected eigenproblem by Householder
 // tridiagonalisation and multisection.  Converged vectors are soft-locked.
 // X, W, P are stored in T (float for the mixed-precision setup, double for
 // the plain form); their A-images are always FP64, so the projection stays
@@ -282,75 +282,149 @@ __device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double
                : "+d"(d0), "+d"(d1)
                : "d"(a), "d"(b));
 }
+// Two such products with the same B: rows 0-7 of A(16x4) in a0, 8-15 in a1, of D in d[0..1] and d[2..3].  One
+// m16n8k4 takes the time of one m8n8k4 (73.7 against 36.8 TFLOP/s), so the kernels pair row tiles where they can.
+__device__ __forceinline__ void dmma1684(double (&d)[4], double a0, double a1, double b) {
+  asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+               : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+               : "d"(a0), "d"(a1), "d"(b));
+}
+
+// N consecutive values by 16-byte loads / stores (two FP32 values: 8); p is aligned to N values or 16 bytes
+template <typename T, int N>
+__device__ __forceinline__ void ldv(const T* p, T (&v)[N]) {
+  if constexpr (sizeof(T) == 4 && N == 2) {
+    const float2 f = *reinterpret_cast<const float2*>(p);
+    v[0] = f.x;
+    v[1] = f.y;
+  } else if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(p + i);
+      v[i] = f.x;
+      v[i + 1] = f.y;
+      v[i + 2] = f.z;
+      v[i + 3] = f.w;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+      const double2 f = *reinterpret_cast<const double2*>(p + i);
+      v[i] = f.x;
+      v[i + 1] = f.y;
+    }
+  }
+}
+template <int N>
+__device__ __forceinline__ void stv(float* p, const double (&v)[N]) {
+  static_assert(N == 4, "");
+  *reinterpret_cast<float4*>(p) = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+}
+template <int N>
+__device__ __forceinline__ void stv(double* p, const double (&v)[N]) {
+  static_assert(N == 2, "");
+  *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+}
 
 // Both Rayleigh-Ritz Grams on the FP64 tensor cores:
-//   GM = (w S)^T S,  GA = S^T (A S),  S = [X W P] (ns <= 32 columns).
-// Warp w takes cells 4w + 32i; for each group of 4 cells lane l loads basis
-// row 8t + l/4 at cell l%4, which is at once its A fragment (row of S^T) and
-// its B fragment (column of S / AS): no shared-memory staging.  The per-warp
-// partial tiles are reduced in a fixed order through shared memory, so the
-// result is deterministic.  red: >= 8 * 32 * 32 doubles.
+//   GM = (w S)^T S,  GA = S^T (A S),  S = [X W P] (ns <= 8 NT columns).
+// Warp w takes cells 16w + 128i; of each group of 16, lane l holds of basis row
+// 8t + l/4 the cells 4(l%4) .. +3, one or two 16-byte loads: cell 4(l%4) + q is
+// k-index l%4 of k-step q, at once its A fragment (row of S^T) and its B fragment
+// (column of S / AS), with no shared-memory staging.  (One value per lane and load,
+// four lanes to a 32-byte sector, kept the L1 busy with eight lines per request.)
+// Columns are readable to a multiple of 64 cells, and what lies past ncells is
+// masked.  Both Grams are symmetric: column tile t is multiplied with the row
+// tiles t and t + 1 (mod NT), which for NT = 3 are the six tiles of a triangle in
+// three instructions.  The per-warp partial tiles are reduced in a fixed order
+// through shared memory, so the result is deterministic.  red: >= 8 * 32 * 32
+// doubles.
+//
+// Bound by HBM where many subdomains iterate (per cell and column a value and an
+// FP64 image): all Grams of a 256^3 set-up take 26.9 ms (36.0 with one value per
+// load and one tile per product; their bytes need 17), of one with blocks of ten
+// columns 30.6 (67.8).  Loading a step ahead in halves of the step costs more than
+// it hides (34.1).
+template <int NT>
+__device__ __forceinline__ bool gram_has(int ta, int tb) {
+  return ta == tb || (NT == 2 && ta == 1) || (NT >= 3 && ta == (tb + 1) % NT) || (NT == 4 && tb == ta + 2);
+}
 template <typename TS, typename TA, int NT>
 __device__ __noinline__ void cta_gram2_mma(const Seg3<TS> S, const Seg3<TA> AS, const double* wgt, int ncells,
                                            double* GM, double* GA, double* red) {
+  constexpr int C = NT <= 3 ? 4 : 2;  // cells per lane and step (four tiles: two, within 128 registers)
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int r = lane >> 2, cq = lane & 3;
   const int ns = S.total();
-  const int nt = (ns + 7) >> 3;
   const TS* sp[NT];
   const TA* ap[NT];
 #pragma unroll
   for (int ta = 0; ta < NT; ++ta) {
     const int a = 8 * ta + r;
-    sp[ta] = (ta < nt && a < ns) ? S.col(a) : nullptr;
-    ap[ta] = (ta < nt && a < ns) ? AS.col(a) : nullptr;
+    sp[ta] = a < ns ? S.col(a) + C * cq : nullptr;
+    ap[ta] = a < ns ? AS.col(a) + C * cq : nullptr;
   }
-  // Only the tiles ta <= tb are accumulated (both Grams are symmetric); the
-  // reduction mirrors them.  NT is the exact tile count when nt == NT (the
-  // batched solver dispatches on it); tiles past nt load zeros.
-  constexpr int NP = NT * (NT + 1) / 2;
-  double cm[NP][2], ca[NP][2];
+  double cm[NT][4], ca[NT][4];  // column tile t: rows t (0, 1) and t + 1 (2, 3)
+  double em[2][2], ea[2][2];    // NT = 4: tiles (0, 2) and (1, 3)
 #pragma unroll
-  for (int p = 0; p < NP; ++p) cm[p][0] = cm[p][1] = ca[p][0] = ca[p][1] = 0.0;
-  // Each warp step covers 8 cells (two k-steps of 4): lane l reads cells
-  // c0 + l%4 and c0 + 4 + l%4, so a column's two loads fill whole 32-byte
-  // sectors, and the next step's 16 loads per lane are in flight during the MMAs.
-  double s[NT], as[NT], s2[NT], as2[NT], wv, wv2;
-  auto load = [&](int c0) {
-    const int c = c0 + cq, c2 = c0 + 4 + cq;
-    const bool in = c < ncells, in2 = c2 < ncells;
-    wv = in ? wgt[c] : 0.0;
-    wv2 = in2 ? wgt[c2] : 0.0;
+  for (int t = 0; t < NT; ++t)
 #pragma unroll
-    for (int ta = 0; ta < NT; ++ta) {
-      s[ta] = (in && sp[ta]) ? (double)sp[ta][c] : 0.0;
-      as[ta] = (in && ap[ta]) ? (double)ap[ta][c] : 0.0;
-      s2[ta] = (in2 && sp[ta]) ? (double)sp[ta][c2] : 0.0;
-      as2[ta] = (in2 && ap[ta]) ? (double)ap[ta][c2] : 0.0;
+    for (int h = 0; h < 4; ++h) cm[t][h] = ca[t][h] = 0.0;
+#pragma unroll
+  for (int t = 0; t < 2; ++t) em[t][0] = em[t][1] = ea[t][0] = ea[t][1] = 0.0;
+  for (int c0 = 4 * C * w; c0 < ncells; c0 += 4 * C * nwarp) {
+    TS sv[NT][C];
+    TA av[NT][C];
+    double wv[C];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+#pragma unroll
+      for (int q = 0; q < C; ++q) {
+        sv[t][q] = (TS)0;
+        av[t][q] = (TA)0;
+      }
+      if (sp[t]) {
+        ldv<TS, C>(sp[t] + c0, sv[t]);
+        ldv<TA, C>(ap[t] + c0, av[t]);
+      }
     }
-  };
-  load(8 * w);
-  for (int c0 = 8 * w; c0 < ncells; c0 += 8 * nwarp) {
-    double cs[NT], cas[NT], cs2[NT], cas2[NT];
+    ldv<double, C>(wgt + C * cq + c0, wv);
+    if (c0 + 4 * C > ncells) {
 #pragma unroll
-    for (int ta = 0; ta < NT; ++ta) {
-      cs[ta] = s[ta];
-      cas[ta] = as[ta];
-      cs2[ta] = s2[ta];
-      cas2[ta] = as2[ta];
+      for (int q = 0; q < C; ++q)
+        if (c0 + C * cq + q >= ncells) {
+          wv[q] = 0.0;
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            sv[t][q] = (TS)0;
+            av[t][q] = (TA)0;
+          }
+        }
     }
-    const double cw = wv, cw2 = wv2;
-    if (c0 + 8 * nwarp < ncells) load(c0 + 8 * nwarp);  // next step in flight during the MMAs
 #pragma unroll
-    for (int ta = 0; ta < NT; ++ta) {
-      const double ws = cs[ta] * cw, ws2 = cs2[ta] * cw2;
+    for (int q = 0; q < C; ++q) {
+      double cs[NT], cw[NT];
 #pragma unroll
-      for (int tb = ta; tb < NT; ++tb) {
-        const int p = ta * NT - ta * (ta - 1) / 2 + (tb - ta);
-        dmma884(cm[p][0], cm[p][1], ws, cs[tb]);
-        dmma884(ca[p][0], ca[p][1], cs[ta], cas[tb]);
-        dmma884(cm[p][0], cm[p][1], ws2, cs2[tb]);
-        dmma884(ca[p][0], ca[p][1], cs2[ta], cas2[tb]);
+      for (int t = 0; t < NT; ++t) {
+        cs[t] = (double)sv[t][q];
+        cw[t] = cs[t] * wv[q];
+      }
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        if (NT >= 3 || (NT == 2 && t == 0)) {
+          dmma1684(cm[t], cw[t], cw[(t + 1) % NT], cs[t]);
+          dmma1684(ca[t], cs[t], cs[(t + 1) % NT], (double)av[t][q]);
+        } else {
+          dmma884(cm[t][0], cm[t][1], cw[t], cs[t]);
+          dmma884(ca[t][0], ca[t][1], cs[t], (double)av[t][q]);
+        }
+      }
+      if (NT == 4) {
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          dmma884(em[t][0], em[t][1], cw[t], cs[(t + 2) % NT]);
+          dmma884(ea[t][0], ea[t][1], cs[t], (double)av[(t + 2) % NT][q]);
+        }
       }
     }
   }
@@ -358,22 +432,22 @@ __device__ __noinline__ void cta_gram2_mma(const Seg3<TS> S, const Seg3<TA> AS, 
 #pragma unroll 1
   for (int which = 0; which < 2; ++which) {
     __syncthreads();
+    auto put = [&](int ta, int tb, double d0, double d1) {
+      double* o = red + (w * 32 + 8 * ta + r) * 32 + 8 * tb + 2 * cq;
+      o[0] = d0;
+      o[1] = d1;
+    };
 #pragma unroll
-    for (int ta = 0; ta < NT; ++ta)
-#pragma unroll
-      for (int tb = ta; tb < NT; ++tb) {
-        const int p = ta * NT - ta * (ta - 1) / 2 + (tb - ta);
-        if (tb < nt) {
-          const int row = 8 * ta + r, col = 8 * tb + 2 * cq;
-          red[(w * 32 + row) * 32 + col] = which ? ca[p][0] : cm[p][0];
-          red[(w * 32 + row) * 32 + col + 1] = which ? ca[p][1] : cm[p][1];
-        }
-      }
+    for (int t = 0; t < NT; ++t) {
+      put(t, t, which ? ca[t][0] : cm[t][0], which ? ca[t][1] : cm[t][1]);
+      if (NT >= 3 || (NT == 2 && t == 0)) put((t + 1) % NT, t, which ? ca[t][2] : cm[t][2], which ? ca[t][3] : cm[t][3]);
+      if (NT == 4 && t < 2) put(t, t + 2, which ? ea[t & 1][0] : em[t & 1][0], which ? ea[t & 1][1] : em[t & 1][1]);
+    }
     __syncthreads();
     double* G = which ? GA : GM;
     for (int e = threadIdx.x; e < ns * ns; e += blockDim.x) {
       int a = e / ns, b = e % ns;
-      if ((a >> 3) > (b >> 3)) {  // below the accumulated block triangle: the mirror
+      if (!gram_has<NT>(a >> 3, b >> 3)) {  // the mirror of an accumulated tile
         const int x = a;
         a = b;
         b = x;
@@ -389,134 +463,93 @@ __device__ __noinline__ void cta_gram2_mma(const Seg3<TS> S, const Seg3<TA> AS, 
 // In-place basis update on the FP64 tensor cores:
 //   B0[:, j] <- sum_b S_b Y[b][j]            (b < ns, S = [B0 | B1 | B2])
 //   B2[:, j] <- sum_{b >= m0} S_b Y[b][j]    (the new search direction)
-// for j < m (m <= 8 NJ).  Warp w handles groups of 8 cells; lane l's A fragment
-// is S_{k0 + l%4} at cell 8g + l/4 and its B fragments come from Y.  Every warp
-// reads all ns columns of its 8 cells before writing them.
-//
-// Each lane resolves its NK column addresses (b = 4 kk + l%4 in [B0 | B1 | B2])
-// once, and for NJ = 1 keeps its Y fragments in registers, so that a group
-// costs NK predicated loads, 2 NK MMAs and the stores: no per-load selection
-// among the three blocks and no loop bounds known only at run time.  Columns
-// b >= ns load as zero and meet zero rows of Y (NK k-steps always run).
-template <typename T, int NK, int NJ, int STAGES>
+// for j < m (m <= 8 NJ).  The product is taken transposed, Y^T S^T: rows 0-7 of a
+// tile are eight columns j of B0 and rows 8-15 the same columns of B2, so one
+// m16n8k4 makes both, and the n-index is the cell.  A warp takes groups of 8 V
+// cells (V values in 16 bytes); lane l loads columns 4 kk + l%4 at cells
+// V (l/4) .. +V-1, cell V n + t being column n of tile t, and its results are the
+// cells V 2(l%4) .. +2V-1 of column l/4 of both outputs: 16-byte loads and stores
+// throughout.  Every warp reads all ns columns of its cells before writing them;
+// the next group is loading meanwhile.  Columns b >= ns load as zero and meet zero
+// rows of Y (NK k-steps always run); cells past ncells are computed from whatever
+// the padding holds, in their own columns of the tiles, and not written.  Bound by
+// HBM: all updates of a 256^3 set-up take 14.0 ms (29.9 with one value per load and
+// separate products for the two outputs; their bytes need 9).
+template <typename T, int NK, int NJ>
 __device__ __noinline__ void cta_update_mma(T* B0, T* B1, T* B2, int m0, int n1, int n2, int m, const double* Y,
                                             int ncells, size_t ld) {
+  constexpr int V = 16 / sizeof(T);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int r = lane >> 2, cq = lane & 3;
   const int ns = m0 + n1 + n2;
-  const int ngrp = (ncells + 7) >> 3;
   const T* colp[NK];
-  double yx[NK], yq[NK];  // Y fragments of tile 0 (NJ = 1)
 #pragma unroll
   for (int kk = 0; kk < NK; ++kk) {
     const int b = 4 * kk + cq;
-    colp[kk] = b >= ns        ? nullptr
+    colp[kk] = b >= ns       ? nullptr
                : b < m0      ? B0 + (size_t)b * ld
                : b < m0 + n1 ? B1 + (size_t)(b - m0) * ld
                              : B2 + (size_t)(b - m0 - n1) * ld;
-    const double y = (NJ == 1 && b < ns && r < m) ? Y[b * LB_LD + r] : 0.0;
-    yx[kk] = y;
-    yq[kk] = b >= m0 ? y : 0.0;
+    if (colp[kk]) colp[kk] += V * r;
   }
-  // STAGES groups ahead are loading while group gi is multiplied.
-  double av[NK], an[NK], an2[NK];
-  auto load = [&](int gi, double* dst) {
-    const int cell = 8 * gi + r;
-    const bool in = cell < ncells;
-#pragma unroll
-    for (int kk = 0; kk < NK; ++kk) dst[kk] = (in && colp[kk]) ? (double)colp[kk][cell] : 0.0;
+  // A fragments, rows j and 8 + j (kept in registers for one tile of columns)
+  auto yfrag = [&](int kk, int tj) {
+    const int b = 4 * kk + cq, j = 8 * tj + r;
+    return (b < ns && j < m) ? Y[b * LB_LD + j] : 0.0;
   };
-  if (w < ngrp) load(w, an);
-  if (STAGES > 1 && w + nwarp < ngrp) load(w + nwarp, an2);
-  for (int gi = w; gi < ngrp; gi += nwarp) {
-    const int cell = 8 * gi + r;
-    const bool in = cell < ncells;
+  double y0[NK];
 #pragma unroll
-    for (int kk = 0; kk < NK; ++kk) {
-      av[kk] = an[kk];
-      if (STAGES > 1) an[kk] = an2[kk];
-    }
-    if (STAGES > 1) {
-      if (gi + 2 * nwarp < ngrp) load(gi + 2 * nwarp, an2);
-    } else {
-      if (gi + nwarp < ngrp) load(gi + nwarp, an);
-    }
-    double dx[NJ][2], dp[NJ][2];
-#pragma unroll
-    for (int tj = 0; tj < NJ; ++tj) dx[tj][0] = dx[tj][1] = dp[tj][0] = dp[tj][1] = 0.0;
+  for (int kk = 0; kk < NK; ++kk) y0[kk] = NJ == 1 ? yfrag(kk, 0) : 0.0;
+  T nx[NK][V];
+  auto load = [&](int c0) {
 #pragma unroll
     for (int kk = 0; kk < NK; ++kk) {
 #pragma unroll
-      for (int tj = 0; tj < NJ; ++tj) {
-        double y = yx[kk], yp = yq[kk];
-        if (NJ > 1) {
-          const int bb = 4 * kk + cq, jj = 8 * tj + r;
-          y = (bb < ns && jj < m) ? Y[bb * LB_LD + jj] : 0.0;
-          yp = bb >= m0 ? y : 0.0;
-        }
-        dmma884(dx[tj][0], dx[tj][1], av[kk], y);
-        dmma884(dp[tj][0], dp[tj][1], av[kk], yp);
-      }
+      for (int q = 0; q < V; ++q) nx[kk][q] = (T)0;
+      if (colp[kk]) ldv<T, V>(colp[kk] + c0, nx[kk]);
     }
-    // D fragment: rows = cells 8gi + r, columns j = 8tj + 2cq + {0, 1}
+  };
+  const int step = 8 * V * nwarp;
+  if (8 * V * w < ncells) load(8 * V * w);
+  for (int c0 = 8 * V * w; c0 < ncells; c0 += step) {
+    T cu[NK][V];
+#pragma unroll
+    for (int kk = 0; kk < NK; ++kk)
+#pragma unroll
+      for (int q = 0; q < V; ++q) cu[kk][q] = nx[kk][q];
+    if (c0 + step < ncells) load(c0 + step);
 #pragma unroll
     for (int tj = 0; tj < NJ; ++tj) {
+      double d[V][4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int j = 8 * tj + 2 * cq + h;
-        if (in && j < m) {
-          B0[(size_t)j * ld + cell] = (T)dx[tj][h];
-          B2[(size_t)j * ld + cell] = (T)dp[tj][h];
-        }
+      for (int t = 0; t < V; ++t)
+#pragma unroll
+        for (int h = 0; h < 4; ++h) d[t][h] = 0.0;
+#pragma unroll
+      for (int kk = 0; kk < NK; ++kk) {
+        const double y = NJ == 1 ? y0[kk] : yfrag(kk, tj), yp = 4 * kk + cq >= m0 ? y : 0.0;
+#pragma unroll
+        for (int t = 0; t < V; ++t) dmma1684(d[t], y, yp, (double)cu[kk][t]);
       }
-    }
-  }
-}
-
-// The same update on the CUDA cores, one cell per thread (FP64 arithmetic):
-// each thread loads the ns values of its cell (independent, coalesced loads:
-// consecutive threads on consecutive cells), then accumulates both outputs
-// with Y broadcast from shared memory, and writes them.  Every value of a
-// cell is read before the cell is written, as in cta_update_mma.
-template <typename T, int MM>
-__device__ __noinline__ void cta_update_cc(T* B0, T* B1, T* B2, int m0, int n1, int n2, int m, const double* Y,
-                                           int ncells, size_t ld) {
-  const int ns = m0 + n1 + n2;
-  for (int cell = threadIdx.x; cell < ncells; cell += blockDim.x) {
-    double sv[3 * MM];
-#pragma unroll
-    for (int b = 0; b < 3 * MM; ++b) {
-      double v = 0.0;
-      if (b < ns) {
-        if (b < m0)
-          v = (double)B0[(size_t)b * ld + cell];
-        else if (b < m0 + n1)
-          v = (double)B1[(size_t)(b - m0) * ld + cell];
-        else
-          v = (double)B2[(size_t)(b - m0 - n1) * ld + cell];
-      }
-      sv[b] = v;
-    }
-    double ax[MM], ap[MM];
-#pragma unroll
-    for (int j = 0; j < MM; ++j) ax[j] = ap[j] = 0.0;
-#pragma unroll
-    for (int b = 0; b < 3 * MM; ++b) {
-      if (b < ns) {
-#pragma unroll
-        for (int j = 0; j < MM; ++j) {
-          const double y = Y[b * LB_LD + j];
-          ax[j] += sv[b] * y;
-          if (b >= m0) ap[j] += sv[b] * y;
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < MM; ++j)
+      const int j = 8 * tj + r;
       if (j < m) {
-        B0[(size_t)j * ld + cell] = (T)ax[j];
-        B2[(size_t)j * ld + cell] = (T)ap[j];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {  // h & 1: which of the two runs of V cells; h >> 1: B0 or B2
+          const int cell = c0 + V * (2 * cq + (h & 1));
+          T* o = (h >> 1 ? B2 : B0) + (size_t)j * ld + cell;
+          double v[V];
+#pragma unroll
+          for (int t = 0; t < V; ++t) v[t] = d[t][h];
+          if (cell + V <= ncells) {
+            stv<V>(o, v);
+          } else {
+#pragma unroll
+            for (int t = 0; t < V; ++t)
+              if (cell + t < ncells) o[t] = (T)v[t];
+          }
+        }
       }
+    }
   }
 }
 
@@ -1162,10 +1195,10 @@ __global__ void __launch_bounds__(LB_THREADS) k_lobpcg(LobpcgArgs a, unsigned ch
       // ---- X <- S Y, P <- [W P] Y_WP, same for AX / AP (per cell, in place)
       // X <- S Y, P <- [W P] Y_WP and the same combination of the FP64 A-images, on the
       // FP64 tensor cores
-      cta_update_mma<T, 8, 2, 1>(X, W, P, m, nact, np, m, mt.Y, nc, ld);
+      cta_update_mma<T, 8, 2>(X, W, P, m, nact, np, m, mt.Y, nc, ld);
       pc.lap(14);
       if (sizeof(T) == 8) {
-        cta_update_mma<double, 8, 2, 1>(AX, AW, AP, m, nact, np, m, mt.Y, nc, ld);
+        cta_update_mma<double, 8, 2>(AX, AW, AP, m, nact, np, m, mt.Y, nc, ld);
         __syncthreads();
       } else {
         // FP32 storage rounds X and P: their A-images are recomputed from the stored values
@@ -1694,10 +1727,9 @@ static void launch_eb_rr(const EbArgs& e, int nact, double drop, cudaStream_t st
 }
 
 // X <- S Y, P <- [W P] Y_WP (and the FP64 A-images in FP64 storage), per chunk.
-// NK / NJ: k-steps and 8-column tiles of the tensor-core update (6 / 1 for m <= 8);
-// ST: groups of 8 cells each warp has loading while it multiplies one (1 or 2).
-template <typename T, int NK, int NJ, int ST>
-__global__ void __launch_bounds__(256, (NJ == 1 && ST == 1) ? 3 : 2) k_eb_update(EbArgs a) {
+// NK / NJ: k-steps and 8-column tiles of the tensor-core update (6 / 1 for m <= 8).
+template <typename T, int NK, int NJ>
+__global__ void __launch_bounds__(256, 2) k_eb_update(EbArgs a) {
   __shared__ double Ys[LB_LD * LB_LD];
   const int s = eb_sub(a, blockIdx.y);
   const EbState& es = a.state[s];
@@ -1712,31 +1744,9 @@ __global__ void __launch_bounds__(256, (NJ == 1 && ST == 1) ? 3 : 2) k_eb_update
   __syncthreads();
   EbSlab<T> sl(a.slab + (size_t)s * a.slab_stride, a.m, a.ld);
   const int m = a.m;
-  cta_update_mma<T, NK, NJ, ST>(sl.X + c0, sl.W + c0, sl.P + c0, m, es.nact, es.np, m, Ys, cn, a.ld);
+  cta_update_mma<T, NK, NJ>(sl.X + c0, sl.W + c0, sl.P + c0, m, es.nact, es.np, m, Ys, cn, a.ld);
   if (sizeof(T) == 8)
-    cta_update_mma<double, NK, NJ, ST>(sl.AX + c0, sl.AW + c0, sl.AP + c0, m, es.nact, es.np, m, Ys, cn, a.ld);
-}
-
-// k_eb_update with the CUDA-core update (m <= 8 block columns)
-template <typename T>
-__global__ void __launch_bounds__(256, 2) k_eb_update_cc(EbArgs a) {
-  __shared__ double Ys[LB_LD * LB_LD];
-  const int s = eb_sub(a, blockIdx.y);
-  const EbState& es = a.state[s];
-  if (es.done || es.restart) return;
-  const SubInfo S = a.subs[s];
-  const int nc = S.nx * S.ny * S.nz;
-  const int c0 = blockIdx.x * EB_CHUNK;
-  if (c0 >= nc) return;
-  const int cn = min(nc - c0, EB_CHUNK);
-  const double* Y = a.Ybuf + (size_t)s * LB_LD * LB_LD;
-  for (int e = threadIdx.x; e < es.nS * LB_LD; e += blockDim.x) Ys[e] = Y[e];
-  __syncthreads();
-  EbSlab<T> sl(a.slab + (size_t)s * a.slab_stride, a.m, a.ld);
-  const int m = a.m;
-  cta_update_cc<T, 8>(sl.X + c0, sl.W + c0, sl.P + c0, m, es.nact, es.np, m, Ys, cn, a.ld);
-  if (sizeof(T) == 8)
-    cta_update_cc<double, 8>(sl.AX + c0, sl.AW + c0, sl.AP + c0, m, es.nact, es.np, m, Ys, cn, a.ld);
+    cta_update_mma<double, NK, NJ>(sl.AX + c0, sl.AW + c0, sl.AP + c0, m, es.nact, es.np, m, Ys, cn, a.ld);
 }
 
 // ---- final phase (k_lobpcg mode 2 as phase kernels over every subdomain of
@@ -2200,16 +2210,11 @@ int launch_lobpcg_batched(const LobpcgArgs& a_in, const EbBuffers& b, const int*
   for (int q = 0; q < nmb; ++q) pre_smem_max = std::max(pre_smem_max, coef + (size_t)4 * e.ldc * mb_c[q]);
   const size_t gram_smem = (size_t)8 * 32 * 32 * sizeof(double);
   cudaFuncSetAttribute(k_eb_precond<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pre_smem_max);
-  // basis update tiles: <6,1> (3 CTAs per SM) is the built-in for m <= 8, <8,2> the alternative;
-  // candidates 2 / 3 are the same tiles with two groups of cells loading ahead per warp
-  // candidate 4 (m <= 8): the CUDA-core update, one cell per thread
-  const int nupd = a.m <= 8 ? 5 : 2;
-  char kpre[96], kupd[96];
+  char kpre[96];
   snprintf(kpre, sizeof(kpre), "eb_precond|%s|m%d|c%d", sizeof(T) == 4 ? "f32" : "f64", a.m, e.ldc);
-  snprintf(kupd, sizeof(kupd), "eb_update|%s|m%d|c%d|cc", sizeof(T) == 4 ? "f32" : "f64", a.m, e.ldc);
-  cudaEvent_t tev[4];
+  cudaEvent_t tev[2];
   for (auto& x : tev) cudaEventCreate(&x);
-  int prev_pc = -1, prev_uc = -1, prev_cols = 0, prev_ns = 0;
+  int prev_pc = -1, prev_cols = 0;
   // time per unit of work of the previous iteration's launches, read after the
   // iteration's own synchronisation (no extra host waits)
   auto report_prev = [&]() {
@@ -2217,8 +2222,6 @@ int launch_lobpcg_batched(const LobpcgArgs& a_in, const EbBuffers& b, const int*
     float ms = 0.0f;
     if (cudaEventElapsedTime(&ms, tev[0], tev[1]) == cudaSuccess && prev_cols > 0)
       tune_online_report(kpre, nmb, prev_pc, 1e3f * ms / (float)prev_cols);
-    if (cudaEventElapsedTime(&ms, tev[2], tev[3]) == cudaSuccess && prev_ns > 0)
-      tune_online_report(kupd, nupd, prev_uc, 1e3f * ms / (float)prev_ns);
     prev_pc = -1;
   };
   cudaFuncSetAttribute(k_eb_gram<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gram_smem);
@@ -2254,7 +2257,7 @@ int launch_lobpcg_batched(const LobpcgArgs& a_in, const EbBuffers& b, const int*
     nact = b.h_nactive[0];
     if (nact == 0) break;
     ++lockstep;
-    const int pc = tune_online_pick(kpre, nmb), uc = tune_online_pick(kupd, nupd);
+    const int pc = tune_online_pick(kpre, nmb);
     EbArgs ep = e;
     ep.mb = mb_c[pc];
     const dim3 gchunk(e.nchunk, nact), gpre((a.m + ep.mb - 1) / ep.mb, nact);
@@ -2269,22 +2272,12 @@ int launch_lobpcg_batched(const LobpcgArgs& a_in, const EbBuffers& b, const int*
     launch_eb_rr(e, nact, drop, st);
     mark(5);
     note_launch();
-    cudaEventRecord(tev[2], st);
-    if (a.m <= 8 && uc == 4)
-      k_eb_update_cc<T><<<gchunk, 256, 0, st>>>(e);
-    else if (a.m <= 8 && uc == 0)
-      k_eb_update<T, 6, 1, 1><<<gchunk, 256, 0, st>>>(e);
-    else if (a.m <= 8 && uc == 2)
-      k_eb_update<T, 6, 1, 2><<<gchunk, 256, 0, st>>>(e);
-    else if (uc == 3 || (a.m > 8 && uc == 1))
-      k_eb_update<T, 8, 2, 2><<<gchunk, 256, 0, st>>>(e);
+    if (a.m <= 8)
+      k_eb_update<T, 6, 1><<<gchunk, 256, 0, st>>>(e);
     else
-      k_eb_update<T, 8, 2, 1><<<gchunk, 256, 0, st>>>(e);
-    cudaEventRecord(tev[3], st);
+      k_eb_update<T, 8, 2><<<gchunk, 256, 0, st>>>(e);
     prev_pc = pc;
-    prev_uc = uc;
     prev_cols = b.h_nactive[1];
-    prev_ns = b.h_nactive[2];
     mark(6);
     if (sizeof(T) == 4) { note_launch(); k_eb_aimg<T><<<dim3(2 * a.m, nact), 256, 0, st>>>(e, 1); }
     mark(7);
