@@ -477,7 +477,7 @@ int Solver::build_partition() {
   const int GX = px * sx, GY = py * sy, GZ = pz * sz;
   std::vector<int> gmap((size_t)GX * GY * GZ, -1);
   max_cells = 0;
-  max_lines = 0;
+  max_lines = max_nxny = 0;
   for (int kz = 0; kz < pz; ++kz)
     for (int ky = 0; ky < py; ++ky)
       for (int kx_ = 0; kx_ < px; ++kx_) {
@@ -510,6 +510,7 @@ int Solver::build_partition() {
               gmap[((size_t)gz * GY + gy) * GX + gx] = s;
               max_cells = std::max(max_cells, S.nx * S.ny * S.nz);
               max_lines = std::max(max_lines, S.ny * S.nz);
+              max_nxny = std::max(max_nxny, S.nx * S.ny);
             }
       }
   for (int s = 0; s < nsub; ++s) {
@@ -543,7 +544,7 @@ int Solver::build_partition_batch() {
   rank_grid[1] = rank_grid[2] = 1;
   subs.clear();
   rank_first.assign(nprob + 1, 0);
-  max_cells = max_lines = 0;
+  max_cells = max_lines = max_nxny = 0;
   spr = 0;
   for (int q = 0; q < nprob; ++q) {
     ProbInfo& pq = probs[q];
@@ -584,6 +585,7 @@ int Solver::build_partition_batch() {
           S.nb[5] = at(cx, cy, cz + 1);
           max_cells = std::max(max_cells, S.nx * S.ny * S.nz);
           max_lines = std::max(max_lines, S.ny * S.nz);
+          max_nxny = std::max(max_nxny, S.nx * S.ny);
           subs.push_back(S);
         }
     pq.s1 = (int)subs.size();
@@ -1141,6 +1143,7 @@ int Solver::setup() {
   la.rel_floor = opt.eig_rel_floor;
   la.final_batched = opt.eig_final;
   la.init_batched = opt.eig_init;
+  la.max_nxny = max_nxny;
   la.slab = nullptr;
   la.slab_stride = 0;
   la.state = nullptr;

@@ -105,7 +105,7 @@ class Solver {
   Options opt;
   cudaStream_t st = nullptr;
   std::vector<SubInfo> subs;
-  int nsub = 0, nrank = 0, spr = 0, kmax = 0, max_cells = 0, max_lines = 0, nr = 0, en2 = 0, n3 = 0;
+  int nsub = 0, nrank = 0, spr = 0, kmax = 0, max_cells = 0, max_lines = 0, max_nxny = 0, nr = 0, en2 = 0, n3 = 0;
   int rank_grid[3];
   bool is_setup = false;
   std::vector<double> eig1, eig3;  // per subdomain k values / per rank en2 values
