@@ -769,9 +769,9 @@ static bool gj_inverse(int nb, GjShape sh, double* a, double tol, int* nnull, cu
   return true;
 }
 
-void launch_spd_inverse_r(const RankLayout& L, int nrank, int nr_max, double* dense, double tol, int* nnull,
+bool launch_spd_inverse_r(const RankLayout& L, int nrank, int nr_max, double* dense, double tol, int* nnull,
                           cudaStream_t st) {
-  gj_inverse(nrank, GjShape{L.first, L.off2, nr_max, L.kmax}, dense, tol, nnull, st);
+  return gj_inverse(nrank, GjShape{L.first, L.off2, nr_max, L.kmax}, dense, tol, nnull, st);
 }
 
 void launch_spd_inverse(int nb, int n, double* a, double tol, int* nnull, cudaStream_t st) {
@@ -1052,9 +1052,12 @@ __global__ void k_l3_init(RankLayout L, int p, const double* A_all, double* work
   }
 }
 
-// Out = M In (REFINE: X - M In), blocks src / dst of the rank's workspace (0 X, 1 Y, 2 R or A Y).  Lane (r, q) of a warp holds of
-// row r the entries k0 + 4 q + t, t < 4, of each 16: whole 128-byte row segments per load, used as the A
-// fragments of four k-steps (the order of k within a dot product is free as long as B follows it).
+// Out = M In (REFINE: X - M In), blocks src / dst of the rank's workspace (0 X,
+// 1 Y, 2 R or A Y).  Lane (r, q) of a warp holds of row r the entries k0 + 4 q + t,
+// t < 4, of each 16: whole 128-byte row segments per load, used as the A fragments
+// of four k-steps (the order of k within a dot product is free as long as B follows
+// it).  m16n8k4 products, here and in the inverses, measured the same: neither
+// kernel is bound by the tensor cores.
 template <bool REFINE>
 __global__ void __launch_bounds__(128) k_l3_mm(RankLayout L, int p, const double* M_all, double* work_all, int src,
                                                int dst, const L3Rank* st) {

@@ -213,8 +213,8 @@ void launch_assemble_dense_r(const SubInfo* subs, int nrank, const RankLayout& L
                              const double* gface, int mode, double* dense, cudaStream_t st);
 // dense[r] += mu (relative != 0: mu x max |diag| of the block) on the diagonal, one CTA per rank
 void launch_add_diag_r(const RankLayout& L, int nrank, double* dense, double mu, int relative, cudaStream_t st);
-// Gauss-Jordan inverses of the ragged blocks (the multi-CTA form of launch_spd_inverse)
-void launch_spd_inverse_r(const RankLayout& L, int nrank, int nr_max, double* dense, double tol, int* nnull,
+// Gauss-Jordan inverses of the ragged blocks (false: no room for the scratch, nothing done)
+bool launch_spd_inverse_r(const RankLayout& L, int nrank, int nr_max, double* dense, double tol, int* nnull,
                           cudaStream_t st);
 void launch_axpy(long long n, double a, const double* x, double* y, const int* done, cudaStream_t st);
 void launch_copy(long long n, const double* x, double* y, const int* done, cudaStream_t st);

@@ -1318,18 +1318,22 @@ int Solver::setup() {
     return finish();
   }
   launch_assemble_dense_r(d_subs, nrank, rl, tot2, blk, gface, 0, A2inv, st);
-  if (ragged)
-    launch_spd_inverse_r(rl, nrank, nr, A2inv, 1e-14, d_flag + 1, st);
-  else
+  auto no_scratch = [&]() {
+    err = "not enough device memory for the scratch of the coarse inverses";
+    return 76;
+  };
+  if (ragged) {
+    if (!launch_spd_inverse_r(rl, nrank, nr, A2inv, 1e-14, d_flag + 1, st)) return no_scratch();
+  } else
     launch_spd_inverse(nrank, nr, A2inv, 1e-14, d_flag + 1, st);
   cudaEventRecord(e[3], st);
   // level 3: rank-Neumann HEP
   launch_assemble_dense_r(d_subs, nrank, rl, tot2, blk, gface, 1, AN, st);
   cudaMemcpyAsync(ANinv, AN, sizeof(double) * tot2, cudaMemcpyDeviceToDevice, st);
   launch_add_diag_r(rl, nrank, ANinv, 1e-8, 1, st);
-  if (ragged)
-    launch_spd_inverse_r(rl, nrank, nr, ANinv, 1e-14, d_flag + 2, st);
-  else
+  if (ragged) {
+    if (!launch_spd_inverse_r(rl, nrank, nr, ANinv, 1e-14, d_flag + 2, st)) return no_scratch();
+  } else
     launch_spd_inverse(nrank, nr, ANinv, 1e-14, d_flag + 2, st);
   if (!l3work) {
     if (int er = check(cudaMalloc(&l3work, sizeof(double) * totw), "cudaMalloc l3 work")) return er;

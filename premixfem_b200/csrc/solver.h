@@ -35,7 +35,7 @@ struct Options {
   double l3_tol = 1e-10;
   unsigned long long seed = 20240611ull;
   int pcg_chunk = 4;
-  int pcg_graph = 1;  // replay each chunk of PCG iterations as one CUDA graph
+  int pcg_graph = 1;  // PCG iterations as one CUDA graph that repeats itself
   int eig_final = 1;  // batched eigensolver: final Rayleigh-Ritz and output as phase kernels (0: one persistent launch)
   double eig_rel_floor = 0.0;  // > 0: eigen residual test relative to max(|lambda|, floor x lscale)
   int eig_init = 0;   // batched eigensolver: 1 = set-up as phase kernels, 0 = one persistent launch
