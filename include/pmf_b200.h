@@ -59,9 +59,10 @@ typedef struct pmf_solver pmf_solver;
  * test, instead of tol x lscale with lscale = max diag(A_N)/M; experimental,
  * off by default),
  * -pmf_eig_profile 1 (per-phase timing, pmf_get_eig_phases), -pmf_pcg_graph
- * 0|1 (PCG iterations replayed as CUDA graphs, on by default), -pmf_autotune
+ * 0|1 (PCG iterations as a CUDA graph that repeats itself, on by default), -pmf_autotune
  * 0|1 (launch-shape tuning, on by default; pmf_tune_report), -pmf_lv1_kernel
- * auto|natural|blocked|staged (level-1 solve kernel: the tuner's choice, the
+ * auto|natural|blocked|staged (level-1 solve kernel: the tuner's choice, which
+ * also tries one warp per subdomain where ny <= 32 and nx >= 4, the
  * natural-order kernel, the kernel that stages each subdomain's IC(0) factor
  * with one TMA bulk copy, which needs every subdomain 16 cells wide in x with
  * x0 and M multiples of 4, or that kernel with all of its other global loads
