@@ -282,11 +282,11 @@ __device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double
                : "+d"(d0), "+d"(d1)
                : "d"(a), "d"(b));
 }
-// Two such products with the same B: rows 0-7 of A(16x4) in a0, 8-15 in a1, of D in d[0..1] and d[2..3].  One
+// Two such products with the same B: rows 0-7 of A(16x4) in a0, 8-15 in a1, of D in d0 and d1.  One
 // m16n8k4 takes the time of one m8n8k4 (73.7 against 36.8 TFLOP/s), so the kernels pair row tiles where they can.
-__device__ __forceinline__ void dmma1684(double (&d)[4], double a0, double a1, double b) {
+__device__ __forceinline__ void dmma1684(double (&d0)[2], double (&d1)[2], double a0, double a1, double b) {
   asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
-               : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+               : "+d"(d0[0]), "+d"(d0[1]), "+d"(d1[0]), "+d"(d1[1])
                : "d"(a0), "d"(a1), "d"(b));
 }
 
@@ -334,21 +334,18 @@ __device__ __forceinline__ void stv(double* p, const double (&v)[N]) {
 // (column of S / AS), with no shared-memory staging.  (One value per lane and load,
 // four lanes to a 32-byte sector, kept the L1 busy with eight lines per request.)
 // Columns are readable to a multiple of 64 cells, and what lies past ncells is
-// masked.  Both Grams are symmetric: column tile t is multiplied with the row
-// tiles t and t + 1 (mod NT), which for NT = 3 are the six tiles of a triangle in
-// three instructions.  The per-warp partial tiles are reduced in a fixed order
+// masked.  Both Grams are symmetric: only the row tiles up to the column tile's own
+// are accumulated, two per instruction.  It has to be that triangle: its images are
+// those of the later columns, AW's and not AX's, which in FP64 storage are updated
+// from iteration to iteration and drift.  The per-warp partial tiles are reduced in a fixed order
 // through shared memory, so the result is deterministic.  red: >= 8 * 32 * 32
 // doubles.
 //
 // Bound by HBM where many subdomains iterate (per cell and column a value and an
 // FP64 image): all Grams of a 256^3 set-up take 26.9 ms (36.0 with one value per
 // load and one tile per product; their bytes need 17), of one with blocks of ten
-// columns 30.6 (67.8).  Loading a step ahead in halves of the step costs more than
+// columns 31.4 (67.8).  Loading a step ahead in halves of the step costs more than
 // it hides (34.1).
-template <int NT>
-__device__ __forceinline__ bool gram_has(int ta, int tb) {
-  return ta == tb || (NT == 2 && ta == 1) || (NT >= 3 && ta == (tb + 1) % NT) || (NT == 4 && tb == ta + 2);
-}
 template <typename TS, typename TA, int NT>
 __device__ __noinline__ void cta_gram2_mma(const Seg3<TS> S, const Seg3<TA> AS, const double* wgt, int ncells,
                                            double* GM, double* GA, double* red) {
@@ -364,14 +361,10 @@ __device__ __noinline__ void cta_gram2_mma(const Seg3<TS> S, const Seg3<TA> AS, 
     sp[ta] = a < ns ? S.col(a) + C * cq : nullptr;
     ap[ta] = a < ns ? AS.col(a) + C * cq : nullptr;
   }
-  double cm[NT][4], ca[NT][4];  // column tile t: rows t (0, 1) and t + 1 (2, 3)
-  double em[2][2], ea[2][2];    // NT = 4: tiles (0, 2) and (1, 3)
+  constexpr int NP = NT * (NT + 1) / 2;
+  double cm[NP][2], ca[NP][2];  // tile (ta, tb), ta <= tb, at tb (tb + 1) / 2 + ta
 #pragma unroll
-  for (int t = 0; t < NT; ++t)
-#pragma unroll
-    for (int h = 0; h < 4; ++h) cm[t][h] = ca[t][h] = 0.0;
-#pragma unroll
-  for (int t = 0; t < 2; ++t) em[t][0] = em[t][1] = ea[t][0] = ea[t][1] = 0.0;
+  for (int p = 0; p < NP; ++p) cm[p][0] = cm[p][1] = ca[p][0] = ca[p][1] = 0.0;
   for (int c0 = 4 * C * w; c0 < ncells; c0 += 4 * C * nwarp) {
     TS sv[NT][C];
     TA av[NT][C];
@@ -410,20 +403,18 @@ __device__ __noinline__ void cta_gram2_mma(const Seg3<TS> S, const Seg3<TA> AS, 
         cw[t] = cs[t] * wv[q];
       }
 #pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        if (NT >= 3 || (NT == 2 && t == 0)) {
-          dmma1684(cm[t], cw[t], cw[(t + 1) % NT], cs[t]);
-          dmma1684(ca[t], cs[t], cs[(t + 1) % NT], (double)av[t][q]);
-        } else {
-          dmma884(cm[t][0], cm[t][1], cw[t], cs[t]);
-          dmma884(ca[t][0], ca[t][1], cs[t], (double)av[t][q]);
-        }
-      }
-      if (NT == 4) {
+      for (int tb = 0; tb < NT; ++tb) {
+        const double ab = (double)av[tb][q];
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          dmma884(em[t][0], em[t][1], cw[t], cs[(t + 2) % NT]);
-          dmma884(ea[t][0], ea[t][1], cs[t], (double)av[(t + 2) % NT][q]);
+        for (int ta = 0; ta <= tb; ta += 2) {
+          const int p = tb * (tb + 1) / 2 + ta;
+          if (ta < tb) {
+            dmma1684(cm[p], cm[p + 1], cw[ta], cw[ta + 1], cs[tb]);
+            dmma1684(ca[p], ca[p + 1], cs[ta], cs[ta + 1], ab);
+          } else {
+            dmma884(cm[p][0], cm[p][1], cw[ta], cs[tb]);
+            dmma884(ca[p][0], ca[p][1], cs[ta], ab);
+          }
         }
       }
     }
@@ -432,22 +423,20 @@ __device__ __noinline__ void cta_gram2_mma(const Seg3<TS> S, const Seg3<TA> AS, 
 #pragma unroll 1
   for (int which = 0; which < 2; ++which) {
     __syncthreads();
-    auto put = [&](int ta, int tb, double d0, double d1) {
-      double* o = red + (w * 32 + 8 * ta + r) * 32 + 8 * tb + 2 * cq;
-      o[0] = d0;
-      o[1] = d1;
-    };
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      put(t, t, which ? ca[t][0] : cm[t][0], which ? ca[t][1] : cm[t][1]);
-      if (NT >= 3 || (NT == 2 && t == 0)) put((t + 1) % NT, t, which ? ca[t][2] : cm[t][2], which ? ca[t][3] : cm[t][3]);
-      if (NT == 4 && t < 2) put(t, t + 2, which ? ea[t & 1][0] : em[t & 1][0], which ? ea[t & 1][1] : em[t & 1][1]);
-    }
+    for (int tb = 0; tb < NT; ++tb)
+#pragma unroll
+      for (int ta = 0; ta <= tb; ++ta) {
+        const int p = tb * (tb + 1) / 2 + ta;
+        double* o = red + (w * 32 + 8 * ta + r) * 32 + 8 * tb + 2 * cq;
+        o[0] = which ? ca[p][0] : cm[p][0];
+        o[1] = which ? ca[p][1] : cm[p][1];
+      }
     __syncthreads();
     double* G = which ? GA : GM;
     for (int e = threadIdx.x; e < ns * ns; e += blockDim.x) {
       int a = e / ns, b = e % ns;
-      if (!gram_has<NT>(a >> 3, b >> 3)) {  // the mirror of an accumulated tile
+      if ((a >> 3) > (b >> 3)) {  // below the accumulated block triangle: the mirror
         const int x = a;
         a = b;
         b = x;
@@ -520,16 +509,14 @@ __device__ __noinline__ void cta_update_mma(T* B0, T* B1, T* B2, int m0, int n1,
     if (c0 + step < ncells) load(c0 + step);
 #pragma unroll
     for (int tj = 0; tj < NJ; ++tj) {
-      double d[V][4];
+      double d0[V][2], d1[V][2];  // the tiles' halves: B0 and B2
 #pragma unroll
-      for (int t = 0; t < V; ++t)
-#pragma unroll
-        for (int h = 0; h < 4; ++h) d[t][h] = 0.0;
+      for (int t = 0; t < V; ++t) d0[t][0] = d0[t][1] = d1[t][0] = d1[t][1] = 0.0;
 #pragma unroll
       for (int kk = 0; kk < NK; ++kk) {
         const double y = NJ == 1 ? y0[kk] : yfrag(kk, tj), yp = 4 * kk + cq >= m0 ? y : 0.0;
 #pragma unroll
-        for (int t = 0; t < V; ++t) dmma1684(d[t], y, yp, (double)cu[kk][t]);
+        for (int t = 0; t < V; ++t) dmma1684(d0[t], d1[t], y, yp, (double)cu[kk][t]);
       }
       const int j = 8 * tj + r;
       if (j < m) {
@@ -539,7 +526,7 @@ __device__ __noinline__ void cta_update_mma(T* B0, T* B1, T* B2, int m0, int n1,
           T* o = (h >> 1 ? B2 : B0) + (size_t)j * ld + cell;
           double v[V];
 #pragma unroll
-          for (int t = 0; t < V; ++t) v[t] = d[t][h];
+          for (int t = 0; t < V; ++t) v[t] = h >> 1 ? d1[t][h & 1] : d0[t][h & 1];
           if (cell + V <= ncells) {
             stv<V>(o, v);
           } else {
