@@ -15,8 +15,9 @@
 // tensor cores (mma.sync m16n8k4), the projected eigenproblem by Householder
 // tridiagonalisation and multisection.  Converged vectors are soft-locked.
 // X, W, P are stored in T (float for the mixed-precision setup, double for
-// the plain form); their A-images are always FP64, so the projection stays
-// consistent without recomputation.  A final FP64 Rayleigh-Ritz fixes the
+// the plain form); their A-images are always FP64, and the phase-batched form
+// computes them from the stored vectors in every iteration (the persistent one in
+// FP32 storage only).  A final FP64 Rayleigh-Ritz fixes the
 // returned eigenvalues and the normalisation v^T M v = 1 (the GHEP
 // normalisation SLEPc returns).
 #include <algorithm>
@@ -335,11 +336,9 @@ __device__ __forceinline__ void stv(double* p, const double (&v)[N]) {
 // four lanes to a 32-byte sector, kept the L1 busy with eight lines per request.)
 // Columns are readable to a multiple of 64 cells, and what lies past ncells is
 // masked.  Both Grams are symmetric: only the row tiles up to the column tile's own
-// are accumulated, two per instruction.  It has to be that triangle: its images are
-// those of the later columns, AW's and not AX's, which in FP64 storage are updated
-// from iteration to iteration and drift.  The per-warp partial tiles are reduced in a fixed order
-// through shared memory, so the result is deterministic.  red: >= 8 * 32 * 32
-// doubles.
+// are accumulated, two per instruction.  The per-warp partial tiles are reduced in a
+// fixed order through shared memory, so the result is deterministic.  red: >= 8 * 32
+// * 32 doubles.
 //
 // Bound by HBM where many subdomains iterate (per cell and column a value and an
 // FP64 image): all Grams of a 256^3 set-up take 26.9 ms (36.0 with one value per
@@ -1364,14 +1363,15 @@ struct EbArgs {
 // Phase kernels index the compacted active list; the control kernel the full list.
 __device__ __forceinline__ int eb_sub(const EbArgs& a, int idx) { return a.alist[idx]; }
 
-// Partial ||AX_j - lambda_j M X_j||^2_{M^-1} over one chunk of cells.
+// Partial ||AX_j - lambda_j M X_j||^2_{M^-1} over one chunk of cells: the first
+// iteration's, whose A X the set-up formed.
 // All m columns at once: a full chunk gives each thread four consecutive cells
 // (vector loads, every column's loads in flight together); the per-column
 // sums are reduced per warp by shuffles and across the warps in a fixed order.
 template <typename T>
-__global__ void __launch_bounds__(256) k_eb_resid(EbArgs a, int use_alist) {
+__global__ void __launch_bounds__(256) k_eb_resid(EbArgs a) {
   __shared__ double red[32][LB_MM];
-  const int s = use_alist ? a.alist[blockIdx.y] : (a.list ? a.list[blockIdx.y] : (int)blockIdx.y);
+  const int s = a.list ? a.list[blockIdx.y] : (int)blockIdx.y;
   const EbState& es = a.state[s];
   if (es.done) return;
   const SubInfo S = a.subs[s];
@@ -1610,9 +1610,19 @@ __global__ void __launch_bounds__(256) k_eb_aimg(EbArgs a) {
                     S.nx * S.ny * S.nz);
 }
 
-// FP32 storage: AX = A X and AP = A P with the FP32-rounded couplings, and the
-// partial residual norms ||AX_j - lambda_j M X_j||^2_{M^-1} of the next iteration's
-// convergence test while AX is at hand.
+// AX = A X and AP = A P, with the FP64 operator in FP64 storage and the FP32-rounded
+// couplings in FP32 storage, and the partial residual norms ||AX_j - lambda_j M
+// X_j||^2_{M^-1} of the next iteration's convergence test while AX is at hand.
+//
+// The images are computed from the stored vectors in every iteration, never combined
+// with the vectors' coefficients: a direction of P is a difference that shrinks to
+// rounding as its vector converges, and what is left of a combined image then does not
+// belong to what is left of the direction.  Scaled to unit norm in the Rayleigh-Ritz
+// step such a pair has an arbitrary Ritz value.  (With combined images in FP64 storage,
+// 42 of 7 776 subdomains of 16..216 cells had wrong eigenvalues at the iteration limit,
+// 39 of them of 32 cells with blocks of ten; computed, none, in 22 iterations at most.
+// The layered field of 60 x 220 x 85 cells, 15 seeds: 1 to 8 subdomains at the limit
+// instead of 4 to 18.)
 //
 // A CTA takes two columns of X and of P over the whole subdomain, a thread the
 // cells above one (x, y) place, marching in z: the four columns share a cell's
@@ -1621,8 +1631,11 @@ __global__ void __launch_bounds__(256) k_eb_aimg(EbArgs a) {
 // per result at sixteen per clock and SM, this 6.25.  All images and residual norms
 // of a 256^3 set-up: 29.1 ms instead of 46.9 (their bytes need 13); with a chunk of
 // cells and all columns per CTA, couplings widened once, the planes of sixteen
-// columns do not stay in L1: 44.5.
+// columns do not stay in L1: 44.5.  In FP64 storage at 150^3 this, the update and the
+// control step take 24.5 ms, 24.8 with the images combined and the residuals apart.
+template <typename T>
 __global__ void __launch_bounds__(256) k_eb_aimg_resid(EbArgs a) {
+  constexpr bool F32 = sizeof(T) == 4;
   __shared__ double red[8][2];
   const int s = eb_sub(a, blockIdx.y);
   const EbState& es = a.state[s];
@@ -1630,20 +1643,32 @@ __global__ void __launch_bounds__(256) k_eb_aimg_resid(EbArgs a) {
   const SubInfo S = a.subs[s];
   const int nx = S.nx, ny = S.ny, nz = S.nz, nxny = nx * ny;
   const int ld = a.ld, m = a.m, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  EbSlab<float> sl(a.slab + (size_t)s * a.slab_stride, m, ld);
+  EbSlab<T> sl(a.slab + (size_t)s * a.slab_stride, m, ld);
   const int ja = 2 * blockIdx.x, jb = min(ja + 1, m - 1);  // odd m: the last column twice
-  const float* __restrict__ v[4] = {sl.X + (size_t)ja * ld, sl.X + (size_t)jb * ld, sl.P + (size_t)ja * ld,
-                                    sl.P + (size_t)jb * ld};
+  const T* __restrict__ v[4] = {sl.X + (size_t)ja * ld, sl.X + (size_t)jb * ld, sl.P + (size_t)ja * ld,
+                                sl.P + (size_t)jb * ld};
   double* __restrict__ o[4] = {sl.AX + (size_t)ja * ld, sl.AX + (size_t)jb * ld, sl.AP + (size_t)ja * ld,
                                sl.AP + (size_t)jb * ld};
-  const float *__restrict__ ctx = sl.ctx, *__restrict__ cty = sl.cty, *__restrict__ ctz = sl.ctz;
-  const double *__restrict__ dN = sl.dN32, *__restrict__ Md = sl.Md;
+  // couplings: the slab's (natural order of the subdomain) or the mesh's, from the subdomain's first cell on
+  const long long g0 = ((long long)S.z0 * a.g.N + S.y0) * a.g.M + S.x0;
+  const T *__restrict__ ctx, *__restrict__ cty, *__restrict__ ctz;
+  if constexpr (F32) {
+    ctx = sl.ctx;
+    cty = sl.cty;
+    ctz = sl.ctz;
+  } else {
+    ctx = a.tx + g0;
+    cty = a.ty + g0;
+    ctz = a.tz + g0;
+  }
+  const int sy = F32 ? nx : a.g.M, sz = F32 ? nxny : a.g.M * a.g.N;  // their strides in y and z
+  const double *__restrict__ dN = F32 ? sl.dN32 : sl.dN, *__restrict__ Md = sl.Md;
   const double lam[2] = {es.lam[ja], es.lam[jb]};
   double acc[2] = {0.0, 0.0};
   for (int p = threadIdx.x; p < nxny; p += blockDim.x) {
     const int j = p / nx, i = p - j * nx;
     const bool xm = i > 0, xp = i < nx - 1, ym = j > 0, yp = j < ny - 1;
-    const int ixm = xm ? -1 : 0, ixp = xp ? 1 : 0, iym = ym ? -nx : 0, iyp = yp ? nx : 0;
+    const int ixm = xm ? -1 : 0, ixp = xp ? 1 : 0, iym = ym ? -nx : 0, iyp = yp ? nx : 0, cyo = yp ? sy : 0;
     double um[4], uc[4], czm = 0.0;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -1651,10 +1676,10 @@ __global__ void __launch_bounds__(256) k_eb_aimg_resid(EbArgs a) {
       uc[q] = (double)v[q][p];
     }
 #pragma unroll 1
-    for (int k = 0, cl = p; k < nz; ++k, cl += nxny) {
+    for (int k = 0, cl = p, cg = j * sy + i; k < nz; ++k, cl += nxny, cg += sz) {
       const bool zp = k < nz - 1;
       const int up = zp ? cl + nxny : cl;
-      float n[4][5];
+      T n[4][5];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         n[q][0] = v[q][cl + ixm];
@@ -1663,7 +1688,7 @@ __global__ void __launch_bounds__(256) k_eb_aimg_resid(EbArgs a) {
         n[q][3] = v[q][cl + iyp];
         n[q][4] = v[q][up];
       }
-      const float fxm = ctx[cl], fxp = ctx[cl + ixp], fym = cty[cl], fyp = cty[cl + iyp], fzp = ctz[up];
+      const T fxm = ctx[cg], fxp = ctx[cg + ixp], fym = cty[cg], fyp = cty[cg + cyo], fzp = ctz[zp ? cg + sz : cg];
       const double d = dN[cl], md = Md[cl], imd = 1.0 / md;
       const double cxm = xm ? (double)fxm : 0.0, cxp = xp ? (double)fxp : 0.0, cym = ym ? (double)fym : 0.0,
                    cyp = yp ? (double)fyp : 0.0, czp = zp ? (double)fzp : 0.0;
@@ -1770,7 +1795,7 @@ static void launch_eb_rr(const EbArgs& e, int nact, double drop, cudaStream_t st
     k_eb_rr<32, 10><<<nact, 32, 0, st>>>(e, drop);
 }
 
-// X <- S Y, P <- [W P] Y_WP (and the FP64 A-images in FP64 storage), per chunk.
+// X <- S Y, P <- [W P] Y_WP, per chunk (their images: k_eb_aimg_resid).
 // NK / NJ: k-steps and 8-column tiles of the tensor-core update (6 / 1 for m <= 8).
 template <typename T, int NK, int NJ>
 __global__ void __launch_bounds__(256, 2) k_eb_update(EbArgs a) {
@@ -1789,8 +1814,6 @@ __global__ void __launch_bounds__(256, 2) k_eb_update(EbArgs a) {
   EbSlab<T> sl(a.slab + (size_t)s * a.slab_stride, a.m, a.ld);
   const int m = a.m;
   cta_update_mma<T, NK, NJ>(sl.X + c0, sl.W + c0, sl.P + c0, m, es.nact, es.np, m, Ys, cn, a.ld);
-  if (sizeof(T) == 8)
-    cta_update_mma<double, NK, NJ>(sl.AX + c0, sl.AW + c0, sl.AP + c0, m, es.nact, es.np, m, Ys, cn, a.ld);
 }
 
 // ---- final phase (k_lobpcg mode 2 as phase kernels over every subdomain of
@@ -2286,10 +2309,10 @@ int launch_lobpcg_batched(const LobpcgArgs& a_in, const EbBuffers& b, const int*
   for (int it = 0; it < a.max_it; ++it) {
     // residual norms of the subdomains still iterating (all of them at it = 0)
     mark(1);
-    // (FP32 storage: formed with the A-images of the iteration before, except at the start)
-    if (sizeof(T) == 8 || it == 0) {
+    // (formed with the A-images of the iteration before, except at the start)
+    if (it == 0) {
       note_launch();
-      k_eb_resid<T><<<dim3(e.nchunk, nact), 256, 0, st>>>(e, it > 0 ? 1 : 0);
+      k_eb_resid<T><<<dim3(e.nchunk, nact), 256, 0, st>>>(e);
     }
     cudaMemsetAsync(b.nactive, 0, 3 * sizeof(int), st);
     { note_launch(); k_eb_control<<<(nlist + 127) / 128, 128, 0, st>>>(e, nlist, it); }
@@ -2328,10 +2351,7 @@ int launch_lobpcg_batched(const LobpcgArgs& a_in, const EbBuffers& b, const int*
     prev_pc = pc;
     prev_cols = b.h_nactive[1];
     mark(6);
-    if (sizeof(T) == 4) {
-      note_launch();
-      k_eb_aimg_resid<<<dim3((a.m + 1) / 2, nact), aimg_threads, 0, st>>>(e);
-    }
+    { note_launch(); k_eb_aimg_resid<T><<<dim3((a.m + 1) / 2, nact), aimg_threads, 0, st>>>(e); }
     mark(7);
     if (prof) {
       cudaEventSynchronize(pev[7]);

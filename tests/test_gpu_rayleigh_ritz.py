@@ -53,3 +53,23 @@ def test_basis_wider_than_the_space(native, tile, k):
         err = np.abs(ev - ref) / np.maximum(np.abs(ref), 1e-3 * scale)
         assert (status != 1).all()
         assert err.max() <= 1e-6, f"max rel eigen error {err.max():.2e}"
+
+
+@pytest.mark.parametrize("tile,k", [((3, 3, 3), 6), ((5, 3, 2), 6), ((4, 4, 2), 8), ((3, 3, 4), 8)],
+                         ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else str(v))
+def test_images_belong_to_the_block(native, tile, k):
+    """Blocks whose basis takes nearly all of the space: search directions shrink to rounding, and an image that is
+    carried along with them instead of computed from them no longer belongs to its vector; the Ritz values are then
+    wrong and the block stops converging.  216 subdomains; the bars of the tests above."""
+    for seed in range(8):
+        prob = fields.random_box(tuple(3 * n for n in tile), seed=seed, sigma=[0.5, 1.5, 3.0, 4.0][seed % 4])
+        s = DarcySolver.from_problem(prob, options_string({"sd": 3, "en_lv1": k, "en_lv2": 2}))
+        s.setup()
+        ev, _, _, status = s.eigen_lv1()
+        boxes, _ = s.subdomains()
+        s.close()
+        ref = O.local_eigenvalues(prob, [tuple(b) for b in boxes], k, method="dense")
+        scale = np.abs(ref).max(axis=1, keepdims=True)
+        err = np.abs(ev - ref) / np.maximum(np.abs(ref), 1e-3 * scale)
+        assert (status != 1).all()
+        assert err.max() <= 1e-6, f"max rel eigen error {err.max():.2e}"
