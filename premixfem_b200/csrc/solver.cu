@@ -448,7 +448,7 @@ Solver::~Solver() {
   if (ev1) cudaEventDestroy(ev1);
   for (auto& e : prof_ev)
     if (e) cudaEventDestroy(e);
-  for (void* q : {(void*)d_coff, ic_coef, (void*)d_woff, ic_wcoef, rt, (void*)r32, (void*)d_kerr, (void*)phi64,
+  for (void* q : {(void*)d_coff, ic_coef, (void*)d_woff, ic_wcoef, (void*)r32, (void*)d_kerr, (void*)phi64,
                   (void*)d_rl_first, (void*)d_rl_off, (void*)d_rl_dof_rank, (void*)d_rl_chunk, (void*)d_rl_chunks,
                   (void*)d_probs, (void*)d_layer_prob})
     if (q) cudaFree(q);
@@ -749,7 +749,6 @@ int Solver::alloc_fine() {
                          {(void**)&z, n * 8, "z"},        {(void**)&p0, n * 8, "p0"},
                          {(void**)&p1, n * 8, "p1"},      {(void**)&w, n * 8, "w"},
                          {(void**)&y0, n * pb, "y0"},     {(void**)&y1, n * pb, "y1"},
-                         {&rt, n * pb, "rt"},
                          {(void**)&phi, n * kmax * pb, "phi"},
                          {(void**)&part, (size_t)(nparts + cell_blocks(g.ncell)) * 8, "part"},
                          {(void**)&state, sizeof(PcgState), "state"}};
@@ -1077,7 +1076,8 @@ int Solver::setup() {
   }
   if (!opt.use_full_Cholesky_lv1) {
     if (int er = setup_ic_blocked(mixed)) return er;
-    if (int er = setup_ic_warp(mixed)) return er;
+    check_ic_warp(mixed);
+    if (ic_wcoef) pack_ic_warp(mixed);  // kept from a set-up before
     if (opt.lv1_kernel == 2 && !ic_blk_ok) {
       err = "-pmf_lv1_kernel blocked needs every subdomain 16 cells wide in x with x0 % 4 == 0, M % 4 == 0 and "
             "ny*nz <= 256";
@@ -1514,42 +1514,64 @@ int Solver::setup_ic_blocked(bool mixed) {
   return 0;
 }
 
-// The step-ordered copy of the IC(0) factor for k_ic_warp, rebuilt by every
-// set-up, unless another kernel is forced by option.
-int Solver::setup_ic_warp(bool mixed) {
+// Whether k_ic_warp is a candidate: it needs ny <= 32 and nx >= 4, and its factor's
+// step order fills out idle lanes.  It is offered up to four entries per cell: 2 million
+// cells in subdomains that give 4.9, 5.1 and 9.5 took 36 to 103 us a visit against 34
+// to 48 of the natural-order kernel, those that give 1.4 to 3.8 15 to 60 against 16 to 77.
+void Solver::check_ic_warp(bool mixed) {
+  ic_wrp_packed = false;
   ic_wrp_ok = opt.lv1_kernel == 0;
   ic_wrp_smem = ic_wrp_face = 0;
+  long long entries = 0;
   for (const SubInfo& S : subs) {
     if (S.ny > 32 || S.nx < 4) ic_wrp_ok = false;
-    if (!ic_wrp_ok) return 0;
+    if (!ic_wrp_ok) return;
     ic_wrp_smem = std::max(ic_wrp_smem, ic_warp_smem_len(S.nx, S.ny, S.nz));
     ic_wrp_face = std::max(ic_wrp_face, S.nx * S.ny);
+    entries += ic_warp_coef_len(S.nx, S.ny, S.nz);
   }
-  const size_t tb = mixed ? 4 : 8;
-  if (ic_warp_smem_bytes(ic_wrp_smem, ic_wrp_face, (int)tb) > 227 * 1024) ic_wrp_ok = false;
-  if (!ic_wrp_ok) return 0;
-  if (!d_woff) {
+  if (entries > 4 * (long long)g.ncell) ic_wrp_ok = false;
+  if (ic_warp_smem_bytes(ic_wrp_smem, ic_wrp_face, mixed ? 4 : 8) > 227 * 1024) ic_wrp_ok = false;
+}
+
+// The step-ordered copy of this set-up's IC(0) factor for k_ic_warp, made when the
+// tuner times that kernel or has chosen it (false: no room for it, another kernel
+// runs) and given back where neither visit kind takes it.
+bool Solver::pack_ic_warp(bool mixed) {
+  if (!ic_wrp_ok) return false;
+  if (ic_wrp_packed) return true;
+  if (!ic_wcoef) {
     std::vector<long long> off(nsub);
     long long acc = 0;
     for (int s = 0; s < nsub; ++s) {
       off[s] = acc;
       acc += ic_warp_coef_len(subs[s].nx, subs[s].ny, subs[s].nz);
     }
-    if (int e = dalloc((void**)&d_woff, sizeof(long long) * nsub, "step-ordered factor offsets")) return e;
-    if (int e = dalloc(&ic_wcoef, (size_t)acc * 4 * tb, "step-ordered IC(0) factor")) {
-      cudaFree(d_woff);
-      d_woff = nullptr;
-      return e;
+    if (dalloc((void**)&d_woff, sizeof(long long) * nsub, "step-ordered factor offsets") ||
+        dalloc(&ic_wcoef, (size_t)acc * 4 * (mixed ? 4 : 8), "step-ordered IC(0) factor")) {
+      err.clear();
+      free_ic_warp();
+      return false;
     }
     cudaMemcpyAsync(d_woff, off.data(), sizeof(long long) * nsub, cudaMemcpyHostToDevice, st);
     // the host vector must outlive the asynchronous copy
-    if (int e = check(cudaStreamSynchronize(st), "step-ordered factor offsets")) return e;
+    if (cudaStreamSynchronize(st) != cudaSuccess) return false;
   }
   if (mixed)
     launch_pack_ic_warp<float>(g, d_subs, nsub, d_woff, tx32, ty32, tz32, inv32, ic_wcoef, st);
   else
     launch_pack_ic_warp<double>(g, d_subs, nsub, d_woff, tx, ty, tz, inv64, ic_wcoef, st);
-  return 0;
+  ic_wrp_packed = true;
+  return true;
+}
+
+void Solver::free_ic_warp() {
+  if (ic_wcoef) drop_graphs();
+  cudaFree(d_woff);
+  cudaFree(ic_wcoef);
+  d_woff = nullptr;
+  ic_wcoef = nullptr;
+  ic_wrp_packed = false;
 }
 
 // A bounded wait inside a kernel ran out (the kernel recorded it and returned
@@ -1575,9 +1597,9 @@ void Solver::launch_lv1(const double* x, const T* xt, const T* yin, T* out_t, do
   const T* ttz = f32 ? (const T*)tz32 : (const T*)tz;
   const T* tdg = f32 ? (const T*)diag32 : (const T*)diag;
   const int kind = yin ? 1 : 0;
-  if (ic_variant[kind] == 3 && ic_wrp_ok) {
+  if (ic_variant[kind] == 3 && ic_wrp_packed) {
     launch_ic_warp<T>(g, d_subs, nsub, ic_wrp_smem, ic_wrp_face, d_woff, ic_wcoef, ttx, tty, ttz, tdg, x, xt, yin,
-                      (T*)rt, out_t, out_d, partial, done, st);
+                      (T*)w, out_t, out_d, partial, done, st);
   } else if (ic_variant[kind] == 2 && ic_stg_ok) {
     launch_ic_apply_stg<T>(g, d_subs, nsub, max_cells, d_coff, ic_coef, ttx, tty, ttz, tdg, x, yin, out_t, out_d,
                            partial, done, d_kerr, st);
@@ -1655,9 +1677,11 @@ void Solver::tune_pc() {
         else if (v == 2)
           launch_ic_apply_stg<T>(g, d_subs, nsub, max_cells, d_coff, ic_coef, ttx, tty, ttz, tdg, z, yi, o_t, o_d, o_p,
                                  nullptr, d_kerr, st);
-        else
+        else if (pack_ic_warp(f32))
           launch_ic_warp<T>(g, d_subs, nsub, ic_wrp_smem, ic_wrp_face, d_woff, ic_wcoef, ttx, tty, ttz, tdg, z, zt, yi,
-                            (T*)rt, o_t, o_d, o_p, nullptr, st);
+                            (T*)w, o_t, o_d, o_p, nullptr, st);
+        else
+          return false;
         return true;
       }, st);
       ic_variant[kind] = follow ? ic_variant[1] : variant(ci);
@@ -1665,6 +1689,10 @@ void Solver::tune_pc() {
       if (kind == 1) ic_threads = cand[std::min(ci, nnat - 1)];
       if (opt.lv1_kernel > 0) ic_variant[kind] = opt.lv1_kernel - 1;  // eligibility checked by setup()
     }
+    if ((ic_variant[0] == 3 || ic_variant[1] == 3) && !pack_ic_warp(f32))
+      for (int& v : ic_variant)
+        if (v == 3) v = ic_blk_ok ? 1 : 0;  // chosen before, no room now
+    if (ic_variant[0] != 3 && ic_variant[1] != 3) free_ic_warp();
   }
   const int rcand[3] = {256, 128, 512};
   snprintf(key, sizeof(key), "resid_restrict|%s|n%d|c%d|k%d", prec, nsub, max_cells, kmax);

@@ -216,13 +216,15 @@ class Solver {
   long long* d_coff = nullptr;  // per subdomain: first cell in the blocked arrays
   void* ic_coef = nullptr;      // blocked {tx, ty, tz, 1/D} (precision of the preconditioner)
   // level-1 solve by one warp per subdomain (k_ic_warp): the factor in step order
-  bool ic_wrp_ok = false;
+  bool ic_wrp_ok = false;      // a candidate for this mesh
+  bool ic_wrp_packed = false;  // d_woff and ic_wcoef hold this set-up's factor
   int ic_wrp_smem = 0, ic_wrp_face = 0;
   long long* d_woff = nullptr;
   void* ic_wcoef = nullptr;
-  void* rt = nullptr;     // residual x - A y of the level-1 visits with an iterate (k_lv1_resid)
   float* r32 = nullptr;   // mixed form: FP32 copy of the vector the preconditioner is applied to
-  int setup_ic_warp(bool mixed);
+  void check_ic_warp(bool mixed);
+  bool pack_ic_warp(bool mixed);
+  void free_ic_warp();
   int* d_kerr = nullptr;        // set by a kernel whose bounded wait ran out
   int check_kernel_flag(const char* what);
   int setup_ic_blocked(bool mixed);

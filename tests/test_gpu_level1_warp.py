@@ -50,3 +50,56 @@ def test_warp_level1_matches_natural(native, monkeypatch, name, precision):
     rel = np.linalg.norm(out[1][0] - out[0][0]) / np.linalg.norm(out[0][0])
     assert rel <= (1e-12 if precision == "fp64" else 1e-5), rel
     assert abs(out[0][1] - out[1][1]) <= 1
+
+
+def test_no_room_for_the_step_ordered_factor(native, monkeypatch):
+    """The factor's copy is this kernel's alone: where it does not fit beside what the other kernels need, one of them
+    runs.  118 MB of copy for 3.3 million FP64 cells, 16 MB left (and what the stream-ordered pools give back)."""
+    import torch
+    prob = fields.random_box((160, 160, 128), seed=7, sigma=1.5)
+
+    def solve(kernel):
+        s = DarcySolver.from_problem(prob, options_string({"pmf_sd": (10, 10, 8), "en_lv1": 3, "en_lv2": 2,
+                                                           "pmf_lv1_kernel": kernel}))
+        s.setup()
+        its = s.solve(s.rhs(prob["source"].ravel()))[1]
+        used = free - torch.cuda.mem_get_info()[0]
+        s.close()
+        return its, used
+
+    monkeypatch.setenv("PMF_TUNE_FORCE", "100")
+    free = torch.cuda.mem_get_info()[0]
+    solve("natural")  # warms the pools
+    free = torch.cuda.mem_get_info()[0]
+    its, used = solve("natural")
+    its_warp, used_warp = solve("auto")
+    assert used_warp - used > 100 << 20
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - used - (16 << 20), dtype=torch.uint8, device="cuda")
+    free = torch.cuda.mem_get_info()[0]
+    try:
+        assert abs(solve("auto")[0] - its) <= 1
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert abs(its_warp - its) <= 1
+
+
+@pytest.mark.parametrize("tile,offered", [((4, 4, 4), False), ((4, 8, 8), False), ((8, 8, 8), True)],
+                         ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else str(v))
+def test_idle_lanes_take_no_memory(native, monkeypatch, tile, offered):
+    """A shape that leaves most of a warp's lanes idle would fill its factor's copy with nothing: it is not offered."""
+    import torch
+    monkeypatch.setenv("PMF_TUNE_FORCE", "100")
+    mesh = tuple(64 for _ in tile)
+    prob = fields.random_box(mesh, seed=7, sigma=1.0)
+    used = []
+    for kernel in ("natural", "natural", "auto"):  # the first one warms the pools
+        free = torch.cuda.mem_get_info()[0]
+        s = DarcySolver.from_problem(prob, options_string({
+            "pmf_vranks": (2, 2, 2), "pmf_sd": tuple(32 // t for t in tile), "en_lv1": 2, "en_lv2": 2,
+            "pmf_lv1_kernel": kernel}))
+        s.setup()
+        used.append(free - torch.cuda.mem_get_info()[0])
+        s.close()
+    # 262 144 cells: 1.6 entries of 32 bytes a cell are 13 MB, 4.9 and 9.5 are 41 and 80; cudaMalloc's blocks are 2 MB
+    assert (used[2] - used[1] > 8 << 20) == offered
