@@ -626,7 +626,7 @@ struct WgradArgs {
 // dW[t][ci][co] = sum over output rows of in[gather(row, t)][ci] * dz[row][co], in FP32 on the CUDA cores.
 // blockIdx.y = group of G taps, blockIdx.x = chunk of rows; a thread holds TA x TB outputs of each of the G
 // taps, so that a row's dz is read from shared memory once for all of them (one tap of 32 x 32 channels alone
-// gives a thread four multiply-adds for four reads, nine taps 36 for ten).  The rows' chunks are as many as
+// gives a thread four multiply-adds for four reads, nine taps 36 for ten).  The rows' chunks are at least as many as
 // fill the chip, their sums added atomically.
 // 64 patches, the 16^3 32 -> 32 layer: 2.33 ms with one tap per CTA, 0.73 ms.
 template <int CIN, int COUT, int TA, int TB, int G>
@@ -709,9 +709,9 @@ __global__ void __launch_bounds__((CIN / TA) * (COUT / TB)) k_net_wgrad(WgradArg
 }
 template <int CIN, int COUT, int TA, int TB, int G>
 static void wgrad_launch(WgradArgs w, long long rows, int taps, cudaStream_t st) {
-  // about four CTAs per SM, chunks of at least 64 rows
+  // about four CTAs per SM, chunks of 64 rows at least and 2 048 at most: a chunk is one chain of FP32 additions
   const long long chunks = std::max<long long>(1, std::min<long long>(rows / 64, (148LL * 4 * G + taps - 1) / taps));
-  w.rows_per_chunk = (int)(((rows + chunks - 1) / chunks + 15) & ~15LL);
+  w.rows_per_chunk = (int)std::min<long long>(2048, ((rows + chunks - 1) / chunks + 15) & ~15LL);
   const dim3 grid((unsigned)((rows + w.rows_per_chunk - 1) / w.rows_per_chunk), taps / G);
   note_launch();
   k_net_wgrad<CIN, COUT, TA, TB, G><<<grid, (CIN / TA) * (COUT / TB), 0, st>>>(w);

@@ -150,3 +150,32 @@ def test_trained_network_reduces_eigensolver_iterations(native, torch):
     assert l["fallbacks"] <= 0.05 * 512, res
     assert abs(l["pcg_iters"] - r["pcg_iters"]) <= 1, res
     assert res["solution_rel_diff"] < 1e-6, res
+
+
+def test_weight_gradient_of_a_large_batch(native, torch):
+    """512 patches: the rows of a weight gradient's FP32 sums are added in chains of at most 2 048, the chains' results
+    one after another.  Weights and biases that make the input of the second convolution at 16^3 one everywhere and its
+    output's gradient dy: the centre tap's entries are then sums of dy over all rows.  dy is a constant whose
+    additions round the same way for long stretches.  The tolerance is half a unit in the last place of every partial
+    sum, added up."""
+    B, c = 512, np.float32(0.7429176568984985)
+    net = learned.Net(seed=7)
+    for l in range(9):
+        w, b = net.weights(l)
+        w[:] = 0.0
+        b[:] = 1.0 if l in (6, 7) else 0.0
+        if l == 8:
+            w[0, :16, :] = np.eye(16)
+        net.set_weights(l, w, b)
+    y = torch.empty((B, 4096, 16), dtype=torch.float32, device="cuda")
+    net.forward(torch.zeros((B, 4096, 16), dtype=torch.bfloat16, device="cuda"), y)
+    assert float(y.min()) == 1.0 and float(y.max()) == 1.0
+    net.backward(torch.full_like(y, float(c)))
+    got = net.grads(7)[0][13, :, :16].astype(np.float64)
+    rows, chain = B * 4096, 2048
+    half_ulp = lambda s: 0.5 * np.spacing(s.astype(np.float32)).astype(np.float64)
+    per_chain = half_ulp(float(c) * np.arange(1, chain + 1)).sum()
+    nchain = rows // chain
+    tol = nchain * per_chain + half_ulp(float(c) * chain * np.arange(1, nchain + 1)).sum()
+    exact = rows * float(c)
+    assert np.abs(got - exact).max() <= tol, (np.abs(got - exact).max() / exact, tol / exact)
