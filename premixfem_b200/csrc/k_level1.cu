@@ -450,8 +450,8 @@ __global__ void __launch_bounds__(BD, sizeof(T) == 4 ? 2 : 1)
 // (shuffles), except below kl = 0, where the value comes from shared memory,
 // written nx - KL + 1 >= 4 steps before.  A sweep is one stream of
 // nx nz / KL + ny + KL - 2 steps with no CTA barrier and no drained pipeline
-// between groups of lines, and about ten warps per SM hide each other's
-// latency.
+// between groups of lines, and eight warps per SM (what the shared memory of 16^3
+// FP32 cells admits) hide each other's latency.
 //
 // The factor {tx, ty, tz, 1/D}, masked at the subdomain's faces so that the
 // sweeps have no branches, is stored in step order (entry step * 32 + lane):
@@ -463,16 +463,17 @@ __global__ void __launch_bounds__(BD, sizeof(T) == 4 ? 2 : 1)
 // holds only the vector, at pitch 34 per position: consecutive positions of a
 // line and consecutive lines at one step then both fall on different banks.
 //
-// The backward sweep passes the products t_ij z_j down instead of z_j, because
-// the coupling belongs to the upper cell: its sums round the products where the
-// other kernels contract them into multiply-adds (1e-12 in FP64, 1e-5 in mixed
-// precision per application, the bar between those kernels).
+// The couplings of the backward sweep belong to the upper cells: they go down
+// beside the values (a shuffle each, and for the group above a place in shared memory
+// beside the vector), so that the sums are the multiply-adds of the other kernels in
+// the same order.
 //
 // Measured against the better of the other kernels: 256^3 cells in 4 096 mixed-
-// precision subdomains, 165 us the first visit (270) and 303 with the iterate,
-// its residual kernel included (411; the bytes of one pass need 72 and 113);
-// 192^3 FP64, 140 and 230 (219 and 320); 128^3 mixed, 512 subdomains, 30 and 56
-// (37 and 58).
+// precision subdomains, 167 us the first visit (270) and 306 with the iterate,
+// its residual kernel included (409; the bytes of one pass need 72 and 113);
+// 192^3 FP64, 140 and 230 (224 and 320); 128^3 mixed, 512 subdomains, 30 and 57
+// (37 and 58).  (165 and 304 at 256^3 with the products t_ij z_j passed down, one
+// shuffle a direction, which rounds each of them before it is added.)
 namespace {
 constexpr int kWarpPitch = 34;
 constexpr int kWarpBatch = 4;  // steps between warp synchronisations
@@ -529,7 +530,7 @@ __global__ void __launch_bounds__(32, 8) k_ic_warp(Grid g, const SubInfo* subs, 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   V4* ring = reinterpret_cast<V4*>(smem_raw);  // ring[(batch % NB) * BS * 32 + step * 32 + lane]
   T* us = reinterpret_cast<T*>(ring + NB * BS * 32);  // us[position * P + lane]
-  T* pzs = us + ldu;                                  // products to the group below, [i * ny + j]
+  T* pzs = us + ldu;                                  // tz of the first plane of the group above, [i * ny + j]
   const unsigned full = 0xffffffffu;
   const SubInfo S = subs[blockIdx.x];
   const int nx = S.nx, ny = S.ny, nz = S.nz, nc = nx * ny * nz;
@@ -561,7 +562,6 @@ __global__ void __launch_bounds__(32, 8) k_ic_warp(Grid g, const SubInfo* subs, 
       cp_async_elem<sizeof(T)>(us + q.slot, rs + q.loc);
     }
     cp_async_commit();
-    for (int e = lane; e < nx * ny; e += 32) pzs[e] = (T)0;
   }
   const int kl = dny.quot(lane), j = lane - kl * ny, off = j + kl;
   // positions of this lane: whole lines with k = group * KL + kl < nz
@@ -633,15 +633,17 @@ __global__ void __launch_bounds__(32, 8) k_ic_warp(Grid g, const SubInfo* subs, 
   cp_async_wait<0>();
   // backward: (D + L^T) z = D u  ->  z_i = u_i + (sum_{upper} t_ij z_j) / D_i, in batches as well
   {
-    T px = (T)0, py = (T)0, pz = (T)0;
+    // of the lane's step before: value and couplings
+    T ov = (T)0, cxv = (T)0, cyv = (T)0, czv = (T)0;
     const bool top = lane == 31;  // no lane above
+    const int dk = nx * P - (KL - 1) * ny;
 #pragma unroll
     for (int b = 0; b < NB - 1; ++b) stage(nbatch - 1 - b);
     for (int b = nbatch - 1; b >= 0; --b) {
       cp_async_wait<NB - 2>();
       const V4* cb = ring + (b % NB) * BS * 32 + lane;
       V4 cc[BS];
-      T un[BS], gn[BS], o[BS], oz[BS];
+      T un[BS], gn[BS], gc[BS], o[BS];
       bool act[BS];
       T* pp[BS];
       const int p0 = b * BS + BS - 1 - off;  // position of the batch's first step
@@ -650,32 +652,34 @@ __global__ void __launch_bounds__(32, 8) k_ic_warp(Grid g, const SubInfo* subs, 
       for (int q = 0; q < BS; ++q) {
         act[q] = (unsigned)(p0 - q) < (unsigned)np;
         cc[q] = cb[(BS - 1 - q) * 32];
-        un[q] = gn[q] = (T)0;
+        un[q] = gn[q] = gc[q] = (T)0;
         pp[q] = pzs + i * ny + j;
-        if (act[q]) un[q] = u0[(b * BS + BS - 1 - q) * P];
-        if (act[q] && above) gn[q] = *pp[q];
+        const T* s0 = u0 + (b * BS + BS - 1 - q) * P;
+        if (act[q]) un[q] = *s0;
+        if (act[q] && above && p0 - q + nx < w.npos) {
+          gn[q] = s0[dk];
+          gc[q] = *pp[q];
+        }
         i = i == 0 ? nx - 1 : i - 1;
       }
       stage(b - (NB - 1));
 #pragma unroll
       for (int q = 0; q < BS; ++q) {
-        T qy = __shfl_down_sync(full, py, 1);
-        T qz = __shfl_sync(full, pz, (lane + ny) & 31);
-        qy = top ? (T)0 : qy;
-        qz = above ? gn[q] : qz;
-        T s = px;
-        s += qy;
-        s += qz;
+        const T qy = __shfl_down_sync(full, ov, 1), ty = __shfl_down_sync(full, cyv, 1);
+        const T qz = __shfl_sync(full, ov, (lane + ny) & 31), tz = __shfl_sync(full, czv, (lane + ny) & 31);
+        T s = cxv * ov;
+        s += (top ? (T)0 : ty) * qy;
+        s += (above ? gc[q] : tz) * (above ? gn[q] : qz);
         o[q] = un[q] + s * cc[q].w;
-        px = act[q] ? cc[q].x * o[q] : px;
-        py = act[q] ? cc[q].y * o[q] : py;
-        pz = act[q] ? cc[q].z * o[q] : pz;
-        oz[q] = pz;
+        ov = act[q] ? o[q] : ov;
+        cxv = act[q] ? cc[q].x : cxv;
+        cyv = act[q] ? cc[q].y : cyv;
+        czv = act[q] ? cc[q].z : czv;
       }
 #pragma unroll
       for (int q = 0; q < BS; ++q) {
         if (act[q]) u0[(b * BS + BS - 1 - q) * P] = o[q];
-        if (act[q] && below) *pp[q] = oz[q];
+        if (act[q] && below) *pp[q] = cc[q].z;
       }
       __syncwarp();
     }
