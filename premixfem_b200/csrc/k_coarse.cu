@@ -1045,10 +1045,15 @@ __global__ void k_l3_init(RankLayout L, int p, const double* A_all, double* work
     st[r].conv = 0;
     st[r].it = 0;
   }
-  double* R = X + 2 * (long long)nr * p;  // X = 0 and R = -(random columns): Y = inv (random columns)
+  __syncthreads();
+  // Random columns V as X = V / anorm and R = -V, which makes Y = inv V and a little of V: a direction that the inverse
+  // dropped as null (the only one of a floating rank of one unknown, whose matrix is rounding) stays in the block.
+  double* R = X + 2 * (long long)nr * p;
+  const double an = st[r].anorm;
   for (long long e = threadIdx.x; e < (long long)nr * p; e += blockDim.x) {
-    X[e] = 0.0;
-    R[e] = -hash_uniform(((unsigned long long)r << 40) ^ (unsigned long long)e);
+    const double v = hash_uniform(((unsigned long long)r << 40) ^ (unsigned long long)e);
+    X[e] = v / an;
+    R[e] = -v;
   }
 }
 
@@ -1269,7 +1274,7 @@ __global__ void __launch_bounds__(kL3Thr) k_l3_rr(RankLayout L, int en2, int p, 
     for (int c = q; c < p; ++c) {
       double v = rnd(l, c);
       for (int k = 0; k < q; ++k) v -= d[c * 16 + k] * X[(long long)l * p + k];
-      X[(long long)l * p + c] = 0.0;
+      X[(long long)l * p + c] = v / st[rk].anorm;
       AY[(long long)l * p + c] = -v;
     }
 }

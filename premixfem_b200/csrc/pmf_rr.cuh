@@ -115,7 +115,9 @@ __device__ __forceinline__ void warp_sym_lowest(WarpRR<NX, MX>& s, double (&a)[N
     gh = fmax(gh, __shfl_xor_sync(full, gh, o));
     gm = fmax(gm, __shfl_xor_sync(full, gm, o));
   }
-  const double emax = fmax(gm, 1e-300), isc = 1.0 / emax;
+  // a matrix of zeros (a floating rank of one unknown) has its scale set to one: the inverse
+  // iteration's growth, up to 1e19 / emax, is squared below
+  const double emax = gm > 1e-100 ? gm : 1.0, isc = 1.0 / emax;
   // scaled diagonal, and squared couplings to the row before: at least 1e-36, a
   // coupling of 1e-18, which is below the rounding of T
   double *ds = s.ds, *es = s.es;

@@ -55,3 +55,11 @@ def test_coarse_orders(native, monkeypatch, name, contrast):
     y, yr = s.pc_apply(x), pc.apply(x)
     s.close()
     assert np.linalg.norm(y - yr) <= 1e-6 * np.linalg.norm(yr)
+
+
+@pytest.mark.parametrize("contrast", [1.0, 4.0])
+def test_floating_ranks_of_one_unknown(native, monkeypatch, contrast):
+    """64 ranks of one unknown, most of them floating: their 1 x 1 matrix is the rounding of zero, of either sign, and
+    its inverse may drop it as null.  The bars of the test above."""
+    monkeypatch.setitem(CASES, "floating", ((16, 16, 16), (1, 1, 1), (4, 4, 4), 1, 1))
+    test_coarse_orders(native, monkeypatch, "floating", contrast)
