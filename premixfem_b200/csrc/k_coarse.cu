@@ -852,22 +852,28 @@ __global__ void __launch_bounds__(512) k_dense_smallest_eig(RankLayout L, int en
     for (int i = 0; i < nr; ++i) m = fmax(m, fabs(A[(long long)i * nr + i]));
     anorm = m > 0 ? m : 1.0;
   }
-  for (long long e = tid; e < (long long)nr * p; e += nt)
-    X[e] = hash_uniform(((unsigned long long)r << 40) ^ (unsigned long long)e);
+  __syncthreads();
+  for (long long e = tid; e < (long long)nr * p; e += nt) {
+    const double v = hash_uniform(((unsigned long long)r << 40) ^ (unsigned long long)e);
+    X[e] = v / anorm;
+    AY[e] = -v;
+  }
   __syncthreads();
   int it = 0;
   for (; it < max_it; ++it) {
-    // Y = inv X
+    // Y = X - inv R with the residuals R in AY, as k_l3_mm and k_l3_init explain
     if (ldx > 0) {
-      cta_stage_block(X, nr, p, p, xs, ldx);
+      cta_stage_block(AY, nr, p, p, xs, ldx);
       cta_rows_mm(inv, nr, xs, ldx, p, Y, p, nullptr);
+      __syncthreads();
+      for (long long e = tid; e < (long long)nr * p; e += nt) Y[e] = X[e] - Y[e];
     } else {
       for (long long e = tid; e < (long long)nr * p; e += nt) {
         const int i = (int)(e / p), j = (int)(e % p);
         const double* row = inv + (long long)i * nr;
         double acc = 0.0;
-        for (int l = 0; l < nr; ++l) acc += row[l] * X[(long long)l * p + j];
-        Y[e] = acc;
+        for (int l = 0; l < nr; ++l) acc += row[l] * AY[(long long)l * p + j];
+        Y[e] = X[e] - acc;
       }
     }
     __syncthreads();
@@ -976,14 +982,31 @@ __global__ void __launch_bounds__(512) k_dense_smallest_eig(RankLayout L, int en
     }
     if (q < en2 && tid == 0) conv = 0;
     __syncthreads();
-    // pad dropped columns with fresh random directions for the next sweep
+    if (conv) break;
+    // fresh random directions in place of dropped columns, orthogonal to the kept ones: the inverse of a floating
+    // rank, whose constant it takes 1e8 times, would turn others back into copies of the kept ones
     for (long long e = tid; e < (long long)nr * (p - q); e += nt) {
       const int i = (int)(e / (p - q)), c = q + (int)(e % (p - q));
       X[(long long)i * p + c] = hash_uniform(((unsigned long long)(r + 7) << 44) ^ ((unsigned long long)it << 32) ^
                                              (unsigned long long)e);
     }
     __syncthreads();
-    if (conv) break;
+    for (int e = tid; e < (p - q) * q; e += nt) {
+      const int c = q + e / q, k = e % q;
+      double acc = 0.0;
+      for (int l = 0; l < nr; ++l) acc += X[(long long)l * p + c] * X[(long long)l * p + k];
+      G[c * PMF_L3_MAXP + k] = acc;
+    }
+    __syncthreads();
+    for (long long e = tid; e < (long long)nr * (p - q); e += nt) {
+      const long long i = e / (p - q);
+      const int c = q + (int)(e % (p - q));
+      double v = X[i * p + c];
+      for (int k = 0; k < q; ++k) v -= G[c * PMF_L3_MAXP + k] * X[i * p + k];
+      X[i * p + c] = v / anorm;
+      AY[i * p + c] = -v;
+    }
+    __syncthreads();
   }
   double* V = V_all + L.offv[r];
   for (long long e = tid; e < (long long)nr * en2; e += nt) {

@@ -63,3 +63,12 @@ def test_floating_ranks_of_one_unknown(native, monkeypatch, contrast):
     its inverse may drop it as null.  The bars of the test above."""
     monkeypatch.setitem(CASES, "floating", ((16, 16, 16), (1, 1, 1), (4, 4, 4), 1, 1))
     test_coarse_orders(native, monkeypatch, "floating", contrast)
+
+
+@pytest.mark.parametrize("contrast", [1.0, 4.0])
+@pytest.mark.parametrize("vr,en2", [((2, 2, 2), 8), ((3, 3, 3), 8), ((3, 3, 3), 10)])
+def test_wide_blocks_of_floating_ranks(native, monkeypatch, vr, en2, contrast):
+    """Blocks of 20 and 24 columns on ranks of 36 unknowns, most of which touch no Dirichlet face; the bars of the test
+    above."""
+    monkeypatch.setitem(CASES, "floating", (tuple(v * n for v, n in zip(vr, (6, 6, 2))), (3, 3, 1), vr, 4, en2))
+    test_coarse_orders(native, monkeypatch, "floating", contrast)
