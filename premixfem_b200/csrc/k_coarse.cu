@@ -161,8 +161,63 @@ __global__ void __launch_bounds__(256) k_lv3_solve(const CoarseChunk* chunks, co
     Z[ch.g0 + q] = first ? acc : Z[ch.g0 + q] + acc;
   }
 }
-void launch_lv3_solve(const RankLayout& L, int n3, int en2, const double* part, const double* A3inv, const double* V,
-                      double* dz, double* Z, int first, const int* done, cudaStream_t st) {
+// The same in three launches for many ranks, where every CTA's own sums and products cost more than two
+// launches: d by a warp per entry, w = A3^-1 d by a warp per row, then the prolongation.
+__global__ void __launch_bounds__(256) k_lv3_sum(const int* chunk_first, int n3, int en2, const double* part, double* d,
+                                                 const int* done) {
+  if (done && *done) return;
+  const int e = (int)((blockIdx.x * 256u + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (e >= n3) return;
+  const int rr = e / en2, j = e - rr * en2, c1 = chunk_first[rr + 1];
+  double v = 0.0;
+  for (int k = chunk_first[rr] + lane; k < c1; k += 32) v += part[(long long)k * en2 + j];
+  v = warp_sum(v);
+  if (lane == 0) d[e] = v;
+}
+__global__ void __launch_bounds__(256) k_lv3_gemv(int n3, const double* A3inv, const double* d, double* w,
+                                                  const int* done) {
+  if (done && *done) return;
+  const int i = (int)((blockIdx.x * 256u + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (i >= n3) return;
+  const double* row = A3inv + (long long)i * n3;
+  double acc = 0.0;
+#pragma unroll 8
+  for (int e = lane; e < n3; e += 32) acc += row[e] * d[e];
+  acc = warp_sum(acc);
+  if (lane == 0) w[i] = acc;
+}
+__global__ void __launch_bounds__(256) k_lv3_prolong(const CoarseChunk* chunks, int nchunk, int en2, const double* w,
+                                                     const double* V, double* dz, double* Z, int first,
+                                                     const int* done) {
+  if (done && *done) return;
+  const int c = blockIdx.x * 8 + (threadIdx.x >> 5), q = threadIdx.x & 31;  // a warp per chunk, a lane per row
+  static_assert(kCoarseRows == 32, "a lane per row");
+  if (c >= nchunk) return;
+  const CoarseChunk ch = chunks[c];
+  if (q >= ch.rows) return;
+  const double* Vi = V + ch.v_off + (long long)q * en2;
+  const double* wr = w + (long long)ch.rank * en2;
+  double acc = 0.0;
+#pragma unroll 4
+  for (int j = 0; j < en2; ++j) acc += Vi[j] * wr[j];
+  dz[ch.g0 + q] = acc;
+  Z[ch.g0 + q] = first ? acc : Z[ch.g0 + q] + acc;
+}
+
+// Every CTA of the one launch reads en2 (nchunk + n3) values.  Coarse part of an iteration in one launch and in
+// three, by that number: 3 072 (64 ranks of 256 unknowns, four vectors each) 50 us and 55, 4 096 52 and 50 (128
+// ranks of 128) and 67 and 68 (64 of 384), 13 312 458 and 423 (64 of 1 536), 20 480 227 and 128 (512 of 192);
+// 4 096 ranks of four unknowns 1 428 and 152.
+bool lv3_split(const RankLayout& L, int n3, int en2) { return (long long)en2 * (L.nchunk + n3) > 4096; }
+void launch_lv3_solve(const RankLayout& L, int n3, int en2, const double* part, double* dw, const double* A3inv,
+                      const double* V, double* dz, double* Z, int first, const int* done, cudaStream_t st) {
+  if (lv3_split(L, n3, en2)) {
+    const int g = (n3 + 7) / 8;
+    { note_launch(); k_lv3_sum<<<g, 256, 0, st>>>(L.chunk_first, n3, en2, part, dw, done); }
+    { note_launch(); k_lv3_gemv<<<g, 256, 0, st>>>(n3, A3inv, dw, dw + n3, done); }
+    { note_launch(); k_lv3_prolong<<<(L.nchunk + 7) / 8, 256, 0, st>>>(L.chunks, L.nchunk, en2, dw + n3, V, dz, Z, first, done); }
+    return;
+  }
   const int smem = (n3 + en2) * (int)sizeof(double);
   int gs = 1;  // lanes per entry of d: as many as leave no second pass
   while (gs < 32 && n3 * gs * 2 <= 256) gs *= 2;

@@ -206,9 +206,10 @@ void launch_block_gemv_r(const RankLayout& L, const double* inv, const double* i
 // then part[chunk][j] = the chunk's rows of V^T c (V not null)
 void launch_coarse_resid(const RankLayout& L, const SubInfo* subs, const double* blk, const double* dz, double* c,
                          int en2, const double* V, double* part, const int* done, cudaStream_t st);
-// dz = V A3^-1 (sum of part), Z = dz (first) or Z += dz
-void launch_lv3_solve(const RankLayout& L, int n3, int en2, const double* part, const double* A3inv, const double* V,
-                      double* dz, double* Z, int first, const int* done, cudaStream_t st);
+// dz = V A3^-1 (sum of part), Z = dz (first) or Z += dz; dw: 2 n3 values of scratch where lv3_split
+bool lv3_split(const RankLayout& L, int n3, int en2);
+void launch_lv3_solve(const RankLayout& L, int n3, int en2, const double* part, double* dw, const double* A3inv,
+                      const double* V, double* dz, double* Z, int first, const int* done, cudaStream_t st);
 void launch_assemble_dense_r(const SubInfo* subs, int nrank, const RankLayout& L, long long total, const double* blk,
                              const double* gface, int mode, double* dense, cudaStream_t st);
 // dense[r] += mu (relative != 0: mu x max |diag| of the block) on the diagonal, one CTA per rank

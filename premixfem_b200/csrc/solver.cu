@@ -1258,7 +1258,8 @@ int Solver::setup() {
                       {(void**)&c, sizeof(double) * nsub * kmax, "coarse residual"},
                       {(void**)&dz, sizeof(double) * nsub * kmax, "coarse correction"},
                       {(void**)&Zacc, sizeof(double) * nsub * kmax, "coarse accumulator"},
-                      {(void**)&l3part, sizeof(double) * rl.nchunk * en2, "level-3 right-hand side"},
+                      {(void**)&l3part, sizeof(double) * ((size_t)rl.nchunk * en2 + (lv3_split(rl, n3, en2) ? 2 * (size_t)n3 : 0)),
+                       "level-3 right-hand side"},
                       {(void**)&d_rank_nb, sizeof(int) * nrank * 6, "rank neighbours"}};
     const int nl = (int)(sizeof(list) / sizeof(list[0]));
     for (int i = 0; i < nl; ++i) {
@@ -1767,7 +1768,7 @@ void Solver::apply_impl(const double* x, const T* xt, double* out, double* parti
       }
       if (v == 3) {
         launch_coarse_resid(rl, d_subs, blk, dz_pend ? dz : nullptr, c, en2, V3, l3part, done, st);
-        launch_lv3_solve(rl, n3, en2, l3part, A3inv, V3, dz, Zacc, z_pend ? 0 : 1, done, st);
+        launch_lv3_solve(rl, n3, en2, l3part, l3part + (size_t)rl.nchunk * en2, A3inv, V3, dz, Zacc, z_pend ? 0 : 1, done, st);
       } else {
         if (dz_pend) launch_coarse_resid(rl, d_subs, blk, dz, c, en2, nullptr, nullptr, done, st);
         if (v == 2) {

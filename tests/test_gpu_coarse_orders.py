@@ -72,3 +72,23 @@ def test_wide_blocks_of_floating_ranks(native, monkeypatch, vr, en2, contrast):
     above."""
     monkeypatch.setitem(CASES, "floating", (tuple(v * n for v, n in zip(vr, (6, 6, 2))), (3, 3, 1), vr, 4, en2))
     test_coarse_orders(native, monkeypatch, "floating", contrast)
+
+
+@pytest.mark.parametrize("case", [((16, 16, 16), (1, 1, 1), (8, 8, 8), 4, 3), ((48, 24, 8), (3, 3, 1), (8, 4, 4), 4, 8)],
+                         ids=["512_ranks_of_4", "128_ranks_of_36"])
+def test_many_ranks(native, monkeypatch, case):
+    """Level-3 problems of 1 536 and 1 024 unknowns, solved in launches of their own; the bars of the test above."""
+    monkeypatch.setitem(CASES, "many", case)
+    test_coarse_orders(native, monkeypatch, "many", 1.0)
+
+
+def test_cost_of_many_ranks(native):
+    """4 096 ranks of one subdomain each: the level-3 inverse, 537 MB, is streamed once an iteration (about 0.1 ms), not
+    once for every group of rows."""
+    s = DarcySolver.from_problem(fields.random_box((128, 128, 128), seed=3), options_string({
+        "sd": 1, "pmf_vranks": (16, 16, 16), "en_lv1": 4, "en_lv2": 2, "pmf_precision": "mixed", "pmf_eig_max_it": 2}))
+    s.setup()
+    s.profile_iteration(5)
+    ms = s.profile_iteration(20)["coarse"][0]
+    s.close()
+    assert ms <= 0.7, ms
