@@ -83,13 +83,13 @@ __global__ void k_bpcg_beta_fin(const ProbInfo* probs, const double* part, PcgSt
   }
 }
 
-// p <- z (first) or z + (beta/betaold) p; w <- A p: a CTA covers a 32 x 8 tile of
-// one layer of the shared mesh, whose problem is layer_prob[z] (separator
-// layers: none); layers past the grid's y limit are taken in turn.  Tiles past
+// p <- z (first) or z + (beta/betaold) p; w <- A p: a CTA covers 256 places along the
+// rows of one layer of the shared mesh, whose problem is layer_prob[z] (separator
+// layers: none); layers past the grid's y limit are taken in turn.  Places past
 // the problem's own extent (the shared mesh is the largest of all problems in x
-// and y) only report a zero partial; everything there is zero and stays so.
-// Partial z tiles + tile of p.w, so problem q's partials are the contiguous range
-// of its layers.  (A solve of 16 problems of 24..80 cells per axis takes 18.4 ms;
+// and y) add nothing; everything there is zero and stays so.  A partial of p.w per
+// run and layer, so problem q's partials are the contiguous range of its layers.
+// (A solve of 16 problems of 24..80 cells per axis takes 18.4 ms;
 // with this step and the next over the whole shared mesh 25.)
 __global__ void __launch_bounds__(kStX * kStY) k_bpcg_iter_a(Grid g, const ProbInfo* probs, const int* layer_prob,
                                                              const double* tx, const double* ty, const double* tz,
@@ -242,15 +242,15 @@ void launch_bpcg_beta(const ProbInfo* probs, int nprob, const double* part, PcgS
 void launch_bpcg_iter_a(const Grid& g, const ProbInfo* probs, const int* layer_prob, int nprob, const double* tx,
                         const double* ty, const double* tz, const double* diag, const double* z, const double* pin,
                         double* pout, double* w, double* part, PcgState* st, cudaStream_t s) {
-  // a partial per tile and layer: pcg_part_capacity(g) of them at most
-  const dim3 grid((g.M + kStX - 1) / kStX * ((g.N + kStY - 1) / kStY), std::min(g.P, 65535));
+  // a partial per run and layer: pcg_part_capacity(g) of them
+  const dim3 grid(stencil_shape(g).grid.x, std::min(g.P, 65535));
   { note_launch(); k_bpcg_iter_a<<<grid, dim3(kStX, kStY), 0, s>>>(g, probs, layer_prob, tx, ty, tz, diag, z, pin, pout, w, part, st); }
   { note_launch(); k_bpcg_iter_a_fin<<<nprob, 1024, 0, s>>>(probs, part, (int)grid.x, st); }
 }
 void launch_bpcg_iter_b(const Grid& g, const ProbInfo* probs, const int* layer_prob, int nprob, double* r, float* r32,
                         const double* p, const double* w, double* part, PcgState* st, int* all_done, LoopCond loop,
                         cudaStream_t s) {
-  const int sub = std::max(1, std::min(32, (int)(g.MN / 2048)));  // CTAs per layer, fewer than its tiles
+  const int sub = std::max(1, std::min(32, (int)(g.MN / 2048)));  // CTAs per layer, fewer than its runs
   { note_launch(); k_bpcg_iter_b<<<dim3(sub, std::min(g.P, 65535)), kBT, 0, s>>>(g, probs, layer_prob, r, r32, p, w, part, st); }
   { note_launch(); k_bpcg_iter_b_fin<<<1, 1024, 0, s>>>(probs, nprob, part, sub, st, all_done, loop); }
 }

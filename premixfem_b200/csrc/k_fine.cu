@@ -354,9 +354,9 @@ __global__ void __launch_bounds__(1024) k_pcg_iter_a_fin(const double* part, int
     }
   }
 }
-// one partial per x-y tile and plane: the batch's CG step, the largest user
+// one partial per run of places and plane: the batch's CG step, the largest user
 int pcg_part_capacity(const Grid& g) {
-  const long long n = (long long)((g.M + kStX - 1) / kStX) * ((g.N + kStY - 1) / kStY) * g.P;
+  const long long n = (long long)stencil_shape(g).grid.x * g.P;
   return (int)std::max<long long>(cell_blocks(g.ncell), n);
 }
 

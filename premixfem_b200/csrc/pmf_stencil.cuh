@@ -1,10 +1,13 @@
 // The 7-point operator over the whole mesh as a short march in z.
 //
-// A CTA of 32 x 8 threads owns a column of x-y tiles and walks zc planes: the
-// value and the z coupling of the plane above become those of the plane below,
-// so each is loaded once per march instead of at three planes, and the x and y
-// neighbours are read through L1 from the rows the CTA's other threads load.
-// Bound by HBM.  The loop is unrolled twice, which puts the next plane's loads
+// A CTA owns a run of 256 places along the rows of the x-y plane and walks zc
+// planes: the value and the z coupling of the plane above become those of the plane
+// below, so each is loaded once per march instead of at three planes, and the x and
+// y neighbours come from L1 and L2.  Runs along the rows leave no thread idle on any
+// mesh; tiles of 32 x 8 places, which keep the y neighbours of wide meshes in L1,
+// measured the same there (operator at 256^3 146 us either way) and slower where they
+// do not fit: 59 us against 50 at 161 x 163 x 157, 99 against 50 at 8 x 512 x 1024,
+// the CG step 212 against 58 at 2048 x 1 x 2048.  Bound by HBM.  The loop is unrolled twice, which puts the next plane's loads
 // in flight before this plane's arithmetic (the CG step at 256^3: unrolled once
 // 289 us, twice 183, four times 252; one plane per CTA 238) provided the output
 // pointers are __restrict__.  Sixteen planes,
@@ -25,18 +28,18 @@ struct StencilShape {
 };
 inline StencilShape stencil_shape(const Grid& g) {
   StencilShape s;
-  const long long tiles = (long long)((g.M + kStX - 1) / kStX) * ((g.N + kStY - 1) / kStY);
+  const long long runs = (g.MN + kStX * kStY - 1) / (kStX * kStY);
   s.zc = 16;
-  while (s.zc > 1 && tiles * ((g.P + s.zc - 1) / s.zc) < 16 * 148) s.zc /= 2;
+  while (s.zc > 1 && runs * ((g.P + s.zc - 1) / s.zc) < 16 * 148) s.zc /= 2;
   while ((g.P + s.zc - 1) / s.zc > 65535) s.zc *= 2;
-  s.grid = dim3((unsigned)tiles, (g.P + s.zc - 1) / s.zc);  // x: tiles, x fastest; y: stretches of planes
+  s.grid = dim3((unsigned)runs, (g.P + s.zc - 1) / s.zc);  // y: stretches of planes
   return s;
 }
 
-// this thread's (x, y) in tile blockIdx.x
+// this thread's (x, y) in the blockIdx.x-th run of 256 places along the rows
 __device__ __forceinline__ int2 stencil_xy(const Grid& g) {
-  const int nx = (g.M + kStX - 1) / kStX, by = blockIdx.x / nx;
-  return make_int2((blockIdx.x - by * nx) * kStX + threadIdx.x, by * kStY + threadIdx.y);
+  const unsigned c = (blockIdx.x * kStY + threadIdx.y) * kStX + threadIdx.x, y = c / (unsigned)g.M;
+  return make_int2((int)(c - y * g.M), (int)y);
 }
 
 // out(c, v, a) with v = val(c) and a = (A v)(c), evaluated in the order diagonal, x-, x+, y-, y+, z-, z+, for the
@@ -70,7 +73,7 @@ __device__ __forceinline__ void stencil_march(const Grid& g, const T* __restrict
   }
 }
 
-// sum over a 32 x 8 CTA in a fixed order, valid in thread (0, 0)
+// sum over a CTA of 32 x 8 threads in a fixed order, valid in thread (0, 0)
 __device__ __forceinline__ double stencil_sum(double v) {
   __shared__ double red[kStY];
   v = warp_sum(v);

@@ -51,3 +51,42 @@ def test_basis_sizes(native, k, precision):
         s.close()
         assert reason == "converged"
         assert np.linalg.norm(b - op.A @ u) <= 1e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("mesh,tile", [((4, 1024, 1024), (4, 16, 16)), ((8, 512, 1024), (8, 16, 16)),
+                                       ((2048, 1, 2048), (16, 1, 16)), ((2048, 3, 704), (16, 3, 16))],
+                         ids=["4x1024x1024", "8x512x1024", "2048x1x2048", "2048x3x704"])
+def test_thin_meshes_leave_no_threads_idle(native, mesh, tile):
+    """Meshes of a few cells in x or y take no longer than a cube of as many cells (4.2 million; 30 % for the box's
+    surface and the clock): the operator's call and the CG step."""
+    import time
+
+    import torch
+
+    def times(mesh, tile):
+        n = [-(-m // t) for m, t in zip(mesh, tile)]
+        vr = [1, 1, 1]
+        while np.prod([-(-c // v) for c, v in zip(n, vr)]) * 2 > 2000:
+            vr[int(np.argmax([c / v for c, v in zip(n, vr)]))] *= 2
+        sd = [-(-c // v) for c, v in zip(n, vr)]
+        s = DarcySolver((1.0, 1.0, 1.0), mesh, f"-pmf_vranks {vr[0]},{vr[1]},{vr[2]} -pmf_sd {sd[0]},{sd[1]},{sd[2]} "
+                                               "-en_lv1 2 -en_lv2 2 -pmf_eig_max_it 3 -pmf_autotune 0")
+        k = torch.from_numpy(np.exp(np.random.default_rng(0).standard_normal(int(np.prod(mesh))))).cuda()
+        s.set_kappa(k, k, k)
+        s.set_dirichlet("x-", 0.0)
+        s.setup()
+        x, y = torch.ones_like(k), torch.empty_like(k)
+        best = []
+        for _ in range(5):
+            t0 = time.perf_counter()
+            for _ in range(20):
+                s.apply_A(x, y)
+            best.append((time.perf_counter() - t0) / 20)
+        s.profile_iteration(10)
+        step = s.profile_iteration(20)["cg_p_update_Ap"][0]
+        s.close()
+        return min(best), step
+
+    ref = times((161, 163, 160), (16, 16, 16))
+    got = times(mesh, tile)
+    assert got[0] <= 1.3 * ref[0] and got[1] <= 1.3 * ref[1], (got, ref)
