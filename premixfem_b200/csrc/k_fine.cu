@@ -624,9 +624,20 @@ void launch_ic_apply(const Grid& g, const SubInfo* subs, int nsub, int max_lines
 // _PC_apply_vec_lv2, src/PreMixFEM_3D.c:1564) fused with the residual update
 // r = x - A y of PC_apply_vec (:1859-1926): the residual is never stored.
 // KM is the number of basis vectors exactly, and a cell's row of Phi is read by
-// the widest loads that every row's alignment allows: one load per vector under a
-// run-time bound cost the prolongation 94 us at 256^3 with six FP32 vectors, this
-// 90 (its 1.2 GB of traffic need 82); the restriction stays at 185 to 190 either way.
+// the widest loads that every row's alignment allows.  What is left to choose is how
+// many cells a thread has in flight: more hide the latency, and cost the registers
+// that limit the warps.  The restriction's best of one to four, by precision and
+// basis size, over 128^3 cells in tiles of 8, 160^3, 161 x 163 x 157 and 256^3 (us at
+// 160^3, in brackets with the basis rounded up to 4 or 8 and a load per value):
+//   FP32  45 (72)  47 (72)  49 (74)  52 (75)  55 (60)  55 (61)  59 (63)  56 (66)
+//   FP64  59 (74)  68 (74)  64 (76)  72 (78)  76 (93)  84 (95)  87 (96)  97 (108)
+// The wrong one costs up to half as much again (five FP32 vectors, one cell: 84).  The
+// prolongation takes one cell where a row is 16 to 32 bytes, else two: 20 to 32 us
+// (21 to 41) in FP32, 22 to 54 (27 to 72) in FP64.
+__host__ __device__ constexpr int restrict_unroll(int prec_bytes, int km) {
+  constexpr int f32[8] = {1, 1, 1, 3, 3, 3, 4, 2}, f64[8] = {4, 3, 3, 3, 3, 2, 2, 1};
+  return prec_bytes == 4 ? f32[km - 1] : f64[km - 1];
+}
 template <typename T, int KM>
 __device__ __forceinline__ void load_phi(const T* __restrict__ p, T (&v)[KM]) {
   constexpr int B = KM * sizeof(T) % 16 == 0 ? 16 : KM * sizeof(T) % 8 == 0 ? 8 : 4;  // row alignment in bytes
@@ -664,12 +675,13 @@ __global__ void k_resid_restrict(Grid g, const SubInfo* subs, const T* __restric
                                  const T* __restrict__ tz, const T* __restrict__ diag, const T* __restrict__ phi,
                                  const T* __restrict__ x, const T* __restrict__ y, double* c, const int* done) {
   if (done && *done) return;
+  constexpr int U = restrict_unroll(sizeof(T), KM);
   __shared__ double red[KM][33];
   const SubGeom q = sub_geom(subs[blockIdx.x]);
   double acc[KM];
 #pragma unroll
   for (int j = 0; j < KM; ++j) acc[j] = 0.0;
-#pragma unroll 1
+#pragma unroll U
   for (int cl = threadIdx.x; cl < q.ncells; cl += blockDim.x) {
     const int i = cl % q.nx, tt = cl / q.nx, jj = tt % q.ny, k = tt / q.ny;
     const int ex = q.x0 + i, ey = q.y0 + jj, ez = q.z0 + k;
@@ -730,11 +742,12 @@ template <typename T, int KM>
 __global__ void k_prolong(Grid g, const SubInfo* subs, const T* __restrict__ phi, const double* __restrict__ Z,
                           T* __restrict__ y, const int* done) {
   if (done && *done) return;
+  constexpr int R = KM * sizeof(T), U = R >= 16 && R <= 32 ? 1 : 2;
   const SubGeom q = sub_geom(subs[blockIdx.x]);
   T z[KM];
 #pragma unroll
   for (int j = 0; j < KM; ++j) z[j] = (T)Z[(long long)blockIdx.x * KM + j];
-#pragma unroll 2
+#pragma unroll U
   for (int cl = threadIdx.x; cl < q.ncells; cl += blockDim.x) {
     const int i = cl % q.nx, tt = cl / q.nx, jj = tt % q.ny, k = tt / q.ny;
     const long long cg = ((long long)(q.z0 + k) * g.N + (q.y0 + jj)) * g.M + (q.x0 + i);

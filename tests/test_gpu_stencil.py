@@ -90,3 +90,22 @@ def test_thin_meshes_leave_no_threads_idle(native, mesh, tile):
     ref = times((161, 163, 160), (16, 16, 16))
     got = times(mesh, tile)
     assert got[0] <= 1.3 * ref[0] and got[1] <= 1.3 * ref[1], (got, ref)
+
+
+def test_a_basis_vector_costs_its_bytes(native):
+    """The restriction with five to eight FP32 basis vectors against four, on 4.1 million cells: a cell's bytes are
+    those of k + 10 values, and 10 % are left for the clock."""
+    import torch
+    k0 = torch.from_numpy(np.exp(np.random.default_rng(0).standard_normal(160 ** 3))).cuda()
+    us = {}
+    for k in range(4, 9):
+        s = DarcySolver((1.0, 1.0, 1.0), (160, 160, 160), f"-pmf_vranks 4,2,2 -pmf_sd 3,5,5 -en_lv1 {k} -en_lv2 2 "
+                                                          "-pmf_precision mixed -pmf_eig_max_it 3")
+        s.set_kappa(k0, k0, k0)
+        s.set_dirichlet("x-", 0.0)
+        s.setup()
+        s.profile_iteration(10)
+        us[k] = 1e3 * s.profile_iteration(40)["resid_restrict"][0]
+        s.close()
+    for k in range(5, 9):
+        assert us[k] <= 1.1 * (k + 10) / 14 * us[4], us
