@@ -1322,6 +1322,16 @@ __global__ void __launch_bounds__(kL3Thr) k_l3_rr(RankLayout L, int en2, int p, 
       __syncthreads();
       if (tid == 0) sm.G[c] = rr;
     }
+  for (int c = 8; c < nw2; ++c) {  // rarely wanted: from the residuals this thread has just stored
+    double v = 0.0;
+    for (int l = tid; l < nr; l += kL3Thr) {
+      const double d = AY[(long long)l * p + c];
+      v += d * d;
+    }
+    const double rr = block_sum(v, sm.red);
+    __syncthreads();
+    if (tid == 0) sm.G[c] = rr;
+  }
   __syncthreads();
   for (int c = 0; c < nw2; ++c) conv = conv && sqrt(sm.G[c]) <= thr;
   if (tid == 0) {
@@ -1386,7 +1396,7 @@ void launch_dense_smallest_eig(const RankLayout& L, int nrank, int nr, int en2, 
                                double* work, cudaStream_t st) {
   L3Rank* rs = nullptr;
   int* left = nullptr;
-  if (p <= kL3Cols && en2 <= 8 && cudaMallocAsync((void**)&rs, sizeof(L3Rank) * nrank + 16, st) == cudaSuccess) {
+  if (p <= kL3Cols && cudaMallocAsync((void**)&rs, sizeof(L3Rank) * nrank + 16, st) == cudaSuccess) {
     left = reinterpret_cast<int*>(rs + nrank);
     const int gx = (nr + kL3Rows - 1) / kL3Rows;
     cudaFuncSetAttribute(k_l3_rr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(L3Smem));

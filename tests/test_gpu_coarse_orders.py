@@ -92,3 +92,14 @@ def test_cost_of_many_ranks(native):
     ms = s.profile_iteration(20)["coarse"][0]
     s.close()
     assert ms <= 0.7, ms
+
+
+@pytest.mark.parametrize("contrast", [1.0, 4.0])
+@pytest.mark.parametrize("case", [((16, 4, 4), (4, 1, 1), (1, 1, 1), 4, 16), ((24, 16, 8), (3, 1, 1), (2, 2, 2), 4, 12),
+                                  ((24, 12, 12), (3, 1, 1), (3, 3, 3), 3, 9), ((24, 24, 8), (4, 1, 1), (2, 2, 1), 4, 10)],
+                         ids=["16_of_16", "12_of_12", "9_of_9", "10_of_16"])
+def test_most_of_a_small_rank(native, monkeypatch, case, contrast):
+    """More than eight wanted vectors in blocks of at most 16: all or most of the ranks' spaces, floating ranks among
+    them; the bars of the test above."""
+    monkeypatch.setitem(CASES, "small", case)
+    test_coarse_orders(native, monkeypatch, "small", contrast)
