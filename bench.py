@@ -617,6 +617,8 @@ def _lv1_kernel(tune, prec, kind):
         if choice < nnat:
             return "k_ic_apply" + args
         return ("k_ic_apply_blk" if choice - nnat < 2 else "k_ic_apply_stg") + args
+    if kind == 0:  # not tuned where no blocked kernel applies: the first visit takes the other visits' choice
+        return _lv1_kernel(tune, prec, 1).split("<")[0] + args
     return "k_ic_apply" + args
 
 

@@ -34,3 +34,13 @@ def test_level1_kernel_names_follow_the_tuner_table():
     assert b._lv1_kernel(tune, "f64", 1) == "k_ic_apply_blk<double,1,1>"  # b2: last candidate is blocked 256
     # no tuned level-1 shape (tuning off): the natural-order kernel
     assert b._lv1_kernel({}, "f32", 1) == "k_ic_apply<float,1,1>"
+
+
+def test_level1_first_visit_without_a_blocked_kernel():
+    """Where only the natural-order and the warp kernel apply, the first visit has no row of its own and takes the
+    choice of the visits with an iterate."""
+    b = _bench()
+    us = [34.4, 29.7, 35.8, 39.9, 58.3, 28.7]
+    assert b._lv1_kernel({"ic_apply|f32|n512|c1728|l144|b0|w1|y1|f": [5, us]}, "f32", 0) == "k_ic_warp<float,0,0>"
+    assert b._lv1_kernel({"ic_apply|f32|n512|c1728|l144|b0|w1|y1|f": [1, us]}, "f32", 0) == "k_ic_apply<float,0,0>"
+    assert b._lv1_kernel({}, "f64", 0) == "k_ic_apply<double,0,0>"
