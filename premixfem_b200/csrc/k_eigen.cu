@@ -1474,7 +1474,6 @@ __global__ void k_eb_control(EbArgs a, int nlist, int it) {
   es.it = it + 1;  // iterations counted if the iteration limit ends the solve
   a.alist[atomicAdd(a.nactive, 1)] = s;  // order is irrelevant: subdomains are independent
   atomicAdd(a.nactive + 1, na);          // active columns: the preconditioner's work
-  atomicAdd(a.nactive + 2, es.nS);       // basis columns: the Gram's and the update's work
   if (a.colcells) atomicAdd(a.colcells, (unsigned long long)es.nS * (unsigned long long)nc);
 }
 

@@ -189,25 +189,6 @@ __device__ __forceinline__ double fixed_sum_wide(const double* part, int n, doub
   return block_sum(v, scratch);
 }
 
-__global__ void k_dot(const double* a, const double* b, long long n, double* part) {
-  __shared__ double red[32];
-  double v = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    v += a[i] * b[i];
-  v = block_sum(v, red);
-  if (threadIdx.x == 0) part[blockIdx.x] = v;
-}
-__global__ void k_fin_sum(const double* part, int n, double* out) {
-  __shared__ double red[32];
-  double v = fixed_sum(part, n, red);
-  if (threadIdx.x == 0) *out = v;
-}
-void launch_dot(const double* a, const double* b, long long n, double* part, double* out, cudaStream_t st) {
-  int nb = cell_blocks(n);
-  { note_launch(); k_dot<<<nb, kCellThreads, 0, st>>>(a, b, n, part); }
-  { note_launch(); k_fin_sum<<<1, 256, 0, st>>>(part, nb, out); }
-}
-
 // --- KSPSolve_CG (PETSc src/ksp/ksp/impls/cg/cg.c) with the unpreconditioned norm ---
 __global__ void k_pcg_start(long long n, const double* b, double* x, double* r, float* r32, double* part) {
   __shared__ double red[32];

@@ -76,7 +76,6 @@ void launch_pcg_iter_a(const Grid& g, const double* tx, const double* ty, const 
                        cudaStream_t st);
 void launch_pcg_iter_b(long long n, double* r, float* r32, const double* p, const double* w, double* part, PcgState* s,
                        cudaStream_t st);
-void launch_dot(const double* a, const double* b, long long n, double* part, double* out, cudaStream_t st);
 
 // ---- CG over a batch of problems (k_batch.cu): per-problem scalars, 2-D grids
 // (blocks x problems); all_done is set when every problem has stopped
@@ -172,14 +171,6 @@ void launch_prolong(const Grid& g, const SubInfo* subs, int nsub, int kmax, cons
                     const int* done, cudaStream_t st, int threads = 256);
 
 // ---- coarse (FP64) -------------------------------------------------------------
-// Where each virtual rank's coarse data live: rank r owns subdomains
-// first[r] .. first[r+1]-1 (contiguous), so nr_r = (first[r+1] - first[r]) x kmax
-// coarse dofs starting at first[r] x kmax; its dense nr_r x nr_r blocks start
-// at off2[r], its level-3 vectors (nr_r x en2) at offv[r], its level-3 work
-// (3 x nr_r x p) at offw[r].  A grid of ranks of equal size is the special case
-// first[r] = r spr, off2[r] = r nr^2 ...; a batch of problems has one rank per
-// problem and ragged sizes.  All arrays are device arrays of nrank + 1 entries;
-// dof_rank (nsub x kmax) maps a coarse dof to its rank.
 // kCoarseRows rows of one rank's coarse dofs: a CTA of the level-2 / level-3 products
 struct CoarseChunk {
   int rank, rows, nr, pad;
@@ -187,12 +178,19 @@ struct CoarseChunk {
   long long a_off, v_off;  // the chunk's first row in the dense blocks (off2) and in V (offv)
 };
 constexpr int kCoarseRows = 32;
+
+// Where each virtual rank's coarse data live: rank r owns subdomains
+// first[r] .. first[r+1]-1 (contiguous), so nr_r = (first[r+1] - first[r]) x kmax
+// coarse dofs starting at first[r] x kmax; its dense nr_r x nr_r blocks start
+// at off2[r], its level-3 vectors (nr_r x en2) at offv[r], its level-3 work
+// (3 x nr_r x p) at offw[r].  A grid of ranks of equal size is the special case
+// first[r] = r spr, off2[r] = r nr^2 ...; a batch of problems has one rank per
+// problem and ragged sizes.  All arrays are device arrays of nrank + 1 entries.
 struct RankLayout {
   const int* first = nullptr;
   const long long* off2 = nullptr;
   const long long* offv = nullptr;
   const long long* offw = nullptr;
-  const int* dof_rank = nullptr;
   int kmax = 0;
   // chunks of rank r: chunk_first[r] .. chunk_first[r+1]-1
   int nchunk = 0;
@@ -318,7 +316,7 @@ struct EbBuffers {
   double* Ybuf = nullptr;         // nsub x 32 x 32 Rayleigh-Ritz coefficients
   double* gpart = nullptr;        // nsub x nchunk x 2 x 32 x 32 partial Grams
   double* rpart = nullptr;        // nsub x nchunk x LB_MM partial residual norms
-  int* nactive = nullptr;         // device counter
+  int* nactive = nullptr;         // device: subdomains iterating, their active columns, [3] a copy that never landed
   int* alist = nullptr;           // nsub: compacted list of subdomains still iterating
   unsigned long long* colcells = nullptr;  // device: sum of (basis columns x cells) over sub-iterations
   double* phase_ms = nullptr;     // host, optional: accumulated ms of resid+control, preconditioner,

@@ -449,7 +449,7 @@ Solver::~Solver() {
   for (auto& e : prof_ev)
     if (e) cudaEventDestroy(e);
   for (void* q : {(void*)d_coff, ic_coef, (void*)d_woff, ic_wcoef, (void*)r32, (void*)d_kerr, (void*)phi64,
-                  (void*)d_rl_first, (void*)d_rl_off, (void*)d_rl_dof_rank, (void*)d_rl_chunk, (void*)d_rl_chunks,
+                  (void*)d_rl_first, (void*)d_rl_off, (void*)d_rl_chunk, (void*)d_rl_chunks,
                   (void*)d_probs, (void*)d_layer_prob})
     if (q) cudaFree(q);
   if (st) cudaStreamDestroy(st);
@@ -669,7 +669,7 @@ int Solver::rank_layout() {
     off[(nrank + 1) + r + 1] = off[(nrank + 1) + r] + n * en2;
     off[2 * (nrank + 1) + r + 1] = off[2 * (nrank + 1) + r] + 3 * n * l3p;
   }
-  std::vector<int> dof_rank((size_t)nsub * kmax), chunk(nrank + 1, 0);
+  std::vector<int> chunk(nrank + 1, 0);
   for (int r = 0; r < nrank; ++r)
     chunk[r + 1] = chunk[r] + ((rank_first[r + 1] - rank_first[r]) * kmax + kCoarseRows - 1) / kCoarseRows;
   const int nchunk = chunk[nrank];
@@ -682,17 +682,13 @@ int Solver::rank_layout() {
                               off[(nrank + 1) + r] + (long long)i * en2};
     }
   }
-  for (int r = 0; r < nrank; ++r)
-    for (long long g = (long long)rank_first[r] * kmax; g < (long long)rank_first[r + 1] * kmax; ++g) dof_rank[g] = r;
   int e = dalloc((void**)&d_rl_first, sizeof(int) * (nrank + 1), "rank layout");
   if (!e) e = dalloc((void**)&d_rl_off, sizeof(long long) * off.size(), "rank layout");
-  if (!e) e = dalloc((void**)&d_rl_dof_rank, sizeof(int) * dof_rank.size(), "rank layout");
   if (!e) e = dalloc((void**)&d_rl_chunk, sizeof(int) * chunk.size(), "rank layout");
   if (!e) e = dalloc((void**)&d_rl_chunks, sizeof(CoarseChunk) * chunks.size(), "rank layout");
   if (e) return e;
   cudaMemcpyAsync(d_rl_first, rank_first.data(), sizeof(int) * (nrank + 1), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(d_rl_off, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_rl_dof_rank, dof_rank.data(), sizeof(int) * dof_rank.size(), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(d_rl_chunk, chunk.data(), sizeof(int) * chunk.size(), cudaMemcpyHostToDevice, st);
   rl.chunk_first = d_rl_chunk;
   cudaMemcpyAsync(d_rl_chunks, chunks.data(), sizeof(CoarseChunk) * chunks.size(), cudaMemcpyHostToDevice, st);
@@ -702,14 +698,11 @@ int Solver::rank_layout() {
   rl.off2 = d_rl_off;
   rl.offv = d_rl_off + (nrank + 1);
   rl.offw = d_rl_off + 2 * (nrank + 1);
-  rl.dof_rank = d_rl_dof_rank;
   rl.kmax = kmax;
   // the host vectors must outlive the copies
   return check(cudaStreamSynchronize(st), "rank layout");
 }
 
-// cudaMalloc with its return code checked: on failure *p is null, err names
-// the array and the PETSc-style code 76 comes back.
 // The CG graphs hold addresses and launch shapes of what they were captured with.
 void Solver::drop_graphs() {
   if (pcg_exec) cudaGraphExecDestroy(pcg_exec);
@@ -717,6 +710,8 @@ void Solver::drop_graphs() {
   pcg_exec = bpcg_exec = nullptr;
 }
 
+// cudaMalloc with its return code checked: on failure *p is null, err names
+// the array and the PETSc-style code 76 comes back.
 int Solver::dalloc(void** p, size_t bytes, const char* what) {
   drop_graphs();  // the new buffer may replace one that they hold
   *p = nullptr;

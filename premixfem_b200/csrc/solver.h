@@ -139,7 +139,6 @@ class Solver {
   RankLayout rl;
   int* d_rl_first = nullptr;
   long long* d_rl_off = nullptr;  // off2, offv, offw: 3 x (nrank + 1)
-  int* d_rl_dof_rank = nullptr;
   int* d_rl_chunk = nullptr;
   CoarseChunk* d_rl_chunks = nullptr;
   void rank_sizes();   // host: nr, nr_min, en2, n3, l3p, tot2, totv, totw from rank_first
