@@ -225,6 +225,47 @@ void launch_lv3_solve(const RankLayout& L, int n3, int en2, const double* part, 
   { note_launch(); k_lv3_solve<<<L.nchunk, 256, smem, st>>>(L.chunks, L.chunk_first, n3, en2, gs, part, A3inv, V, dz, Z, first, done); }
 }
 
+// nv[s] = 1 / (value of subdomain s's first basis vector, a constant): the constant in the coarse space
+template <typename T>
+__global__ void k_null_coef(Grid g, const SubInfo* subs, int nsub, int kmax, const T* phi, double* nv) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= nsub) return;
+  const SubInfo& S = subs[s];
+  nv[s] = 1.0 / (double)phi[(((long long)S.z0 * g.N + S.y0) * g.M + S.x0) * kmax];
+}
+template <typename T>
+void launch_null_coef(const Grid& g, const SubInfo* subs, int nsub, int kmax, const T* phi, double* nv,
+                      cudaStream_t st) {
+  { note_launch(); k_null_coef<T><<<(nsub + 255) / 256, 256, 0, st>>>(g, subs, nsub, kmax, phi, nv); }
+}
+template void launch_null_coef<float>(const Grid&, const SubInfo*, int, int, const float*, double*, cudaStream_t);
+template void launch_null_coef<double>(const Grid&, const SubInfo*, int, int, const double*, double*, cudaStream_t);
+
+// c <- c - nv (nv.c) / (nv.nv).  nv.c is the sum of the residual, zero up to the rounding of the restriction, and
+// what is left of it the coarse solves multiply by up to 1e12 (the shift of the singular level-3 matrix).  One CTA:
+// a load or two per thread and pass, bound by its own latency (3 us for 2 244 subdomains).
+__global__ void __launch_bounds__(1024) k_coarse_project(int nsub, int kmax, const double* nv, double* c,
+                                                         const int* done) {
+  if (done && *done) return;
+  __shared__ double red[32];
+  double t = 0.0, nn = 0.0;
+  for (int s = threadIdx.x; s < nsub; s += 1024) {
+    const double v = nv[s];
+    t += v * c[(long long)s * kmax];
+    nn += v * v;
+  }
+  t = block_sum(t, red);
+  __syncthreads();
+  nn = block_sum(nn, red);
+  __shared__ double q;
+  if (threadIdx.x == 0) q = t / nn;
+  __syncthreads();
+  for (int s = threadIdx.x; s < nsub; s += 1024) c[(long long)s * kmax] -= q * nv[s];
+}
+void launch_coarse_project(int nsub, int kmax, const double* nv, double* c, const int* done, cudaStream_t st) {
+  { note_launch(); k_coarse_project<<<1, 1024, 0, st>>>(nsub, kmax, nv, c, done); }
+}
+
 __global__ void k_axpy(long long n, double a, const double* x, double* y, const int* done) {
   if (done && *done) return;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)

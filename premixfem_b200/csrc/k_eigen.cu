@@ -1233,14 +1233,19 @@ __global__ void __launch_bounds__(LB_THREADS) k_lobpcg(LobpcgArgs a, unsigned ch
     __syncthreads();
     const int num = sm.ival[1];
     if (threadIdx.x < k) evals[(long long)s * k + threadIdx.x] = sm.lam[threadIdx.x];
-    // FP32 storage: on a subdomain that touches no Dirichlet face, the lowest
-    // eigenvector of A_i^N v = lambda M_i v is exactly the constant (A_i^N 1 = 0),
-    // but FP32 iterations only reach it to ~1e-6.  Write the exact M-normalised
-    // constant instead, so that the coarse spaces contain the global null vector
-    // of a pure-Neumann operator exactly and its coarse pivot stays negligible.
+    // On a subdomain that touches no Dirichlet face the lowest eigenvector of
+    // A_i^N v = lambda M_i v is exactly the constant (A_i^N 1 = 0), but the iterations
+    // only reach it to the tolerance.  Write the exact M-normalised constant instead,
+    // so that the coarse spaces contain the global null vector of a pure-Neumann
+    // operator exactly and its share of a coarse residual can be taken out
+    // (k_coarse_project).  With a nearly exact one the coarse solves multiply that share
+    // by up to 1e12, and the rounding of the result ends the CG's progress: on the
+    // layered field of contrast 1e6, twelve seeds, at 1e-13 to 2e-8 of the right-hand
+    // side in FP64 and 2e-12 to 1e-8 in the mixed form on an FP64 basis, now at 1e-13
+    // to 4e-11 in every form.
     bool snap = false;
     double cval = 0.0;
-    if (sizeof(T) == 4 && num >= 1) {
+    if (num >= 1) {
       const bool touches = touches_dirichlet(eg, S);
       if (!touches) {
         double msum = 0.0, vsum = 0.0;
@@ -1900,11 +1905,11 @@ __global__ void __launch_bounds__(256) k_eb_fin_rr(EbArgs a, double eb, int dmas
     const int r = e / m, c = e % m;
     Y[r * LB_LD + c] = mt.Y[r * LB_LD + c];
   }
-  // FP32 storage, subdomain touching no Dirichlet face: the lowest vector is
-  // the constant; write it exactly (M-normalised, sign of the computed one)
+  // a subdomain touching no Dirichlet face: the lowest vector is the constant; write
+  // it exactly (M-normalised, sign of the computed one), as k_lobpcg explains
   bool snap = false;
   double cval = 0.0;
-  if (sizeof(T) == 4 && num >= 1) {
+  if (num >= 1) {
     const bool touches = touches_dirichlet(eig_geom(a.probs, a.g, 0.0, 0.0, 0.0, 0.0, dmask, S), S);
     if (!touches) {
       EbSlab<T> sl(a.slab + (size_t)s * a.slab_stride, a.m, a.ld);

@@ -421,7 +421,7 @@ int Solver::upload_probs() {
 Solver::~Solver() {
   if (st) cudaStreamSynchronize(st);
   void* ptrs[] = {d_subs, kx,    ky,    kz,    tx,     ty,    tz,     diag,     db,       bval,    tx32,  ty32,
-                  tz32,   diag32, inv32, inv64, phi,    blk,   gface,  A2inv,    AN,       ANinv,   V3,    A3inv, a3part,
+                  tz32,   diag32, inv32, inv64, phi,    blk,   gface,  A2inv,    AN,       ANinv,   V3,    A3inv, a3part, nullv,
                   d_eig1, d_eig3, d_ks,  d_iters, d_status, d_l3it, d_flag, d_rank_nb, eig_work, c,     dz,    Zacc,
                   l3part, y0,    y1,    vb,     vx,    r,      z,        p0,       p1,      w,     part,
                   state};
@@ -1250,6 +1250,7 @@ int Solver::setup() {
                       {(void**)&A3inv, sizeof(double) * n3 * n3, "level-3 inverse"},
                       {(void**)&a3part, sizeof(double) * nrank * 7 * ((spr + kA3Chunk - 1) / kA3Chunk) * en2 * en2,
                        "level-3 partial blocks"},
+                      {(void**)&nullv, sizeof(double) * nsub, "coarse null vector"},
                       {(void**)&c, sizeof(double) * nsub * kmax, "coarse residual"},
                       {(void**)&dz, sizeof(double) * nsub * kmax, "coarse correction"},
                       {(void**)&Zacc, sizeof(double) * nsub * kmax, "coarse accumulator"},
@@ -1277,6 +1278,10 @@ int Solver::setup() {
     launch_galerkin<float>(g, d_subs, nsub, kmax, tx, ty, tz, diag, (const float*)phi, blk, gface, st);
   else
     launch_galerkin<double>(g, d_subs, nsub, kmax, tx, ty, tz, diag, (const double*)phi, blk, gface, st);
+  if (mixed)
+    launch_null_coef<float>(g, d_subs, nsub, kmax, (const float*)phi, nullv, st);
+  else
+    launch_null_coef<double>(g, d_subs, nsub, kmax, (const double*)phi, nullv, st);
   auto finish = [&]() -> int {
     if (int er = check(cudaStreamSynchronize(st), "coarse setup")) return er;
     if (int er = check(cudaGetLastError(), "coarse setup launch")) return er;
@@ -1707,7 +1712,7 @@ void Solver::tune_pc() {
 }
 
 template <typename T>
-void Solver::apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done) {
+void Solver::apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done, bool project) {
   const bool f32 = sizeof(T) == 4;
   const T* ttx = f32 ? (const T*)tx32 : (const T*)tx;
   const T* tty = f32 ? (const T*)ty32 : (const T*)ty;
@@ -1759,6 +1764,7 @@ void Solver::apply_impl(const double* x, const T* xt, double* out, double* parti
         launch_resid_restrict<T>(g, d_subs, nsub, kmax, ttx, tty, ttz, tdg, tphi, xt, y_zero ? nullptr : yb[cur], c,
                                  done, st, rr_threads);
         prof_mark(PROF_RESTRICT);
+        if (project) launch_coarse_project(nsub, kmax, nullv, c, done, st);
         c_valid = true;
       }
       if (v == 3) {
@@ -1960,7 +1966,7 @@ int Solver::profile_iteration(int reps, double ms[PROF_SLOTS], int launches[PROF
     prof_mark(PROF_CG_A);
     launch_pcg_iter_b(g.ncell, vb, r32, p1, w, part, state, st);
     prof_mark(PROF_CG_B);
-    apply(vb, z, part, nullptr);
+    apply(vb, z, part, nullptr, singular());
     if (opt.null_space)
       launch_pcg_null_beta(z, vb, g.ncell, part, zpart, state, LoopCond(), st);
     else
@@ -1984,11 +1990,13 @@ int Solver::profile_iteration(int reps, double ms[PROF_SLOTS], int launches[PROF
 }
 
 // In the mixed form r32 holds x in FP32 (written by the CG kernels with the residual).
-void Solver::apply(const double* x, double* out, double* partial, const int* done) {
+// project: x is a residual of a singular operator (-ksp_constant_null_space without a
+// Dirichlet face), whose sum is zero.
+void Solver::apply(const double* x, double* out, double* partial, const int* done, bool project) {
   if (opt.precision == 1)
-    apply_impl<float>(x, r32, out, partial, done);
+    apply_impl<float>(x, r32, out, partial, done, project);
   else
-    apply_impl<double>(x, x, out, partial, done);
+    apply_impl<double>(x, x, out, partial, done, project);
 }
 
 int Solver::rhs(const double* source, double* out, bool on_device) {
@@ -2077,7 +2085,8 @@ int Solver::solve(const double* b_in, double* x_out, bool on_device, int* its, d
     else
       launch_pcg_beta_fin(part, nparts_apply(), state, loop, st);
   };
-  apply(r, z, part, done);
+  const bool project = singular();
+  apply(r, z, part, done, project);
   beta(LoopCond());
   double* pin = p0;
   double* pout = p1;
@@ -2086,7 +2095,7 @@ int Solver::solve(const double* b_in, double* x_out, bool on_device, int* its, d
     for (int c_ = 0; c_ < chunk; ++c_) {
       launch_pcg_iter_a(g, tx, ty, tz, diag, z, pin, pout, w, part, state, st);
       launch_pcg_iter_b(g.ncell, r, r32, pout, w, part, state, st);
-      apply(r, z, part, done);
+      apply(r, z, part, done, project);
       beta(loop);
       std::swap(pin, pout);
     }
@@ -2097,11 +2106,12 @@ int Solver::solve(const double* b_in, double* x_out, bool on_device, int* its, d
   // their roles.
   const bool use_graph = opt.pcg_graph && chunk % 2 == 0;
   if (use_graph) {
-    if (!pcg_exec || pcg_graph_ns != opt.null_space) {
+    if (!pcg_exec || pcg_graph_ns != opt.null_space || pcg_graph_project != project) {
       if (pcg_exec) cudaGraphExecDestroy(pcg_exec);
       pcg_exec = nullptr;
       if (int e = loop_graph(&pcg_exec, &pcg_graph_kernels, enqueue_chunk)) return e;
       pcg_graph_ns = opt.null_space;
+      pcg_graph_project = project;
     }
     if (int e = check(cudaGraphLaunch(pcg_exec, st), "graph launch")) return e;
     cudaMemcpyAsync(h_state, state, sizeof(PcgState), cudaMemcpyDeviceToHost, st);

@@ -126,7 +126,7 @@ class Solver {
   long long band_len = 0;
   void* phi = nullptr;
   double *blk = nullptr, *gface = nullptr, *A2inv = nullptr, *AN = nullptr, *ANinv = nullptr, *V3 = nullptr,
-         *A3inv = nullptr, *a3part = nullptr, *d_eig1 = nullptr, *d_eig3 = nullptr;
+         *A3inv = nullptr, *a3part = nullptr, *nullv = nullptr, *d_eig1 = nullptr, *d_eig3 = nullptr;
   int *d_ks = nullptr, *d_iters = nullptr, *d_status = nullptr, *d_l3it = nullptr, *d_flag = nullptr;
   int* d_rank_nb = nullptr;
   bool coarse_ok = false;  // the level-2/3 arrays above are allocated
@@ -182,10 +182,16 @@ class Solver {
   int alloc_fine();
   void assemble_launch();
   template <typename T>
-  void apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done);
-  void apply(const double* x, double* out, double* partial, const int* done);
+  void apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done, bool project);
+  void apply(const double* x, double* out, double* partial, const int* done, bool project = false);
   std::vector<int> schedule() const;
   int dir_on_[6] = {0, 0, 0, 0, 0, 0};
+  // the constant is the operator's null space and the solve says so
+  bool singular() const {
+    for (int on : dir_on_)
+      if (on) return false;
+    return opt.null_space;
+  }
   double dir_val_[6] = {0, 0, 0, 0, 0, 0};
   double last_setup_ms = 0, last_solve_ms = 0;
   int last_its = 0;
@@ -197,7 +203,8 @@ class Solver {
   EbBuffers eb;  // phase-batched eigensolver storage
   double eig_phase_ms[8] = {0};
   cudaGraphExec_t pcg_exec = nullptr;  // PCG iterations, repeated on the device
-  bool pcg_graph_ns = false;  // the null-space setting the graph was captured with
+  // the null-space setting the graph was captured with, and whether its coarse residuals are projected
+  bool pcg_graph_ns = false, pcg_graph_project = false;
   unsigned long long pcg_graph_kernels = 0;
   unsigned long long eig_colcells = 0;
   int alloc_eb(int m, bool mixed);

@@ -46,3 +46,26 @@ def test_constant_null_space_option_values(native):
     with pytest.raises(PmfError) as e:
         DarcySolver((1.0, 1.0, 1.0), (8, 8, 8), "-sd 2 -ksp_constant_null_space maybe")
     assert e.value.code == 62
+
+
+@pytest.mark.parametrize("form", [{"pmf_precision": "fp64"}, {"pmf_precision": "mixed"},
+                                  {"pmf_precision": "mixed", "pmf_eig_precision": "fp64"}],
+                         ids=["fp64", "mixed", "mixed_fp64_basis"])
+@pytest.mark.parametrize("seed", [1, 2, 3, 4])
+def test_constant_is_in_the_coarse_space(native, seed, form):
+    """Channels of contrast 1e6 without a Dirichlet face: every subdomain's first basis vector is the constant to the
+    last bits, so that the coarse operator's null vector is the operator's own, and CG gets to 1e-10 of the right-hand
+    side."""
+    prob = fields.layered(seed=seed, M=30, N=44, P=30, smooth_layers=10)
+    s = DarcySolver.from_problem(prob, options_string(dict(form, pmf_vranks=(2, 2, 1), pmf_sd=(2, 2, 6), en_lv1=4,
+                                                           en_lv2=4, ksp_constant_null_space=True, ksp_rtol=1e-10,
+                                                           ksp_max_it=2000)))
+    s.setup()
+    phi = s.phi()[:, 0].reshape(prob["kappa"][0].shape)
+    boxes, _ = s.subdomains()
+    for x0, nx, y0, ny, z0, nz in boxes:
+        v = phi[z0:z0 + nz, y0:y0 + ny, x0:x0 + nx]
+        assert np.ptp(v) <= 1e-13 * np.abs(v).max()
+    _, its, _, reason = s.solve(s.rhs(prob["source"].ravel()))
+    s.close()
+    assert reason == "converged", its
