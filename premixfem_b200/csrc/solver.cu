@@ -1990,8 +1990,7 @@ int Solver::profile_iteration(int reps, double ms[PROF_SLOTS], int launches[PROF
 }
 
 // In the mixed form r32 holds x in FP32 (written by the CG kernels with the residual).
-// project: x is a residual of a singular operator (-ksp_constant_null_space without a
-// Dirichlet face), whose sum is zero.
+// project: x is a residual of a singular operator, whose sum is zero.
 void Solver::apply(const double* x, double* out, double* partial, const int* done, bool project) {
   if (opt.precision == 1)
     apply_impl<float>(x, r32, out, partial, done, project);

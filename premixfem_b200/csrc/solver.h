@@ -186,11 +186,11 @@ class Solver {
   void apply(const double* x, double* out, double* partial, const int* done, bool project = false);
   std::vector<int> schedule() const;
   int dir_on_[6] = {0, 0, 0, 0, 0, 0};
-  // the constant is the operator's null space and the solve says so
+  // no Dirichlet face: the constant is the operator's null space, whether or not the solve projects z
   bool singular() const {
     for (int on : dir_on_)
       if (on) return false;
-    return opt.null_space;
+    return true;
   }
   double dir_val_[6] = {0, 0, 0, 0, 0, 0};
   double last_setup_ms = 0, last_solve_ms = 0;

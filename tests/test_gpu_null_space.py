@@ -69,3 +69,20 @@ def test_constant_is_in_the_coarse_space(native, seed, form):
     _, its, _, reason = s.solve(s.rhs(prob["source"].ravel()))
     s.close()
     assert reason == "converged", its
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("seed", [1, 2, 3, 4])
+def test_singular_operator_without_the_option(native, seed, precision):
+    """The same channels without -ksp_constant_null_space and with the default shift of the level-3 matrix, which the
+    coarse solve multiplies the constant by 1e12 with: a consistent right-hand side is solved to the default 1e-8."""
+    prob = fields.layered(seed=seed, M=30, N=44, P=30, smooth_layers=10)
+    s = DarcySolver.from_problem(prob, options_string(dict(sd=3, en_lv1=4, en_lv2=4, pmf_precision=precision,
+                                                           ksp_max_it=600)))
+    s.setup()
+    b = s.rhs(prob["source"].ravel())
+    x, its, _, reason = s.solve(b)
+    r = b - s.apply_A(x)
+    s.close()
+    assert reason == "converged", its
+    assert np.linalg.norm(r) <= 1.1e-8 * np.linalg.norm(b)
