@@ -243,13 +243,16 @@ template void launch_null_coef<double>(const Grid&, const SubInfo*, int, int, co
 
 // c <- c - nv (nv.c) / (nv.nv).  nv.c is the sum of the residual, zero up to the rounding of the restriction, and
 // what is left of it the coarse solves multiply by up to 1e12 (the shift of the singular level-3 matrix).  One CTA:
-// a load or two per thread and pass, bound by its own latency (3 us for 2 244 subdomains).
-__global__ void __launch_bounds__(1024) k_coarse_project(int nsub, int kmax, const double* nv, double* c,
-                                                         const int* done) {
+// a load or two per thread and pass, bound by its own latency (3 us for 2 244 subdomains).  A batch has one CTA
+// per problem, whose subdomains are a rank's; problems with a Dirichlet face are left alone.
+__global__ void __launch_bounds__(1024) k_coarse_project(int nsub, int kmax, const int* first, const ProbInfo* probs,
+                                                         const double* nv, double* c, const int* done) {
   if (done && *done) return;
+  if (probs && probs[blockIdx.x].dmask) return;
+  const int s0 = probs ? first[blockIdx.x] : 0, s1 = probs ? first[blockIdx.x + 1] : nsub;
   __shared__ double red[32];
   double t = 0.0, nn = 0.0;
-  for (int s = threadIdx.x; s < nsub; s += 1024) {
+  for (int s = s0 + threadIdx.x; s < s1; s += 1024) {
     const double v = nv[s];
     t += v * c[(long long)s * kmax];
     nn += v * v;
@@ -260,10 +263,11 @@ __global__ void __launch_bounds__(1024) k_coarse_project(int nsub, int kmax, con
   __shared__ double q;
   if (threadIdx.x == 0) q = t / nn;
   __syncthreads();
-  for (int s = threadIdx.x; s < nsub; s += 1024) c[(long long)s * kmax] -= q * nv[s];
+  for (int s = s0 + threadIdx.x; s < s1; s += 1024) c[(long long)s * kmax] -= q * nv[s];
 }
-void launch_coarse_project(int nsub, int kmax, const double* nv, double* c, const int* done, cudaStream_t st) {
-  { note_launch(); k_coarse_project<<<1, 1024, 0, st>>>(nsub, kmax, nv, c, done); }
+void launch_coarse_project(int nsub, int kmax, const RankLayout& L, const ProbInfo* probs, int nprob, const double* nv,
+                           double* c, const int* done, cudaStream_t st) {
+  { note_launch(); k_coarse_project<<<probs ? nprob : 1, 1024, 0, st>>>(nsub, kmax, L.first, probs, nv, c, done); }
 }
 
 __global__ void k_axpy(long long n, double a, const double* x, double* y, const int* done) {

@@ -216,11 +216,12 @@ void launch_add_diag_r(const RankLayout& L, int nrank, double* dense, double mu,
 bool launch_spd_inverse_r(const RankLayout& L, int nrank, int nr_max, double* dense, double tol, int* nnull,
                           cudaStream_t st);
 // The operator's constant null space in the coarse space: nv (nsub values) from the first basis vectors, which are
-// constants; c <- c - nv (nv.c) / (nv.nv)
+// constants; c <- c - nv (nv.c) / (nv.nv), in a batch per problem without a Dirichlet face
 template <typename T>
 void launch_null_coef(const Grid& g, const SubInfo* subs, int nsub, int kmax, const T* phi, double* nv,
                       cudaStream_t st);
-void launch_coarse_project(int nsub, int kmax, const double* nv, double* c, const int* done, cudaStream_t st);
+void launch_coarse_project(int nsub, int kmax, const RankLayout& L, const ProbInfo* probs, int nprob, const double* nv,
+                           double* c, const int* done, cudaStream_t st);
 void launch_axpy(long long n, double a, const double* x, double* y, const int* done, cudaStream_t st);
 void launch_copy(long long n, const double* x, double* y, const int* done, cudaStream_t st);
 

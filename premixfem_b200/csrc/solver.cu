@@ -1764,7 +1764,7 @@ void Solver::apply_impl(const double* x, const T* xt, double* out, double* parti
         launch_resid_restrict<T>(g, d_subs, nsub, kmax, ttx, tty, ttz, tdg, tphi, xt, y_zero ? nullptr : yb[cur], c,
                                  done, st, rr_threads);
         prof_mark(PROF_RESTRICT);
-        if (project) launch_coarse_project(nsub, kmax, nullv, c, done, st);
+        if (project) launch_coarse_project(nsub, kmax, rl, d_probs, nprob, nullv, c, done, st);
         c_valid = true;
       }
       if (v == 3) {
@@ -1829,7 +1829,7 @@ int Solver::solve_batch(const double* b_in, double* x_out, bool on_device, int* 
   const int nblk = bpcg_blocks();
   cudaEventRecord(ev0, st);
   launch_bpcg_start(d_probs, nprob, bs, xs, r, r32, part, bstate, opt.rtol, opt.atol, opt.max_it, d_all_done, nblk, st);
-  apply(r, z, part, d_all_done);
+  apply(r, z, part, d_all_done, singular());
   launch_bpcg_beta(d_probs, nprob, part, bstate, st);
   double* pin = p0;
   double* pout = p1;
@@ -1838,7 +1838,7 @@ int Solver::solve_batch(const double* b_in, double* x_out, bool on_device, int* 
     for (int c_ = 0; c_ < chunk; ++c_) {
       launch_bpcg_iter_a(g, d_probs, d_layer_prob, nprob, tx, ty, tz, diag, z, pin, pout, w, part, bstate, st);
       launch_bpcg_iter_b(g, d_probs, d_layer_prob, nprob, r, r32, pout, w, part, bstate, d_all_done, loop, st);
-      apply(r, z, part, d_all_done);
+      apply(r, z, part, d_all_done, singular());
       launch_bpcg_beta(d_probs, nprob, part, bstate, st);
       std::swap(pin, pout);
     }

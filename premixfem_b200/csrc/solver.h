@@ -187,7 +187,11 @@ class Solver {
   std::vector<int> schedule() const;
   int dir_on_[6] = {0, 0, 0, 0, 0, 0};
   // no Dirichlet face: the constant is the operator's null space, whether or not the solve projects z
+  // (a batch: of at least one problem)
   bool singular() const {
+    for (const ProbInfo& p : probs)
+      if (!p.dmask) return true;
+    if (nprob) return false;
     for (int on : dir_on_)
       if (on) return false;
     return true;

@@ -86,3 +86,22 @@ def test_singular_operator_without_the_option(native, seed, precision):
     s.close()
     assert reason == "converged", its
     assert np.linalg.norm(r) <= 1.1e-8 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("seed", [1, 3, 5])
+def test_batch_of_singular_problems(native, seed, precision):
+    """Three channel problems without a Dirichlet face and one with, in one batch (which has no null space option): each
+    converges to the default 1e-8."""
+    from premixfem_b200.solver import BatchSolver
+    probs = [fields.layered(seed=seed * 10 + q, M=18 + 2 * q, N=24, P=16, smooth_layers=5) for q in range(4)]
+    probs[2]["dirichlet"] = {"z-": 1.0}
+    rng = np.random.default_rng(seed)
+    srcs = [v - v.mean() for v in (rng.standard_normal(p["source"].shape) for p in probs)]
+    s = BatchSolver(probs, [tuple(-(-n // 8) for n in p["mesh"]) for p in probs],
+                    options_string({"en_lv1": 4, "en_lv2": 3, "pmf_precision": precision, "ksp_max_it": 800}))
+    s.set_kappa(*[s.pack([p["kappa"][d] for p in probs]) for d in range(3)])
+    s.setup()
+    _, its, _, reason = s.solve(s.rhs(s.pack(srcs)))
+    s.close()
+    assert list(reason) == ["converged"] * 4, (its, reason)
