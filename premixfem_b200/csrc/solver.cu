@@ -1712,8 +1712,8 @@ void Solver::tune_pc() {
 }
 
 template <typename T>
-void Solver::apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done, bool project) {
-  const bool f32 = sizeof(T) == 4;
+void Solver::apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done) {
+  const bool f32 = sizeof(T) == 4, project = singular();
   const T* ttx = f32 ? (const T*)tx32 : (const T*)tx;
   const T* tty = f32 ? (const T*)ty32 : (const T*)ty;
   const T* ttz = f32 ? (const T*)tz32 : (const T*)tz;
@@ -1829,7 +1829,7 @@ int Solver::solve_batch(const double* b_in, double* x_out, bool on_device, int* 
   const int nblk = bpcg_blocks();
   cudaEventRecord(ev0, st);
   launch_bpcg_start(d_probs, nprob, bs, xs, r, r32, part, bstate, opt.rtol, opt.atol, opt.max_it, d_all_done, nblk, st);
-  apply(r, z, part, d_all_done, singular());
+  apply(r, z, part, d_all_done);
   launch_bpcg_beta(d_probs, nprob, part, bstate, st);
   double* pin = p0;
   double* pout = p1;
@@ -1838,7 +1838,7 @@ int Solver::solve_batch(const double* b_in, double* x_out, bool on_device, int* 
     for (int c_ = 0; c_ < chunk; ++c_) {
       launch_bpcg_iter_a(g, d_probs, d_layer_prob, nprob, tx, ty, tz, diag, z, pin, pout, w, part, bstate, st);
       launch_bpcg_iter_b(g, d_probs, d_layer_prob, nprob, r, r32, pout, w, part, bstate, d_all_done, loop, st);
-      apply(r, z, part, d_all_done, singular());
+      apply(r, z, part, d_all_done);
       launch_bpcg_beta(d_probs, nprob, part, bstate, st);
       std::swap(pin, pout);
     }
@@ -1966,7 +1966,7 @@ int Solver::profile_iteration(int reps, double ms[PROF_SLOTS], int launches[PROF
     prof_mark(PROF_CG_A);
     launch_pcg_iter_b(g.ncell, vb, r32, p1, w, part, state, st);
     prof_mark(PROF_CG_B);
-    apply(vb, z, part, nullptr, singular());
+    apply(vb, z, part, nullptr);
     if (opt.null_space)
       launch_pcg_null_beta(z, vb, g.ncell, part, zpart, state, LoopCond(), st);
     else
@@ -1990,12 +1990,13 @@ int Solver::profile_iteration(int reps, double ms[PROF_SLOTS], int launches[PROF
 }
 
 // In the mixed form r32 holds x in FP32 (written by the CG kernels with the residual).
-// project: x is a residual of a singular operator, whose sum is zero.
-void Solver::apply(const double* x, double* out, double* partial, const int* done, bool project) {
+// Of a singular operator every application has its coarse residuals projected, a caller's own as well: the residuals
+// of a consistent system have no share of the constant, and what rounding puts there must not be amplified.
+void Solver::apply(const double* x, double* out, double* partial, const int* done) {
   if (opt.precision == 1)
-    apply_impl<float>(x, r32, out, partial, done, project);
+    apply_impl<float>(x, r32, out, partial, done);
   else
-    apply_impl<double>(x, x, out, partial, done, project);
+    apply_impl<double>(x, x, out, partial, done);
 }
 
 int Solver::rhs(const double* source, double* out, bool on_device) {
@@ -2084,8 +2085,7 @@ int Solver::solve(const double* b_in, double* x_out, bool on_device, int* its, d
     else
       launch_pcg_beta_fin(part, nparts_apply(), state, loop, st);
   };
-  const bool project = singular();
-  apply(r, z, part, done, project);
+  apply(r, z, part, done);
   beta(LoopCond());
   double* pin = p0;
   double* pout = p1;
@@ -2094,7 +2094,7 @@ int Solver::solve(const double* b_in, double* x_out, bool on_device, int* its, d
     for (int c_ = 0; c_ < chunk; ++c_) {
       launch_pcg_iter_a(g, tx, ty, tz, diag, z, pin, pout, w, part, state, st);
       launch_pcg_iter_b(g.ncell, r, r32, pout, w, part, state, st);
-      apply(r, z, part, done, project);
+      apply(r, z, part, done);
       beta(loop);
       std::swap(pin, pout);
     }
@@ -2105,12 +2105,12 @@ int Solver::solve(const double* b_in, double* x_out, bool on_device, int* its, d
   // their roles.
   const bool use_graph = opt.pcg_graph && chunk % 2 == 0;
   if (use_graph) {
-    if (!pcg_exec || pcg_graph_ns != opt.null_space || pcg_graph_project != project) {
+    if (!pcg_exec || pcg_graph_ns != opt.null_space || pcg_graph_project != singular()) {
       if (pcg_exec) cudaGraphExecDestroy(pcg_exec);
       pcg_exec = nullptr;
       if (int e = loop_graph(&pcg_exec, &pcg_graph_kernels, enqueue_chunk)) return e;
       pcg_graph_ns = opt.null_space;
-      pcg_graph_project = project;
+      pcg_graph_project = singular();
     }
     if (int e = check(cudaGraphLaunch(pcg_exec, st), "graph launch")) return e;
     cudaMemcpyAsync(h_state, state, sizeof(PcgState), cudaMemcpyDeviceToHost, st);

@@ -182,11 +182,11 @@ class Solver {
   int alloc_fine();
   void assemble_launch();
   template <typename T>
-  void apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done, bool project);
-  void apply(const double* x, double* out, double* partial, const int* done, bool project = false);
+  void apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done);
+  void apply(const double* x, double* out, double* partial, const int* done);
   std::vector<int> schedule() const;
   int dir_on_[6] = {0, 0, 0, 0, 0, 0};
-  // no Dirichlet face: the constant is the operator's null space, whether or not the solve projects z
+  // no Dirichlet face: the constant is the operator's null space, whether or not the caller projects z
   // (a batch: of at least one problem)
   bool singular() const {
     for (const ProbInfo& p : probs)

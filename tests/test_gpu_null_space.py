@@ -88,6 +88,40 @@ def test_singular_operator_without_the_option(native, seed, precision):
     assert np.linalg.norm(r) <= 1.1e-8 * np.linalg.norm(b)
 
 
+@pytest.mark.parametrize("project", [True, False], ids=["null_space", "plain"])
+@pytest.mark.parametrize("form", [{"pmf_precision": "fp64"}, {"pmf_precision": "mixed"},
+                                  {"pmf_precision": "mixed", "pmf_eig_precision": "fp64"}],
+                         ids=["fp64", "mixed", "mixed_fp64_basis"])
+@pytest.mark.parametrize("seed", [1, 2, 5])
+def test_callers_own_cg_on_a_singular_operator(native, seed, form, project):
+    """CG of a caller's own through apply_A and pc_apply on the same channels, with and without the null space taken out
+    of z: the 1e-8 that the library's own solve reaches, in its iterations give or take a tenth."""
+    prob = fields.layered(seed=seed, M=30, N=44, P=30, smooth_layers=10)
+    s = DarcySolver.from_problem(prob, options_string(dict(form, sd=3, en_lv1=4, en_lv2=4, ksp_max_it=600,
+                                                           ksp_constant_null_space=project)))
+    s.setup()
+    b = s.rhs(prob["source"].ravel())
+    _, its, _, reason = s.solve(b)
+    assert reason == "converged"
+
+    def precondition(r):
+        z = s.pc_apply(r)
+        return z - z.mean() if project else z
+
+    x, r = np.zeros_like(b), b.copy()
+    p = z = precondition(r)
+    rz, n = r @ z, 0
+    while np.linalg.norm(r) > 1e-8 * np.linalg.norm(b) and n < 1.1 * its:
+        w = s.apply_A(p)
+        x, r, n = x + rz / (p @ w) * p, r - rz / (p @ w) * w, n + 1
+        z = precondition(r)
+        rz, old = r @ z, rz
+        p = z + rz / old * p
+    r = b - s.apply_A(x)
+    s.close()
+    assert np.linalg.norm(r) <= 1.1e-8 * np.linalg.norm(b), n
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("seed", [1, 3, 5])
 def test_batch_of_singular_problems(native, seed, precision):
