@@ -222,6 +222,9 @@ void launch_null_coef(const Grid& g, const SubInfo* subs, int nsub, int kmax, co
                       cudaStream_t st);
 void launch_coarse_project(int nsub, int kmax, const RankLayout& L, const ProbInfo* probs, int nprob, const double* nv,
                            double* c, const int* done, cudaStream_t st);
+// the dense blocks of ranks that hold a whole singular problem made regular along nv
+void launch_lift_null(int nrank, const RankLayout& L, const ProbInfo* probs, const double* nv, double* dense,
+                      cudaStream_t st);
 void launch_axpy(long long n, double a, const double* x, double* y, const int* done, cudaStream_t st);
 void launch_copy(long long n, const double* x, double* y, const int* done, cudaStream_t st);
 

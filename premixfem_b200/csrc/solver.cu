@@ -1319,6 +1319,7 @@ int Solver::setup() {
     return finish();
   }
   launch_assemble_dense_r(d_subs, nrank, rl, tot2, blk, gface, 0, A2inv, st);
+  if (singular() && (nprob || nrank == 1)) launch_lift_null(nrank, rl, d_probs, nullv, A2inv, st);
   auto no_scratch = [&]() {
     err = "not enough device memory for the scratch of the coarse inverses";
     return 76;

@@ -123,6 +123,26 @@ def test_callers_own_cg_on_a_singular_operator(native, seed, form, project):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("mesh,sd,seed", [((20, 22, 18), 5, 2), ((20, 22, 18), 5, 8), ((16, 16, 16), 4, 4),
+                                          ((30, 28, 26), 6, 3)], ids=lambda v: str(v).replace(", ", "x"))
+def test_one_rank_holds_the_singular_problem(native, mesh, sd, seed, precision):
+    """A single rank's coarse block is the whole singular operator's: its inverse must not depend on how the rounding of
+    its last pivot falls.  Iterations within +-1 of the oracle's."""
+    prob = fields.random_box(mesh, seed=seed, sigma=1.5)
+    prob["dirichlet"] = {}
+    src = np.random.default_rng(seed).standard_normal(prob["kappa"][0].shape)
+    prob["source"] = src - src.mean()
+    d = {"sd": sd, "en_lv1": 4, "en_lv2": 4}
+    ref = O.solve(prob, O.Options(**d, constant_null_space=True))
+    s = DarcySolver.from_problem(prob, options_string(dict(d, pmf_precision=precision, ksp_constant_null_space=True,
+                                                           ksp_max_it=100)))
+    s.setup()
+    _, its, _, reason = s.solve(s.rhs(prob["source"].ravel()))
+    s.close()
+    assert reason == "converged" and abs(its - ref["its"]) <= 1, (its, ref["its"])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("seed", [1, 3, 5])
 def test_batch_of_singular_problems(native, seed, precision):
     """Three channel problems without a Dirichlet face and one with, in one batch (which has no null space option): each
