@@ -96,7 +96,7 @@ WORKLOADS = {
              "channels (contrast 1e6), +/-1 injector/producer columns, no-flux walls (-ksp_constant_null_space); "
              "6x22x17 subdomains of 10x10x5 on a 2x2x1 virtual rank grid, en_lv1=4, en_lv2=4; the mixed form "
              "computes the local basis in FP64 (-pmf_eig_precision fp64: with the FP32 eigensolver's 1e-6 "
-             "residual the near-zero channel modes are too inexact and CG stalls)",
+             "residual the near-zero channel modes are inexact and CG takes up to a third more iterations)",
         mixed_opts={"pmf_eig_precision": "fp64"},
         # the pure-Neumann operator's FP64 CG levels off between 1e-11 and 1e-10 (1e-11 was not reached in
         # 20 000 iterations); solutions are compared modulo constants

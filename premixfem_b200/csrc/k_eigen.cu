@@ -341,7 +341,7 @@ __device__ __forceinline__ void stv(double* p, const double (&v)[N]) {
 // * 32 doubles.
 //
 // Bound by HBM where many subdomains iterate (per cell and column a value and an
-// FP64 image): all Grams of a 256^3 set-up take 26.9 ms (36.0 with one value per
+// FP64 image): all Grams of a 256^3 set-up take 26.5 ms (36.0 with one value per
 // load and one tile per product; their bytes need 17), of one with blocks of ten
 // columns 31.4 (67.8).  Loading a step ahead in halves of the step costs more than
 // it hides (34.1).
@@ -1633,7 +1633,7 @@ __global__ void __launch_bounds__(256) k_eb_aimg(EbArgs a) {
 // couplings, the values of three planes stay in registers, and the planes in use
 // stay in L1.  A column per CTA and a cell at a time widens thirteen FP32 values
 // per result at sixteen per clock and SM, this 6.25.  All images and residual norms
-// of a 256^3 set-up: 29.1 ms instead of 46.9 (their bytes need 13); with a chunk of
+// of a 256^3 set-up: 27 to 29 ms instead of 46.9 (their bytes need 13); with a chunk of
 // cells and all columns per CTA, couplings widened once, the planes of sixteen
 // columns do not stay in L1: 44.5.  In FP64 storage at 150^3 this, the update and the
 // control step take 24.5 ms, 24.8 with the images combined and the residuals apart.

@@ -148,7 +148,7 @@ __device__ __forceinline__ T apply_A(const Grid& g, long long c, int ex, int ey,
   return v;
 }
 
-// 135 us at 256^3 (5.96 TB/s of its 48 B per cell); one cell per thread with a decoded index took 185.
+// 146 us at 256^3 (5.5 TB/s of its 48 B per cell); one cell per thread with a decoded index took 185.
 __global__ void __launch_bounds__(kStX * kStY) k_spmv(Grid g, const double* tx, const double* ty, const double* tz,
                                                       const double* diag, const double* __restrict__ x,
                                                       double* __restrict__ y, int zc) {
