@@ -79,8 +79,9 @@ int pmf_setup(pmf_solver* s);
 /* rhs = source + Dirichlet boundary contributions (needs pmf_setup). */
 int pmf_rhs(pmf_solver* s, const double* source, double* rhs, int on_device);
 int pmf_apply_A(pmf_solver* s, const double* x, double* y, int on_device);
-/* Without a Dirichlet face the operator is singular: the share of the constant in
- * the coarse residuals, zero for a residual of a consistent system, is taken out. */
+/* Without a Dirichlet face the operator is singular: the share of the constant in the
+ * coarse residuals, zero for a residual of a consistent system, is taken out (with
+ * -no_shift_A_cc only where the sum of x is rounding). */
 int pmf_pc_apply(pmf_solver* s, const double* x, double* y, int on_device);
 /* reason: 1 converged (residual test), 2 max_it, 3 indefinite, 4 nan/inf, 5 converged because the
  * preconditioned residual's dot z.r is exactly zero (PETSc's KSP_CONVERGED_ATOL for KSPCG) */

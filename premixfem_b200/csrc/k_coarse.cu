@@ -270,35 +270,18 @@ void launch_coarse_project(int nsub, int kmax, const RankLayout& L, const ProbIn
   { note_launch(); k_coarse_project<<<probs ? nprob : 1, 1024, 0, st>>>(nsub, kmax, L.first, probs, nv, c, done); }
 }
 
-// A += max|diag A| n n^T with n = nv / |nv| on the block of a rank that holds a whole singular problem, whose null vector
-// nv is: a product of the block's inverse with a projected residual is then that of its pseudo-inverse.  Left singular,
-// the block's last pivot is its rounding, kept or dropped as it falls (1e-14 of the diagonal): of 48 boxes without a
-// Dirichlet face in one rank, 1e-8 took one 17 instead of 12 iterations in FP64 and five of them 38 to 100 in mixed
-// precision.  One CTA per rank.
-__global__ void __launch_bounds__(1024) k_lift_null(RankLayout L, const ProbInfo* probs, const double* nv, double* dense) {
+// The block of a rank that holds a whole singular problem has its null pivot at the last unknown of the null vector, the
+// last subdomain's constant.  Its rounding would be kept or dropped as it falls (1e-14 of the diagonal): of 48 boxes
+// without a Dirichlet face in one rank, 1e-8 took one 17 instead of 12 iterations in FP64 and five of them 38 to 100 in
+// mixed precision.  With row and column set to zero the inverse's rule drops it always.  One CTA per rank.
+__global__ void __launch_bounds__(256) k_pin_null(RankLayout L, const ProbInfo* probs, double* dense) {
   if (probs && probs[blockIdx.x].dmask) return;
-  const int r = blockIdx.x, n = rank_nr(L, r), s0 = L.first[r], ns = L.first[r + 1] - s0;
+  const int r = blockIdx.x, n = rank_nr(L, r), e = n - L.kmax;
   double* A = dense + L.off2[r];
-  __shared__ double red[32];
-  double t = 0.0, m = 0.0;
-  for (int s = threadIdx.x; s < ns; s += 1024) t += nv[s0 + s] * nv[s0 + s];
-  t = block_sum(t, red);
-  __shared__ double q;
-  if (threadIdx.x == 0) q = 1.0 / t;
-  for (int i = threadIdx.x; i < n; i += 1024) m = fmax(m, fabs(A[(long long)i * n + i]));
-  __syncthreads();
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  for (int w = 0; w < 32; ++w) m = fmax(m, red[w]);
-  for (long long e = threadIdx.x; e < (long long)ns * ns; e += 1024) {
-    const long long i = e / ns, j = e - i * ns;
-    A[i * L.kmax * n + j * L.kmax] += m * q * nv[s0 + i] * nv[s0 + j];
-  }
+  for (int i = threadIdx.x; i < n; i += 256) A[(long long)e * n + i] = A[(long long)i * n + e] = 0.0;
 }
-void launch_lift_null(int nrank, const RankLayout& L, const ProbInfo* probs, const double* nv, double* dense,
-                      cudaStream_t st) {
-  { note_launch(); k_lift_null<<<nrank, 1024, 0, st>>>(L, probs, nv, dense); }
+void launch_pin_null(int nrank, const RankLayout& L, const ProbInfo* probs, double* dense, cudaStream_t st) {
+  { note_launch(); k_pin_null<<<nrank, 256, 0, st>>>(L, probs, dense); }
 }
 
 __global__ void k_axpy(long long n, double a, const double* x, double* y, const int* done) {

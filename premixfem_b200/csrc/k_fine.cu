@@ -189,6 +189,26 @@ __device__ __forceinline__ double fixed_sum_wide(const double* part, int n, doub
   return block_sum(v, scratch);
 }
 
+__global__ void k_sum_abs(const double* x, long long n, double* part) {
+  __shared__ double red[32];
+  double v = 0.0, a = 0.0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    v += x[i];
+    a += fabs(x[i]);
+  }
+  v = block_sum(v, red);
+  a = block_sum(a, red);
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = v;
+    part[2 * blockIdx.x + 1] = a;
+  }
+}
+int launch_sum_abs(const double* x, long long n, double* part, cudaStream_t st) {
+  const int nb = std::min(cell_blocks(n), 1184);
+  { note_launch(); k_sum_abs<<<nb, kCellThreads, 0, st>>>(x, n, part); }
+  return nb;
+}
+
 // --- KSPSolve_CG (PETSc src/ksp/ksp/impls/cg/cg.c) with the unpreconditioned norm ---
 __global__ void k_pcg_start(long long n, const double* b, double* x, double* r, float* r32, double* part) {
   __shared__ double red[32];

@@ -55,6 +55,8 @@ void launch_zero_padding(const Grid& g, const ProbInfo* probs, const int* layer_
                          double* kz, cudaStream_t st);
 void launch_assemble(const AssembleArgs& a, double* tx, double* ty, double* tz, double* diag, double* db,
                      double* bval, cudaStream_t st);
+// part[2b], part[2b + 1]: block b's share of the sum of x and of |x|; the number of blocks
+int launch_sum_abs(const double* x, long long n, double* part, cudaStream_t st);
 void launch_to_f32(const double* in, float* out, long long n, cudaStream_t st);
 void launch_to_f64(const float* in, double* out, long long n, cudaStream_t st);
 
@@ -222,9 +224,8 @@ void launch_null_coef(const Grid& g, const SubInfo* subs, int nsub, int kmax, co
                       cudaStream_t st);
 void launch_coarse_project(int nsub, int kmax, const RankLayout& L, const ProbInfo* probs, int nprob, const double* nv,
                            double* c, const int* done, cudaStream_t st);
-// the dense blocks of ranks that hold a whole singular problem made regular along nv
-void launch_lift_null(int nrank, const RankLayout& L, const ProbInfo* probs, const double* nv, double* dense,
-                      cudaStream_t st);
+// the null unknown of the dense blocks of ranks that hold a whole singular problem taken out
+void launch_pin_null(int nrank, const RankLayout& L, const ProbInfo* probs, double* dense, cudaStream_t st);
 void launch_axpy(long long n, double a, const double* x, double* y, const int* done, cudaStream_t st);
 void launch_copy(long long n, const double* x, double* y, const int* done, cudaStream_t st);
 

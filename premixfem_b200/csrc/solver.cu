@@ -1319,7 +1319,7 @@ int Solver::setup() {
     return finish();
   }
   launch_assemble_dense_r(d_subs, nrank, rl, tot2, blk, gface, 0, A2inv, st);
-  if (singular() && (nprob || nrank == 1)) launch_lift_null(nrank, rl, d_probs, nullv, A2inv, st);
+  if (singular() && (nprob || nrank == 1)) launch_pin_null(nrank, rl, d_probs, A2inv, st);
   auto no_scratch = [&]() {
     err = "not enough device memory for the scratch of the coarse inverses";
     return 76;
@@ -1713,8 +1713,8 @@ void Solver::tune_pc() {
 }
 
 template <typename T>
-void Solver::apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done) {
-  const bool f32 = sizeof(T) == 4, project = singular();
+void Solver::apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done, bool project) {
+  const bool f32 = sizeof(T) == 4;
   const T* ttx = f32 ? (const T*)tx32 : (const T*)tx;
   const T* tty = f32 ? (const T*)ty32 : (const T*)ty;
   const T* ttz = f32 ? (const T*)tz32 : (const T*)tz;
@@ -1830,7 +1830,7 @@ int Solver::solve_batch(const double* b_in, double* x_out, bool on_device, int* 
   const int nblk = bpcg_blocks();
   cudaEventRecord(ev0, st);
   launch_bpcg_start(d_probs, nprob, bs, xs, r, r32, part, bstate, opt.rtol, opt.atol, opt.max_it, d_all_done, nblk, st);
-  apply(r, z, part, d_all_done);
+  apply(r, z, part, d_all_done, singular());
   launch_bpcg_beta(d_probs, nprob, part, bstate, st);
   double* pin = p0;
   double* pout = p1;
@@ -1839,7 +1839,7 @@ int Solver::solve_batch(const double* b_in, double* x_out, bool on_device, int* 
     for (int c_ = 0; c_ < chunk; ++c_) {
       launch_bpcg_iter_a(g, d_probs, d_layer_prob, nprob, tx, ty, tz, diag, z, pin, pout, w, part, bstate, st);
       launch_bpcg_iter_b(g, d_probs, d_layer_prob, nprob, r, r32, pout, w, part, bstate, d_all_done, loop, st);
-      apply(r, z, part, d_all_done);
+      apply(r, z, part, d_all_done, singular());
       launch_bpcg_beta(d_probs, nprob, part, bstate, st);
       std::swap(pin, pout);
     }
@@ -1967,7 +1967,7 @@ int Solver::profile_iteration(int reps, double ms[PROF_SLOTS], int launches[PROF
     prof_mark(PROF_CG_A);
     launch_pcg_iter_b(g.ncell, vb, r32, p1, w, part, state, st);
     prof_mark(PROF_CG_B);
-    apply(vb, z, part, nullptr);
+    apply(vb, z, part, nullptr, singular());
     if (opt.null_space)
       launch_pcg_null_beta(z, vb, g.ncell, part, zpart, state, LoopCond(), st);
     else
@@ -1991,13 +1991,13 @@ int Solver::profile_iteration(int reps, double ms[PROF_SLOTS], int launches[PROF
 }
 
 // In the mixed form r32 holds x in FP32 (written by the CG kernels with the residual).
-// Of a singular operator every application has its coarse residuals projected, a caller's own as well: the residuals
-// of a consistent system have no share of the constant, and what rounding puts there must not be amplified.
-void Solver::apply(const double* x, double* out, double* partial, const int* done) {
+// project: x is a residual of a consistent system of a singular operator and has no share of the constant; what
+// rounding puts into its coarse residuals must not be amplified.
+void Solver::apply(const double* x, double* out, double* partial, const int* done, bool project) {
   if (opt.precision == 1)
-    apply_impl<float>(x, r32, out, partial, done);
+    apply_impl<float>(x, r32, out, partial, done, project);
   else
-    apply_impl<double>(x, x, out, partial, done);
+    apply_impl<double>(x, x, out, partial, done, project);
 }
 
 int Solver::rhs(const double* source, double* out, bool on_device) {
@@ -2045,7 +2045,23 @@ int Solver::pc_apply(const double* x_in, double* y_out, bool on_device) {
   }
   cudaEventRecord(ev0, st);
   if (opt.precision == 1) launch_to_f32(xs, r32, g.ncell, st);
-  apply(xs, ys, part, nullptr);
+  // Singular operator: with the shift of the coarse matrix the answer to a share of the constant is 1e12 times the
+  // constant, and every vector is projected, as the residuals of the solves are.  Without the shift that answer is as
+  // large as others: a vector's own sum (about Sigma |x| / sqrt(n) for random entries) is kept, and only one of a
+  // hundredth of that, which CG residuals stay below to 1e-8, is taken for rounding.
+  bool project = singular() && !(nprob && opt.no_shift_A_cc);
+  if (project && opt.no_shift_A_cc) {
+    std::vector<double> h(2 * (size_t)launch_sum_abs(xs, g.ncell, part, st));
+    cudaMemcpyAsync(h.data(), part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
+    if (int e = check(cudaStreamSynchronize(st), "PC_apply_vec")) return e;
+    double sum = 0.0, mag = 0.0;
+    for (size_t i = 0; i < h.size(); i += 2) {
+      sum += h[i];
+      mag += h[i + 1];
+    }
+    project = fabs(sum) <= 1e-2 / sqrt((double)g.ncell) * mag;
+  }
+  apply(xs, ys, part, nullptr, project);
   cudaEventRecord(ev1, st);
   if (!on_device) cudaMemcpyAsync(y_out, ys, n * 8, cudaMemcpyDeviceToHost, st);
   int e = check(cudaStreamSynchronize(st), "PC_apply_vec");
@@ -2086,7 +2102,7 @@ int Solver::solve(const double* b_in, double* x_out, bool on_device, int* its, d
     else
       launch_pcg_beta_fin(part, nparts_apply(), state, loop, st);
   };
-  apply(r, z, part, done);
+  apply(r, z, part, done, singular());
   beta(LoopCond());
   double* pin = p0;
   double* pout = p1;
@@ -2095,7 +2111,7 @@ int Solver::solve(const double* b_in, double* x_out, bool on_device, int* its, d
     for (int c_ = 0; c_ < chunk; ++c_) {
       launch_pcg_iter_a(g, tx, ty, tz, diag, z, pin, pout, w, part, state, st);
       launch_pcg_iter_b(g.ncell, r, r32, pout, w, part, state, st);
-      apply(r, z, part, done);
+      apply(r, z, part, done, singular());
       beta(loop);
       std::swap(pin, pout);
     }

@@ -182,8 +182,8 @@ class Solver {
   int alloc_fine();
   void assemble_launch();
   template <typename T>
-  void apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done);
-  void apply(const double* x, double* out, double* partial, const int* done);
+  void apply_impl(const double* x, const T* xt, double* out, double* partial, const int* done, bool project);
+  void apply(const double* x, double* out, double* partial, const int* done, bool project);
   std::vector<int> schedule() const;
   int dir_on_[6] = {0, 0, 0, 0, 0, 0};
   // no Dirichlet face: the constant is the operator's null space, whether or not the caller projects z

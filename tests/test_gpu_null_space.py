@@ -143,6 +143,25 @@ def test_one_rank_holds_the_singular_problem(native, mesh, sd, seed, precision):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("mesh,vranks,sd,seed", [((24, 24, 24), (2, 2, 1), 2, 1), ((24, 20, 16), (2, 1, 1), 2, 2),
+                                                 ((16, 16, 16), (2, 2, 2), 1, 3), ((16, 16, 16), (1, 1, 1), 2, 3)],
+                         ids=lambda v: str(v).replace(", ", "x"))
+def test_pc_apply_of_a_vector_with_a_sum(native, mesh, vranks, sd, seed, precision):
+    """One application to a vector whose sum is not zero, without the shift that would drown it: the oracle's to the 1e-6
+    of the other applications (a projection would take part of it away)."""
+    prob = fields.random_box(mesh, seed=seed, sigma=1.5)
+    prob["dirichlet"] = {}
+    d = {"sd": sd, "en_lv1": 4, "en_lv2": 4, "no_shift_A_cc": True}
+    x = np.random.default_rng(seed).standard_normal(int(np.prod(mesh)))
+    y = O.Preconditioner(O.Operator(prob), O.Options(**d, vranks=vranks)).apply(x)
+    s = DarcySolver.from_problem(prob, options_string(dict(d, pmf_vranks=vranks, pmf_precision=precision)))
+    s.setup()
+    z = s.pc_apply(x)
+    s.close()
+    assert np.linalg.norm(z - y) <= 1e-6 * np.linalg.norm(y)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("seed", [1, 3, 5])
 def test_batch_of_singular_problems(native, seed, precision):
     """Three channel problems without a Dirichlet face and one with, in one batch (which has no null space option): each
